@@ -147,3 +147,77 @@ def test_stabilizer_with_learned_upsampler(vsc, cuda):
     a.close()
     b.close()
     up.close()
+
+
+def _reference_steps(params, batches, lr):
+    """Adam steps of the L1 loss in float64 (torch autograd on the CPU): parameters after each."""
+    import torch
+
+    p = torch.from_numpy(params.astype(np.float64)).requires_grad_()
+    m, v = torch.zeros_like(p), torch.zeros_like(p)
+    out = []
+    for k, (inp, tgt) in enumerate(batches, 1):
+        x = torch.from_numpy(inp.astype(np.float64)).permute(0, 3, 1, 2)
+        at = 0
+        for li, (ci, co) in enumerate(LAYERS):
+            w = p[at:at + co * 9 * ci].reshape(co, 3, 3, ci).permute(0, 3, 1, 2)
+            at += co * 9 * ci
+            x = torch.nn.functional.conv2d(x, w, p[at:at + co], padding=1)
+            at += co
+            x = x.relu() if li < 3 else x
+        d = torch.from_numpy(inp[..., :2].astype(np.float64)) + x.permute(0, 2, 3, 1) - torch.from_numpy(tgt)
+        loss = d.abs().sum() / (d.numel() // 2)
+        (g,) = torch.autograd.grad(loss, p)
+        with torch.no_grad():
+            m = 0.9 * m + 0.1 * g
+            v = 0.999 * v + 0.001 * g * g
+            p -= lr * (m / (1 - 0.9 ** k)) / ((v / (1 - 0.999 ** k)).sqrt() + 1e-8)
+        out.append((float(loss.detach()), p.detach().numpy().copy()))
+    return out
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("n,h,w", [(1, 1, 1), (1, 2, 31), (2, 9, 33), (3, 7, 50), (1, 33, 64), (5, 8, 32)])
+def test_training_steps_match_float64(vsc, cuda, n, h, w):
+    """Two steps on different batches (the first Adam step alone shows only the
+    gradients' signs) at the edges of the 32 x 8 and 32 x 2 pixel tiles.  The
+    FP32 gradients' rounding (about 1e-5 of a layer's gradient scale) moves an
+    update by lr * 1e-5 * scale / |g|: 1e-4 lr in the median, and more than
+    1e-2 lr only where |g| is below a thousandth of its layer's scale."""
+    import torch
+
+    rng = np.random.Generator(np.random.PCG64(100 * n + 10 * h + w))
+    lr = 1e-4
+    params = rng.normal(0, 0.1, vsc.Upsampler.param_count()).astype(np.float32)
+    batches = [(rng.normal(0, 1, (n, h, w, 3)).astype(np.float32), rng.normal(0, 1, (n, h, w, 2)).astype(np.float32))
+               for _ in range(2)]
+    up = vsc.Upsampler(params)
+    for (inp, tgt), (loss, ref) in zip(batches, _reference_steps(params, batches, lr)):
+        got = up.train_step(torch.from_numpy(inp).to(cuda), torch.from_numpy(tgt).to(cuda), lr)
+        assert abs(got - loss) <= 1e-5 * loss
+        # less the parameters' own rounding (|p| < 1: half a unit is 6e-8 at most)
+        err = np.maximum(np.abs(up.params() - ref) - 6e-8, 0) / lr
+        assert np.median(err) <= 1e-4 and np.quantile(err, 0.99) <= 1e-2 and err.max() <= 2.5, (err.max(), h, w)
+    up.close()
+
+
+@pytest.mark.gpu
+def test_training_ignores_values_where_the_gradient_is_zero(vsc, cuda):
+    """An infinite input inside a region without a loss gradient (its targets
+    are NaN: neither sign) adds nothing to the weight gradients: the step is
+    the one with a finite value in its place."""
+    import torch
+
+    h, w = 40, 48
+    inp = RNG.normal(0, 1, (1, h, w, 3)).astype(np.float32)
+    tgt = RNG.normal(0, 1, (1, h, w, 2)).astype(np.float32)
+    tgt[0, 10:31, 10:31] = np.nan  # further than the net's four pixels around (20, 20)
+    got = []
+    for value in (0.5, np.inf):
+        inp[0, 20, 20, 0] = value
+        up = vsc.Upsampler("default")
+        up.train_step(torch.from_numpy(inp).to(cuda), torch.from_numpy(tgt).to(cuda), 1e-3)
+        got.append(up.params())
+        up.close()
+    assert np.all(np.isfinite(got[1]))
+    assert np.quantile(np.abs(got[0] - got[1]), 0.99) <= 1e-5  # the sums' order varies

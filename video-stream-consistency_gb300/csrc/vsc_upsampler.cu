@@ -11,9 +11,9 @@
 // training and rounded to FP16 for inference.
 //
 // The training kernels are written here, in FP32: direct convolutions on the
-// CUDA cores over NHWC activations (one thread per pixel, the layer's weights
-// in shared memory, fused multiply-adds), a backward pass for the data and
-// the weights, an L1 loss against the full-resolution flow and Adam.  The
+// CUDA cores over planar activations (register tiles of pixels and channels
+// fed from shared memory, fused multiply-adds), a backward pass for the data
+// and the weights, an L1 loss against the full-resolution flow and Adam.  The
 // input preparation is shared with the inference, which runs on the tensor
 // cores (vsc_upsampler_tc.cu).  Nothing here has a bit-exact contract
 // (contraction is spelled out with __fmaf_rn, the library being built
@@ -23,15 +23,15 @@
 
 #include <cuda_fp16.h>
 
+#include <algorithm>
 #include <cmath>
-#include <vector>
+#include <mutex>
 
 namespace vsc {
 namespace {
 
 constexpr int kParams = 19970;
 static_assert(kUpLayers[3].b_off + 2 == kParams, "parameter layout");
-constexpr int kThreads = 128;
 
 __device__ __forceinline__ float luma(const float* p) { return 0.299f * p[0] + 0.587f * p[1] + 0.114f * p[2]; }
 
@@ -65,150 +65,463 @@ __global__ void prepare_kernel(const float* __restrict__ coarse, int cw, int ch,
     o[2] = luma(img + n * s_img + pix_index(x, y, w) * 3);
 }
 
-// ---- forward: one 3x3 convolution, NHWC, batch n along blockIdx.y ---------------------
-template <int CI, int CO, bool kRelu, typename WT>
-__global__ void __launch_bounds__(kThreads) conv_fwd_kernel(const float* __restrict__ x, const WT* __restrict__ wts,
-    const float* __restrict__ bias, float* __restrict__ y, int H, int W)
+// ---- training: 3x3 convolutions on register tiles ---------------------------------------
+// Inner activations and their gradients are planes ([image][channel][y][x]);
+// the input (NHWC, 3 channels) is read as the caller holds it.
+//
+// The convolutions (forward, and backward for the data with the taps
+// flipped) and the weight gradients are FP32 contractions of 9 CI CO products
+// a pixel, bound by the FMA issue rate as long as shared memory keeps up.
+// One thread per pixel with the weights read one by one from shared memory
+// (one 4-byte broadcast load per FMA) ran the 32 -> 32 layer of a 32 x 64 x
+// 64 batch in 274 us forward and 369 us backward; weight gradients with one
+// block per (output, tap), which re-read the whole activation with a stride
+// for each of the 288 blocks, took 919 us.  The layer's 1.2 G FMAs are 30 us
+// at 152 x 128 lanes.
+
+__device__ __forceinline__ void cp_async4(float* dst, const float* src, bool valid)
 {
-    __shared__ float sw[CO * 9 * CI];
-    __shared__ float sb[CO];
-    for (int i = threadIdx.x; i < CO * 9 * CI; i += blockDim.x)
-        sw[i] = static_cast<float>(wts[i]);
-    for (int i = threadIdx.x; i < CO; i += blockDim.x)
-        sb[i] = bias[i];
-    __syncthreads();
-    const int64_t HW = static_cast<int64_t>(H) * W;
-    const int64_t p = blockIdx.x * static_cast<int64_t>(blockDim.x) + threadIdx.x;
-    if (p >= HW)
-        return;
-    const int n = blockIdx.y;
-    const int py = static_cast<int>(p / W), px = static_cast<int>(p % W);
-    const float* xb = x + n * HW * CI;
-    float acc[CO];
-#pragma unroll
-    for (int o = 0; o < CO; ++o)
-        acc[o] = sb[o];
-    for (int t = 0; t < 9; ++t) {
-        const int yy = py + t / 3 - 1, xx = px + t % 3 - 1;
-        if (yy < 0 || yy >= H || xx < 0 || xx >= W)
-            continue;
-        const float* xs = xb + (static_cast<int64_t>(yy) * W + xx) * CI;
-#pragma unroll 4
-        for (int c = 0; c < CI; ++c) {
-            const float xv = xs[c];
-#pragma unroll
-            for (int o = 0; o < CO; ++o)
-                acc[o] = __fmaf_rn(sw[(o * 9 + t) * CI + c], xv, acc[o]);
-        }
-    }
-    float* yo = y + (n * HW + p) * CO;
-#pragma unroll
-    for (int o = 0; o < CO; ++o)
-        yo[o] = kRelu ? fmaxf(acc[o], 0.0f) : acc[o];
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;" ::"r"(
+                     static_cast<uint32_t>(__cvta_generic_to_shared(dst))),
+        "l"(src), "r"(valid ? 4 : 0)
+        : "memory");
+}
+__device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
+template <int N>
+__device__ __forceinline__ void cp_async_wait()
+{
+    asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory");
 }
 
-// ---- backward ---------------------------------------------------------------------------
-// dz_prev = (sum over taps and output channels of w * dz) * (a_prev > 0)
-template <int CI, int CO, bool kMask>
-__global__ void __launch_bounds__(kThreads) conv_bwd_data_kernel(const float* __restrict__ dz,
-    const float* __restrict__ wts, const float* __restrict__ a_prev, float* __restrict__ dz_prev, int H, int W)
+__device__ __forceinline__ bool finite_f(float v) { return fabsf(v) <= 3.402823466e38f; }
+
+constexpr int kTileW = 32;   // pixels of a tile row
+constexpr int kPitch = 36;   // its shared-memory pitch: 34 with the halo; 4 mod 32 keeps 16-byte reads of
+                             // 4 groups x 8 rows free of bank conflicts
+
+enum ConvMode { kConvRelu, kConvLoss, kConvBwd };
+
+// The convolution of one 32 x (8 PG) pixel tile.  A thread keeps 8 adjacent
+// pixels x OCT output channels; a warp covers 32 x 8 pixels of one channel
+// group, so its weight reads are broadcasts and its pixel reads (10 values
+// for the 8 pixels' three horizontal taps) conflict-free 16-byte words: per
+// input channel and tap row, 2.5 + 3 OCT / 4 reads for 24 OCT FMAs.  Channels
+// stream in chunks of CC through two cp.async buffers (zero outside the
+// image, the convolution's padding).
+template <int CI, int CO, int OCT>
+struct ConvShape {
+    static constexpr int CC = CI < 8 ? CI : 8;
+    static constexpr int chunks = (CI + CC - 1) / CC;
+    static constexpr int OG = CO / OCT;          // channel groups
+    static constexpr int PG = 4 / OG;            // 32 x 8 pixel groups of the tile
+    static constexpr int rows = 8 * PG;
+    static constexpr int plane = (rows + 2) * kPitch;
+    static constexpr int wp = 9 * CO + 4;        // weights [c][tap][o]; + 4 spreads the transposing writes
+    static constexpr int buf = (CC * plane + CC * wp + 3) / 4 * 4;
+    static constexpr int bufs = chunks > 1 ? 2 : 1;
+    static constexpr int smem = bufs * buf * 4;
+    static_assert(CI % CC == 0 && OG * PG == 4 && (CC * plane) % 4 == 0 && wp % (OCT < 4 ? 2 : 4) == 0, "tile");
+};
+
+// x: planes (kInter: interleaved CI-channel pixels).  kConvRelu: y = ReLU(conv
+// + bias).  kConvLoss (the last layer): the L1 loss of base + r against the
+// target and its gradient dr = sign / pixels as planes in y.  kConvBwd: x is
+// dz of the layer's CI outputs, y = dz of its CO inputs where a_prev > 0.
+// nonfinite: set when a value the weight gradients will multiply (the input
+// or an activation) is not finite.
+template <int CI, int CO, int OCT, int kMode, bool kInter>
+__global__ void __launch_bounds__(128, 4) conv3x3_kernel(const float* __restrict__ x, const float* __restrict__ wts,
+    const float* __restrict__ bias, const float* __restrict__ a_prev, float* __restrict__ y, int H, int W, int tiles_x,
+    const float* __restrict__ input, const float* __restrict__ target, float* __restrict__ loss, float inv,
+    int* __restrict__ nonfinite)
 {
-    __shared__ float sw[CO * 9 * CI];
-    for (int i = threadIdx.x; i < CO * 9 * CI; i += blockDim.x)
-        sw[i] = wts[i];
-    __syncthreads();
+    using S = ConvShape<CI, CO, OCT>;
+    extern __shared__ __align__(16) float sm[];
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const int og = warp % S::OG, pg = warp / S::OG;
+    const int g = lane & 3, r = pg * 8 + (lane >> 2);  // this thread's 8-pixel group and tile row
+    const int x0 = (blockIdx.x % tiles_x) * kTileW, y0 = (blockIdx.x / tiles_x) * S::rows;
     const int64_t HW = static_cast<int64_t>(H) * W;
-    const int64_t p = blockIdx.x * static_cast<int64_t>(blockDim.x) + threadIdx.x;
-    if (p >= HW)
-        return;
     const int n = blockIdx.y;
-    const int py = static_cast<int>(p / W), px = static_cast<int>(p % W);
-    float acc[CI];
-#pragma unroll
-    for (int c = 0; c < CI; ++c)
-        acc[c] = 0.0f;
-    for (int t = 0; t < 9; ++t) {
-        // the output pixel whose tap t read this pixel
-        const int yy = py - (t / 3 - 1), xx = px - (t % 3 - 1);
-        if (yy < 0 || yy >= H || xx < 0 || xx >= W)
-            continue;
-        const float* g = dz + (n * HW + static_cast<int64_t>(yy) * W + xx) * CO;
-        for (int o = 0; o < CO; ++o) {
-            const float gv = g[o];
-#pragma unroll
-            for (int c = 0; c < CI; ++c)
-                acc[c] = __fmaf_rn(sw[(o * 9 + t) * CI + c], gv, acc[c]);
+    const float* xn = x + static_cast<int64_t>(n) * HW * CI;
+
+    auto stage = [&](int chunk, float* b) {
+        const int c0 = chunk * S::CC;
+        for (int i = tid; i < S::CC * (S::rows + 2) * 34; i += 128) {
+            const int c = i / ((S::rows + 2) * 34), rem = i % ((S::rows + 2) * 34);
+            const int row = rem / 34, col = rem % 34;
+            const int gy = y0 - 1 + row, gx = x0 - 1 + col;
+            const bool ok = gy >= 0 && gy < H && gx >= 0 && gx < W;
+            const int64_t p = ok ? static_cast<int64_t>(gy) * W + gx : 0;
+            cp_async4(b + c * S::plane + row * kPitch + col, xn + (kInter ? p * CI + c0 + c : (c0 + c) * HW + p), ok);
         }
-    }
-    const float* ap = a_prev + (n * HW + p) * CI;
-    float* out = dz_prev + (n * HW + p) * CI;
+        float* sw = b + S::CC * S::plane;
+        for (int i = tid; i < S::CC * 9 * CO; i += 128) {
+            if (kMode == kConvBwd) {  // the layer's weights [in = its outputs][tap][out], taps flipped
+                const int o = i % CO, t = (i / CO) % 9, c = i / (9 * CO);
+                cp_async4(sw + c * S::wp + t * CO + o, wts + ((c0 + c) * 9 + 8 - t) * CO + o, true);
+            } else {
+                const int c = i % S::CC, t = (i / S::CC) % 9, o = i / (9 * S::CC);
+                cp_async4(sw + c * S::wp + t * CO + o, wts + (o * 9 + t) * CI + c0 + c, true);
+            }
+        }
+        cp_async_commit();
+    };
+
+    float acc[8][OCT];
 #pragma unroll
-    for (int c = 0; c < CI; ++c)
-        out[c] = (!kMask || ap[c] > 0.0f) ? acc[c] : 0.0f;
+    for (int o = 0; o < OCT; ++o) {
+        const float b = kMode == kConvBwd ? 0.0f : bias[og * OCT + o];
+#pragma unroll
+        for (int i = 0; i < 8; ++i)
+            acc[i][o] = b;
+    }
+    stage(0, sm);
+    bool bad = false;
+    for (int k = 0; k < S::chunks; ++k) {
+        float* b = sm + (k % S::bufs) * S::buf;
+        if (k + 1 < S::chunks)
+            stage(k + 1, sm + ((k + 1) % S::bufs) * S::buf);
+        if (k + 1 < S::chunks)
+            cp_async_wait<1>();
+        else
+            cp_async_wait<0>();
+        __syncthreads();
+        if (kInter && kMode == kConvRelu)  // the layer's own input feeds its weight gradient
+            for (int i = tid; i < S::CC * (S::rows + 2) * 34; i += 128) {
+                const int c = i / ((S::rows + 2) * 34), rem = i % ((S::rows + 2) * 34);
+                bad = bad || !finite_f(b[c * S::plane + rem / 34 * kPitch + rem % 34]);
+            }
+        const float* xp = b + r * kPitch + 8 * g;
+        const float* wq = b + S::CC * S::plane + og * OCT;
+#pragma unroll 1
+        for (int c = 0; c < S::CC; ++c, xp += S::plane, wq += S::wp) {
+#pragma unroll
+            for (int ky = 0; ky < 3; ++ky) {
+                const float4 v0 = *reinterpret_cast<const float4*>(xp + ky * kPitch);
+                const float4 v1 = *reinterpret_cast<const float4*>(xp + ky * kPitch + 4);
+                const float2 v2 = *reinterpret_cast<const float2*>(xp + ky * kPitch + 8);
+                const float v[10] = {v0.x, v0.y, v0.z, v0.w, v1.x, v1.y, v1.z, v1.w, v2.x, v2.y};
+#pragma unroll
+                for (int kx = 0; kx < 3; ++kx) {
+                    float w[OCT];
+                    const float* wt = wq + (ky * 3 + kx) * CO;
+                    if constexpr (OCT % 4 == 0) {
+#pragma unroll
+                        for (int q = 0; q < OCT / 4; ++q) {
+                            const float4 f = *reinterpret_cast<const float4*>(wt + 4 * q);
+                            w[4 * q] = f.x;
+                            w[4 * q + 1] = f.y;
+                            w[4 * q + 2] = f.z;
+                            w[4 * q + 3] = f.w;
+                        }
+                    } else {
+                        const float2 f = *reinterpret_cast<const float2*>(wt);
+                        w[0] = f.x;
+                        w[1] = f.y;
+                    }
+#pragma unroll
+                    for (int i = 0; i < 8; ++i)
+#pragma unroll
+                        for (int o = 0; o < OCT; ++o)
+                            acc[i][o] = __fmaf_rn(w[o], v[i + kx], acc[i][o]);
+                }
+            }
+        }
+        __syncthreads();  // the buffer is refilled two chunks on
+    }
+
+    const int py = y0 + r, px = x0 + 8 * g;
+    const bool row_in = py < H;
+    const int64_t p = static_cast<int64_t>(py) * W + px;
+    if constexpr (kMode == kConvLoss) {
+        float l = 0.0f;
+#pragma unroll
+        for (int i = 0; i < 8; ++i) {
+            if (!row_in || px + i >= W)
+                continue;
+            const int64_t q = n * HW + p + i;
+#pragma unroll
+            for (int o = 0; o < OCT; ++o) {
+                const float d = input[q * 3 + o] + acc[i][o] - target[q * 2 + o];
+                l += fabsf(d);
+                y[(static_cast<int64_t>(n) * CO + o) * HW + p + i] = d > 0.0f ? inv : (d < 0.0f ? -inv : 0.0f);
+            }
+        }
+        for (int o = 16; o > 0; o >>= 1)
+            l += __shfl_xor_sync(0xffffffffu, l, o);
+        if (lane == 0)
+            atomicAdd(loss, l * inv);
+    } else {
+        const bool vec = (W & 3) == 0;  // planes and rows then start on the 16-byte grid
+#pragma unroll
+        for (int o = 0; o < OCT; ++o) {
+            const int64_t q = (static_cast<int64_t>(n) * CO + og * OCT + o) * HW + p;
+            float v[8];
+#pragma unroll
+            for (int i = 0; i < 8; ++i) {
+                const bool in = row_in && px + i < W;
+                v[i] = acc[i][o];
+                if (kMode == kConvRelu) {
+                    v[i] = fmaxf(v[i], 0.0f);
+                    bad = bad || (in && !finite_f(v[i]));
+                } else {
+                    v[i] = in && a_prev[q + i] > 0.0f ? v[i] : 0.0f;
+                }
+            }
+#pragma unroll
+            for (int h = 0; h < 2; ++h) {
+                if (vec && row_in && px + 4 * h + 3 < W) {
+                    *reinterpret_cast<float4*>(y + q + 4 * h) =
+                        make_float4(v[4 * h], v[4 * h + 1], v[4 * h + 2], v[4 * h + 3]);
+                } else {
+#pragma unroll
+                    for (int i = 4 * h; i < 4 * h + 4; ++i)
+                        if (row_in && px + i < W)
+                            y[q + i] = v[i];
+                }
+            }
+        }
+        if (kMode == kConvRelu && bad)
+            atomicOr(nonfinite, 1);
+    }
 }
 
+// ---- weight gradients ---------------------------------------------------------------
 // dw[o][t][c] += sum over pixels of dz[o] * x[tap t][c]; db[o] += sum dz[o].
-// Block (o, t) over a slice of the pixels (blockIdx.z), reduced in shared
-// memory, one atomic add per weight and block.
-template <int CI, int CO>
-__global__ void __launch_bounds__(kThreads) conv_wgrad_kernel(const float* __restrict__ x, const float* __restrict__ dz,
-    float* __restrict__ dw, float* __restrict__ db, int N, int H, int W)
+// Blocks walk 32 x 2 pixel tiles, two cp.async buffers, and add their sums to
+// the gradient once at the end.  A pixel with dz = 0 adds nothing, whatever x
+// holds there (kSafe, taken when some x is not finite; else 0 * x is 0 anyway).
+constexpr int kWgRows = 2;
+constexpr int kWgPx = kTileW * kWgRows;
+constexpr int kWgPlane = 148;  // x plane: 4 rows x 36, + 4: 20 mod 32, 16-byte reads across channels conflict-free
+
+// CI = 32: a lane is an input channel with OGT outputs x 9 taps in registers,
+// a warp one group of outputs (its dz reads are broadcasts); with fewer than
+// four groups the warps split the tile's columns.  Per 4 pixels a thread
+// reads 3 + OGT 16-byte words for 36 OGT FMAs.
+template <int CO, int OGT>
+struct WgShape {
+    static constexpr int NOG = CO / OGT, KS = 4 / NOG;
+    static constexpr int dzp = kWgPx;  // dz pitch
+    static constexpr int buf = 32 * kWgPlane + CO * dzp;
+    static constexpr int smem = 2 * buf * 4;
+};
+
+__device__ __forceinline__ float wg_add(bool safe, float g, float v, float acc)
 {
-    __shared__ float red[kThreads][CI + 1];
-    const int o = blockIdx.x, t = blockIdx.y;
-    const int dy = t / 3 - 1, dx = t % 3 - 1;
-    const int64_t HW = static_cast<int64_t>(H) * W, total = N * HW;
-    const int64_t chunk = (total + gridDim.z - 1) / gridDim.z;
-    const int64_t p0 = blockIdx.z * chunk, p1 = min(total, p0 + chunk);
-    float acc[CI + 1];
+    return safe && g == 0.0f ? acc : __fmaf_rn(g, v, acc);
+}
+
+template <int CO, int OGT, bool kSafe>
+__device__ __forceinline__ void wg_tile(const float* sx, const float* sz, int ks, int lane, float (&acc)[OGT][9])
+{
+    using S = WgShape<CO, OGT>;
+    constexpr int J = 8 / S::KS;  // 4-pixel groups of a row this warp takes
+#pragma unroll 1
+    for (int row = 0; row < kWgRows; ++row) {
+        const float* xr = sx + lane * kWgPlane + row * kPitch + 4 * J * ks;
+        const float* zr = sz + row * kTileW + 4 * J * ks;
+        float4 cur[3];
 #pragma unroll
-    for (int c = 0; c <= CI; ++c)
-        acc[c] = 0.0f;
-    for (int64_t q = p0 + threadIdx.x; q < p1; q += blockDim.x) {
-        const int64_t n = q / HW, p = q % HW;
-        const int py = static_cast<int>(p / W), px = static_cast<int>(p % W);
-        const float g = dz[q * CO + o];
-        acc[CI] += g;
-        const int yy = py + dy, xx = px + dx;
-        if (g == 0.0f || yy < 0 || yy >= H || xx < 0 || xx >= W)
-            continue;
-        const float* xs = x + (n * HW + static_cast<int64_t>(yy) * W + xx) * CI;
+        for (int ky = 0; ky < 3; ++ky)
+            cur[ky] = *reinterpret_cast<const float4*>(xr + ky * kPitch);
+#pragma unroll 2
+        for (int j = 0; j < J; ++j) {
+            float v[3][6];
 #pragma unroll
-        for (int c = 0; c < CI; ++c)
-            acc[c] = __fmaf_rn(g, xs[c], acc[c]);
-    }
+            for (int ky = 0; ky < 3; ++ky) {
+                const float4 nx = *reinterpret_cast<const float4*>(xr + ky * kPitch + 4 * j + 4);
+                v[ky][0] = cur[ky].x;
+                v[ky][1] = cur[ky].y;
+                v[ky][2] = cur[ky].z;
+                v[ky][3] = cur[ky].w;
+                v[ky][4] = nx.x;
+                v[ky][5] = nx.y;
+                cur[ky] = nx;
+            }
 #pragma unroll
-    for (int c = 0; c <= CI; ++c)
-        red[threadIdx.x][c] = acc[c];
-    __syncthreads();
-    for (int c = threadIdx.x; c <= CI; c += blockDim.x) {
-        float s = 0.0f;
-        for (int i = 0; i < kThreads; ++i)
-            s += red[i][c];
-        if (c < CI)
-            atomicAdd(&dw[(o * 9 + t) * CI + c], s);
-        else if (t == 0)
-            atomicAdd(&db[o], s);
+            for (int o = 0; o < OGT; ++o) {
+                const float4 z = *reinterpret_cast<const float4*>(zr + o * S::dzp + 4 * j);
+                const float gz[4] = {z.x, z.y, z.z, z.w};
+#pragma unroll
+                for (int i = 0; i < 4; ++i)
+#pragma unroll
+                    for (int t = 0; t < 9; ++t)
+                        acc[o][t] = wg_add(kSafe, gz[i], v[t / 3][i + t % 3], acc[o][t]);
+            }
+        }
     }
 }
 
-// L1 loss of base + r against the target flow; dr = sign / (pixels); loss summed.
-__global__ void loss_kernel(const float* __restrict__ input, const float* __restrict__ r,
-    const float* __restrict__ target, float* __restrict__ dr, float* __restrict__ loss, int64_t npx, float inv)
+template <int CO, int OGT>
+__global__ void __launch_bounds__(128, 4) wgrad_kernel(const float* __restrict__ x, const float* __restrict__ dz,
+    float* __restrict__ dw, float* __restrict__ db, int H, int W, int tiles_x, int tiles, int N,
+    const int* __restrict__ nonfinite)
 {
-    const int64_t p = blockIdx.x * static_cast<int64_t>(blockDim.x) + threadIdx.x;
-    float l = 0.0f;
-    if (p < npx) {
-        for (int k = 0; k < 2; ++k) {
-            const float d = input[p * 3 + k] + r[p * 2 + k] - target[p * 2 + k];
-            l += fabsf(d);
-            dr[p * 2 + k] = d > 0.0f ? inv : (d < 0.0f ? -inv : 0.0f);
+    using S = WgShape<CO, OGT>;
+    extern __shared__ __align__(16) float sm[];
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const int og = warp % S::NOG, ks = warp / S::NOG;
+    const int64_t HW = static_cast<int64_t>(H) * W;
+    const int total = tiles * N;
+
+    auto stage = [&](int tile, float* b) {
+        const int n = tile / tiles, rem = tile % tiles;
+        const int x0 = (rem % tiles_x) * kTileW, y0 = (rem / tiles_x) * kWgRows;
+        const float* xn = x + static_cast<int64_t>(n) * HW * 32;
+        const float* zn = dz + static_cast<int64_t>(n) * HW * CO;
+        for (int i = tid; i < 32 * 4 * 34; i += 128) {
+            const int c = i / (4 * 34), q = i % (4 * 34), row = q / 34, col = q % 34;
+            const int gy = y0 - 1 + row, gx = x0 - 1 + col;
+            const bool ok = gy >= 0 && gy < H && gx >= 0 && gx < W;
+            cp_async4(b + c * kWgPlane + row * kPitch + col,
+                ok ? xn + c * HW + static_cast<int64_t>(gy) * W + gx : xn, ok);
+        }
+        float* sz = b + 32 * kWgPlane;
+        for (int i = tid; i < CO * kWgPx; i += 128) {
+            const int o = i / kWgPx, q = i % kWgPx, gy = y0 + q / kTileW, gx = x0 + q % kTileW;
+            const bool ok = gy < H && gx < W;
+            cp_async4(sz + o * S::dzp + q, ok ? zn + o * HW + static_cast<int64_t>(gy) * W + gx : zn, ok);
+        }
+    };
+
+    float acc[OGT][9], bsum[OGT];
+#pragma unroll
+    for (int o = 0; o < OGT; ++o) {
+        bsum[o] = 0.0f;
+#pragma unroll
+        for (int t = 0; t < 9; ++t)
+            acc[o][t] = 0.0f;
+    }
+    const bool safe = *nonfinite != 0;
+    int tile = blockIdx.x, k = 0;
+    if (tile < total)
+        stage(tile, sm);
+    cp_async_commit();
+    for (; tile < total; tile += gridDim.x, ++k) {
+        const float* b = sm + (k & 1) * S::buf;
+        if (tile + static_cast<int>(gridDim.x) < total)
+            stage(tile + gridDim.x, sm + ((k + 1) & 1) * S::buf);
+        cp_async_commit();
+        cp_async_wait<1>();
+        __syncthreads();
+        const float* sz = b + 32 * kWgPlane + og * OGT * S::dzp;
+        if (safe)
+            wg_tile<CO, OGT, true>(b, sz, ks, lane, acc);
+        else
+            wg_tile<CO, OGT, false>(b, sz, ks, lane, acc);
+        if (ks == 0)
+#pragma unroll
+            for (int o = 0; o < OGT; ++o)
+                bsum[o] += sz[o * S::dzp + lane] + sz[o * S::dzp + 32 + lane];
+        __syncthreads();
+    }
+#pragma unroll
+    for (int o = 0; o < OGT; ++o) {
+        const int oc = og * OGT + o;
+#pragma unroll
+        for (int t = 0; t < 9; ++t)
+            atomicAdd(&dw[(oc * 9 + t) * 32 + lane], acc[o][t]);  // a warp's 32 channels: one 128-byte line
+        if (ks == 0) {
+            float s = bsum[o];
+            for (int d = 16; d > 0; d >>= 1)
+                s += __shfl_xor_sync(0xffffffffu, s, d);
+            if (lane == 0)
+                atomicAdd(&db[oc], s);
         }
     }
-    for (int o = 16; o > 0; o >>= 1)
-        l += __shfl_xor_sync(0xffffffffu, l, o);
-    if ((threadIdx.x & 31) == 0)
-        atomicAdd(loss, l * inv);
+}
+
+// The first layer (3 -> 32, interleaved input): a lane is an output with 3 x 9
+// sums, the warps split each tile's columns.
+constexpr int kWg1Dz = kWgPx + 4;  // dz pitch: 4 mod 32, 16-byte reads across outputs conflict-free
+constexpr int kWg1X = 3 * 4 * kPitch;
+constexpr int kWg1Buf = 32 * kWg1Dz + kWg1X;
+
+__global__ void __launch_bounds__(128) wgrad_first_kernel(const float* __restrict__ x, const float* __restrict__ dz,
+    float* __restrict__ dw, float* __restrict__ db, int H, int W, int tiles_x, int tiles, int N,
+    const int* __restrict__ nonfinite)
+{
+    __shared__ __align__(16) float sm[2 * kWg1Buf];
+    __shared__ float red[32 * 28];
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const int64_t HW = static_cast<int64_t>(H) * W;
+    const int total = tiles * N;
+    for (int i = tid; i < 32 * 28; i += 128)
+        red[i] = 0.0f;
+
+    auto stage = [&](int tile, float* b) {
+        const int n = tile / tiles, rem = tile % tiles;
+        const int x0 = (rem % tiles_x) * kTileW, y0 = (rem / tiles_x) * kWgRows;
+        const float* xn = x + static_cast<int64_t>(n) * HW * 3;
+        const float* zn = dz + static_cast<int64_t>(n) * HW * 32;
+        for (int i = tid; i < 32 * kWgPx; i += 128) {
+            const int o = i / kWgPx, q = i % kWgPx, gy = y0 + q / kTileW, gx = x0 + q % kTileW;
+            const bool ok = gy < H && gx < W;
+            cp_async4(b + o * kWg1Dz + q, ok ? zn + o * HW + static_cast<int64_t>(gy) * W + gx : zn, ok);
+        }
+        float* sx = b + 32 * kWg1Dz;
+        for (int i = tid; i < 3 * 4 * 34; i += 128) {
+            const int c = i % 3, q = i / 3, row = q / 34, col = q % 34;
+            const int gy = y0 - 1 + row, gx = x0 - 1 + col;
+            const bool ok = gy >= 0 && gy < H && gx >= 0 && gx < W;
+            cp_async4(sx + (c * 4 + row) * kPitch + col, ok ? xn + (static_cast<int64_t>(gy) * W + gx) * 3 + c : xn, ok);
+        }
+    };
+
+    float acc[27], bsum = 0.0f;
+#pragma unroll
+    for (int t = 0; t < 27; ++t)
+        acc[t] = 0.0f;
+    const bool safe = *nonfinite != 0;
+    int tile = blockIdx.x, k = 0;
+    if (tile < total)
+        stage(tile, sm);
+    cp_async_commit();
+    for (; tile < total; tile += gridDim.x, ++k) {
+        const float* b = sm + (k & 1) * kWg1Buf;
+        if (tile + static_cast<int>(gridDim.x) < total)
+            stage(tile + gridDim.x, sm + ((k + 1) & 1) * kWg1Buf);
+        cp_async_commit();
+        cp_async_wait<1>();
+        __syncthreads();
+        const float* sx = b + 32 * kWg1Dz;
+#pragma unroll 1
+        for (int q = 2 * warp; q < 2 * warp + 2; ++q)  // this warp's 4-pixel groups of each row
+#pragma unroll
+            for (int row = 0; row < kWgRows; ++row) {
+                const float4 z = *reinterpret_cast<const float4*>(b + lane * kWg1Dz + row * kTileW + 4 * q);
+                const float gz[4] = {z.x, z.y, z.z, z.w};
+                bsum += (z.x + z.y) + (z.z + z.w);
+#pragma unroll
+                for (int c = 0; c < 3; ++c)
+#pragma unroll
+                    for (int ky = 0; ky < 3; ++ky) {
+                        const float* xr = sx + (c * 4 + row + ky) * kPitch + 4 * q;
+                        const float4 v0 = *reinterpret_cast<const float4*>(xr);
+                        const float2 v1 = *reinterpret_cast<const float2*>(xr + 4);
+                        const float v[6] = {v0.x, v0.y, v0.z, v0.w, v1.x, v1.y};
+#pragma unroll
+                        for (int i = 0; i < 4; ++i)
+#pragma unroll
+                            for (int kx = 0; kx < 3; ++kx)
+                                acc[(ky * 3 + kx) * 3 + c] = wg_add(safe, gz[i], v[i + kx], acc[(ky * 3 + kx) * 3 + c]);
+                    }
+            }
+        __syncthreads();
+    }
+    __syncthreads();
+    // the four warps' sums, then one coalesced addition per weight and block
+#pragma unroll
+    for (int t = 0; t < 27; ++t)
+        atomicAdd(&red[lane * 27 + t], acc[t]);
+    atomicAdd(&red[32 * 27 + lane], bsum);
+    __syncthreads();
+    for (int i = tid; i < 32 * 27; i += 128)
+        atomicAdd(&dw[i], red[i]);
+    if (tid < 32)
+        atomicAdd(&db[tid], red[32 * 27 + tid]);
 }
 
 __global__ void adam_kernel(float* __restrict__ prm, const float* __restrict__ g, float* __restrict__ m,
@@ -231,22 +544,52 @@ uint64_t splitmix(uint64_t* s)
     return z ^ (z >> 31);
 }
 
-// weights: the layers' weight arrays (parameter layout offsets) in type WT
-template <typename WT>
-cudaError_t forward(const WT* wts, const float* prm, const float* input, float* a1, float* a2, float* a3, float* r,
-    int N, int H, int W, cudaStream_t st)
+// Dynamic shared memory of the training kernels, opted into once per device.
+cudaError_t train_prepare_device(int* sms)
 {
-    const int64_t HW = static_cast<int64_t>(H) * W;
-    const dim3 g(static_cast<unsigned>((HW + kThreads - 1) / kThreads), N);
-    const WT* w0 = wts + kUpLayers[0].w_off;
-    const WT* w1 = wts + kUpLayers[1].w_off;
-    const WT* w2 = wts + kUpLayers[2].w_off;
-    const WT* w3 = wts + kUpLayers[3].w_off;
-    conv_fwd_kernel<3, 32, true, WT><<<g, kThreads, 0, st>>>(input, w0, prm + kUpLayers[0].b_off, a1, H, W);
-    conv_fwd_kernel<32, 32, true, WT><<<g, kThreads, 0, st>>>(a1, w1, prm + kUpLayers[1].b_off, a2, H, W);
-    conv_fwd_kernel<32, 32, true, WT><<<g, kThreads, 0, st>>>(a2, w2, prm + kUpLayers[2].b_off, a3, H, W);
-    conv_fwd_kernel<32, 2, false, WT><<<g, kThreads, 0, st>>>(a3, w3, prm + kUpLayers[3].b_off, r, H, W);
-    return cudaGetLastError();
+    static std::mutex mu;
+    static int count[64] = {};
+    int dev = 0;
+    cudaError_t e = cudaGetDevice(&dev);
+    if (e != cudaSuccess)
+        return e;
+    if (dev < 0 || dev >= 64)
+        return cudaErrorInvalidDevice;
+    std::lock_guard<std::mutex> lock(mu);
+    if (!count[dev]) {
+        constexpr auto kAttr = cudaFuncAttributeMaxDynamicSharedMemorySize;
+        auto set = [&](auto* k, int smem) {
+            if (e == cudaSuccess)
+                e = cudaFuncSetAttribute(k, kAttr, smem);
+        };
+        set(conv3x3_kernel<3, 32, 8, kConvRelu, true>, ConvShape<3, 32, 8>::smem);
+        set(conv3x3_kernel<32, 32, 8, kConvRelu, false>, ConvShape<32, 32, 8>::smem);
+        set(conv3x3_kernel<32, 2, 2, kConvLoss, false>, ConvShape<32, 2, 2>::smem);
+        set(conv3x3_kernel<2, 32, 8, kConvBwd, false>, ConvShape<2, 32, 8>::smem);
+        set(conv3x3_kernel<32, 32, 8, kConvBwd, false>, ConvShape<32, 32, 8>::smem);
+        set(wgrad_kernel<2, 2>, WgShape<2, 2>::smem);
+        set(wgrad_kernel<32, 8>, WgShape<32, 8>::smem);
+        int n = 0;
+        if (e == cudaSuccess)
+            e = cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev);
+        if (e != cudaSuccess)
+            return e;
+        count[dev] = n;
+    }
+    *sms = count[dev];
+    return cudaSuccess;
+}
+
+template <int CI, int CO, int OCT, int kMode, bool kInter>
+void launch_conv(const float* x, const float* prm, int layer, const float* a_prev, float* y, int N, int H, int W,
+    int* nonfinite, cudaStream_t st, const float* input = nullptr, const float* target = nullptr,
+    float* loss = nullptr, float inv = 0.0f)
+{
+    using S = ConvShape<CI, CO, OCT>;
+    const int tx = (W + kTileW - 1) / kTileW, ty = (H + S::rows - 1) / S::rows;
+    conv3x3_kernel<CI, CO, OCT, kMode, kInter><<<dim3(static_cast<unsigned>(tx) * ty, N), 128, S::smem, st>>>(x,
+        prm + kUpLayers[layer].w_off, prm + kUpLayers[layer].b_off, a_prev, y, H, W, tx, input, target, loss, inv,
+        nonfinite);
 }
 
 }  // namespace
@@ -277,47 +620,50 @@ cudaError_t launch_upsampler_prepare(const float* coarse, int cw, int ch, int cf
     return cudaGetLastError();
 }
 
-// One Adam step on a batch: forward, L1 loss, backward, update.
-// work: upsampler_act_floats(N,H,W) * 2 + kParams * 2 (+ slack) floats.
+// One Adam step on a batch: forward, L1 loss, backward, update.  work:
+// upsampler_train_work_floats floats; state: the loss and, as an int, the
+// non-finite flag.
 cudaError_t upsampler_train_step(float* prm, float* grad, float* m, float* v, int step, const float* input,
-    const float* target, int N, int H, int W, float lr, float* work, float* loss_dev, cudaStream_t st)
+    const float* target, int N, int H, int W, float lr, float* work, float* state, cudaStream_t st)
 {
+    int sms = 0;
+    cudaError_t e = train_prepare_device(&sms);
+    if (e != cudaSuccess)
+        return e;
     const int64_t px = static_cast<int64_t>(N) * H * W;
     float* a1 = work;
     float* a2 = a1 + px * 32;
     float* a3 = a2 + px * 32;
-    float* r = a3 + px * 32;
-    float* dr = r + px * 2;
-    float* dz3 = dr + px * 2;
+    float* dz3 = a3 + px * 32;
     float* dz2 = dz3 + px * 32;
     float* dz1 = dz2 + px * 32;
-    cudaError_t e = forward<float>(prm, prm, input, a1, a2, a3, r, N, H, W, st);
-    if (e != cudaSuccess)
-        return e;
+    float* dr = dz1 + px * 32;
+    int* bad = reinterpret_cast<int*>(state + 1);
     if ((e = cudaMemsetAsync(grad, 0, kParams * sizeof(float), st)) != cudaSuccess)
         return e;
-    if ((e = cudaMemsetAsync(loss_dev, 0, sizeof(float), st)) != cudaSuccess)
+    if ((e = cudaMemsetAsync(state, 0, 2 * sizeof(float), st)) != cudaSuccess)
         return e;
-    loss_kernel<<<static_cast<unsigned>((px + 255) / 256), 256, 0, st>>>(input, r, target, dr, loss_dev, px,
+    launch_conv<3, 32, 8, kConvRelu, true>(input, prm, 0, nullptr, a1, N, H, W, bad, st);
+    launch_conv<32, 32, 8, kConvRelu, false>(a1, prm, 1, nullptr, a2, N, H, W, bad, st);
+    launch_conv<32, 32, 8, kConvRelu, false>(a2, prm, 2, nullptr, a3, N, H, W, bad, st);
+    launch_conv<32, 2, 2, kConvLoss, false>(a3, prm, 3, nullptr, dr, N, H, W, bad, st, input, target, state,
         1.0f / static_cast<float>(px));
-    const int64_t HW = static_cast<int64_t>(H) * W;
-    const dim3 g(static_cast<unsigned>((HW + kThreads - 1) / kThreads), N);
-    const unsigned slices = static_cast<unsigned>(std::min<int64_t>(64, (px + 4095) / 4096));
-    // layer 4 (32 -> 2)
-    conv_wgrad_kernel<32, 2><<<dim3(2, 9, slices), kThreads, 0, st>>>(a3, dr, grad + kUpLayers[3].w_off,
-        grad + kUpLayers[3].b_off, N, H, W);
-    conv_bwd_data_kernel<32, 2, true><<<g, kThreads, 0, st>>>(dr, prm + kUpLayers[3].w_off, a3, dz3, H, W);
-    // layer 3
-    conv_wgrad_kernel<32, 32><<<dim3(32, 9, slices), kThreads, 0, st>>>(a2, dz3, grad + kUpLayers[2].w_off,
-        grad + kUpLayers[2].b_off, N, H, W);
-    conv_bwd_data_kernel<32, 32, true><<<g, kThreads, 0, st>>>(dz3, prm + kUpLayers[2].w_off, a2, dz2, H, W);
-    // layer 2
-    conv_wgrad_kernel<32, 32><<<dim3(32, 9, slices), kThreads, 0, st>>>(a1, dz2, grad + kUpLayers[1].w_off,
-        grad + kUpLayers[1].b_off, N, H, W);
-    conv_bwd_data_kernel<32, 32, true><<<g, kThreads, 0, st>>>(dz2, prm + kUpLayers[1].w_off, a1, dz1, H, W);
-    // layer 1 (3 -> 32): weights only
-    conv_wgrad_kernel<3, 32><<<dim3(32, 9, slices), kThreads, 0, st>>>(input, dz1, grad + kUpLayers[0].w_off,
-        grad + kUpLayers[0].b_off, N, H, W);
+    // weight gradients: resident blocks walk the tiles, so a block's sums are added once
+    const int tx = (W + kTileW - 1) / kTileW, tiles = tx * ((H + kWgRows - 1) / kWgRows);
+    const int wb = static_cast<int>(std::min<int64_t>(static_cast<int64_t>(tiles) * N, 4 * sms));
+    float* gw[4];
+    float* gb[4];
+    for (int l = 0; l < 4; ++l) {
+        gw[l] = grad + kUpLayers[l].w_off;
+        gb[l] = grad + kUpLayers[l].b_off;
+    }
+    wgrad_kernel<2, 2><<<wb, 128, WgShape<2, 2>::smem, st>>>(a3, dr, gw[3], gb[3], H, W, tx, tiles, N, bad);
+    launch_conv<2, 32, 8, kConvBwd, false>(dr, prm, 3, a3, dz3, N, H, W, bad, st);
+    wgrad_kernel<32, 8><<<wb, 128, WgShape<32, 8>::smem, st>>>(a2, dz3, gw[2], gb[2], H, W, tx, tiles, N, bad);
+    launch_conv<32, 32, 8, kConvBwd, false>(dz3, prm, 2, a2, dz2, N, H, W, bad, st);
+    wgrad_kernel<32, 8><<<wb, 128, WgShape<32, 8>::smem, st>>>(a1, dz2, gw[1], gb[1], H, W, tx, tiles, N, bad);
+    launch_conv<32, 32, 8, kConvBwd, false>(dz2, prm, 1, a1, dz1, N, H, W, bad, st);
+    wgrad_first_kernel<<<wb, 128, 0, st>>>(input, dz1, gw[0], gb[0], H, W, tx, tiles, N, bad);
     const float b1 = 0.9f, b2 = 0.999f;
     const float c1 = 1.0f - std::pow(b1, static_cast<float>(step)), c2 = 1.0f - std::pow(b2, static_cast<float>(step));
     adam_kernel<<<(kParams + 255) / 256, 256, 0, st>>>(prm, grad, m, v, kParams, lr, b1, b2, c1, c2, 1e-8f);
@@ -327,7 +673,7 @@ cudaError_t upsampler_train_step(float* prm, float* grad, float* m, float* v, in
 size_t upsampler_train_work_floats(int N, int H, int W)
 {
     const size_t px = static_cast<size_t>(N) * H * W;
-    return px * (32 * 3 + 2 + 2 + 32 * 3);
+    return px * (32 * 6 + 2);
 }
 
 }  // namespace vsc
