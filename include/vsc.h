@@ -280,7 +280,10 @@ VSC_API vsc_status vsc_get_consist_out(const vsc_image* crnt_pr, const vsc_image
 /* vsc_get_consist_out in the VSC_SOLVER_FMA form: same arguments; its
  * workspace (vsc_consist_out_fma_workspace_size bytes, 16-byte aligned, or
  * NULL for the library's stream-ordered pool) holds the solve as planes, 18
- * floats a pixel.  Results within the tolerance stated at VSC_SOLVER_FMA of
+ * floats a pixel.  Where the width is not a multiple of 4, the TMA-fed solve
+ * needs the bytes of the width rounded up to one: NULL takes them, and so does
+ * a workspace that has them; a smaller one is solved with plain loads (same
+ * bits, about 2.5 times the time).  Results within the tolerance stated at VSC_SOLVER_FMA of
  * vsc_get_consist_out's.  No counterpart in the reference. */
 VSC_API size_t vsc_consist_out_fma_workspace_size(int32_t width, int32_t height);
 VSC_API vsc_status vsc_get_consist_out_fma(const vsc_image* crnt_pr, const vsc_image* prev_stab_warp,

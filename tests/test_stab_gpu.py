@@ -195,6 +195,24 @@ def test_consist_out_fma(vsc, oracle, cuda, h, w, iters):
     assert np.array_equal(O2.cpu().numpy().view(np.uint32), got.view(np.uint32))
 
 
+@pytest.mark.parametrize("w,h", [(113, 57), (114, 64), (115, 73), (119, 130), (121, 65), (225, 120), (238, 61),
+                                 (853, 60), (1, 70), (5, 200)])
+def test_consist_out_fma_any_width(vsc, oracle, cuda, w, h):
+    """Widths that are not a multiple of 4 run the TMA-fed solve on planes of
+    padded rows: the frame's last two columns in any column of a lane and in
+    the tile before the last (113, 225), a partial last tile, one column."""
+    import torch
+
+    P, A, Wt, O0 = _img(h, w), _img(h, w), _img(h, w, hi=2.0), _img(h, w)
+    for iters in (8, 27):
+        O = _t(O0, cuda)
+        vsc.get_consist_out(_t(P, cuda), _t(A, cuda), _t(Wt, cuda), iters, 0.15, 0.15, O, form="fma")
+        ref = oracle.consist_out(P, A, Wt, iters, 0.15, 0.15, O0, form="fma")
+        assert np.array_equal(O.cpu().numpy().view(np.uint32), ref.view(np.uint32))
+    torch.cuda.synchronize()
+    vsc.check_device()
+
+
 def test_consist_out_fma_single_tile_shape(vsc, cuda):
     """The FMA form has one tile shape (128 x 72 of a plane); the autotuner
     reports it without measuring."""

@@ -517,6 +517,7 @@ vsc_status consist_out_form(int form, const vsc_image* crnt_pr, const vsc_image*
     const int w = consis_out->width, h = consis_out->height;
     const size_t need = solver_workspace_floats(w, h, form) * sizeof(float);
     void* ws = workspace;
+    size_t ws_bytes = workspace_bytes;
     bool pooled = false;
     if (ws) {
         if (workspace_bytes < need)
@@ -524,12 +525,13 @@ vsc_status consist_out_form(int form, const vsc_image* crnt_pr, const vsc_image*
         if (reinterpret_cast<uintptr_t>(ws) & 15)
             return set_error(VSC_EINVAL, "consist_out: workspace not 16-byte aligned");
     } else if (num_iter > 0) {
-        if ((s = check_cuda(pool_alloc(&ws, need, cs(stream)), "consist_out workspace")))
+        ws_bytes = solver_workspace_full_floats(w, h, form) * sizeof(float);
+        if ((s = check_cuda(pool_alloc(&ws, ws_bytes, cs(stream)), "consist_out workspace")))
             return s;
         pooled = true;
     }
     cudaError_t e = run_solver(crnt_pr->data, prev_stab_warp->data, cons_wt->data, consis_out->data, w, h, num_iter,
-        step_size, mom_fac, static_cast<float*>(ws), cs(stream), nullptr, nullptr, form);
+        step_size, mom_fac, static_cast<float*>(ws), ws_bytes / sizeof(float), cs(stream), nullptr, nullptr, form);
     if (pooled)
         cudaFreeAsync(ws, cs(stream));
     return check_cuda(e, "consist_out launch");
@@ -907,7 +909,7 @@ vsc_status alloc_all(vsc_stabilizer* s)
         A(dalloc(&s->pyrW[j], m));
         A(dalloc(&s->pyrO[j], m));
     }
-    A(dalloc(&s->solver_ws, solver_workspace_floats(s->w, s->h, kSolverFma)));  // room for either form
+    A(dalloc(&s->solver_ws, solver_workspace_any_floats(s->w, s->h)));
     if (s->compute_flow) {
         s->fd = flow_dims(s->fw, s->fh);
         // the three frames' features in one allocation, so a flow pair can
@@ -1281,6 +1283,7 @@ cudaError_t enqueue_step(vsc_stabilizer* s, const vsc_hyper_params& hp, uint8_t*
     float** A = lv.A;
     float** W = lv.W;
     float** O = lv.O;
+    const size_t ws_floats = solver_workspace_any_floats(s->w, s->h);
     // The solution is initialised with the processed frame and carried down
     // with the same bilinear chain, so at the coarsest level it equals P.
     run(cudaMemcpyAsync(O[L - 1], P[L - 1], static_cast<size_t>(s->lw[L - 1]) * s->lh[L - 1] * 3 * sizeof(float),
@@ -1294,15 +1297,15 @@ cudaError_t enqueue_step(vsc_stabilizer* s, const vsc_hyper_params& hp, uint8_t*
         if (j != L - 1 && s->solver_form == kSolverFma && iters > 0) {
             // the FMA form upsamples the coarser solution in its setup pass
             run(run_solver_from_coarse(P[j], A[j], W[j], O[j], s->lw[j], s->lh[j], O[j + 1], s->lw[j + 1],
-                s->lh[j + 1], iters, hp.step_size, hp.mom_fac, s->solver_ws, st, &nl, rgba));
+                s->lh[j + 1], iters, hp.step_size, hp.mom_fac, s->solver_ws, ws_floats, st, &nl, rgba));
             continue;
         }
         if (j != L - 1) {
             run(launch_bilinear(Img{O[j + 1], s->lw[j + 1], s->lh[j + 1], 3}, Img{O[j], s->lw[j], s->lh[j], 3}, st));
             ++nl;
         }
-        run(run_solver(P[j], A[j], W[j], O[j], s->lw[j], s->lh[j], iters, hp.step_size, hp.mom_fac, s->solver_ws, st,
-            &nl, rgba, s->solver_form));
+        run(run_solver(P[j], A[j], W[j], O[j], s->lw[j], s->lh[j], iters, hp.step_size, hp.mom_fac, s->solver_ws,
+            ws_floats, st, &nl, rgba, s->solver_form));
     }
     mark(s, kEvStep1);
     *launches = nl;
@@ -1867,7 +1870,7 @@ float* ms_level_ws(vsc_multistream* m, size_t i, int j)
         return s->solver_ws;
     float* p = m->lvl_ws[i];
     for (int k = 1; k < j; ++k)
-        p += solver_workspace_floats(s->lw[k], s->lh[k], kSolverFma);
+        p += solver_workspace_any_floats(s->lw[k], s->lh[k]);
     return p;
 }
 
@@ -2105,7 +2108,7 @@ VSC_API vsc_status vsc_multistream_create(const vsc_stream_desc* desc, int32_t n
         vsc_stabilizer* st = m->st[i];
         size_t floats = 0;
         for (int j = 1; j < st->levels_alloc; ++j)
-            floats += solver_workspace_floats(st->lw[j], st->lh[j], kSolverFma);  // room for either form
+            floats += solver_workspace_any_floats(st->lw[j], st->lh[j]);
         float* p = nullptr;
         if (floats && (s = check_cuda(dalloc(&p, floats), "multistream_create level workspaces")))
             break;

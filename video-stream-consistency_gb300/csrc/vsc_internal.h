@@ -147,6 +147,11 @@ cudaError_t launch_bilinear_group(const Img* in, const Img* out, int n, cudaStre
 //                 6 * w*h*3 floats.
 enum SolverForm { kSolverExact = 0, kSolverFma = 1 };
 size_t solver_workspace_floats(int w, int h, int form = kSolverExact);
+// The same with room for the FMA form's planes at a row pitch on the 16-byte
+// grid, which the TMA-fed solve wants: more than the above for widths that are
+// not a multiple of 4 only.  A workspace between the two takes plain loads.
+size_t solver_workspace_full_floats(int w, int h, int form);
+size_t solver_workspace_any_floats(int w, int h);  // the larger form's
 int solver_steps_per_launch();  // Jacobi steps one solver launch performs (temporal blocking)
 // Tile-shape autotuner of the persistent solver kernels (same results either
 // way): solver_autotune times both shapes at (w, h) on scratch images and
@@ -162,16 +167,16 @@ cudaError_t solver_group_autotune(const int* w, const int* h, int n, cudaStream_
     int form = kSolverExact);
 int solver_group_tile_rows(const int* w, const int* h, int n, bool* tuned, int form = kSolverExact);
 // Runs num_iter iterations; O holds the initial solution and receives the
-// result.  Returns the number of kernels launched through *launches.
+// result; workspace: ws_floats floats, at least solver_workspace_floats.  Returns the number of kernels launched through *launches.
 cudaError_t run_solver(const float* P, const float* A, const float* Wt, float* O, int w, int h, int num_iter,
-    float step, float mom, float* workspace, cudaStream_t st, int* launches, uint8_t* rgba_out = nullptr,
-    int form = kSolverExact);
+    float step, float mom, float* workspace, size_t ws_floats, cudaStream_t st, int* launches,
+    uint8_t* rgba_out = nullptr, int form = kSolverExact);
 // The FMA form started from the cw x ch solution Oc upsampled to w x h with
 // kernel_bilinear's expression (the pyramid's next level), the upsampling
 // fused into the solve's setup; O receives the result only.  num_iter >= 1.
 cudaError_t run_solver_from_coarse(const float* P, const float* A, const float* Wt, float* O, int w, int h,
-    const float* Oc, int cw, int ch, int num_iter, float step, float mom, float* workspace, cudaStream_t st,
-    int* launches, uint8_t* rgba_out);
+    const float* Oc, int cw, int ch, int num_iter, float step, float mom, float* workspace, size_t ws_floats,
+    cudaStream_t st, int* launches, uint8_t* rgba_out);
 
 // Grouped solve: n images of any sizes, the same iterations, each launch of
 // the persistent kernel walking the tiles of all of them (up to 16 images

@@ -874,32 +874,48 @@ __global__ void __launch_bounds__(kPThreads, 1)
 //
 // The three colour channels of the step never interact, so the form solves
 // each channel as its own image: the workspace holds O, U, Cs and nK as
-// planes (channel-major, solver_to_planar / solver_from_planar convert O at
-// the ends of a solve).  A tile is 128 x 72 pixels of one plane: each of the
-// 384 threads keeps a 4-column x 6-row block of O, U, Cs and nK in registers
-// (96 floats), a warp spans the tile's width, so the 8-pixel ring of the
-// temporal blocking leaves a 112 x 56 interior (68 % of the tile; the
-// interleaved 64 x 48 tile of three channels kept 50 %), horizontal
-// neighbours cost two shuffles per row for four pixels, and each warp
-// publishes its top and bottom row as two 16-byte stores per thread.
+// planes (channel-major, planar_group_kernel converts O at the ends of a
+// solve).  A tile is 128 x 72 pixels of one plane: each of 256 threads keeps a
+// 4-column x 9-row block of O, U, Cs and nK in registers (144 floats), a warp
+// spans the tile's width, so the 8-pixel ring of the temporal blocking leaves
+// a 112 x 56 interior (68 % of the tile), horizontal neighbours cost two
+// shuffles per row for four pixels, and each warp publishes its top and
+// bottom row as two 16-byte stores per thread.
 
 constexpr int kPlW = 128;                 // tile width (a warp: 32 lanes x 4 columns)
 constexpr int kPlIW = kPlW - 2 * kTbT;    // interior width (112)
-constexpr int kPlPX = kPlW + 8;           // edge-row pitch (a 16-byte apron each side)
-constexpr int kPlWarps = 12;
-constexpr int kPlThreads = 32 * kPlWarps;
-constexpr int kPlRPT = 6;                 // rows per thread
-constexpr int kPlRows = kPlRPT * kPlWarps;  // 72
-constexpr int kPlIRows = kPlRows - 2 * kTbT;  // 56
-constexpr int kPlStage = kPlRows * kPlW;  // floats of one input tile
-constexpr int kPlStageBytes = kPlStage * static_cast<int>(sizeof(float));
-constexpr int kPlSlotPlane = (kPlWarps + 2) * 2 * kPlPX;  // edge-row slots of one buffer
-constexpr int kPlOut = kPlIRows * kPlIW;  // floats of one interior tile
-constexpr int kPlSmem = 4 * kPlStageBytes + (2 * kPlSlotPlane + 2 * kPlOut) * static_cast<int>(sizeof(float)) + 16;
-static_assert(kPlSmem <= 232448, "dynamic shared memory per CTA");
+
+// A form's tile: kPlanes input planes, kWarps warps of kRPT rows each.
+template <int kForm>
+struct PlG;
+template <>
+struct PlG<kSolverFma> {
+    static constexpr int kPlanes = 4, kWarps = 8, kRPT = 9;
+};
+
+template <int kForm>
+struct PlGeo : PlG<kForm> {
+    using PlG<kForm>::kPlanes;
+    using PlG<kForm>::kWarps;
+    using PlG<kForm>::kRPT;
+    static constexpr int kRows = kRPT * kWarps;          // 72
+    static constexpr int kIRows = kRows - 2 * kTbT;      // interior rows (56)
+    static constexpr int kStage = kRows * kPlW;          // floats of one input tile
+    static constexpr int kStageBytes = kStage * static_cast<int>(sizeof(float));
+    static constexpr int kSlots = (kWarps + 2) * 2 * kPlW;  // edge-row slots of one buffer
+    static constexpr int kOut = kIRows * kPlIW;          // floats of one interior tile
+    static constexpr int kSmem =
+        kPlanes * kStageBytes + (2 * kSlots + 2 * kOut) * static_cast<int>(sizeof(float)) + 128;
+    static_assert(kSmem <= 232448, "dynamic shared memory per CTA");
+    static_assert((kPlanes * kStageBytes) % 128 == 0 && (2 * kSlots * 4) % 128 == 0 && (kOut * 4) % 128 == 0,
+        "TMA sources and destinations on the 128-byte grid");
+    // rows of the tile that the frame's rows 0 (tiles at oy = -8) and h - 2, h - 1
+    // (tiles that end on the frame's last row) sit in, as warp and row
+    static constexpr int kTopWarp = kTbT / kRPT, kTopRow = kTbT % kRPT;
+    static constexpr int kBot2Warp = (kRows - kTbT - 2) / kRPT, kBot2Row = (kRows - kTbT - 2) % kRPT;
+    static constexpr int kBot1Warp = (kRows - kTbT - 1) / kRPT, kBot1Row = (kRows - kTbT - 1) % kRPT;
+};
 static_assert((kPlIW * 4) % 16 == 0 && (kTbT * 4) % 16 == 0, "TMA x coordinates must be 16-byte aligned");
-static_assert((4 * kPlStageBytes) % 128 == 0 && (2 * kPlSlotPlane * 4) % 128 == 0 && (kPlOut * 4) % 128 == 0,
-    "TMA sources and destinations on the 128-byte grid");
 
 // Cs = step * fma(wt, A, -lap P) and nK = -(step * (cnt + wt)) as planes
 // (lap P, cnt as lap_pr_kernel computes them); with O non-null, also O as
@@ -909,7 +925,7 @@ static_assert((4 * kPlStageBytes) % 128 == 0 && (2 * kPlSlotPlane * 4) % 128 == 
 // solve counters zeroed.
 __global__ void solver_prep_fma_kernel(const float* __restrict__ P, const float* __restrict__ A,
     const float* __restrict__ Wt, const float* __restrict__ O, float* __restrict__ Cs, float* __restrict__ nK,
-    float* __restrict__ Op, int w, int h, float step, unsigned* __restrict__ cnt, int ncnt,
+    float* __restrict__ Op, int w, int h, int pitch, float step, unsigned* __restrict__ cnt, int ncnt,
     const float* __restrict__ Oc, int cw, int ch)
 {
     pdl_enter();
@@ -922,8 +938,8 @@ __global__ void solver_prep_fma_kernel(const float* __restrict__ P, const float*
         return;
     const int64_t i0 = pix_index(x, y, w) * 3;
     const int64_t rs = static_cast<int64_t>(w) * 3;
-    const int64_t plane = static_cast<int64_t>(w) * h;
-    const int64_t q = pix_index(x, y, w);
+    const int64_t plane = static_cast<int64_t>(pitch) * h;
+    const int64_t q = pix_index(x, y, pitch);
     float up[3];
     if (Oc)
         bilinear_px(Oc, cw, ch, w, h, 3, x, y, up);
@@ -960,7 +976,7 @@ __global__ void solver_prep_fma_kernel(const float* __restrict__ P, const float*
 
 // Interleaved <-> planar copies of the images of up to kPlanarGroupMax solves
 // (one launch per level of a multi-stream step): to_planar = 1 reads the
-// interleaved src and writes dst as planes; 0 the reverse, and writes the
+// interleaved src and writes dst as planes of `pitch`-float rows; 0 the reverse, and writes the
 // RGBA8 copy when rgba is non-null.
 constexpr int kPlanarGroupMax = 16;
 struct PlanarGroup {
@@ -970,6 +986,8 @@ struct PlanarGroup {
     unsigned* cnt[kPlanarGroupMax];  // solve counters zeroed on the way in, or null
     int ncnt[kPlanarGroupMax];
     int64_t npix[kPlanarGroupMax];
+    int w[kPlanarGroupMax], pitch[kPlanarGroupMax];  // of an image row, of a plane's row
+    int64_t plane[kPlanarGroupMax];                  // floats of a plane
     int block0[kPlanarGroupMax + 1];
     int count;
 };
@@ -987,14 +1005,18 @@ __global__ void __launch_bounds__(256) planar_group_kernel(const __grid_constant
     const int64_t n = g.npix[p];
     if (i >= n)
         return;
+    const int64_t pl = g.plane[p];
+    int64_t q = i;  // the pixel's place in a plane
+    if (g.pitch[p] != g.w[p])
+        q += (n < (int64_t{1} << 31) ? static_cast<int>(i) / g.w[p] : i / g.w[p]) * (g.pitch[p] - g.w[p]);
     if (to_planar) {
         const float* s = g.src[p] + i * 3;
-        g.dst[p][i] = s[0];
-        g.dst[p][n + i] = s[1];
-        g.dst[p][2 * n + i] = s[2];
+        g.dst[p][q] = s[0];
+        g.dst[p][pl + q] = s[1];
+        g.dst[p][2 * pl + q] = s[2];
         return;
     }
-    const float r = g.src[p][i], gg = g.src[p][n + i], b = g.src[p][2 * n + i];
+    const float r = g.src[p][q], gg = g.src[p][pl + q], b = g.src[p][2 * pl + q];
     float* d = g.dst[p] + i * 3;
     d[0] = r;
     d[1] = gg;
@@ -1003,8 +1025,10 @@ __global__ void __launch_bounds__(256) planar_group_kernel(const __grid_constant
         reinterpret_cast<uint32_t*>(g.rgba[p])[i] = pack_rgba(r, gg, b);
 }
 
+template <int kForm>
 struct PlState {
-    float4 o[kPlRPT], u[kPlRPT], c[kPlRPT], nk[kPlRPT];  // [row] = (column 0 .. 3)
+    static constexpr int kR = PlGeo<kForm>::kRPT;
+    float4 o[kR], u[kR], c[kR], nk[kR];  // [row] = (column 0 .. 3)
 };
 
 __device__ __forceinline__ float& f4(float4& v, int j) { return j == 0 ? v.x : j == 1 ? v.y : j == 2 ? v.z : v.w; }
@@ -1023,137 +1047,231 @@ __device__ __forceinline__ float f4c(const float4& v, int j) { return j == 0 ? v
 //             a multiple of 4: column 0 is then column j = 0 of the thread
 //             with gx0 = 0 and columns w - 2, w - 1 are j = 2, 3 of the thread
 //             with gx0 = w - 4 (three selects a row); row 0 of a tile at
-//             oy = -8 is row 2 of warp 1 and rows h - 2, h - 1 of a tile at
-//             oy = h - 64 are rows 2, 3 of warp 10 (a select of a row's up or
-//             down neighbours in every warp, true only in that one).  A tile
+//             oy = -8 and rows h - 2, h - 1 of a tile at oy = h - 64 are fixed
+//             rows of fixed warps (kTopRow ..: a select of a row's up or down
+//             neighbours in every warp, true only in that one).  A tile
 //             holding row 0, h - 2 or h - 1 elsewhere (frames of few rows)
-//             takes kPlEvery.  Same bits as kPlEvery for every pixel inside
-//             the frame, without its four tests a pixel.
-//   kPlEvery: every neighbour tested.
-enum { kPlAll, kPlLanes, kPlEvery };
+//             takes kPlEvery.
+//   kPlCols:  the same for any other width: columns w - 2 and w - 1 may be any
+//             column of a thread (five selects a row).
+//   kPlEvery: rows 0, h - 2 and h - 1 anywhere, too (a select of every row's up
+//             and down neighbours).
+enum { kPlAll, kPlLanes, kPlCols, kPlEvery };
 
-// One step of a thread's 4 x 6 block: the previous iterate's edge rows of the
-// neighbouring warps come from `src`, the new top and bottom rows go to `dst`.
-// zl / zr (kPlLanes): this thread holds column 0 / columns w - 4 .. w - 1;
-// zt / zb: its row 2 is row 0 / its rows 2 and 3 are rows h - 2 and h - 1.
-template <int kMode>
-__device__ __forceinline__ void pl_step(PlState& s, const float* src, float* dst, bool mom_on, float step, float mom,
-    int lane, int warp, int gx0, int gy0, int w, int h, bool zl, bool zr, bool zt, bool zb)
+// What a step needs to know of its thread's place.  zl / zr: it holds column 0 /
+// columns w - 4 .. w - 1; zt / zb2 / zb1 (kPlLanes, kPlCols): its row kTopRow /
+// kBot2Row / kBot1Row is the frame's row 0 / h - 2 / h - 1.
+struct PlPlace {
+    int xlim;      // its first column that is column w - 2 or beyond
+    int top, bot;  // kPlEvery: its row that is row 0, its first one that is row h - 2 or beyond
+    bool zl, zr, zt, zb2, zb1;
+};
+
+// The columns left and right of a thread's block, from the neighbouring lanes
+// (the outer lanes keep their own value: the tile's outer columns never reach
+// the interior).
+template <int kForm>
+struct PlSides {
+    float l[PlGeo<kForm>::kRPT], r[PlGeo<kForm>::kRPT];
+};
+
+// One step of row r of a thread's block: the new row in `on`, U in place;
+// then the lanes exchange the new row's end columns for the next step.
+template <int kForm, int kMode>
+__device__ __forceinline__ void pl_row(PlState<kForm>& s, PlSides<kForm>& x, float4* on, int r, float4 up, float4 dn,
+    float step, float mom, const PlPlace& t)
 {
-    const float4 up = *reinterpret_cast<const float4*>(&src[(warp * 2 + 1) * kPlPX + 4 * lane + 4]);
-    const float4 dn = *reinterpret_cast<const float4*>(&src[((warp + 2) * 2) * kPlPX + 4 * lane + 4]);
-    float L[kPlRPT], R[kPlRPT];
-#pragma unroll
-    for (int r = 0; r < kPlRPT; ++r) {
-        L[r] = __shfl_up_sync(0xffffffffu, s.o[r].w, 1);
-        R[r] = __shfl_down_sync(0xffffffffu, s.o[r].x, 1);
-    }
-    float4 on[kPlRPT];
-#pragma unroll
-    for (int r = 0; r < kPlRPT; ++r) {
-        const float4 o = s.o[r];
-        float4 u = r == 0 ? up : s.o[r - 1];
-        float4 d = r == kPlRPT - 1 ? dn : s.o[r + 1];
-        if (kMode == kPlLanes && r == 2 && zt)
-            u = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-        if (kMode == kPlLanes && (r == 2 || r == 3) && zb)
-            d = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-        bool vu = true, vd = true;
-        if (kMode == kPlEvery) {
-            vu = (gy0 + r - 1) >= 0;
-            vd = (gy0 + r + 1) < (h - 1);
-        }
-        float lft = L[r], rgt = R[r], o3 = o.w;  // left of column 0, right of columns 3 and 2
-        if (kMode == kPlLanes) {
-            lft = zl ? 0.0f : lft;
-            rgt = zr ? 0.0f : rgt;
-            o3 = zr ? 0.0f : o3;
-        }
-#pragma unroll
-        for (int j = 0; j < 4; ++j) {
-            float left = j == 0 ? lft : f4c(o, j - 1);
-            float right = j == 3 ? rgt : (j == 2 ? o3 : f4c(o, j + 1));
-            float upv = f4c(u, j), dnv = f4c(d, j);
-            if (kMode == kPlEvery) {
-                const int gx = gx0 + j;
-                left = (gx - 1) >= 0 ? left : 0.0f;
-                right = (gx + 1) < (w - 1) ? right : 0.0f;
-                upv = vu ? upv : 0.0f;
-                dnv = vd ? dnv : 0.0f;
-            }
-            const float oj = f4c(o, j);
-            const float g = __fmaf_rn(f4c(s.nk[r], j), oj,
-                __fmaf_rn(step, __fadd_rn(__fadd_rn(left, right), __fadd_rn(upv, dnv)), f4c(s.c[r], j)));
-            float n = __fadd_rn(oj, g);
-            if (mom_on)
-                n = __fmaf_rn(mom, f4c(s.u[r], j), n);
-            f4(s.u[r], j) = g;
-            f4(on[r], j) = n;
-        }
+    using G = PlGeo<kForm>;
+    const float4 o = s.o[r];
+    float4 u = r == 0 ? up : s.o[r - 1];
+    float4 d = r == G::kRPT - 1 ? dn : s.o[r + 1];
+    constexpr bool kFixed = kMode == kPlLanes || kMode == kPlCols;
+    if (kFixed && r == G::kTopRow && t.zt)
+        u = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+    if (kFixed && ((r == G::kBot2Row && t.zb2) || (r == G::kBot1Row && t.zb1)))
+        d = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+    if (kMode == kPlEvery && r == t.top)
+        u = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+    if (kMode == kPlEvery && r >= t.bot)
+        d = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+    float lft = x.l[r], rgt = x.r[r], o3 = o.w;  // left of column 0, right of columns 3 and 2
+    if (kMode != kPlAll)
+        lft = t.zl ? 0.0f : lft;
+    if (kMode == kPlLanes) {
+        rgt = t.zr ? 0.0f : rgt;
+        o3 = t.zr ? 0.0f : o3;
     }
 #pragma unroll
-    for (int r = 0; r < kPlRPT; ++r)
+    for (int j = 0; j < 4; ++j) {
+        const float left = j == 0 ? lft : f4c(o, j - 1);
+        float right = j == 3 ? rgt : (j == 2 ? o3 : f4c(o, j + 1));
+        if (kMode == kPlCols || kMode == kPlEvery)
+            right = j < t.xlim ? right : 0.0f;
+        const float oj = f4c(o, j);
+        const float g = __fmaf_rn(f4c(s.nk[r], j), oj,
+            __fmaf_rn(step, __fadd_rn(__fadd_rn(left, right), __fadd_rn(f4c(u, j), f4c(d, j))), f4c(s.c[r], j)));
+        f4(on[r], j) = __fmaf_rn(mom, f4c(s.u[r], j), __fadd_rn(oj, g));
+        f4(s.u[r], j) = g;
+    }
+    x.l[r] = __shfl_up_sync(0xffffffffu, on[r].w, 1);
+    x.r[r] = __shfl_down_sync(0xffffffffu, on[r].x, 1);
+}
+
+// One step of a thread's block; `up` and `dn` are the previous iterate's rows
+// above and below it.  The rows between go first, while those two arrive; each
+// row's shuffles for the next step run beside the following rows' arithmetic.
+template <int kForm, int kMode>
+__device__ __forceinline__ void pl_step(PlState<kForm>& s, PlSides<kForm>& x, float4 up, float4 dn, float step,
+    float mom, const PlPlace& t)
+{
+    constexpr int kR = PlGeo<kForm>::kRPT;
+    float4 on[kR];
+#pragma unroll
+    for (int q = 0; q < kR; ++q)
+        pl_row<kForm, kMode>(s, x, on, q < kR - 2 ? q + 1 : (q == kR - 2 ? 0 : kR - 1), up, dn, step, mom, t);
+#pragma unroll
+    for (int r = 0; r < kR; ++r)
         s.o[r] = on[r];
-    float* D = dst + ((warp + 1) * 2) * kPlPX + 4 * lane + 4;
-    *reinterpret_cast<float4*>(D) = on[0];                   // top row
-    *reinterpret_cast<float4*>(D + kPlPX) = on[kPlRPT - 1];  // bottom row
 }
 
 // The planar step's test mode for a tile at (ox, oy) of a w x h frame.
+template <int kForm>
 __device__ __forceinline__ int pl_mode(int ox, int oy, int w, int h)
 {
-    if (ox >= 1 && oy >= 1 && ox + kPlW - 1 <= w - 3 && oy + kPlRows - 1 <= h - 3)
+    constexpr int kRows = PlGeo<kForm>::kRows;
+    if (ox >= 1 && oy >= 1 && ox + kPlW - 1 <= w - 3 && oy + kRows - 1 <= h - 3)
         return kPlAll;
-    const bool row0 = oy <= 0 && oy + kPlRows - 1 >= 0;
-    const bool last2 = oy <= h - 1 && oy + kPlRows - 1 >= h - 2;
-    if ((w & 3) == 0 && (ox & 3) == 0 && (!row0 || oy == -kTbT) && (!last2 || oy == h - kPlRows + kTbT))
-        return kPlLanes;
+    const bool row0 = oy <= 0 && oy + kRows - 1 >= 0;
+    const bool last2 = oy <= h - 1 && oy + kRows - 1 >= h - 2;
+    if ((!row0 || oy == -kTbT) && (!last2 || oy == h - kRows + kTbT))  // ox is a multiple of 4
+        return (w & 3) == 0 ? kPlLanes : kPlCols;
     return kPlEvery;
 }
 
-// Iteration k is needed on rows [ring - T + k + 1, kPlRows - ring + T - k - 1)
-// (ring = kTbT); a warp whose rows all lie outside skips it.  idle(k) runs in
-// the warps that skip the last three steps k of a full round (warps 0 and
-// 11: work a caller keeps off the steps' critical path, as long as each part
-// fits a step); in a shorter round idle(kTbT - 3) runs before its steps and
-// the other two after them.
-template <int kMode, class Idle>
-__device__ __forceinline__ void pl_iterate(PlState& s, float* slots, int T, int k0, float step, float mom, int lane,
-    int warp, int gx0, int gy0, int w, int h, int oy, Idle&& idle)
+// The steps of one tile's round.  After each step a warp publishes its top and
+// bottom row to a slot buffer (slot w + 1 is warp w's; even steps write buffer
+// 0 and odd ones buffer 1) and bar() joins the warps; `up` and `dn` are the
+// rows above and below the thread's block in the initial iterate.
+//
+// The steps of a full round are a loop of two: unrolled to eight, its code (24
+// KB a test mode) missed the instruction cache for 10 % of the warps' time,
+// and with a condition in it (momentum off in a solve's first step, steps left
+// out) the two steps' registers meet in moves.  A solve's first step has U = +0
+// and takes mom = -0: fma(-0, +0, n) is n, whatever n is.
+template <int kForm, int kMode, class Bar>
+__device__ __forceinline__ void pl_steps(PlState<kForm>& s, float4 up, float4 dn, float* slots, int T, int k0,
+    float step, float mom, int lane, int warp, const PlPlace& t, Bar&& bar)
 {
-    const int r0 = kPlRPT * warp;
-    const bool zl = gx0 == 0, zr = gx0 == w - 4;
-    const bool zt = oy == -kTbT && warp == 1, zb = oy == h - kPlRows + kTbT && warp == 10;
-    auto one = [&](int k, bool mom_on) {
-        pl_step<kMode>(s, slots + (k & 1) * kPlSlotPlane, slots + ((k & 1) ^ 1) * kPlSlotPlane, mom_on, step, mom,
-            lane, warp, gx0, gy0, w, h, zl, zr, zt, zb);
-    };
-    if (T == kTbT) {
-        // full launches, unrolled; momentum is off only in the first step of a solve
-        const bool later = k0 > 0;
+    using G = PlGeo<kForm>;
+    PlSides<kForm> x;
 #pragma unroll
-        for (int k = 0; k < kTbT; ++k) {
-            if (!(r0 + kPlRPT - 1 < k + 1 || r0 >= kPlRows - k - 1))
-                one(k, k > 0 || later);
-            else if (k >= kTbT - 3)
-                idle(k);
-            __syncthreads();
-        }
+    for (int r = 0; r < G::kRPT; ++r) {
+        x.l[r] = __shfl_up_sync(0xffffffffu, s.o[r].w, 1);
+        x.r[r] = __shfl_down_sync(0xffffffffu, s.o[r].x, 1);
+    }
+    float* const top = slots + ((warp + 1) * 2) * kPlW + 4 * lane;  // slot of this warp: top row, bottom row
+    auto exchange = [&](float* b) {
+        *reinterpret_cast<float4*>(b) = s.o[0];
+        *reinterpret_cast<float4*>(b + kPlW) = s.o[G::kRPT - 1];
+        bar();
+        up = *reinterpret_cast<const float4*>(b - kPlW);      // slot w, bottom row
+        dn = *reinterpret_cast<const float4*>(b + 2 * kPlW);  // slot w + 2, top row
+    };
+    float m = k0 > 0 ? mom : -0.0f;
+#pragma unroll 1
+    for (int k = 0; k + 1 < T; k += 2) {
+        pl_step<kForm, kMode>(s, x, up, dn, step, m, t);
+        exchange(top);
+        pl_step<kForm, kMode>(s, x, up, dn, step, mom, t);
+        exchange(top + G::kSlots);
+        m = mom;
+    }
+    if (T & 1)  // a short last round
+        pl_step<kForm, kMode>(s, x, up, dn, step, m, t);
+}
+
+template <int kForm, class Bar>
+__device__ __forceinline__ void pl_round(int mode, PlState<kForm>& s, float4 up, float4 dn, float* slots, int T,
+    int k0, float step, float mom, int lane, int warp, const PlPlace& t, Bar&& bar)
+{
+    if (mode == kPlAll)
+        pl_steps<kForm, kPlAll>(s, up, dn, slots, T, k0, step, mom, lane, warp, t, bar);
+    else if (mode == kPlLanes)
+        pl_steps<kForm, kPlLanes>(s, up, dn, slots, T, k0, step, mom, lane, warp, t, bar);
+    else if (mode == kPlCols)
+        pl_steps<kForm, kPlCols>(s, up, dn, slots, T, k0, step, mom, lane, warp, t, bar);
+    else
+        pl_steps<kForm, kPlEvery>(s, up, dn, slots, T, k0, step, mom, lane, warp, t, bar);
+}
+
+// A thread's place in a tile at (ox, oy).
+template <int kForm>
+__device__ __forceinline__ PlPlace pl_place(int ox, int oy, int w, int h, int lane, int warp)
+{
+    using G = PlGeo<kForm>;
+    const int gx0 = ox + 4 * lane, gy0 = oy + G::kRPT * warp;
+    PlPlace t;
+    t.xlim = w - 2 - gx0;
+    t.top = -gy0;
+    t.bot = h - 2 - gy0;
+    t.zl = gx0 == 0;
+    t.zr = gx0 == w - 4;
+    t.zt = oy == -kTbT && warp == G::kTopWarp;
+    t.zb2 = oy == h - G::kRows + kTbT && warp == G::kBot2Warp;
+    t.zb1 = oy == h - G::kRows + kTbT && warp == G::kBot1Warp;
+    return t;
+}
+
+// A thread's block out of the staged tile, with the O rows above and below it
+// (zero outside the tile: values the ring never passes on to the interior).
+template <int kForm>
+__device__ __forceinline__ void pl_take(PlState<kForm>& s, float4& up, float4& dn, const float* stage, int k0, int lane,
+    int warp)
+{
+    using G = PlGeo<kForm>;
+    const float* base = stage + PlGeo<kForm>::kRPT * warp * kPlW + 4 * lane;
+#pragma unroll
+    for (int r = 0; r < PlGeo<kForm>::kRPT; ++r) {
+        const float* row = base + r * kPlW;
+        s.o[r] = *reinterpret_cast<const float4*>(row);
+        s.u[r] = *reinterpret_cast<const float4*>(row + G::kStage);
+        s.nk[r] = *reinterpret_cast<const float4*>(row + 2 * G::kStage);
+        s.c[r] = *reinterpret_cast<const float4*>(row + 3 * G::kStage);
+    }
+    if (k0 == 0)  // no U yet
+#pragma unroll
+        for (int r = 0; r < PlGeo<kForm>::kRPT; ++r)
+            s.u[r] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+    up = dn = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+    if (warp > 0)
+        up = *reinterpret_cast<const float4*>(base - kPlW);
+    if (warp < G::kWarps - 1)
+        dn = *reinterpret_cast<const float4*>(base + PlGeo<kForm>::kRPT * kPlW);
+}
+
+// A thread's interior pixels of O and U into the out staging.
+template <int kForm>
+__device__ __forceinline__ void pl_put(const PlState<kForm>& s, float* so, float* su, int lane, int warp)
+{
+    const int ix = 4 * lane - kTbT;
+    if (ix < 0 || ix >= kPlIW)
         return;
+#pragma unroll
+    for (int r = 0; r < PlGeo<kForm>::kRPT; ++r) {
+        const int iy = PlGeo<kForm>::kRPT * warp + r - kTbT;
+        if (iy < 0 || iy >= PlGeo<kForm>::kIRows)
+            continue;
+        *reinterpret_cast<float4*>(so + iy * kPlIW + ix) = s.o[r];
+        *reinterpret_cast<float4*>(su + iy * kPlIW + ix) = s.u[r];
     }
-    idle(kTbT - 3);
-    for (int k = 0; k < T; ++k) {
-        const int lo = kTbT - T + k + 1, hi = kPlRows - kTbT + T - k - 1;
-        if (!(r0 + kPlRPT - 1 < lo || r0 >= hi))
-            one(k, (k0 + k) > 0);
-        __syncthreads();
-    }
-    idle(kTbT - 2);
-    idle(kTbT - 1);
 }
 
 int pl_tiles_x(int w) { return (w + kPlIW - 1) / kPlIW; }
-int pl_tiles(int w, int h) { return 3 * pl_tiles_x(w) * ((h + kPlIRows - 1) / kPlIRows); }
+template <int kForm>
+int pl_tiles(int w, int h)
+{
+    return 3 * pl_tiles_x(w) * ((h + PlGeo<kForm>::kIRows - 1) / PlGeo<kForm>::kIRows);
+}
 
 __device__ __forceinline__ void tma_load_3d(void* dst, const CUtensorMap* map, int x, int y, int z, uint64_t* bar)
 {
@@ -1183,33 +1301,37 @@ struct PlPlain {
 // Stage <- tile (c, ox, oy) of the four planes, zero outside the image.
 __device__ __forceinline__ void pl_plain_load(float* stage, const PlPlain& p, int c, int ox, int oy)
 {
+    using G = PlGeo<kSolverFma>;
     const float* src[4] = {p.O, p.U, p.K, p.C};
     const int64_t base = static_cast<int64_t>(c) * p.w * p.h;
-    for (int i = threadIdx.x; i < kPlStage; i += kPlThreads) {
+#pragma unroll 4
+    for (int i = threadIdx.x; i < G::kStage; i += 32 * G::kWarps) {
         const int row = i / kPlW, col = i - row * kPlW;
         const int gy = oy + row, gx = ox + col;
         const bool in = gx >= 0 && gx < p.w && gy >= 0 && gy < p.h;
         const int64_t idx = in ? base + pix_index(gx, gy, p.w) : 0;
 #pragma unroll
         for (int a = 0; a < 4; ++a)
-            stage[a * kPlStage + i] = in ? src[a][idx] : 0.0f;
+            stage[a * G::kStage + i] = in ? src[a][idx] : 0.0f;
     }
 }
 
-// The plain-load form (widths that are not a multiple of 4, or a workspace off
-// the 16-byte grid): one launch per round of up to kTbT steps, each CTA
-// walking the round's tiles with plain loads and stores.
-__device__ __forceinline__ void pl_plain_body(const PlPlain& pl, int T, int k0, float step, float mom)
+// The plain-load form (widths that are not a multiple of 4 in a caller's
+// workspace, whose planes then have no room for a 16-byte row pitch): one
+// launch per round of up to kTbT steps, each CTA walking the round's tiles
+// with plain loads and stores.
+__global__ void __launch_bounds__(32 * PlGeo<kSolverFma>::kWarps, 1)
+    solver_fma_plain_kernel(const __grid_constant__ PlPlain pl, int T, int k0, float step, float mom)
 {
+    using G = PlGeo<kSolverFma>;
     extern __shared__ __align__(128) unsigned char smem_raw[];
     float* stage = reinterpret_cast<float*>(smem_raw);
-    float* slots = stage + 4 * kPlStage;
-    float* so = slots + 2 * kPlSlotPlane;
-    float* su = so + kPlOut;
+    float* slots = stage + 4 * G::kStage;
+    float* so = slots + 2 * G::kSlots;
+    float* su = so + G::kOut;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const int px0 = 4 * lane, py0 = kPlRPT * warp;
 
-    for (int i = threadIdx.x; i < 2 * kPlSlotPlane; i += kPlThreads)
+    for (int i = threadIdx.x; i < 2 * G::kSlots; i += blockDim.x)
         slots[i] = 0.0f;  // the apron slots stay zero
     grid_dependency_wait();
     const int per_plane = pl.ntiles / 3;
@@ -1217,47 +1339,21 @@ __device__ __forceinline__ void pl_plain_body(const PlPlain& pl, int T, int k0, 
         if (tile + static_cast<int>(gridDim.x) >= pl.ntiles)
             allow_dependent_launch();
         const int c = tile / per_plane, r = tile - c * per_plane;
-        const int ox = (r % pl.tiles_x) * kPlIW - kTbT, oy = (r / pl.tiles_x) * kPlIRows - kTbT;
+        const int ox = (r % pl.tiles_x) * kPlIW - kTbT, oy = (r / pl.tiles_x) * G::kIRows - kTbT;
         const int w = pl.w, h = pl.h;
-        __syncthreads();  // the previous tile has left the staging and the slots
+        __syncthreads();  // the previous tile has left the staging
         pl_plain_load(stage, pl, c, ox, oy);
         __syncthreads();
-        const int gx0 = ox + px0, gy0 = oy + py0;
-        const bool interior = ox >= 1 && oy >= 1 && ox + kPlW - 1 <= w - 3 && oy + kPlRows - 1 <= h - 3;
-
-        PlState s;
-#pragma unroll
-        for (int rr = 0; rr < kPlRPT; ++rr) {
-            const float* row = stage + (py0 + rr) * kPlW + px0;
-            s.o[rr] = *reinterpret_cast<const float4*>(row);
-            s.u[rr] = *reinterpret_cast<const float4*>(row + kPlStage);
-            s.nk[rr] = *reinterpret_cast<const float4*>(row + 2 * kPlStage);
-            s.c[rr] = *reinterpret_cast<const float4*>(row + 3 * kPlStage);
-        }
-        {
-            float* D = slots + ((warp + 1) * 2) * kPlPX + px0 + 4;  // buffer 0
-            *reinterpret_cast<float4*>(D) = s.o[0];
-            *reinterpret_cast<float4*>(D + kPlPX) = s.o[kPlRPT - 1];
-        }
-        __syncthreads();  // edge rows published
-        if (interior)
-            pl_iterate<kPlAll>(s, slots, T, k0, step, mom, lane, warp, gx0, gy0, w, h, oy, [](int) {});
-        else
-            pl_iterate<kPlEvery>(s, slots, T, k0, step, mom, lane, warp, gx0, gy0, w, h, oy, [](int) {});
-        {
-            const int ix = px0 - kTbT;
-#pragma unroll
-            for (int rr = 0; rr < kPlRPT; ++rr) {
-                const int iy = py0 + rr - kTbT;
-                if (ix < 0 || ix >= kPlIW || iy < 0 || iy >= kPlIRows)
-                    continue;
-                *reinterpret_cast<float4*>(so + iy * kPlIW + ix) = s.o[rr];
-                *reinterpret_cast<float4*>(su + iy * kPlIW + ix) = s.u[rr];
-            }
-        }
+        PlState<kSolverFma> s;
+        float4 up, dn;
+        pl_take<kSolverFma>(s, up, dn, stage, k0, lane, warp);
+        const bool interior = ox >= 1 && oy >= 1 && ox + kPlW - 1 <= w - 3 && oy + G::kRows - 1 <= h - 3;
+        pl_round<kSolverFma>(interior ? kPlAll : kPlEvery, s, up, dn, slots, T, k0, step, mom, lane, warp,
+            pl_place<kSolverFma>(ox, oy, w, h, lane, warp), [] { __syncthreads(); });
+        pl_put<kSolverFma>(s, so, su, lane, warp);
         __syncthreads();
         const int64_t base = static_cast<int64_t>(c) * w * h;
-        for (int i = threadIdx.x; i < kPlOut; i += kPlThreads) {
+        for (int i = threadIdx.x; i < G::kOut; i += blockDim.x) {
             const int iy = i / kPlIW, ix = i - iy * kPlIW;
             const int gy = oy + kTbT + iy, gx = ox + kTbT + ix;
             if (gx < w && gy < h) {
@@ -1269,13 +1365,7 @@ __device__ __forceinline__ void pl_plain_body(const PlPlain& pl, int T, int k0, 
     }
 }
 
-__global__ void __launch_bounds__(kPlThreads, 1)
-    solver_fma_plain_kernel(const __grid_constant__ PlPlain pl, int T, int k0, float step, float mom)
-{
-    pl_plain_body(pl, T, k0, step, mom);
-}
-
-// ---- the FMA form's solve in one persistent launch -----------------------------
+// ---- a solve in one persistent launch -------------------------------------------
 // A solve of L launches' worth of 8-step rounds over N tiles is one kernel:
 // each CTA takes (round k, tile t) tickets in order from a global counter
 // (k = ticket / N, t = ticket % N), waits until the tile's 3x3 neighbourhood
@@ -1290,13 +1380,28 @@ __global__ void __launch_bounds__(kPlThreads, 1)
 // same.  Rounds overlap: a CTA moves on to round k + 1 while the last tiles of
 // round k finish elsewhere, which removes the per-launch tail (1,080 tiles
 // per round at 1920x1080 leave the eighth of eight rounds 11 % full) and the
-// launch boundaries.  The next ticket's loads are issued while the current
-// tile iterates when its neighbours are ready (normally: they finished about
-// N / #SMs tiles earlier); otherwise warp 0 looks again during the steps it
-// skips, and failing that the CTA first finishes and signals its current
-// tile, then waits.  The tickets' bookkeeping (decoding, neighbour checks,
-// and with many tiles a round the fence that publishes a tile) runs in those
-// skipped steps, not between a tile's data and its first step.
+// launch boundaries.
+//
+// The compute warps only run steps: they wait for a tile's data, take it into
+// registers, hand the staging back, iterate, and put the interior into the
+// out staging.  Two control warps do the rest, overlapping it with the steps.
+// One takes and decodes tickets, watches the neighbours' counters (nine lanes,
+// one look per L2 round trip), and loads the next tile as soon as the staging
+// is free and its neighbours are done.  The other stores a finished interior
+// and publishes its round when the stores are complete.  With that work in a
+// compute warp's idle steps the counters were looked at three times a tile, a
+// tile whose neighbours were late was loaded only after the tile before it,
+// its nine counters read one after the other, and a finished tile was
+// published at the end of the next one.
+//
+// A tile takes 4.7 us at 1920x1080: 6,500 cycles of steps (4,030 of FP32 issue;
+// the exchange between warps and two warps a scheduler the rest), 2,100 of
+// moving 147 KB out of the staging and 50 KB into the other, 700 of waits.
+// Microseconds per 8-step round before (12 warps of 4 x 6 blocks, unrolled
+// steps, the bookkeeping in warp 0) and now: 1920x1080 38.2 -> 32.8, 3840x2160
+// 144 -> 129, 1280x720 21.5 -> 14.2, 960x540 13.9 -> 11.5, 640x360 12.3 -> 9.8.
+// Two CTAs of 6 warps on 64 x 72 tiles an SM, tried in place of this: 41.3 at
+// 1920x1080.
 enum { kPmO0, kPmO1, kPmU0, kPmU1, kPmK, kPmC, kPmOo0, kPmOo1, kPmUo0, kPmUo1, kPlMaps };
 
 template <int kN>
@@ -1315,17 +1420,17 @@ struct PlJob {
     int ox, oy, w, h;
 };
 
-template <int kN>
+template <int kForm, int kN>
 __device__ __forceinline__ PlJob pl_job(const PlSolve<kN>& g, int ticket)
 {
+    using G = PlGeo<kForm>;
     const int N = g.tile0[g.count];
     PlJob j;
     j.k = ticket / N;
     const int tile = ticket - j.k * N;
     int p = 0;
     if (kN > 1) {
-        // the last problem whose first tile is <= tile (binary search: a job is
-        // decoded several times per tile, partly on thread 0's critical path)
+        // the last problem whose first tile is <= tile (binary search)
         int hi = g.count - 1;
 #pragma unroll 1
         while (p < hi) {
@@ -1344,110 +1449,47 @@ __device__ __forceinline__ PlJob pl_job(const PlSolve<kN>& g, int ticket)
     j.tx = r % g.tiles_x[p];
     j.ty = r / g.tiles_x[p];
     j.ox = j.tx * kPlIW - kTbT;
-    j.oy = j.ty * kPlIRows - kTbT;
+    j.oy = j.ty * G::kIRows - kTbT;
     j.w = g.w[p];
     j.h = g.h[p];
     // The bottom row of tiles is moved up until its interior ends on the
-    // frame's last row (rows h - 2 and h - 1 then sit in warp 10, rows 2 and 3,
-    // where pl_step tests them without per-pixel tests), when its 8-row top
-    // ring still lies in the row of tiles above (the 3 x 3 dependency holds).
-    // Its interior then overlaps that row's: both compute the shared rows from
-    // the same inputs with the same arithmetic and store the same bits.
+    // frame's last row (rows h - 2 and h - 1 then sit in the last but one warp,
+    // rows 2 and 3, where pl_step tests them without per-pixel tests), when its
+    // 8-row top ring still lies in the row of tiles above (the 3 x 3 dependency
+    // holds).  Its interior then overlaps that row's: both compute the shared
+    // rows from the same inputs with the same arithmetic and store the same bits.
     const int ty_n = per_plane / g.tiles_x[p];
-    if (j.ty == ty_n - 1 && j.ty > 0 && j.h - j.ty * kPlIRows >= kTbT)
-        j.oy = j.h - kPlRows + kTbT;
+    if (j.ty == ty_n - 1 && j.ty > 0 && j.h - j.ty * G::kIRows >= kTbT)
+        j.oy = j.h - G::kRows + kTbT;
     return j;
 }
 
-__device__ __forceinline__ unsigned ld_acquire_u32(const unsigned* p)
-{
-    unsigned v;
-    asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
-    return v;
-}
-
-__device__ __forceinline__ void st_release_u32(unsigned* p, unsigned v)
-{
-    asm volatile("st.release.gpu.global.u32 [%0], %1;" ::"l"(p), "r"(v) : "memory");
-}
-
-// Round k - 1 finished on the tile's 3x3 neighbourhood (spins <= 1: one look).
-template <int kN>
-__device__ __forceinline__ bool pl_deps(const PlSolve<kN>& g, const PlJob& j, int spins)
-{
-    if (j.k == 0)
-        return true;
-    const int tx_n = g.tiles_x[j.p];
-    const int per_plane = (g.tile0[j.p + 1] - g.tile0[j.p]) / 3;
-    const int ty_n = per_plane / tx_n;
-    const unsigned* d = g.done[j.p] + j.c * per_plane;
-    for (int dy = -1; dy <= 1; ++dy) {
-        const int y = j.ty + dy;
-        if (y < 0 || y >= ty_n)
-            continue;
-        for (int dx = -1; dx <= 1; ++dx) {
-            const int x = j.tx + dx;
-            if (x < 0 || x >= tx_n)
-                continue;
-            const unsigned* f = d + y * tx_n + x;
-            int i = 0;
-            while (ld_acquire_u32(f) < static_cast<unsigned>(j.k)) {
-                if (++i >= spins)
-                    return false;
-                if (i > 32)
-                    __nanosleep(256);
-            }
-        }
-    }
-    return true;
-}
-
-// the tile's four input planes for its round, after its neighbours' stores
-template <int kN>
+// the tile's input planes for its round, after its neighbours' stores
+template <int kForm, int kN>
 __device__ __forceinline__ void pl_job_loads(float* stage, const PlSolve<kN>& g, const PlJob& j, uint64_t* bar)
 {
+    using G = PlGeo<kForm>;
     asm volatile("fence.proxy.async.global;" ::: "memory");  // the acquired stores, before the async-proxy reads
     const CUtensorMap* m = g.map[j.p];
     const int par = j.k & 1;
-    mbar_expect_tx(bar, 4 * kPlStageBytes);
+    mbar_expect_tx(bar, G::kPlanes * G::kStageBytes);
     tma_load_3d(stage, m + (par ? kPmO1 : kPmO0), j.ox, j.oy, j.c, bar);
-    tma_load_3d(stage + kPlStage, m + (par ? kPmU1 : kPmU0), j.ox, j.oy, j.c, bar);
-    tma_load_3d(stage + 2 * kPlStage, m + kPmK, j.ox, j.oy, j.c, bar);
-    tma_load_3d(stage + 3 * kPlStage, m + kPmC, j.ox, j.oy, j.c, bar);
+    tma_load_3d(stage + G::kStage, m + (par ? kPmU1 : kPmU0), j.ox, j.oy, j.c, bar);
+    tma_load_3d(stage + 2 * G::kStage, m + kPmK, j.ox, j.oy, j.c, bar);
+    tma_load_3d(stage + 3 * G::kStage, m + kPmC, j.ox, j.oy, j.c, bar);
 }
 
-__device__ __forceinline__ void st_relaxed_u32(unsigned* p, unsigned v)
-{
-    asm volatile("st.relaxed.gpu.global.u32 [%0], %1;" ::"l"(p), "r"(v) : "memory");
-}
-
-// the tile's stores are complete: publish its round (the release store
-// orders the completed async-proxy writes, brought into the generic proxy
-// by the proxy fence, before the counter)
+// Round k - 1 finished on the tile's 3x3 neighbourhood, seen by the whole
+// control warp in one L2 round trip: lanes 0..8 each read one neighbour's
+// counter (relaxed; a lane without a neighbour, or a job that waits for
+// nothing, counts as finished).  A yes is followed by an acquire fence in the
+// lanes that read the counters and a warp barrier, which order the counters'
+// published stores before the warp's later accesses (lane 0's TMA loads).
 template <int kN>
-__device__ __forceinline__ void pl_job_signal(const PlSolve<kN>& g, const PlJob& j)
-{
-    bulk_wait_all();
-    asm volatile("fence.proxy.async.global;" ::: "memory");
-    st_release_u32(g.done[j.p] + j.local, static_cast<unsigned>(j.k + 1));
-}
-
-__device__ __forceinline__ void pl_counter_signal(unsigned* done, unsigned v)
-{
-    bulk_wait_all();
-    asm volatile("fence.proxy.async.global;" ::: "memory");
-    st_release_u32(done, v);
-}
-
-// Warp 0 looks at the 3x3 neighbourhood of job j in two halves, so that the
-// L2 round trip can overlap a tile's steps.  Issue: lanes 0..8 each start one
-// relaxed load of a neighbour's counter (a lane without a neighbour, or a job
-// that waits for nothing, yields ~0u).
-template <int kN>
-__device__ __forceinline__ unsigned pl_deps_issue(const PlSolve<kN>& g, const PlJob& j, bool valid, int lane)
+__device__ __forceinline__ bool pl_deps(const PlSolve<kN>& g, const PlJob& j, int lane)
 {
     unsigned v = ~0u;
-    if (valid && j.k > 0 && lane < 9) {
+    if (j.k > 0 && lane < 9) {
         const int tx_n = g.tiles_x[j.p];
         const int per_plane = (g.tile0[j.p + 1] - g.tile0[j.p]) / 3;
         const int ty_n = per_plane / tx_n;
@@ -1458,16 +1500,7 @@ __device__ __forceinline__ unsigned pl_deps_issue(const PlSolve<kN>& g, const Pl
                          : "l"(g.done[j.p] + j.c * per_plane + y * tx_n + x)
                          : "memory");
     }
-    return v;
-}
-
-// Take, all lanes of warp 0: every neighbour has finished round k - 1.  A yes
-// is followed by an acquire fence in the lanes that read the counters and a
-// warp barrier, which order the counters' published stores before the
-// warp's later accesses (lane 0's TMA loads of the job).
-__device__ __forceinline__ bool pl_deps_take(unsigned v, int k)
-{
-    const bool ok = __all_sync(0xffffffffu, v >= static_cast<unsigned>(k));
+    const bool ok = __all_sync(0xffffffffu, v >= static_cast<unsigned>(j.k));
     if (ok) {
         asm volatile("fence.acq_rel.gpu;" ::: "memory");
         __syncwarp();
@@ -1475,254 +1508,205 @@ __device__ __forceinline__ bool pl_deps_take(unsigned v, int k)
     return ok;
 }
 
-template <int kN>
-__global__ void __launch_bounds__(kPlThreads, 1)
-    solver_fma_solve_kernel(const __grid_constant__ PlSolve<kN> g, float step, float mom)
+__device__ __forceinline__ void st_release_u32(unsigned* p, unsigned v)
 {
+    asm volatile("st.release.gpu.global.u32 [%0], %1;" ::"l"(p), "r"(v) : "memory");
+}
+
+__device__ __forceinline__ void mbar_arrive(uint64_t* bar)
+{
+    asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(bar)) : "memory");
+}
+
+// What the loading warp tells the others of a tile (visible to the compute
+// warps with its full_in barrier, to the storing warp with its full_out).
+struct PlTile {
+    int ox, oy, w, h, k0, T, mode;
+    int k, p, c, local;
+    int valid;  // 0: no more tiles
+};
+
+// Bounded wait that also gives up once another role has aborted; a wait that
+// runs out raises the abort for everyone.
+__device__ __forceinline__ bool pl_wait(uint64_t* bar, uint32_t parity, volatile int* abort)
+{
+    for (int i = 0; i < kWaitSpins; ++i) {
+        if (mbar_try_wait(bar, parity))
+            return true;
+        if ((i & 63) == 63 && *abort)
+            return false;
+        if (i > 64)
+            __nanosleep(64);
+    }
+    *abort = 1;
+    return false;
+}
+
+// The block: the compute warps and one warpgroup whose first two warps control
+// (registers are handed out per warpgroup).  All start with 168 registers a
+// thread; the control group gives up what the compute warps need beyond that
+// (setmaxnreg: 256 x 216 + 128 x 72 = 384 x 168).
+constexpr int kPlStartRegs = 168, kPlComputeRegs = 216, kPlControlRegs = 72;
+
+template <int kForm, int kN>
+__global__ void __launch_bounds__(32 * (PlGeo<kForm>::kWarps + 4), 1)
+    solver_solve_kernel(const __grid_constant__ PlSolve<kN> g, float step, float mom)
+{
+    using G = PlGeo<kForm>;
+    static_assert(G::kWarps % 4 == 0 &&
+            G::kWarps * kPlComputeRegs + 4 * kPlControlRegs <= (G::kWarps + 4) * kPlStartRegs &&
+            32 * (G::kWarps + 4) * kPlStartRegs <= 65536,
+        "the warpgroups' registers within the block's");
     extern __shared__ __align__(128) unsigned char smem_raw[];
     float* stage = reinterpret_cast<float*>(smem_raw);
-    float* slots = stage + 4 * kPlStage;
-    float* so = slots + 2 * kPlSlotPlane;
-    float* su = so + kPlOut;
-    uint64_t* bar = reinterpret_cast<uint64_t*>(su + kPlOut);
-    __shared__ int s_next, s_deferred, s_abort;
-    // decoded jobs: the next tile's (read by every thread at its top) and the
-    // one after it (decoded by warp 0 while the current tile runs)
-    __shared__ PlJob s_job, s_job2;
+    float* slots = stage + G::kPlanes * G::kStage;
+    float* so = slots + 2 * G::kSlots;
+    float* su = so + G::kOut;
+    uint64_t* full_in = reinterpret_cast<uint64_t*>(su + G::kOut);  // the tile's data is staged
+    uint64_t* empty_in = full_in + 1;   // every compute warp has taken it
+    uint64_t* full_out = full_in + 2;   // every compute warp has put its interior
+    uint64_t* empty_out = full_in + 3;  // the out staging has been stored
+    // Tile i's entry is i % 4: entry i is written again for tile i + 4, whose
+    // load follows the taking of tile i + 3, the putting of tile i + 2 and so
+    // the storing of tile i + 1.
+    __shared__ PlTile s_tile[4];
+    __shared__ volatile int s_abort;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const int px0 = 4 * lane, py0 = kPlRPT * warp;
-    const int total = g.tile0[g.count] * g.nround;
-    // Many tiles a round (ticketed several tiles' time before their
-    // dependents): a tile's round is published while the next tile runs, in
-    // steps warp 0 skips, instead of on that tile's critical path.
-    const bool lag = g.tile0[g.count] >= 3 * static_cast<int>(gridDim.x);
 
-    for (int i = threadIdx.x; i < 2 * kPlSlotPlane; i += kPlThreads)
+    for (int i = threadIdx.x; i < 2 * G::kSlots; i += blockDim.x)
         slots[i] = 0.0f;  // the apron slots stay zero
     if (threadIdx.x == 0) {
-        mbar_init(bar, 1);
+        mbar_init(full_in, 1);
+        mbar_init(empty_in, G::kWarps);
+        mbar_init(full_out, G::kWarps);
+        mbar_init(empty_out, 1);
         s_abort = 0;
     }
     __syncthreads();
     grid_dependency_wait();
-    // Tickets are taken two ahead: while a CTA runs its current tile, warp 0
-    // holds the next ticket (t1, loaded during the current tile) and takes the
-    // one after (t2), which it decodes and whose neighbours it checks in the
-    // steps it skips; the atomic, the divisions and the counter reads stay off
-    // the critical path.
-    int t1 = 0;
-    bool t1_ready = false;  // warp 0: t1's neighbours were seen finished
-    if (warp == 0) {
-        int a = 0, b = 0;
-        if (lane == 0) {
-            a = static_cast<int>(atomicAdd(g.ticket, 1u));
-            b = static_cast<int>(atomicAdd(g.ticket, 1u));
-        }
-        a = __shfl_sync(0xffffffffu, a, 0);
-        t1 = __shfl_sync(0xffffffffu, b, 0);
-        if (lane == 0) {
-            s_next = a;
-            if (a < total) {
-                const PlJob n = pl_job(g, a);
-                s_job = n;
-                if (pl_deps(g, n, kWaitSpins)) {
-                    pl_job_loads(stage, g, n, bar);
-                } else {
-                    atomicExch(&g_device_timeout, 1);
-                    s_abort = 1;
+
+    if (warp >= G::kWarps) {
+        asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(kPlControlRegs));
+        if (warp == G::kWarps) {
+            // ---- loading warp ---------------------------------------------------------
+            const int total = g.tile0[g.count] * g.nround;
+            int ticket = 0, phases = 0;  // full_in phases armed
+            if (lane == 0)
+                ticket = static_cast<int>(atomicAdd(g.ticket, 1u));
+            for (int i = 0;; ++i) {
+                ticket = __shfl_sync(0xffffffffu, ticket, 0);
+                const bool valid = ticket < total;
+                PlJob j{};
+                if (valid) {
+                    j = pl_job<kForm>(g, ticket);
+                    int spins = 0;
+                    bool ready;
+                    while (!(ready = pl_deps(g, j, lane)) && ++spins < kWaitSpins && !s_abort)
+                        __nanosleep(20);
+                    if (!ready && lane == 0)
+                        s_abort = 1;
                 }
+                if (lane == 0) {
+                    if (i > 0)
+                        pl_wait(empty_in, (i - 1) & 1, &s_abort);
+                    PlTile t{};
+                    if (valid) {
+                        t.ox = j.ox;
+                        t.oy = j.oy;
+                        t.w = j.w;
+                        t.h = j.h;
+                        t.k0 = j.k * kTbT;
+                        t.T = min(kTbT, g.num_iter - t.k0);
+                        t.mode = pl_mode<kForm>(j.ox, j.oy, j.w, j.h);
+                        t.k = j.k;
+                        t.p = j.p;
+                        t.c = j.c;
+                        t.local = j.local;
+                        t.valid = !s_abort;
+                    }
+                    s_tile[i & 3] = t;
+                    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+                    ++phases;
+                    if (t.valid) {
+                        pl_job_loads<kForm>(stage, g, j, full_in);
+                        ticket = static_cast<int>(atomicAdd(g.ticket, 1u));
+                    } else {
+                        mbar_arrive(full_in);
+                    }
+                }
+                __syncwarp();
+                if (!valid || s_abort)
+                    break;
             }
-        }
-        const bool valid = t1 < total;
-        const PlJob n = valid ? pl_job(g, t1) : PlJob{};
-        if (lane == 0)
-            s_job2 = n;
-        t1_ready = pl_deps_take(pl_deps_issue(g, n, valid, lane), n.k);
-    }
-    __syncthreads();
-    int cur = s_next;
-    uint32_t parity = 0;
-    // thread 0: the counter and value of a tile whose round is not yet published
-    unsigned* prev_done = nullptr;
-    unsigned prev_val = 0;
-    while (cur < total && !s_abort) {
-        const PlJob j = s_job;
-        int t2 = 0;
-        if (warp == 0 && lane == 0)
-            t2 = static_cast<int>(atomicAdd(g.ticket, 1u));  // used after the tile's first barrier
-        if (!mbar_wait_bounded(bar, parity, kWaitSpins)) {
-            // the outputs are invalid and vsc_check_device reports VSC_ETIMEOUT
-            if (threadIdx.x == 0) {
+            if (s_abort && lane == 0) {
+                // the outputs are invalid and vsc_check_device reports VSC_ETIMEOUT; let
+                // the copies in flight land before the CTA exits
                 atomicExch(&g_device_timeout, 1);
-                bulk_wait_all();
+                mbar_wait_bounded(full_in, (phases - 1) & 1, kWaitSpins);
             }
-            mbar_wait_bounded(bar, parity, kWaitSpins);  // let copies still in flight land
-            return;
-        }
-        parity ^= 1;
-        if (warp == 0 && !lag) {
-            // One fence a tile, taken while the other warps stage their
-            // registers: it releases the previous tile's completed stores
-            // (published by the relaxed counter store after it) and acquires
-            // the neighbour counters read for t1 during that tile's steps.
-            // (With `lag`, the same happens in the previous tile's last step.)
-            if (lane == 0 && prev_done) {
+        } else if (warp == G::kWarps + 1 && lane == 0) {
+            // ---- storing warp ---------------------------------------------------------
+            for (int i = 0; pl_wait(full_out, i & 1, &s_abort); ++i) {
+                const PlTile t = s_tile[i & 3];
+                if (!t.valid || s_abort)
+                    break;
+                const CUtensorMap* m = g.map[t.p];
+                const int par = (t.k + 1) & 1;
+                tma_store_3d(m + (par ? kPmOo1 : kPmOo0), t.ox + kTbT, t.oy + kTbT, t.c, so);
+                tma_store_3d(m + (par ? kPmUo1 : kPmUo0), t.ox + kTbT, t.oy + kTbT, t.c, su);
+                bulk_commit();
+                // publish: the release store orders the completed async-proxy writes,
+                // brought into the generic proxy by the proxy fence, before the counter
                 bulk_wait_all();
                 asm volatile("fence.proxy.async.global;" ::: "memory");
-            }
-            __syncwarp();
-            asm volatile("fence.acq_rel.gpu;" ::: "memory");
-            __syncwarp();
-            if (lane == 0 && prev_done)
-                st_relaxed_u32(prev_done, prev_val);
-            prev_done = nullptr;
-        }
-        const int w = j.w, h = j.h;
-        const int gx0 = j.ox + px0, gy0 = j.oy + py0;
-
-        PlState s;
-#pragma unroll
-        for (int r = 0; r < kPlRPT; ++r) {
-            const float* row = stage + (py0 + r) * kPlW + px0;
-            s.o[r] = *reinterpret_cast<const float4*>(row);
-            s.u[r] = *reinterpret_cast<const float4*>(row + kPlStage);
-            s.nk[r] = *reinterpret_cast<const float4*>(row + 2 * kPlStage);
-            s.c[r] = *reinterpret_cast<const float4*>(row + 3 * kPlStage);
-        }
-        if (threadIdx.x == 0)
-            bulk_wait_read();  // the previous tile's TMA stores have read the out staging
-        __syncthreads();       // staging consumed
-        {
-            float* D = slots + ((warp + 1) * 2) * kPlPX + px0 + 4;  // buffer 0
-            *reinterpret_cast<float4*>(D) = s.o[0];
-            *reinterpret_cast<float4*>(D + kPlPX) = s.o[kPlRPT - 1];
-        }
-        if (warp == 0) {
-            // load the next tile now if its neighbours are finished (seen
-            // across the previous tile, else one look now)
-            const bool valid = t1 < total;
-            const PlJob n = s_job2;  // decoded while the previous tile ran
-            const bool ready = t1_ready || pl_deps_take(pl_deps_issue(g, n, valid, lane), n.k);
-            if (lane == 0) {
-                s_next = t1;
-                s_job = n;
-                s_deferred = 0;
-                if (valid) {
-                    if (ready) {
-                        asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-                        pl_job_loads(stage, g, n, bar);
-                    } else {
-                        s_deferred = 1;
-                    }
-                }
+                st_release_u32(g.done[t.p] + t.local, static_cast<unsigned>(t.k + 1));
+                mbar_arrive(empty_out);
             }
         }
-        __syncthreads();  // edge rows published
-        unsigned t2_look = ~0u, t1_look = ~0u;
-        int t2_round = 0;
-        // warp 0, in the steps it skips: decode t2 and start reading its
-        // neighbours' counters; with `lag`, wait for the previous tile's
-        // stores (long complete by then); take the counters and, with `lag`,
-        // one fence that acquires them (for t2's loads at the top of the next
-        // tile) and releases the previous tile's stores, published after it
-        auto idle = [&](int k) {
-            if (warp != 0)
-                return;
-            if (k == kTbT - 3) {
-                t2 = __shfl_sync(0xffffffffu, t2, 0);
-                const bool valid = t2 < total;
-                const PlJob n = valid ? pl_job(g, t2) : PlJob{};
-                if (lane == 0)
-                    s_job2 = n;
-                t2_look = pl_deps_issue(g, n, valid, lane);
-                t2_round = n.k;
-                // a deferred next tile (few tiles a round): look again now
-                if (!lag && s_deferred)
-                    t1_look = pl_deps_issue(g, s_job, true, lane);
-            } else if (k == kTbT - 2) {
-                if (lag && lane == 0 && prev_done) {
-                    bulk_wait_all();
-                    asm volatile("fence.proxy.async.global;" ::: "memory");
-                }
-                if (!lag && s_deferred) {
-                    // its neighbours finished during this tile's steps: load it
-                    // now instead of after the tile (ordered as at the top)
-                    const PlJob n = s_job;
-                    if (__all_sync(0xffffffffu, t1_look >= static_cast<unsigned>(n.k))) {
-                        __syncwarp();
-                        asm volatile("fence.acq_rel.gpu;" ::: "memory");
-                        __syncwarp();
-                        if (lane == 0) {
-                            asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-                            pl_job_loads(stage, g, n, bar);
-                            s_deferred = 0;
-                        }
-                    }
-                }
-            } else {
-                t1_ready = __all_sync(0xffffffffu, t2_look >= static_cast<unsigned>(t2_round));
-                if (lag) {
-                    __syncwarp();
-                    asm volatile("fence.acq_rel.gpu;" ::: "memory");
-                    __syncwarp();
-                    if (lane == 0 && prev_done)
-                        st_relaxed_u32(prev_done, prev_val);
-                    prev_done = nullptr;
-                }
-            }
-        };
-        const int k0 = j.k * kTbT, T = min(kTbT, g.num_iter - k0);
-        const int mode = pl_mode(j.ox, j.oy, w, h);
-        if (mode == kPlAll)
-            pl_iterate<kPlAll>(s, slots, T, k0, step, mom, lane, warp, gx0, gy0, w, h, j.oy, idle);
-        else if (mode == kPlLanes)
-            pl_iterate<kPlLanes>(s, slots, T, k0, step, mom, lane, warp, gx0, gy0, w, h, j.oy, idle);
-        else
-            pl_iterate<kPlEvery>(s, slots, T, k0, step, mom, lane, warp, gx0, gy0, w, h, j.oy, idle);
-        {
-            const int ix = px0 - kTbT;
-#pragma unroll
-            for (int r = 0; r < kPlRPT; ++r) {
-                const int iy = py0 + r - kTbT;
-                if (ix < 0 || ix >= kPlIW || iy < 0 || iy >= kPlIRows)
-                    continue;
-                *reinterpret_cast<float4*>(so + iy * kPlIW + ix) = s.o[r];
-                *reinterpret_cast<float4*>(su + iy * kPlIW + ix) = s.u[r];
-            }
-        }
-        if (warp == 0)
-            t1 = t2;  // t1_ready: taken in the last step, acquired by its fence or the next top's
-        asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-        __syncthreads();
-        if (threadIdx.x == 0) {
-            const CUtensorMap* m = g.map[j.p];
-            const int par = (j.k + 1) & 1;
-            tma_store_3d(m + (par ? kPmOo1 : kPmOo0), j.ox + kTbT, j.oy + kTbT, j.c, so);
-            tma_store_3d(m + (par ? kPmUo1 : kPmUo0), j.ox + kTbT, j.oy + kTbT, j.c, su);
-            bulk_commit();
-            prev_done = g.done[j.p] + j.local;
-            prev_val = static_cast<unsigned>(j.k + 1);
-            if (s_deferred) {
-                // the next tile's neighbours were not finished: publish this
-                // tile first (the next one may need it), then wait
-                pl_job_signal(g, j);
-                prev_done = nullptr;
-                const PlJob n = s_job;
-                if (pl_deps(g, n, kWaitSpins)) {
-                    pl_job_loads(stage, g, n, bar);
-                } else {
-                    atomicExch(&g_device_timeout, 1);
-                    s_abort = 1;
-                }
-            }
-        }
-        __syncthreads();  // s_next, s_abort
-        cur = s_next;
+        return;
     }
-    if (threadIdx.x == 0) {
-        if (prev_done)
-            pl_counter_signal(prev_done, prev_val);
-        bulk_wait_all();
+
+    // ---- compute warps --------------------------------------------------------------------
+    asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(kPlComputeRegs));
+    bool ok = true;
+    for (int i = 0;; ++i) {
+        ok = pl_wait(full_in, i & 1, &s_abort) && ok;
+        // the warps leave together: one whose wait gave up takes the others with it
+        int any;
+        asm volatile(
+            "{\n"
+            " .reg .pred p, q;\n"
+            " setp.ne.s32 p, %1, 0;\n"
+            " barrier.cta.red.or.pred q, 1, %2, p;\n"
+            " selp.s32 %0, 1, 0, q;\n"
+            "}\n"
+            : "=r"(any)
+            : "r"(ok ? 0 : 1), "n"(32 * G::kWarps)
+            : "memory");
+        const PlTile& t = s_tile[i & 3];
+        if (any || !t.valid) {
+            __syncwarp();
+            if (lane == 0)
+                mbar_arrive(full_out);  // the storing warp leaves, too
+            break;
+        }
+        const int T = t.T, k0 = t.k0, mode = t.mode;
+        const PlPlace place = pl_place<kForm>(t.ox, t.oy, t.w, t.h, lane, warp);
+        PlState<kForm> s;
+        float4 up, dn;
+        pl_take<kForm>(s, up, dn, stage, k0, lane, warp);
+        __syncwarp();
+        if (lane == 0)
+            mbar_arrive(empty_in);
+        pl_round<kForm>(mode, s, up, dn, slots, T, k0, step, mom, lane, warp, place,
+            [] { asm volatile("barrier.cta.sync 1, %0;" ::"n"(32 * G::kWarps) : "memory"); });
+        if (i > 0)
+            ok = pl_wait(empty_out, (i - 1) & 1, &s_abort);
+        pl_put<kForm>(s, so, su, lane, warp);
+        asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+        __syncwarp();
+        if (lane == 0)
+            mbar_arrive(full_out);
     }
 }
 
@@ -1778,7 +1762,7 @@ bool set_group_smem()
     constexpr auto kAttr = cudaFuncAttributeMaxDynamicSharedMemorySize;
     return cudaFuncSetAttribute(solver_persistent_kernel<kN>, kAttr, kPsSmem) == cudaSuccess &&
            cudaFuncSetAttribute(solver_tall_kernel<kN>, kAttr, kPSmem) == cudaSuccess &&
-           cudaFuncSetAttribute(solver_fma_solve_kernel<kN>, kAttr, kPlSmem) == cudaSuccess;
+           cudaFuncSetAttribute(solver_solve_kernel<kSolverFma, kN>, kAttr, PlGeo<kSolverFma>::kSmem) == cudaSuccess;
 }
 
 struct DeviceInfo {
@@ -1809,7 +1793,7 @@ cudaError_t device_info(DeviceInfo** out)
             return e;
         d.ps_smem = set_group_smem<1>() && set_group_smem<4>() && set_group_smem<kGroupMax>() &&
                     cudaFuncSetAttribute(solver_fma_plain_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                        kPlSmem) == cudaSuccess;
+                        PlGeo<kSolverFma>::kSmem) == cudaSuccess;
         cudaGetLastError();
     }
     *out = &d;
@@ -1853,7 +1837,7 @@ int tiles_of(int w, int h, int ir) { return ((w + kIW - 1) / kIW) * ((h + ir - 1
 int model_rows(const int* w, const int* h, int n, int sms, int form)
 {
     if (form == kSolverFma)
-        return kPlRows;
+        return PlGeo<kSolverFma>::kRows;
     int64_t n_short = 0, n_tall = 0;
     for (int i = 0; i < n; ++i) {
         n_short += tiles_of(w[i], h[i], kIH);
@@ -1894,15 +1878,16 @@ bool encode_solve(SolveMaps* m, float* const O[2], float* const U[2], const floa
     return ok;
 }
 
-// 3D map over the three w x h planes of a planar image (x, y, channel).
-bool encode_plane_map(CUtensorMap* m, const float* base, int w, int h, int box_w, int box_h)
+// 3D map over the three w x h planes of a planar image (x, y, channel) of
+// `pitch`-float rows (a multiple of 4).
+bool encode_plane_map(CUtensorMap* m, const float* base, int w, int h, int pitch, int box_w, int box_h)
 {
     EncodeTiledFn fn = encode_fn();
     if (!fn)
         return false;
     const cuuint64_t dims[3] = {static_cast<cuuint64_t>(w), static_cast<cuuint64_t>(h), 3};
-    const cuuint64_t strides[2] = {static_cast<cuuint64_t>(w) * sizeof(float),
-        static_cast<cuuint64_t>(w) * h * sizeof(float)};
+    const cuuint64_t strides[2] = {static_cast<cuuint64_t>(pitch) * sizeof(float),
+        static_cast<cuuint64_t>(pitch) * h * sizeof(float)};
     const cuuint32_t box[3] = {static_cast<cuuint32_t>(box_w), static_cast<cuuint32_t>(box_h), 1};
     const cuuint32_t estr[3] = {1, 1, 1};
     return fn(m, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 3, const_cast<float*>(base), dims, strides, box, estr,
@@ -2125,12 +2110,30 @@ cudaError_t solver_autotune(int w, int h, cudaStream_t st, int* rows_out, int fo
 // The FMA form's workspace ends in the solve kernel's counters: the ticket,
 // padding to 64 bytes, one finished-round counter per tile; rounded up to
 // 256 bytes so that a workspace placed after it stays aligned.
-int pl_counter_floats(int w, int h) { return (16 + pl_tiles(w, h) + 63) / 64 * 64; }
+int pl_counter_floats(int w, int h) { return (16 + pl_tiles<kSolverFma>(w, h) + 63) / 64 * 64; }
+
+// A plane's row in floats where the workspace has room for rows on the 16-byte
+// grid (TMA's), whatever the width.
+// 854x480, 150 steps: 218 us; with plain loads, which a tile's steps wait for,
+// and a launch a round 542 us.
+int pl_pitch(int w) { return (w + 3) & ~3; }
 
 size_t solver_workspace_floats(int w, int h, int form)
 {
     const size_t img = static_cast<size_t>(w) * h * 3;
     return form == kSolverFma ? 6 * img + pl_counter_floats(w, h) : 4 * img;
+}
+
+size_t solver_workspace_full_floats(int w, int h, int form)
+{
+    if (form != kSolverFma)
+        return solver_workspace_floats(w, h, form);
+    return 6 * static_cast<size_t>(pl_pitch(w)) * h * 3 + pl_counter_floats(w, h);
+}
+
+size_t solver_workspace_any_floats(int w, int h)
+{
+    return std::max(solver_workspace_full_floats(w, h, kSolverExact), solver_workspace_full_floats(w, h, kSolverFma));
 }
 
 int solver_steps_per_launch() { return kTbT; }
@@ -2150,18 +2153,18 @@ WsView ws_view(float* ws, int w, int h)
     return WsView{ws, ws + n, ws + 2 * n, ws + 3 * n};
 }
 
-// The FMA form's workspace: six planar images (three w x h planes each),
-// then the solve kernel's counters.
+// The FMA form's workspace: six planar images (three planes of h rows of
+// `pitch` floats each), then the solve kernel's counters.
 struct PlWs {
     float *C, *K, *U[2], *O[2];
     unsigned* cnt;
-    int ncnt;
+    int ncnt, pitch;
 };
-PlWs pl_view(float* ws, int w, int h)
+PlWs pl_view(float* ws, int w, int h, int pitch)
 {
-    const size_t n = static_cast<size_t>(w) * h * 3;
+    const size_t n = static_cast<size_t>(pitch) * h * 3;
     return PlWs{ws, ws + n, {ws + 2 * n, ws + 3 * n}, {ws + 4 * n, ws + 5 * n},
-        reinterpret_cast<unsigned*>(ws + 6 * n), pl_counter_floats(w, h)};
+        reinterpret_cast<unsigned*>(ws + 6 * n), pl_counter_floats(w, h), pitch};
 }
 
 bool tma_eligible(const DeviceInfo* di, int w, const float* O, const WsView& v, const float* A, const float* Wt)
@@ -2170,15 +2173,19 @@ bool tma_eligible(const DeviceInfo* di, int w, const float* O, const WsView& v, 
            aligned16p(v.U1) && aligned16p(A) && aligned16p(Wt) && aligned16p(v.L);
 }
 
-// planes of a width that is a multiple of 4 in a 16-byte aligned workspace
-// (each plane then starts on the 16-byte grid)
-bool pl_tma_eligible(const DeviceInfo* di, int w, const float* ws) { return di->ps_smem && (w % 4) == 0 && aligned16p(ws); }
+// A solve in planes of rows on the 16-byte grid: a 16-byte aligned workspace of
+// solver_workspace_full_floats (for a width that is a multiple of 4 the same
+// as solver_workspace_floats).
+bool pl_tma_eligible(const DeviceInfo* di, int w, int h, const float* ws, size_t ws_floats)
+{
+    return di->ps_smem && aligned16p(ws) && ws_floats >= solver_workspace_full_floats(w, h, kSolverFma);
+}
 
 struct PlanarCopy {
     const float* src;
     float* dst;
     uint8_t* rgba;
-    int64_t npix;
+    int w, h, pitch;
     unsigned* cnt = nullptr;  // solve counters to zero on the way in
     int ncnt = 0;
 };
@@ -2196,8 +2203,11 @@ cudaError_t launch_planar(const PlanarCopy* c, int n, int to_planar, cudaStream_
             g.rgba[p] = c[b0 + p].rgba;
             g.cnt[p] = c[b0 + p].cnt;
             g.ncnt[p] = c[b0 + p].ncnt;
-            g.npix[p] = c[b0 + p].npix;
-            g.block0[p + 1] = g.block0[p] + static_cast<int>((c[b0 + p].npix + 255) / 256);
+            g.npix[p] = static_cast<int64_t>(c[b0 + p].w) * c[b0 + p].h;
+            g.w[p] = c[b0 + p].w;
+            g.pitch[p] = c[b0 + p].pitch;
+            g.plane[p] = static_cast<int64_t>(c[b0 + p].pitch) * c[b0 + p].h;
+            g.block0[p + 1] = g.block0[p] + static_cast<int>((g.npix[p] + 255) / 256);
         }
         const cudaError_t e = launch_pdl(planar_group_kernel, dim3(g.block0[g.count]), dim3(256), 0, st, g, to_planar);
         if (e != cudaSuccess)
@@ -2209,10 +2219,11 @@ cudaError_t launch_planar(const PlanarCopy* c, int n, int to_planar, cudaStream_
 
 // One launch of the FMA form's solve kernel per kN members (each member's
 // counters zeroed beforehand; the first member's ticket serves the launch).
-template <int kN>
+template <int kForm, int kN>
 cudaError_t launch_solve(const std::vector<PlWs>& v, const int* w, const int* h, int n, int num_iter, float step,
     float mom, int sms, cudaStream_t st, int* nl)
 {
+    using G = PlGeo<kForm>;
     const int nround = solve_launches(num_iter);
     for (int b0 = 0; b0 < n; b0 += kN) {
         PlSolve<kN> g{};
@@ -2224,18 +2235,18 @@ cudaError_t launch_solve(const std::vector<PlWs>& v, const int* w, const int* h,
             CUtensorMap* mp = g.map[p];
             bool ok = true;
             for (int c = 0; c < 2 && ok; ++c)
-                ok = encode_plane_map(&mp[c ? kPmO1 : kPmO0], m.O[c], W, H, kPlW, kPlRows) &&
-                     encode_plane_map(&mp[c ? kPmU1 : kPmU0], m.U[c], W, H, kPlW, kPlRows) &&
-                     encode_plane_map(&mp[c ? kPmOo1 : kPmOo0], m.O[c], W, H, kPlIW, kPlIRows) &&
-                     encode_plane_map(&mp[c ? kPmUo1 : kPmUo0], m.U[c], W, H, kPlIW, kPlIRows);
-            if (!ok || !encode_plane_map(&mp[kPmK], m.K, W, H, kPlW, kPlRows) ||
-                !encode_plane_map(&mp[kPmC], m.C, W, H, kPlW, kPlRows))
+                ok = encode_plane_map(&mp[c ? kPmO1 : kPmO0], m.O[c], W, H, m.pitch, kPlW, G::kRows) &&
+                     encode_plane_map(&mp[c ? kPmU1 : kPmU0], m.U[c], W, H, m.pitch, kPlW, G::kRows) &&
+                     encode_plane_map(&mp[c ? kPmOo1 : kPmOo0], m.O[c], W, H, m.pitch, kPlIW, G::kIRows) &&
+                     encode_plane_map(&mp[c ? kPmUo1 : kPmUo0], m.U[c], W, H, m.pitch, kPlIW, G::kIRows);
+            if (!ok || !encode_plane_map(&mp[kPmK], m.K, W, H, m.pitch, kPlW, G::kRows) ||
+                !encode_plane_map(&mp[kPmC], m.C, W, H, m.pitch, kPlW, G::kRows))
                 return cudaErrorInvalidValue;
             g.done[p] = m.cnt + 16;
             g.w[p] = W;
             g.h[p] = H;
             g.tiles_x[p] = pl_tiles_x(W);
-            g.tile0[p + 1] = g.tile0[p] + pl_tiles(W, H);
+            g.tile0[p + 1] = g.tile0[p] + pl_tiles<kForm>(W, H);
         }
         g.nround = nround;
         g.num_iter = num_iter;
@@ -2248,9 +2259,9 @@ cudaError_t launch_solve(const std::vector<PlWs>& v, const int* w, const int* h,
         cfg.attrs = attr;
         cfg.numAttrs = 1;
         cfg.gridDim = dim3(static_cast<unsigned>(std::min<int64_t>(static_cast<int64_t>(g.tile0[g.count]) * nround, sms)));
-        cfg.blockDim = dim3(kPlThreads);
-        cfg.dynamicSmemBytes = kPlSmem;
-        const cudaError_t e = cudaLaunchKernelEx(&cfg, solver_fma_solve_kernel<kN>, g, step, mom);
+        cfg.blockDim = dim3(32 * (G::kWarps + 4));
+        cfg.dynamicSmemBytes = G::kSmem;
+        const cudaError_t e = cudaLaunchKernelEx(&cfg, solver_solve_kernel<kForm, kN>, g, step, mom);
         if (e != cudaSuccess)
             return e;
         ++*nl;
@@ -2262,33 +2273,35 @@ cudaError_t launch_solve(const std::vector<PlWs>& v, const int* w, const int* h,
 // solution Oc) and zeroed counters, the solve (one launch; per round on the
 // plain-load path), O (and the RGBA8 copy) back from its planes.
 cudaError_t run_solver_fma(const DeviceInfo* di, const float* P, const float* A, const float* Wt, float* O, int w,
-    int h, int num_iter, float step, float mom, float* workspace, cudaStream_t st, int* nl, uint8_t* rgba_out,
-    const float* Oc, int cw, int ch)
+    int h, int num_iter, float step, float mom, float* workspace, size_t ws_floats, cudaStream_t st, int* nl,
+    uint8_t* rgba_out, const float* Oc, int cw, int ch)
 {
-    const PlWs v = pl_view(workspace, w, h);
+    const bool tma = pl_tma_eligible(di, w, h, workspace, ws_floats);
+    const PlWs v = pl_view(workspace, w, h, tma ? pl_pitch(w) : w);
     const dim3 b(32, 8);
     cudaError_t e = launch_pdl(solver_prep_fma_kernel, grid2d(w, h, b), b, 0, st, P, A, Wt,
-        static_cast<const float*>(O), v.C, v.K, v.O[0], w, h, step, v.cnt, v.ncnt, Oc, cw, ch);
+        static_cast<const float*>(O), v.C, v.K, v.O[0], w, h, v.pitch, step, v.cnt, v.ncnt, Oc, cw, ch);
     ++*nl;
     const int nlaunch = solve_launches(num_iter);
-    if (e == cudaSuccess && pl_tma_eligible(di, w, workspace)) {
+    if (e == cudaSuccess && tma) {
         const std::vector<PlWs> one(1, v);
-        e = launch_solve<1>(one, &w, &h, 1, num_iter, step, mom, di->sms, st, nl);
+        e = launch_solve<kSolverFma, 1>(one, &w, &h, 1, num_iter, step, mom, di->sms, st, nl);
     } else if (e == cudaSuccess) {
-        // plain loads and stores (widths not a multiple of 4, an unaligned workspace)
-        const int tx = pl_tiles_x(w), nt = pl_tiles(w, h);
+        // plain loads and stores
+        const int tx = pl_tiles_x(w), nt = pl_tiles<kSolverFma>(w, h);
         int k0 = 0;
         for (int li = 0; li < nlaunch && e == cudaSuccess; ++li) {
             const int T = std::min(kTbT, num_iter - k0);
             const PlPlain pl{v.O[li & 1], v.U[li & 1], v.K, v.C, v.O[(li + 1) & 1], v.U[(li + 1) & 1], w, h, tx, nt};
-            e = launch_pdl(solver_fma_plain_kernel, dim3(std::min(nt, di->sms)), dim3(kPlThreads), kPlSmem, st, pl, T,
+            e = launch_pdl(solver_fma_plain_kernel, dim3(std::min(nt, di->sms)), dim3(32 * PlGeo<kSolverFma>::kWarps),
+                PlGeo<kSolverFma>::kSmem, st, pl, T,
                 k0, step, mom);
             ++*nl;
             k0 += T;
         }
     }
     if (e == cudaSuccess) {
-        const PlanarCopy back{v.O[nlaunch & 1], O, rgba_out, static_cast<int64_t>(w) * h};
+        const PlanarCopy back{v.O[nlaunch & 1], O, rgba_out, w, h, v.pitch};
         e = launch_planar(&back, 1, 0, st, nl);
     }
     return e != cudaSuccess ? e : cudaGetLastError();
@@ -2323,10 +2336,10 @@ cudaError_t solver_prep(int form, const float* P, const float* A, const float* W
 {
     if (form != kSolverFma)
         return solver_lap(P, w, h, workspace, st);
-    const PlWs v = pl_view(workspace, w, h);
+    const PlWs v = pl_view(workspace, w, h, pl_pitch(w));  // w is a multiple of 4 in a grouped solve
     const dim3 b(32, 8);
     const cudaError_t e = launch_pdl(solver_prep_fma_kernel, grid2d(w, h, b), b, 0, st, P, A, Wt,
-        static_cast<const float*>(nullptr), v.C, v.K, static_cast<float*>(nullptr), w, h, step,
+        static_cast<const float*>(nullptr), v.C, v.K, static_cast<float*>(nullptr), w, h, v.pitch, step,
         static_cast<unsigned*>(nullptr), 0, static_cast<const float*>(nullptr), 0, 0);
     if (e != cudaSuccess)
         return e;
@@ -2340,7 +2353,8 @@ bool solver_group_eligible(const SolverImage* im, int n, int form)
         return false;
     for (int i = 0; i < n; ++i) {
         const bool ok = form == kSolverFma
-                            ? pl_tma_eligible(di, im[i].w, im[i].workspace)
+                            ? im[i].w % 4 == 0 && pl_tma_eligible(di, im[i].w, im[i].h, im[i].workspace,
+                                                        solver_workspace_floats(im[i].w, im[i].h, form))
                             : tma_eligible(di, im[i].w, im[i].O, ws_view(im[i].workspace, im[i].w, im[i].h), im[i].A,
                                   im[i].Wt);
         if (!ok)
@@ -2384,15 +2398,14 @@ cudaError_t run_solver_group(const SolverImage* im, int n, int num_iter, float s
         std::vector<PlWs> v(n);
         std::vector<PlanarCopy> to(n), back(n);
         for (int i = 0; i < n; ++i) {
-            v[i] = pl_view(im[i].workspace, im[i].w, im[i].h);
-            const int64_t np = static_cast<int64_t>(im[i].w) * im[i].h;
-            to[i] = PlanarCopy{im[i].O, v[i].O[0], nullptr, np, v[i].cnt, v[i].ncnt};
-            back[i] = PlanarCopy{v[i].O[solve_launches(num_iter) & 1], im[i].O, im[i].rgba, np};
+            v[i] = pl_view(im[i].workspace, im[i].w, im[i].h, im[i].w);
+            to[i] = PlanarCopy{im[i].O, v[i].O[0], nullptr, im[i].w, im[i].h, im[i].w, v[i].cnt, v[i].ncnt};
+            back[i] = PlanarCopy{v[i].O[solve_launches(num_iter) & 1], im[i].O, im[i].rgba, im[i].w, im[i].h, im[i].w};
         }
         e = launch_planar(to.data(), n, 1, st, &nl);
         if (e == cudaSuccess)
-            e = n <= 4 ? launch_solve<4>(v, ws.data(), hs.data(), n, num_iter, step, mom, di->sms, st, &nl)
-                       : launch_solve<kGroupMax>(v, ws.data(), hs.data(), n, num_iter, step, mom, di->sms, st, &nl);
+            e = n <= 4 ? launch_solve<kSolverFma, 4>(v, ws.data(), hs.data(), n, num_iter, step, mom, di->sms, st, &nl)
+                       : launch_solve<kSolverFma, kGroupMax>(v, ws.data(), hs.data(), n, num_iter, step, mom, di->sms, st, &nl);
         if (e == cudaSuccess)
             e = launch_planar(back.data(), n, 0, st, &nl);
         if (launches)
@@ -2421,8 +2434,8 @@ cudaError_t run_solver_group(const SolverImage* im, int n, int num_iter, float s
 }
 
 cudaError_t run_solver_from_coarse(const float* P, const float* A, const float* Wt, float* O, int w, int h,
-    const float* Oc, int cw, int ch, int num_iter, float step, float mom, float* workspace, cudaStream_t st,
-    int* launches, uint8_t* rgba_out)
+    const float* Oc, int cw, int ch, int num_iter, float step, float mom, float* workspace, size_t ws_floats,
+    cudaStream_t st, int* launches, uint8_t* rgba_out)
 {
     if (num_iter <= 0 || !Oc || cw <= 0 || ch <= 0)
         return cudaErrorInvalidValue;
@@ -2433,14 +2446,14 @@ cudaError_t run_solver_from_coarse(const float* P, const float* A, const float* 
     if (!di->ps_smem)
         return cudaErrorNotSupported;
     int nl = 0;
-    e = run_solver_fma(di, P, A, Wt, O, w, h, num_iter, step, mom, workspace, st, &nl, rgba_out, Oc, cw, ch);
+    e = run_solver_fma(di, P, A, Wt, O, w, h, num_iter, step, mom, workspace, ws_floats, st, &nl, rgba_out, Oc, cw, ch);
     if (launches)
         *launches += nl;
     return e;
 }
 
 cudaError_t run_solver(const float* P, const float* A, const float* Wt, float* O, int w, int h, int num_iter,
-    float step, float mom, float* workspace, cudaStream_t st, int* launches, uint8_t* rgba_out, int form)
+    float step, float mom, float* workspace, size_t ws_floats, cudaStream_t st, int* launches, uint8_t* rgba_out, int form)
 {
     const size_t n = static_cast<size_t>(w) * h * 3;
     const WsView v = ws_view(workspace, w, h);
@@ -2461,8 +2474,8 @@ cudaError_t run_solver(const float* P, const float* A, const float* Wt, float* O
     if (form == kSolverFma) {
         if (!di->ps_smem)
             return cudaErrorNotSupported;
-        const cudaError_t e = run_solver_fma(di, P, A, Wt, O, w, h, num_iter, step, mom, workspace, st, &nl, rgba_out,
-            nullptr, 0, 0);
+        const cudaError_t e = run_solver_fma(di, P, A, Wt, O, w, h, num_iter, step, mom, workspace, ws_floats, st, &nl,
+            rgba_out, nullptr, 0, 0);
         if (launches)
             *launches += nl;
         return e;
@@ -2600,7 +2613,8 @@ cudaError_t run_solver_noalloc(const float* P, const float* A, const float* Wt, 
         return e;
     // Every workspace element (lap P, both momentum images, the second Jacobi
     // buffer) is written before it is read, so nothing is cleared.
-    return run_solver(P, A, Wt, O, w, h, num_iter, step, mom, ws, st, nullptr, nullptr, kSolverExact);
+    return run_solver(P, A, Wt, O, w, h, num_iter, step, mom, ws, kNoAllocWorkspaceFloats, st, nullptr, nullptr,
+        kSolverExact);
 }
 
 cudaError_t device_timeout_flag(int** flag)
