@@ -68,8 +68,10 @@ VSC_API vsc_status vsc_selftest_bounded_wait(int32_t spins, vsc_stream_t stream)
  * a property of the build, for profiling tools. */
 VSC_API int32_t vsc_solver_steps_per_launch(void);
 
-/* Tile-shape autotuner of the blend solver (vsc_get_consist_out and the
- * stabilizer).  Its two persistent kernels, on 64 x 32 and 64 x 48 pixel
+/* Tile-shape autotuner of the blend solver's exact form on interleaved images
+ * (vsc_get_consist_out on small images, or in a caller's workspace of
+ * vsc_consist_out_workspace_size bytes; other solves run on planes, in one
+ * tile shape).  Its two persistent kernels, on 64 x 32 and 64 x 48 pixel
  * tiles, give the same results bit for bit; which is faster at a size
  * depends on how the tiles fill the GPU's waves.  vsc_solver_autotune times
  * both at width x height on scratch images and keeps the faster for the
@@ -272,7 +274,12 @@ VSC_API size_t vsc_consist_out_workspace_size(int32_t width, int32_t height);
  * result).  Replaces get_consist_out / kernel_consist_out
  * (flowconsistency.cu:193-258, :350-374).  workspace: device memory of at
  * least vsc_consist_out_workspace_size bytes, or NULL to let the library
- * take it from the stream-ordered memory pool of the current device. */
+ * take it from the stream-ordered memory pool of the current device.  The
+ * faster solve, each channel as its own plane in one launch, needs 7/4 of
+ * those bytes (the width rounded up to a multiple of 4) and 4 bytes per tile:
+ * NULL takes them, a workspace that has them is used so, a smaller one is
+ * solved on interleaved images (same bits, about 1.6 times the time at
+ * 1920x1080). */
 VSC_API vsc_status vsc_get_consist_out(const vsc_image* crnt_pr, const vsc_image* prev_stab_warp,
     const vsc_image* cons_wt, int32_t num_iter, float step_size, float mom_fac, const vsc_image* consis_out,
     void* workspace, size_t workspace_bytes, vsc_stream_t stream);
@@ -473,10 +480,9 @@ VSC_API vsc_status vsc_stabilizer_set_upsampler(vsc_stabilizer* s, vsc_upsampler
  * Stabilizes n independent videos of any sizes in lockstep: each step runs
  * every stream's doOneStep.  Each video's flows, warps, combination and
  * pyramid run on a CUDA stream of its own, forked from `stream`; the solves
- * are grouped: per pyramid level, each launch of the persistent solver
- * kernel (8 Jacobi steps) walks the tiles of every video's image, so one
- * launch sequence on `stream` solves all videos (up to 16 per launch), with
- * the tile shape autotuned at creation for the list of sizes.  From the
+ * are grouped: per pyramid level, each launch of the solve kernel walks the
+ * tiles of every video's image through all Jacobi steps, so one launch on
+ * `stream` solves up to 16 videos.  From the
  * second step on the whole step is replayed as one CUDA graph (captured once
  * per window position).  Flows are computed by the library (compute_flow =
  * 1); every stream shares the hyper-parameters of

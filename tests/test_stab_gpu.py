@@ -213,6 +213,39 @@ def test_consist_out_fma_any_width(vsc, oracle, cuda, w, h):
     vsc.check_device()
 
 
+# The exact form in planes (sizes of more than one wave of its interleaved
+# tiles, or a width that is not a multiple of 4) and both forms' rounds of 16
+# steps (small frames, more than 8 steps): interiors of 112 x 48 and 96 x 32
+# (exact), 96 x 40 (FMA); one or a few rows left for the last row of tiles,
+# which then reads two rows of tiles up (135 = 4 * 32 + 7, 121 = 3 * 40 + 1);
+# two rows of tiles only; short and odd last rounds.
+@pytest.mark.parametrize("form,w,h,iters", [
+    ("exact", 480, 270, 37), ("exact", 484, 261, 19), ("exact", 640, 337, 27), ("exact", 640, 360, 8),
+    ("exact", 241, 135, 20), ("exact", 99, 33, 17), ("exact", 113, 97, 33), ("exact", 427, 240, 16),
+    ("exact", 853, 199, 25), ("exact", 1, 40, 9), ("exact", 97, 65, 31),
+    ("fma", 240, 121, 20), ("fma", 97, 41, 17), ("fma", 225, 135, 33), ("fma", 96, 40, 16), ("fma", 480, 270, 31),
+    ("fma", 193, 161, 48), ("fma", 100, 122, 9)])
+def test_consist_out_planes(vsc, oracle, cuda, form, w, h, iters):
+    import torch
+
+    P, A, Wt, O0 = _img(h, w), _img(h, w), _img(h, w, hi=2.0), _img(h, w)
+    Wt[Wt < 0.3] = 0.0
+    O = _t(O0, cuda)
+    vsc.get_consist_out(_t(P, cuda), _t(A, cuda), _t(Wt, cuda), iters, 0.15, 0.15, O, form=form)
+    got = O.cpu().numpy()
+    ref = oracle.consist_out(P, A, Wt, iters, 0.15, 0.15, O0, form=form)
+    if form == "exact":
+        assert _equal_up_to_zero_sign(got, ref)
+        # a workspace without room for the planes: interleaved images, the same bits
+        ws = torch.empty(vsc.consist_out_workspace_size(w, h) // 4, dtype=torch.float32, device=cuda)
+        O2 = _t(O0, cuda)
+        vsc.get_consist_out(_t(P, cuda), _t(A, cuda), _t(Wt, cuda), iters, 0.15, 0.15, O2, workspace=ws)
+        assert np.array_equal(O2.cpu().numpy().view(np.uint32), got.view(np.uint32))
+    else:
+        assert np.array_equal(got.view(np.uint32), ref.view(np.uint32))
+    vsc.check_device()
+
+
 def test_consist_out_fma_single_tile_shape(vsc, cuda):
     """The FMA form has one tile shape (128 x 72 of a plane); the autotuner
     reports it without measuring."""

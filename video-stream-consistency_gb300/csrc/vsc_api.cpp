@@ -1284,23 +1284,27 @@ cudaError_t enqueue_step(vsc_stabilizer* s, const vsc_hyper_params& hp, uint8_t*
     float** W = lv.W;
     float** O = lv.O;
     const size_t ws_floats = solver_workspace_any_floats(s->w, s->h);
-    // The solution is initialised with the processed frame and carried down
-    // with the same bilinear chain, so at the coarsest level it equals P.
-    run(cudaMemcpyAsync(O[L - 1], P[L - 1], static_cast<size_t>(s->lw[L - 1]) * s->lh[L - 1] * 3 * sizeof(float),
-        cudaMemcpyDeviceToDevice, st));
     mark(s, kEvFront);
     for (int j = L - 1; j >= 0; --j) {
         if (j == 0)
             mark(s, kEvCoarse);
         const int iters = hp.num_iter / (j + 1);
         uint8_t* rgba = j == 0 ? rgba_dev : nullptr;
-        if (j != L - 1 && s->solver_form == kSolverFma && iters > 0) {
-            // the FMA form upsamples the coarser solution in its setup pass
-            run(run_solver_from_coarse(P[j], A[j], W[j], O[j], s->lw[j], s->lh[j], O[j + 1], s->lw[j + 1],
-                s->lh[j + 1], iters, hp.step_size, hp.mom_fac, s->solver_ws, ws_floats, st, &nl, rgba));
+        // The solution is initialised with the processed frame and carried down
+        // with the same bilinear chain, so at the coarsest level it equals P;
+        // the solve's setup reads it from there, or upsamples the coarser
+        // solution.
+        const bool coarsest = j == L - 1;
+        if (iters > 0 && solver_tma_supported()) {
+            run(run_solver_planes(s->solver_form, P[j], A[j], W[j], coarsest ? P[j] : nullptr, O[j], s->lw[j], s->lh[j],
+                coarsest ? nullptr : O[j + 1], coarsest ? 0 : s->lw[j + 1], coarsest ? 0 : s->lh[j + 1], iters,
+                hp.step_size, hp.mom_fac, s->solver_ws, ws_floats, st, &nl, rgba));
             continue;
         }
-        if (j != L - 1) {
+        if (coarsest) {
+            run(cudaMemcpyAsync(O[j], P[j], static_cast<size_t>(s->lw[j]) * s->lh[j] * 3 * sizeof(float),
+                cudaMemcpyDeviceToDevice, st));
+        } else {
             run(launch_bilinear(Img{O[j + 1], s->lw[j + 1], s->lh[j + 1], 3}, Img{O[j], s->lw[j], s->lh[j], 3}, st));
             ++nl;
         }
@@ -1790,7 +1794,6 @@ struct vsc_multistream {
     bool fused = true;      // requested (vsc_multistream_set_fused)
     bool fused_ok = false;  // every stream's level sizes take the TMA path
     std::vector<float*> lvl_ws;  // per stream: solver workspaces of levels 1 ..
-    int tuned_levels = 0;        // levels whose group tile shape was autotuned
     int solver_form = kSolverExact;
     std::vector<cudaStream_t> side;
     std::vector<cudaEvent_t> loaded, joined;
@@ -1897,12 +1900,9 @@ cudaError_t ms_enqueue_fused(vsc_multistream* m, const std::vector<uint8_t*>& ou
             ++nl;
         }
         // videostabilizer.cpp:212-217: the coarsest level starts from P
-        const int it = hp.num_iter / L;
         if (e == cudaSuccess)
-            e = cudaMemcpyAsync(solver_start_buffer(lv[i].O[L - 1], s->lw[L - 1], s->lh[L - 1], it,
-                                    ms_level_ws(m, i, L - 1), m->solver_form),
-                lv[i].P[L - 1], static_cast<size_t>(s->lw[L - 1]) * s->lh[L - 1] * 3 * sizeof(float),
-                cudaMemcpyDeviceToDevice, s->st);
+            e = cudaMemcpyAsync(lv[i].O[L - 1], lv[i].P[L - 1],
+                static_cast<size_t>(s->lw[L - 1]) * s->lh[L - 1] * 3 * sizeof(float), cudaMemcpyDeviceToDevice, s->st);
         if (e == cudaSuccess && (e = cudaEventRecord(m->joined[i], m->side[i])) == cudaSuccess)
             e = cudaStreamWaitEvent(m->main, m->joined[i], 0);
     }
@@ -1913,12 +1913,10 @@ cudaError_t ms_enqueue_fused(vsc_multistream* m, const std::vector<uint8_t*>& ou
         for (size_t i = 0; i < n; ++i) {
             vsc_stabilizer* s = m->st[i];
             float* ws = ms_level_ws(m, i, j);
-            im[i] = SolverImage{lv[i].P[j], lv[i].A[j], lv[i].W[j], lv[i].O[j], s->lw[j], s->lh[j], ws,
-                j == 0 ? outs[i] : nullptr};
+            im[i] = SolverImage{lv[i].O[j], s->lw[j], s->lh[j], ws, j == 0 ? outs[i] : nullptr};
             if (j != L - 1) {
                 up_in[i] = Img{lv[i].O[j + 1], s->lw[j + 1], s->lh[j + 1], 3};
-                up_out[i] = Img{solver_start_buffer(lv[i].O[j], s->lw[j], s->lh[j], it, ws, m->solver_form), s->lw[j],
-                    s->lh[j], 3};
+                up_out[i] = Img{lv[i].O[j], s->lw[j], s->lh[j], 3};
             }
         }
         if (j != L - 1) {
@@ -1949,34 +1947,6 @@ bool ms_use_fused(vsc_multistream* m)
                 return false;
     }
     return true;
-}
-
-// The tile shape of each level's group for a solver form (a stream being
-// captured, or a failed measurement, keeps the wave model).
-void ms_tune(vsc_multistream* m, int form)
-{
-    cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
-    if (cudaStreamIsCapturing(m->main, &cap) != cudaSuccess || cap != cudaStreamCaptureStatusNone)
-        return;
-    int levels = 4;
-    for (vsc_stabilizer* st : m->st)
-        levels = std::min(levels, st->levels_alloc);
-    std::vector<int> ws(m->st.size()), hs(m->st.size());
-    for (int j = 0; j < levels; ++j) {
-        bool eligible = true;
-        for (size_t i = 0; i < m->st.size(); ++i) {
-            ws[i] = m->st[i]->lw[j];
-            hs[i] = m->st[i]->lh[j];
-            eligible = eligible && ws[i] % 4 == 0;
-        }
-        if (!eligible)
-            break;
-        if (solver_group_autotune(ws.data(), hs.data(), static_cast<int>(ws.size()), m->main, nullptr, form) !=
-            cudaSuccess) {
-            cudaGetLastError();
-            break;
-        }
-    }
 }
 
 void ms_drop_graphs(vsc_multistream* m)
@@ -2114,8 +2084,6 @@ VSC_API vsc_status vsc_multistream_create(const vsc_stream_desc* desc, int32_t n
             break;
         m->lvl_ws.push_back(p);
     }
-    if (!s)
-        ms_tune(m, kSolverExact);
     if (s) {
         const std::string msg = vsc_last_error();
         ms_free(m);
@@ -2171,8 +2139,6 @@ VSC_API vsc_status vsc_multistream_set_solver_form(vsc_multistream* m, int32_t f
         s = vsc_stabilizer_set_solver_form(m->st[i], form);
     if (s)
         return s;
-    if (form != m->solver_form)
-        ms_tune(m, form);
     m->solver_form = form;
     ms_drop_graphs(m);
     return VSC_OK;

@@ -136,71 +136,59 @@ cudaError_t launch_bilinear(Img in, Img out, cudaStream_t st);
 // launch_bilinear for n 3-channel images in one launch per 16 (same bits)
 cudaError_t launch_bilinear_group(const Img* in, const Img* out, int n, cudaStream_t st);
 // Solver.
-//   kSolverExact: kernel_consist_out's expression, bit for bit; workspace:
-//                 the Laplacian of the processed image, two momentum images
-//                 and the second Jacobi buffer, 4 * w*h*3 floats;
+//   kSolverExact: kernel_consist_out's expression, bit for bit;
 //   kSolverFma:   the same step regrouped around per-solve constants with
-//                 fused multiply-adds, each channel solved as its own plane
-//                 (within a tolerance of the exact form; equal to the
-//                 restatement's FMA form); workspace: the constants Cs and
-//                 nK, two momentum images and two iterates, all as planes,
-//                 6 * w*h*3 floats.
+//                 fused multiply-adds (within a tolerance of the exact form;
+//                 equal to the restatement's FMA form).
+// Both solve each channel as its own plane in one launch, in a workspace of
+// solver_workspace_full_floats: two momentum images, two iterates and the
+// form's constants (lap P, consWt and A; Cs and nK) as planes of rows on the
+// 16-byte grid.  In a workspace of solver_workspace_floats only, the exact form
+// (4 images: lap P, two momentum images, the second iterate) runs a launch a
+// round on interleaved images, and the FMA form, where its width is not a
+// multiple of 4 (else the two sizes are the same), one with plain loads.
 enum SolverForm { kSolverExact = 0, kSolverFma = 1 };
 size_t solver_workspace_floats(int w, int h, int form = kSolverExact);
-// The same with room for the FMA form's planes at a row pitch on the 16-byte
-// grid, which the TMA-fed solve wants: more than the above for widths that are
-// not a multiple of 4 only.  A workspace between the two takes plain loads.
 size_t solver_workspace_full_floats(int w, int h, int form);
 size_t solver_workspace_any_floats(int w, int h);  // the larger form's
 int solver_steps_per_launch();  // Jacobi steps one solver launch performs (temporal blocking)
-// Tile-shape autotuner of the persistent solver kernels (same results either
-// way): solver_autotune times both shapes at (w, h) on scratch images and
-// keeps the faster for the current device (synchronises `st`; not during
-// stream capture); solver_tile_rows reports the rows of the tile a solve at
-// (w, h) uses (tuned, or the wave model's choice); per solver form.
+// Tile-shape autotuner of the exact form's kernels on interleaved images (same
+// results either way): solver_autotune times both shapes at (w, h) on scratch
+// images and keeps the faster for the current device (synchronises `st`; not
+// during stream capture); solver_tile_rows reports the rows of the tile a solve
+// at (w, h) in a workspace of solver_workspace_floats uses (tuned, or the wave
+// model's choice); per solver form.
 cudaError_t solver_autotune(int w, int h, cudaStream_t st, int* rows_out, int form = kSolverExact);
 int solver_tile_rows(int w, int h, bool* tuned, int form = kSolverExact);
 void solver_set_autotune(bool on);
-// The same for the sizes one grouped launch solves together (one image per
-// stream of a multi-stream step), keyed by the whole list.
-cudaError_t solver_group_autotune(const int* w, const int* h, int n, cudaStream_t st, int* rows_out,
-    int form = kSolverExact);
-int solver_group_tile_rows(const int* w, const int* h, int n, bool* tuned, int form = kSolverExact);
 // Runs num_iter iterations; O holds the initial solution and receives the
-// result; workspace: ws_floats floats, at least solver_workspace_floats.  Returns the number of kernels launched through *launches.
+// result; workspace: ws_floats floats, at least solver_workspace_floats.
+// Returns the number of kernels launched through *launches.
 cudaError_t run_solver(const float* P, const float* A, const float* Wt, float* O, int w, int h, int num_iter,
     float step, float mom, float* workspace, size_t ws_floats, cudaStream_t st, int* launches,
     uint8_t* rgba_out = nullptr, int form = kSolverExact);
-// The FMA form started from the cw x ch solution Oc upsampled to w x h with
-// kernel_bilinear's expression (the pyramid's next level), the upsampling
-// fused into the solve's setup; O receives the result only.  num_iter >= 1.
-cudaError_t run_solver_from_coarse(const float* P, const float* A, const float* Wt, float* O, int w, int h,
-    const float* Oc, int cw, int ch, int num_iter, float step, float mom, float* workspace, size_t ws_floats,
-    cudaStream_t st, int* launches, uint8_t* rgba_out);
+// run_solver in a workspace of solver_workspace_full_floats, started from the
+// image Oi or, with Oi null, from the cw x ch solution Oc upsampled to w x h with
+// kernel_bilinear's expression (the pyramid's next level), the upsampling fused
+// into the solve's setup; O receives the result only.  num_iter >= 1.
+cudaError_t run_solver_planes(int form, const float* P, const float* A, const float* Wt, const float* Oi, float* O,
+    int w, int h, const float* Oc, int cw, int ch, int num_iter, float step, float mom, float* workspace,
+    size_t ws_floats, cudaStream_t st, int* launches, uint8_t* rgba_out);
 
 // Grouped solve: n images of any sizes, the same iterations, each launch of
-// the persistent kernel walking the tiles of all of them (up to 16 images
-// per launch).  Per image, before run_solver_group on the same stream:
-// solver_prep(form, ...) into its workspace, and the initial solution written to
-// solver_start_buffer(O, ...) (O itself or the workspace's second buffer,
-// whichever makes the last launch write O).  Needs solver_group_eligible
-// (width % 4 == 0 and 16-byte aligned images, the TMA path).
+// the solve kernel walking the tiles of all of them (up to 16 images per
+// launch).  Per image, before run_solver_group on the same stream:
+// solver_prep(form, ...) into its workspace, and the initial solution in O.
 struct SolverImage {
-    const float* P;
-    const float* A;
-    const float* Wt;
     float* O;
     int w, h;
-    float* workspace;  // solver_workspace_floats(w, h, form)
+    float* workspace;  // solver_workspace_full_floats(w, h, form)
     uint8_t* rgba;     // RGBA8 copy of the result, or null
 };
-float* solver_start_buffer(float* O, int w, int h, int num_iter, float* workspace, int form = kSolverExact);
-bool solver_tma_supported();  // the persistent TMA kernels run on the current device
-cudaError_t solver_lap(const float* P, int w, int h, float* workspace, cudaStream_t st);
-// the per-solve precomputation of a form: lap P (exact) or Cs (FMA), into the workspace
+bool solver_tma_supported();  // the solve kernel runs on the current device
+// a form's per-solve constants, into the workspace
 cudaError_t solver_prep(int form, const float* P, const float* A, const float* Wt, int w, int h, float step,
     float* workspace, cudaStream_t st);
-bool solver_group_eligible(const SolverImage* im, int n, int form = kSolverExact);
 cudaError_t run_solver_group(const SolverImage* im, int n, int num_iter, float step, float mom, cudaStream_t st,
     int* launches, int form = kSolverExact);
 

@@ -386,46 +386,23 @@ __device__ __forceinline__ void store_interior(const CUtensorMap* mOo, const CUt
 // (O, U; interior box).
 enum { kMapO, kMapU, kMapA, kMapW, kMapL, kMapOo, kMapUo, kMaps };
 
-// The problems of one launch of a persistent solver kernel: kN images of any
-// sizes (one per video stream at one pyramid level), each with its tensor
-// maps, its size and its first tile in the launch's tile list.  Every problem
-// runs the same iterations (T, k0, step, mom).  Passed by value as a
-// __grid_constant__ parameter, so the maps stay in parameter memory, where
-// TMA reads them.
-template <int kN>
-struct SolverGroup {
-    CUtensorMap map[kN][kMaps];
-    int w[kN], h[kN], tiles_x[kN];
-    int tile0[kN + 1];  // first tile of problem p; tile0[count] = tiles in all
-    uint8_t* rgba[kN];  // RGBA8 output of the last launch, or null
-    int count;
+// One launch of a persistent kernel on interleaved images: the tensor maps, the
+// size and the tiles.  Passed by value as a __grid_constant__ parameter, so the
+// maps stay in parameter memory, where TMA reads them.
+struct SolverLaunch {
+    CUtensorMap map[kMaps];
+    int w, h, tiles_x, tiles;
+    uint8_t* rgba;  // RGBA8 output of the last launch, or null
 };
-constexpr int kGroupMax = 16;
 
 struct TileLoc {
-    int p;       // problem
     int ox, oy;  // tile origin (ring included)
-    int w, h;
 };
 
-// tile -> problem by a scan of the first-tile table (kN <= kGroupMax)
-template <int kN, int kRows>
-__device__ __forceinline__ TileLoc locate(const SolverGroup<kN>& g, int tile)
+template <int kRows>
+__device__ __forceinline__ TileLoc locate(const SolverLaunch& g, int tile)
 {
-    int p = 0;
-    if (kN > 1) {
-#pragma unroll 1
-        while (p + 1 < g.count && tile >= g.tile0[p + 1])
-            ++p;
-    }
-    const int t = tile - g.tile0[p];
-    TileLoc l;
-    l.p = p;
-    l.ox = (t % g.tiles_x[p]) * kIW - kTbT;
-    l.oy = (t / g.tiles_x[p]) * kRows - kTbT;
-    l.w = g.w[p];
-    l.h = g.h[p];
-    return l;
+    return TileLoc{(tile % g.tiles_x) * kIW - kTbT, (tile / g.tiles_x) * kRows - kTbT};
 }
 
 // input tiles first .. last - 1 (map order) of a tile at (ox, oy), into consecutive stages
@@ -463,9 +440,8 @@ __device__ __forceinline__ void issue_first_loads(float* stage, const CUtensorMa
         issue_loads(stage, m, ox, oy, stage_floats, bytes, bar);
 }
 
-template <int kN>
 __global__ void __launch_bounds__(kTbEX / 2 * kTbEY / 2, 1)
-    solver_persistent_kernel(const __grid_constant__ SolverGroup<kN> g, int T, int k0, float step, float mom)
+    solver_persistent_kernel(const __grid_constant__ SolverLaunch g, int T, int k0, float step, float mom)
 {
     extern __shared__ __align__(128) unsigned char smem_raw[];
     float* stage = reinterpret_cast<float*>(smem_raw);
@@ -480,19 +456,19 @@ __global__ void __launch_bounds__(kTbEX / 2 * kTbEY / 2, 1)
     if (tid == 0)
         mbar_init(bar, 1);
     __syncthreads();
-    const int ntiles = g.tile0[g.count];
+    const int ntiles = g.tiles;
     int tile = blockIdx.x;
     if (tid == 0 && tile < ntiles) {
-        const TileLoc n = locate<kN, kIH>(g, tile);
-        issue_first_loads(stage, g.map[n.p], n.ox, n.oy, kStageFloats, kStageBytes, bar, k0 > 0);
+        const TileLoc n = locate<kIH>(g, tile);
+        issue_first_loads(stage, g.map, n.ox, n.oy, kStageFloats, kStageBytes, bar, k0 > 0);
     }
     grid_dependency_wait();
     uint32_t parity = 0;
     for (; tile < ntiles; tile += gridDim.x) {
         if (tile + static_cast<int>(gridDim.x) >= ntiles)
             allow_dependent_launch();
-        const TileLoc c = locate<kN, kIH>(g, tile);
-        const int ox = c.ox, oy = c.oy, w = c.w, h = c.h;
+        const TileLoc c = locate<kIH>(g, tile);
+        const int ox = c.ox, oy = c.oy, w = g.w, h = g.h;
         if (!mbar_wait_bounded(bar, parity, kWaitSpins)) {
             // the outputs are invalid and vsc_check_device reports VSC_ETIMEOUT; the
             // second bounded wait gives copies still in flight a chance to land
@@ -554,8 +530,8 @@ __global__ void __launch_bounds__(kTbEX / 2 * kTbEY / 2, 1)
         __syncthreads();  // staging consumed, O published
         if (tid == 0 && tile + static_cast<int>(gridDim.x) < ntiles) {
             asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-            const TileLoc n = locate<kN, kIH>(g, tile + gridDim.x);
-            issue_loads(stage, g.map[n.p], n.ox, n.oy, kStageFloats, kStageBytes, bar);
+            const TileLoc n = locate<kIH>(g, tile + gridDim.x);
+            issue_loads(stage, g.map, n.ox, n.oy, kStageFloats, kStageBytes, bar);
         }
 
         const bool interior = ox >= 1 && oy >= 1 && ox + kTbEX - 1 <= w - 3 && oy + kTbEY - 1 <= h - 3;
@@ -592,8 +568,8 @@ __global__ void __launch_bounds__(kTbEX / 2 * kTbEY / 2, 1)
         asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
         __syncthreads();
         if (tid == 0)
-            store_interior(g.map[c.p] + kMapOo, g.map[c.p] + kMapUo, ox, oy, so, su);
-        if (uint8_t* rgba = g.rgba[c.p]) {
+            store_interior(g.map + kMapOo, g.map + kMapUo, ox, oy, so, su);
+        if (uint8_t* rgba = g.rgba) {
 #pragma unroll
             for (int q = 0; q < 4; ++q) {
                 const int px = px0 + (q & 1), py = py0 + (q >> 1);
@@ -724,9 +700,8 @@ __device__ __forceinline__ void p8_iterate(P8State& s, float* obuf, int T, int k
     }
 }
 
-template <int kN>
 __global__ void __launch_bounds__(kPThreads, 1)
-    solver_tall_kernel(const __grid_constant__ SolverGroup<kN> g, int T, int k0, float step, float mom)
+    solver_tall_kernel(const __grid_constant__ SolverLaunch g, int T, int k0, float step, float mom)
 {
     extern __shared__ __align__(128) unsigned char smem_raw[];
     float* stage = reinterpret_cast<float*>(smem_raw);
@@ -740,19 +715,19 @@ __global__ void __launch_bounds__(kPThreads, 1)
     if (threadIdx.x == 0)
         mbar_init(bar, 1);
     __syncthreads();
-    const int ntiles = g.tile0[g.count];
+    const int ntiles = g.tiles;
     int tile = blockIdx.x;
     if (threadIdx.x == 0 && tile < ntiles) {
-        const TileLoc n = locate<kN, kPIH>(g, tile);
-        issue_first_loads(stage, g.map[n.p], n.ox, n.oy, kPStageFloats, kPStageBytes, bar, k0 > 0);
+        const TileLoc n = locate<kPIH>(g, tile);
+        issue_first_loads(stage, g.map, n.ox, n.oy, kPStageFloats, kPStageBytes, bar, k0 > 0);
     }
     grid_dependency_wait();
     uint32_t parity = 0;
     for (; tile < ntiles; tile += gridDim.x) {
         if (tile + static_cast<int>(gridDim.x) >= ntiles)
             allow_dependent_launch();
-        const TileLoc c = locate<kN, kPIH>(g, tile);
-        const int ox = c.ox, oy = c.oy, w = c.w, h = c.h;
+        const TileLoc c = locate<kPIH>(g, tile);
+        const int ox = c.ox, oy = c.oy, w = g.w, h = g.h;
         if (!mbar_wait_bounded(bar, parity, kWaitSpins)) {
             // the outputs are invalid and vsc_check_device reports VSC_ETIMEOUT; the
             // second bounded wait gives copies still in flight a chance to land
@@ -799,8 +774,8 @@ __global__ void __launch_bounds__(kPThreads, 1)
         __syncthreads();  // staging consumed, edge rows published
         if (threadIdx.x == 0 && tile + static_cast<int>(gridDim.x) < ntiles) {
             asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-            const TileLoc n = locate<kN, kPIH>(g, tile + gridDim.x);
-            issue_loads(stage, g.map[n.p], n.ox, n.oy, kPStageFloats, kPStageBytes, bar);
+            const TileLoc n = locate<kPIH>(g, tile + gridDim.x);
+            issue_loads(stage, g.map, n.ox, n.oy, kPStageFloats, kPStageBytes, bar);
         }
 
         const int gx0 = ox + px0, gy0 = oy + py0;
@@ -839,8 +814,8 @@ __global__ void __launch_bounds__(kPThreads, 1)
         asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
         __syncthreads();
         if (threadIdx.x == 0)
-            store_interior(g.map[c.p] + kMapOo, g.map[c.p] + kMapUo, ox, oy, so, su);
-        if (uint8_t* rgba = g.rgba[c.p]) {
+            store_interior(g.map + kMapOo, g.map + kMapUo, ox, oy, so, su);
+        if (uint8_t* rgba = g.rgba) {
 #pragma unroll
             for (int q = 0; q < 8; ++q) {
                 const int px = px0 + (q & 1), py = py0 + (q >> 1);
@@ -862,7 +837,7 @@ __global__ void __launch_bounds__(kPThreads, 1)
 // ---- FMA form of the solver ---------------------------------------------------
 // kernel_consist_out's step, g = (lap O - lap P) - w (O - A), O' = O + s g
 // (+ m U), U' = s g, regrouped around two per-pixel constants computed once
-// per solve (solver_prep_fma_kernel):
+// per solve (solver_prep_kernel):
 //   Cs = s * fma(w, A, -lap P),   nK = -(s * (cnt + w))   (cnt = valid neighbours),
 // so that one step is
 //   S = (left + right) + (up + down),  g = fma(nK, O, fma(s, S, Cs)),
@@ -882,50 +857,71 @@ __global__ void __launch_bounds__(kPThreads, 1)
 // shuffles per row for four pixels, and each warp publishes its top and
 // bottom row as two 16-byte stores per thread.
 
+constexpr int kGroupMax = 16;             // images of a grouped solve's launch
 constexpr int kPlW = 128;                 // tile width (a warp: 32 lanes x 4 columns)
-constexpr int kPlIW = kPlW - 2 * kTbT;    // interior width (112)
 
-// A form's tile: kPlanes input planes, kWarps warps of kRPT rows each.
+// How a solve in planes runs: its form (bit 0) and whether its rounds are 16
+// steps with a 16-pixel ring instead of 8 (bit 1).
+constexpr int kPlLong = 2;
+
+// A form's tile: kPlanes input planes, kWarps warps of kRPT rows each, and the
+// registers of the compute and the control warps.
 template <int kForm>
 struct PlG;
 template <>
-struct PlG<kSolverFma> {
+struct PlG<kSolverFma> {  // O, U, nK, Cs
     static constexpr int kPlanes = 4, kWarps = 8, kRPT = 9;
+    static constexpr int kComputeRegs = 216, kControlRegs = 72;
+};
+// The exact form's step needs three constants of a pixel, consWt, lap P and A:
+// 160 registers of state for 4 x 8 blocks, a tile of 128 x 64 (interior 112 x
+// 48, 66 %).
+template <>
+struct PlG<kSolverExact> {  // O, U, consWt, lap P, A
+    static constexpr int kPlanes = 5, kWarps = 8, kRPT = 8;
+    static constexpr int kComputeRegs = 224, kControlRegs = 56;
 };
 
-template <int kForm>
-struct PlGeo : PlG<kForm> {
-    using PlG<kForm>::kPlanes;
-    using PlG<kForm>::kWarps;
-    using PlG<kForm>::kRPT;
-    static constexpr int kRows = kRPT * kWarps;          // 72
-    static constexpr int kIRows = kRows - 2 * kTbT;      // interior rows (56)
+template <int kCfg>
+struct PlGeo : PlG<kCfg & 1> {
+    using B = PlG<kCfg & 1>;
+    using B::kPlanes;
+    using B::kRPT;
+    using B::kWarps;
+    static constexpr bool kFma = (kCfg & 1) == kSolverFma;
+    static constexpr int kT = kCfg & kPlLong ? 2 * kTbT : kTbT;  // steps a round, the ring's width
+    static constexpr int kIW = kPlW - 2 * kT;            // interior columns: 112, 96 in long rounds
+    static constexpr int kRows = kRPT * kWarps;          // 72 (FMA), 64 (exact)
+    static constexpr int kIRows = kRows - 2 * kT;        // interior rows: 56, 48; 40, 32 in long rounds
     static constexpr int kStage = kRows * kPlW;          // floats of one input tile
     static constexpr int kStageBytes = kStage * static_cast<int>(sizeof(float));
     static constexpr int kSlots = (kWarps + 2) * 2 * kPlW;  // edge-row slots of one buffer
-    static constexpr int kOut = kIRows * kPlIW;          // floats of one interior tile
+    static constexpr int kOut = kIRows * kIW;            // floats of one interior tile
     static constexpr int kSmem =
         kPlanes * kStageBytes + (2 * kSlots + 2 * kOut) * static_cast<int>(sizeof(float)) + 128;
     static_assert(kSmem <= 232448, "dynamic shared memory per CTA");
     static_assert((kPlanes * kStageBytes) % 128 == 0 && (2 * kSlots * 4) % 128 == 0 && (kOut * 4) % 128 == 0,
         "TMA sources and destinations on the 128-byte grid");
-    // rows of the tile that the frame's rows 0 (tiles at oy = -8) and h - 2, h - 1
+    static_assert(kT <= kIW && kT <= kIRows, "a tile reads only its 3 x 3 neighbours' interiors");
+    static_assert((kIW * 4) % 16 == 0 && (kT * 4) % 16 == 0, "TMA x coordinates must be 16-byte aligned");
+    // rows of the tile that the frame's rows 0 (tiles at oy = -kT) and h - 2, h - 1
     // (tiles that end on the frame's last row) sit in, as warp and row
-    static constexpr int kTopWarp = kTbT / kRPT, kTopRow = kTbT % kRPT;
-    static constexpr int kBot2Warp = (kRows - kTbT - 2) / kRPT, kBot2Row = (kRows - kTbT - 2) % kRPT;
-    static constexpr int kBot1Warp = (kRows - kTbT - 1) / kRPT, kBot1Row = (kRows - kTbT - 1) % kRPT;
+    static constexpr int kTopWarp = kT / kRPT, kTopRow = kT % kRPT;
+    static constexpr int kBot2Warp = (kRows - kT - 2) / kRPT, kBot2Row = (kRows - kT - 2) % kRPT;
+    static constexpr int kBot1Warp = (kRows - kT - 1) / kRPT, kBot1Row = (kRows - kT - 1) % kRPT;
 };
-static_assert((kPlIW * 4) % 16 == 0 && (kTbT * 4) % 16 == 0, "TMA x coordinates must be 16-byte aligned");
 
 // Cs = step * fma(wt, A, -lap P) and nK = -(step * (cnt + wt)) as planes
 // (lap P, cnt as lap_pr_kernel computes them); with O non-null, also O as
 // planes into Op, or with Oc non-null the cw x ch image Oc upsampled to w x h
 // as kernel_bilinear does (bilinear_px: the pyramid's initial solution of
 // this level, written straight into the planes); with cnt non-null, the ncnt
-// solve counters zeroed.
-__global__ void solver_prep_fma_kernel(const float* __restrict__ P, const float* __restrict__ A,
+// solve counters zeroed.  The exact form's constants: lap P in Cs, wt in nK, A
+// in Ap.
+template <int kForm>
+__global__ void solver_prep_kernel(const float* __restrict__ P, const float* __restrict__ A,
     const float* __restrict__ Wt, const float* __restrict__ O, float* __restrict__ Cs, float* __restrict__ nK,
-    float* __restrict__ Op, int w, int h, int pitch, float step, unsigned* __restrict__ cnt, int ncnt,
+    float* __restrict__ Ap, float* __restrict__ Op, int w, int h, int pitch, float step, unsigned* __restrict__ cnt, int ncnt,
     const float* __restrict__ Oc, int cw, int ch)
 {
     pdl_enter();
@@ -965,8 +961,14 @@ __global__ void solver_prep_fma_kernel(const float* __restrict__ P, const float*
         }
         lap = __fsub_rn(lap, __fmul_rn(static_cast<float>(cnt), P[i]));
         const float wt = Wt[i];
-        Cs[c * plane + q] = __fmul_rn(step, __fmaf_rn(wt, A[i], -lap));
-        nK[c * plane + q] = -__fmul_rn(step, __fadd_rn(static_cast<float>(cnt), wt));
+        if (kForm == kSolverFma) {
+            Cs[c * plane + q] = __fmul_rn(step, __fmaf_rn(wt, A[i], -lap));
+            nK[c * plane + q] = -__fmul_rn(step, __fadd_rn(static_cast<float>(cnt), wt));
+        } else {
+            Cs[c * plane + q] = lap;
+            nK[c * plane + q] = wt;
+            Ap[c * plane + q] = A[i];
+        }
         if (Oc)
             Op[c * plane + q] = up[c];
         else if (O)
@@ -1025,10 +1027,11 @@ __global__ void __launch_bounds__(256) planar_group_kernel(const __grid_constant
         reinterpret_cast<uint32_t*>(g.rgba[p])[i] = pack_rgba(r, gg, b);
 }
 
-template <int kForm>
+template <int kCfg>
 struct PlState {
-    static constexpr int kR = PlGeo<kForm>::kRPT;
-    float4 o[kR], u[kR], c[kR], nk[kR];  // [row] = (column 0 .. 3)
+    static constexpr int kR = PlGeo<kCfg>::kRPT;
+    float4 o[kR], u[kR], c[kR], nk[kR];  // [row] = (column 0 .. 3); exact form: c = lap P, nk = consWt
+    float4 a[!PlGeo<kCfg>::kFma ? kR : 1];
 };
 
 __device__ __forceinline__ float& f4(float4& v, int j) { return j == 0 ? v.x : j == 1 ? v.y : j == 2 ? v.z : v.w; }
@@ -1070,30 +1073,31 @@ struct PlPlace {
 // The columns left and right of a thread's block, from the neighbouring lanes
 // (the outer lanes keep their own value: the tile's outer columns never reach
 // the interior).
-template <int kForm>
+template <int kCfg>
 struct PlSides {
-    float l[PlGeo<kForm>::kRPT], r[PlGeo<kForm>::kRPT];
+    float l[PlGeo<kCfg>::kRPT], r[PlGeo<kCfg>::kRPT];
 };
 
 // One step of row r of a thread's block: the new row in `on`, U in place;
 // then the lanes exchange the new row's end columns for the next step.
-template <int kForm, int kMode>
-__device__ __forceinline__ void pl_row(PlState<kForm>& s, PlSides<kForm>& x, float4* on, int r, float4 up, float4 dn,
+template <int kCfg, int kMode>
+__device__ __forceinline__ void pl_row(PlState<kCfg>& s, PlSides<kCfg>& x, float4* on, int r, float4 up, float4 dn,
     float step, float mom, const PlPlace& t)
 {
-    using G = PlGeo<kForm>;
+    using G = PlGeo<kCfg>;
     const float4 o = s.o[r];
     float4 u = r == 0 ? up : s.o[r - 1];
     float4 d = r == G::kRPT - 1 ? dn : s.o[r + 1];
     constexpr bool kFixed = kMode == kPlLanes || kMode == kPlCols;
-    if (kFixed && r == G::kTopRow && t.zt)
+    float cnt_rows = 4.0f;  // exact form: left, right and the valid ones of up and down
+    if ((kFixed && r == G::kTopRow && t.zt) || (kMode == kPlEvery && r == t.top)) {
         u = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-    if (kFixed && ((r == G::kBot2Row && t.zb2) || (r == G::kBot1Row && t.zb1)))
+        cnt_rows -= 1.0f;
+    }
+    if ((kFixed && ((r == G::kBot2Row && t.zb2) || (r == G::kBot1Row && t.zb1))) || (kMode == kPlEvery && r >= t.bot)) {
         d = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-    if (kMode == kPlEvery && r == t.top)
-        u = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-    if (kMode == kPlEvery && r >= t.bot)
-        d = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+        cnt_rows -= 1.0f;
+    }
     float lft = x.l[r], rgt = x.r[r], o3 = o.w;  // left of column 0, right of columns 3 and 2
     if (kMode != kPlAll)
         lft = t.zl ? 0.0f : lft;
@@ -1108,9 +1112,26 @@ __device__ __forceinline__ void pl_row(PlState<kForm>& s, PlSides<kForm>& x, flo
         if (kMode == kPlCols || kMode == kPlEvery)
             right = j < t.xlim ? right : 0.0f;
         const float oj = f4c(o, j);
-        const float g = __fmaf_rn(f4c(s.nk[r], j), oj,
-            __fmaf_rn(step, __fadd_rn(__fadd_rn(left, right), __fadd_rn(f4c(u, j), f4c(d, j))), f4c(s.c[r], j)));
-        f4(on[r], j) = __fmaf_rn(mom, f4c(s.u[r], j), __fadd_rn(oj, g));
+        float g;
+        if (G::kFma) {
+            g = __fmaf_rn(f4c(s.nk[r], j), oj,
+                __fmaf_rn(step, __fadd_rn(__fadd_rn(left, right), __fadd_rn(f4c(u, j), f4c(d, j))), f4c(s.c[r], j)));
+            f4(on[r], j) = __fmaf_rn(mom, f4c(s.u[r], j), __fadd_rn(oj, g));
+        } else {
+            // jacobi_px's expression; where a neighbour is read as +0, cnt of the
+            // valid ones times o is rounded before the subtraction, as there
+            float lap = __fadd_rn(__fadd_rn(__fadd_rn(right, left), f4c(d, j)), f4c(u, j));
+            if (kMode == kPlAll) {
+                lap = __fmaf_rn(-4.0f, oj, lap);
+            } else {
+                const bool vr = kMode == kPlLanes ? !(j >= 2 && t.zr) : j < t.xlim;
+                const float cnt = cnt_rows - (vr ? 0.0f : 1.0f) - (j == 0 && t.zl ? 1.0f : 0.0f);
+                lap = __fsub_rn(lap, __fmul_rn(cnt, oj));
+            }
+            const float d1 = __fmul_rn(f4c(s.nk[r], j), __fsub_rn(oj, f4c(s.a[r], j)));
+            g = __fmul_rn(step, __fsub_rn(__fsub_rn(lap, f4c(s.c[r], j)), d1));
+            f4(on[r], j) = __fadd_rn(__fadd_rn(oj, g), __fmul_rn(mom, f4c(s.u[r], j)));
+        }
         f4(s.u[r], j) = g;
     }
     x.l[r] = __shfl_up_sync(0xffffffffu, on[r].w, 1);
@@ -1120,30 +1141,31 @@ __device__ __forceinline__ void pl_row(PlState<kForm>& s, PlSides<kForm>& x, flo
 // One step of a thread's block; `up` and `dn` are the previous iterate's rows
 // above and below it.  The rows between go first, while those two arrive; each
 // row's shuffles for the next step run beside the following rows' arithmetic.
-template <int kForm, int kMode>
-__device__ __forceinline__ void pl_step(PlState<kForm>& s, PlSides<kForm>& x, float4 up, float4 dn, float step,
+template <int kCfg, int kMode>
+__device__ __forceinline__ void pl_step(PlState<kCfg>& s, PlSides<kCfg>& x, float4 up, float4 dn, float step,
     float mom, const PlPlace& t)
 {
-    constexpr int kR = PlGeo<kForm>::kRPT;
+    constexpr int kR = PlGeo<kCfg>::kRPT;
     float4 on[kR];
 #pragma unroll
     for (int q = 0; q < kR; ++q)
-        pl_row<kForm, kMode>(s, x, on, q < kR - 2 ? q + 1 : (q == kR - 2 ? 0 : kR - 1), up, dn, step, mom, t);
+        pl_row<kCfg, kMode>(s, x, on, q < kR - 2 ? q + 1 : (q == kR - 2 ? 0 : kR - 1), up, dn, step, mom, t);
 #pragma unroll
     for (int r = 0; r < kR; ++r)
         s.o[r] = on[r];
 }
 
 // The planar step's test mode for a tile at (ox, oy) of a w x h frame.
-template <int kForm>
+template <int kCfg>
 __device__ __forceinline__ int pl_mode(int ox, int oy, int w, int h)
 {
-    constexpr int kRows = PlGeo<kForm>::kRows;
+    using G = PlGeo<kCfg>;
+    constexpr int kRows = G::kRows;
     if (ox >= 1 && oy >= 1 && ox + kPlW - 1 <= w - 3 && oy + kRows - 1 <= h - 3)
         return kPlAll;
     const bool row0 = oy <= 0 && oy + kRows - 1 >= 0;
     const bool last2 = oy <= h - 1 && oy + kRows - 1 >= h - 2;
-    if ((!row0 || oy == -kTbT) && (!last2 || oy == h - kRows + kTbT))  // ox is a multiple of 4
+    if ((!row0 || oy == -G::kT) && (!last2 || oy == h - kRows + G::kT))  // ox is a multiple of 4
         return (w & 3) == 0 ? kPlLanes : kPlCols;
     return kPlEvery;
 }
@@ -1158,12 +1180,12 @@ __device__ __forceinline__ int pl_mode(int ox, int oy, int w, int h)
 // and with a condition in it (momentum off in a solve's first step, steps left
 // out) the two steps' registers meet in moves.  A solve's first step has U = +0
 // and takes mom = -0: fma(-0, +0, n) is n, whatever n is.
-template <int kForm, int kMode, class Bar>
-__device__ __forceinline__ void pl_steps(PlState<kForm>& s, float4 up, float4 dn, float* slots, int T, int k0,
+template <int kCfg, int kMode, class Bar>
+__device__ __forceinline__ void pl_steps(PlState<kCfg>& s, float4 up, float4 dn, float* slots, int T, int k0,
     float step, float mom, int lane, int warp, const PlPlace& t, Bar&& bar)
 {
-    using G = PlGeo<kForm>;
-    PlSides<kForm> x;
+    using G = PlGeo<kCfg>;
+    PlSides<kCfg> x;
 #pragma unroll
     for (int r = 0; r < G::kRPT; ++r) {
         x.l[r] = __shfl_up_sync(0xffffffffu, s.o[r].w, 1);
@@ -1180,35 +1202,35 @@ __device__ __forceinline__ void pl_steps(PlState<kForm>& s, float4 up, float4 dn
     float m = k0 > 0 ? mom : -0.0f;
 #pragma unroll 1
     for (int k = 0; k + 1 < T; k += 2) {
-        pl_step<kForm, kMode>(s, x, up, dn, step, m, t);
+        pl_step<kCfg, kMode>(s, x, up, dn, step, m, t);
         exchange(top);
-        pl_step<kForm, kMode>(s, x, up, dn, step, mom, t);
+        pl_step<kCfg, kMode>(s, x, up, dn, step, mom, t);
         exchange(top + G::kSlots);
         m = mom;
     }
     if (T & 1)  // a short last round
-        pl_step<kForm, kMode>(s, x, up, dn, step, m, t);
+        pl_step<kCfg, kMode>(s, x, up, dn, step, m, t);
 }
 
-template <int kForm, class Bar>
-__device__ __forceinline__ void pl_round(int mode, PlState<kForm>& s, float4 up, float4 dn, float* slots, int T,
+template <int kCfg, class Bar>
+__device__ __forceinline__ void pl_round(int mode, PlState<kCfg>& s, float4 up, float4 dn, float* slots, int T,
     int k0, float step, float mom, int lane, int warp, const PlPlace& t, Bar&& bar)
 {
     if (mode == kPlAll)
-        pl_steps<kForm, kPlAll>(s, up, dn, slots, T, k0, step, mom, lane, warp, t, bar);
+        pl_steps<kCfg, kPlAll>(s, up, dn, slots, T, k0, step, mom, lane, warp, t, bar);
     else if (mode == kPlLanes)
-        pl_steps<kForm, kPlLanes>(s, up, dn, slots, T, k0, step, mom, lane, warp, t, bar);
+        pl_steps<kCfg, kPlLanes>(s, up, dn, slots, T, k0, step, mom, lane, warp, t, bar);
     else if (mode == kPlCols)
-        pl_steps<kForm, kPlCols>(s, up, dn, slots, T, k0, step, mom, lane, warp, t, bar);
+        pl_steps<kCfg, kPlCols>(s, up, dn, slots, T, k0, step, mom, lane, warp, t, bar);
     else
-        pl_steps<kForm, kPlEvery>(s, up, dn, slots, T, k0, step, mom, lane, warp, t, bar);
+        pl_steps<kCfg, kPlEvery>(s, up, dn, slots, T, k0, step, mom, lane, warp, t, bar);
 }
 
 // A thread's place in a tile at (ox, oy).
-template <int kForm>
+template <int kCfg>
 __device__ __forceinline__ PlPlace pl_place(int ox, int oy, int w, int h, int lane, int warp)
 {
-    using G = PlGeo<kForm>;
+    using G = PlGeo<kCfg>;
     const int gx0 = ox + 4 * lane, gy0 = oy + G::kRPT * warp;
     PlPlace t;
     t.xlim = w - 2 - gx0;
@@ -1216,61 +1238,68 @@ __device__ __forceinline__ PlPlace pl_place(int ox, int oy, int w, int h, int la
     t.bot = h - 2 - gy0;
     t.zl = gx0 == 0;
     t.zr = gx0 == w - 4;
-    t.zt = oy == -kTbT && warp == G::kTopWarp;
-    t.zb2 = oy == h - G::kRows + kTbT && warp == G::kBot2Warp;
-    t.zb1 = oy == h - G::kRows + kTbT && warp == G::kBot1Warp;
+    t.zt = oy == -G::kT && warp == G::kTopWarp;
+    t.zb2 = oy == h - G::kRows + G::kT && warp == G::kBot2Warp;
+    t.zb1 = oy == h - G::kRows + G::kT && warp == G::kBot1Warp;
     return t;
 }
 
 // A thread's block out of the staged tile, with the O rows above and below it
 // (zero outside the tile: values the ring never passes on to the interior).
-template <int kForm>
-__device__ __forceinline__ void pl_take(PlState<kForm>& s, float4& up, float4& dn, const float* stage, int k0, int lane,
+template <int kCfg>
+__device__ __forceinline__ void pl_take(PlState<kCfg>& s, float4& up, float4& dn, const float* stage, int k0, int lane,
     int warp)
 {
-    using G = PlGeo<kForm>;
-    const float* base = stage + PlGeo<kForm>::kRPT * warp * kPlW + 4 * lane;
+    using G = PlGeo<kCfg>;
+    const float* base = stage + PlGeo<kCfg>::kRPT * warp * kPlW + 4 * lane;
 #pragma unroll
-    for (int r = 0; r < PlGeo<kForm>::kRPT; ++r) {
+    for (int r = 0; r < PlGeo<kCfg>::kRPT; ++r) {
         const float* row = base + r * kPlW;
         s.o[r] = *reinterpret_cast<const float4*>(row);
         s.u[r] = *reinterpret_cast<const float4*>(row + G::kStage);
         s.nk[r] = *reinterpret_cast<const float4*>(row + 2 * G::kStage);
         s.c[r] = *reinterpret_cast<const float4*>(row + 3 * G::kStage);
+        if constexpr (!PlGeo<kCfg>::kFma)
+            s.a[r] = *reinterpret_cast<const float4*>(row + 4 * G::kStage);
     }
     if (k0 == 0)  // no U yet
 #pragma unroll
-        for (int r = 0; r < PlGeo<kForm>::kRPT; ++r)
+        for (int r = 0; r < PlGeo<kCfg>::kRPT; ++r)
             s.u[r] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
     up = dn = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
     if (warp > 0)
         up = *reinterpret_cast<const float4*>(base - kPlW);
     if (warp < G::kWarps - 1)
-        dn = *reinterpret_cast<const float4*>(base + PlGeo<kForm>::kRPT * kPlW);
+        dn = *reinterpret_cast<const float4*>(base + PlGeo<kCfg>::kRPT * kPlW);
 }
 
 // A thread's interior pixels of O and U into the out staging.
-template <int kForm>
-__device__ __forceinline__ void pl_put(const PlState<kForm>& s, float* so, float* su, int lane, int warp)
+template <int kCfg>
+__device__ __forceinline__ void pl_put(const PlState<kCfg>& s, float* so, float* su, int lane, int warp)
 {
-    const int ix = 4 * lane - kTbT;
-    if (ix < 0 || ix >= kPlIW)
+    using G = PlGeo<kCfg>;
+    const int ix = 4 * lane - G::kT;
+    if (ix < 0 || ix >= G::kIW)
         return;
 #pragma unroll
-    for (int r = 0; r < PlGeo<kForm>::kRPT; ++r) {
-        const int iy = PlGeo<kForm>::kRPT * warp + r - kTbT;
-        if (iy < 0 || iy >= PlGeo<kForm>::kIRows)
+    for (int r = 0; r < PlGeo<kCfg>::kRPT; ++r) {
+        const int iy = PlGeo<kCfg>::kRPT * warp + r - G::kT;
+        if (iy < 0 || iy >= PlGeo<kCfg>::kIRows)
             continue;
-        *reinterpret_cast<float4*>(so + iy * kPlIW + ix) = s.o[r];
-        *reinterpret_cast<float4*>(su + iy * kPlIW + ix) = s.u[r];
+        *reinterpret_cast<float4*>(so + iy * G::kIW + ix) = s.o[r];
+        *reinterpret_cast<float4*>(su + iy * G::kIW + ix) = s.u[r];
     }
 }
 
-int pl_tiles_x(int w) { return (w + kPlIW - 1) / kPlIW; }
-template <int kForm>
+template <int kCfg>
+int pl_tiles_x(int w)
+{
+    return (w + PlGeo<kCfg>::kIW - 1) / PlGeo<kCfg>::kIW;
+}
+template <int kCfg>
 int pl_tiles(int w, int h)
 {
-    return 3 * pl_tiles_x(w) * ((h + PlGeo<kForm>::kIRows - 1) / PlGeo<kForm>::kIRows);
+    return 3 * pl_tiles_x<kCfg>(w) * ((h + PlGeo<kCfg>::kIRows - 1) / PlGeo<kCfg>::kIRows);
 }
 
 __device__ __forceinline__ void tma_load_3d(void* dst, const CUtensorMap* map, int x, int y, int z, uint64_t* bar)
@@ -1318,7 +1347,7 @@ __device__ __forceinline__ void pl_plain_load(float* stage, const PlPlain& p, in
 
 // The plain-load form (widths that are not a multiple of 4 in a caller's
 // workspace, whose planes then have no room for a 16-byte row pitch): one
-// launch per round of up to kTbT steps, each CTA walking the round's tiles
+// launch per round of up to G::kT steps, each CTA walking the round's tiles
 // with plain loads and stores.
 __global__ void __launch_bounds__(32 * PlGeo<kSolverFma>::kWarps, 1)
     solver_fma_plain_kernel(const __grid_constant__ PlPlain pl, int T, int k0, float step, float mom)
@@ -1339,7 +1368,7 @@ __global__ void __launch_bounds__(32 * PlGeo<kSolverFma>::kWarps, 1)
         if (tile + static_cast<int>(gridDim.x) >= pl.ntiles)
             allow_dependent_launch();
         const int c = tile / per_plane, r = tile - c * per_plane;
-        const int ox = (r % pl.tiles_x) * kPlIW - kTbT, oy = (r / pl.tiles_x) * G::kIRows - kTbT;
+        const int ox = (r % pl.tiles_x) * G::kIW - G::kT, oy = (r / pl.tiles_x) * G::kIRows - G::kT;
         const int w = pl.w, h = pl.h;
         __syncthreads();  // the previous tile has left the staging
         pl_plain_load(stage, pl, c, ox, oy);
@@ -1354,8 +1383,8 @@ __global__ void __launch_bounds__(32 * PlGeo<kSolverFma>::kWarps, 1)
         __syncthreads();
         const int64_t base = static_cast<int64_t>(c) * w * h;
         for (int i = threadIdx.x; i < G::kOut; i += blockDim.x) {
-            const int iy = i / kPlIW, ix = i - iy * kPlIW;
-            const int gy = oy + kTbT + iy, gx = ox + kTbT + ix;
+            const int iy = i / G::kIW, ix = i - iy * G::kIW;
+            const int gy = oy + G::kT + iy, gx = ox + G::kT + ix;
             if (gx < w && gy < h) {
                 const int64_t idx = base + pix_index(gx, gy, w);
                 pl.Oo[idx] = so[i];
@@ -1394,15 +1423,17 @@ __global__ void __launch_bounds__(32 * PlGeo<kSolverFma>::kWarps, 1)
 // its nine counters read one after the other, and a finished tile was
 // published at the end of the next one.
 //
-// A tile takes 4.7 us at 1920x1080: 6,500 cycles of steps (4,030 of FP32 issue;
-// the exchange between warps and two warps a scheduler the rest), 2,100 of
-// moving 147 KB out of the staging and 50 KB into the other, 700 of waits.
-// Microseconds per 8-step round before (12 warps of 4 x 6 blocks, unrolled
-// steps, the bookkeeping in warp 0) and now: 1920x1080 38.2 -> 32.8, 3840x2160
-// 144 -> 129, 1280x720 21.5 -> 14.2, 960x540 13.9 -> 11.5, 640x360 12.3 -> 9.8.
-// Two CTAs of 6 warps on 64 x 72 tiles an SM, tried in place of this: 41.3 at
-// 1920x1080.
-enum { kPmO0, kPmO1, kPmU0, kPmU1, kPmK, kPmC, kPmOo0, kPmOo1, kPmUo0, kPmUo1, kPlMaps };
+// An FMA tile takes 4.6 us at 1920x1080: 6,500 cycles of steps (4,030 of FP32
+// issue; the exchange between warps and two warps a scheduler the rest), 2,100
+// of moving 147 KB out of the staging and 50 KB into the other, 700 of waits.
+// Microseconds per 8 steps before (12 warps of 4 x 6 blocks, unrolled steps, the
+// bookkeeping in warp 0) and now: 3840x2160 144 -> 122, 1920x1080 38.2 -> 32.3,
+// 1280x720 21.5 -> 14.2, 960x540 13.9 -> 9.5, 640x360 12.3 -> 6.3.  Two CTAs of
+// 6 warps on 64 x 72 tiles an SM, tried in place of this: 41.3 at 1920x1080.
+// The exact form, before (a launch a round on interleaved images) and now:
+// 3840x2160 256 -> 171, 1920x1080 75.5 -> 45.7, 1280x720 40.3 -> 20.3, 960x540
+// 27.1 -> 12.9, 640x360 18.3 -> 10.2.
+enum { kPmO0, kPmO1, kPmU0, kPmU1, kPmK, kPmC, kPmA, kPmOo0, kPmOo1, kPmUo0, kPmUo1, kPlMaps };
 
 template <int kN>
 struct PlSolve {
@@ -1420,10 +1451,18 @@ struct PlJob {
     int ox, oy, w, h;
 };
 
-template <int kForm, int kN>
+// The moved bottom row of tiles reads two rows of tiles up.
+template <int kCfg>
+__device__ __forceinline__ bool pl_deep(int h, int ty_n)
+{
+    using G = PlGeo<kCfg>;
+    return (kCfg & kPlLong) && ty_n >= 3 && h - (ty_n - 1) * G::kIRows < G::kT;
+}
+
+template <int kCfg, int kN>
 __device__ __forceinline__ PlJob pl_job(const PlSolve<kN>& g, int ticket)
 {
-    using G = PlGeo<kForm>;
+    using G = PlGeo<kCfg>;
     const int N = g.tile0[g.count];
     PlJob j;
     j.k = ticket / N;
@@ -1448,69 +1487,100 @@ __device__ __forceinline__ PlJob pl_job(const PlSolve<kN>& g, int ticket)
     const int r = j.local - j.c * per_plane;
     j.tx = r % g.tiles_x[p];
     j.ty = r / g.tiles_x[p];
-    j.ox = j.tx * kPlIW - kTbT;
-    j.oy = j.ty * G::kIRows - kTbT;
+    j.ox = j.tx * G::kIW - G::kT;
+    j.oy = j.ty * G::kIRows - G::kT;
     j.w = g.w[p];
     j.h = g.h[p];
     // The bottom row of tiles is moved up until its interior ends on the
-    // frame's last row (rows h - 2 and h - 1 then sit in the last but one warp,
-    // rows 2 and 3, where pl_step tests them without per-pixel tests), when its
-    // 8-row top ring still lies in the row of tiles above (the 3 x 3 dependency
-    // holds).  Its interior then overlaps that row's: both compute the shared
-    // rows from the same inputs with the same arithmetic and store the same bits.
+    // frame's last row (rows h - 2 and h - 1 then sit in fixed rows of fixed
+    // warps, where pl_row tests them without per-row tests), when its top ring
+    // still lies in the row of tiles above (the 3 x 3 dependency holds) or, in
+    // long rounds, whose 16-pixel ring reaches further than 40 % of the frames'
+    // last rows of tiles, in the two rows above (pl_watched looks two rows up and
+    // down there).  Its interior then overlaps those rows': both compute the
+    // shared rows from the same inputs with the same arithmetic and store the
+    // same bits.
     const int ty_n = per_plane / g.tiles_x[p];
-    if (j.ty == ty_n - 1 && j.ty > 0 && j.h - j.ty * G::kIRows >= kTbT)
-        j.oy = j.h - G::kRows + kTbT;
+    if (j.ty == ty_n - 1 && j.ty > 0 && (j.h - j.ty * G::kIRows >= G::kT || pl_deep<kCfg>(j.h, ty_n)))
+        j.oy = j.h - G::kRows + G::kT;
     return j;
 }
 
-// the tile's input planes for its round, after its neighbours' stores
-template <int kForm, int kN>
-__device__ __forceinline__ void pl_job_loads(float* stage, const PlSolve<kN>& g, const PlJob& j, uint64_t* bar)
+// A tile's constant planes, which no round writes, and its O and U for its
+// round, after its neighbours' stores; both on one full barrier.
+template <int kCfg, int kN>
+__device__ __forceinline__ void pl_load_constants(float* stage, const PlSolve<kN>& g, const PlJob& j, uint64_t* bar)
 {
-    using G = PlGeo<kForm>;
+    using G = PlGeo<kCfg>;
+    const CUtensorMap* m = g.map[j.p];
+    tma_load_3d(stage + 2 * G::kStage, m + kPmK, j.ox, j.oy, j.c, bar);
+    tma_load_3d(stage + 3 * G::kStage, m + kPmC, j.ox, j.oy, j.c, bar);
+    if (!G::kFma)
+        tma_load_3d(stage + 4 * G::kStage, m + kPmA, j.ox, j.oy, j.c, bar);
+}
+
+template <int kCfg, int kN>
+__device__ __forceinline__ void pl_load_iterate(float* stage, const PlSolve<kN>& g, const PlJob& j, uint64_t* bar)
+{
+    using G = PlGeo<kCfg>;
     asm volatile("fence.proxy.async.global;" ::: "memory");  // the acquired stores, before the async-proxy reads
     const CUtensorMap* m = g.map[j.p];
     const int par = j.k & 1;
-    mbar_expect_tx(bar, G::kPlanes * G::kStageBytes);
     tma_load_3d(stage, m + (par ? kPmO1 : kPmO0), j.ox, j.oy, j.c, bar);
     tma_load_3d(stage + G::kStage, m + (par ? kPmU1 : kPmU0), j.ox, j.oy, j.c, bar);
-    tma_load_3d(stage + 2 * G::kStage, m + kPmK, j.ox, j.oy, j.c, bar);
-    tma_load_3d(stage + 3 * G::kStage, m + kPmC, j.ox, j.oy, j.c, bar);
 }
 
-// Round k - 1 finished on the tile's 3x3 neighbourhood, seen by the whole
-// control warp in one L2 round trip: lanes 0..8 each read one neighbour's
-// counter (relaxed; a lane without a neighbour, or a job that waits for
-// nothing, counts as finished).  A yes is followed by an acquire fence in the
-// lanes that read the counters and a warp barrier, which order the counters'
-// published stores before the warp's later accesses (lane 0's TMA loads).
-template <int kN>
-__device__ __forceinline__ bool pl_deps(const PlSolve<kN>& g, const PlJob& j, int lane)
+// A job waits for round k - 1 of the tile's 3x3 neighbourhood and, where the
+// bottom row of tiles reads two rows up, of the tiles it reads there, whose
+// writers wait for it in turn.  Lanes 0..8, 9..11 of the loading warp each
+// watch one counter (null: none to watch).
+template <int kCfg, int kN>
+__device__ __forceinline__ const unsigned* pl_watched(const PlSolve<kN>& g, const PlJob& j, int lane)
+{
+    if (j.k == 0 || lane >= (kCfg & kPlLong ? 12 : 9))
+        return nullptr;
+    const int tx_n = g.tiles_x[j.p];
+    const int per_plane = (g.tile0[j.p + 1] - g.tile0[j.p]) / 3;
+    const int ty_n = per_plane / tx_n;
+    const int x = j.tx + lane % 3 - 1;
+    int y = j.ty + lane / 3 - 1;
+    if (lane >= 9)
+        y = !pl_deep<kCfg>(j.h, ty_n) ? -1 : j.ty == ty_n - 1 ? ty_n - 3 : j.ty == ty_n - 3 ? ty_n - 1 : -1;
+    return x >= 0 && x < tx_n && y >= 0 && y < ty_n ? g.done[j.p] + j.c * per_plane + y * tx_n + x : nullptr;
+}
+
+// One look by the whole warp, an L2 round trip: the acquiring loads and the
+// warp barrier order the counters' published stores before the warp's later
+// accesses (lane 0's TMA loads).
+__device__ __forceinline__ bool pl_look(const unsigned* f, int k)
 {
     unsigned v = ~0u;
-    if (j.k > 0 && lane < 9) {
-        const int tx_n = g.tiles_x[j.p];
-        const int per_plane = (g.tile0[j.p + 1] - g.tile0[j.p]) / 3;
-        const int ty_n = per_plane / tx_n;
-        const int x = j.tx + lane % 3 - 1, y = j.ty + lane / 3 - 1;
-        if (x >= 0 && x < tx_n && y >= 0 && y < ty_n)
-            asm volatile("ld.relaxed.gpu.global.u32 %0, [%1];"
-                         : "=r"(v)
-                         : "l"(g.done[j.p] + j.c * per_plane + y * tx_n + x)
-                         : "memory");
-    }
-    const bool ok = __all_sync(0xffffffffu, v >= static_cast<unsigned>(j.k));
-    if (ok) {
-        asm volatile("fence.acq_rel.gpu;" ::: "memory");
-        __syncwarp();
-    }
+    if (f)
+        asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(f) : "memory");
+    const bool ok = __all_sync(0xffffffffu, v >= static_cast<unsigned>(k));
+    __syncwarp();
     return ok;
 }
 
 __device__ __forceinline__ void st_release_u32(unsigned* p, unsigned v)
 {
     asm volatile("st.release.gpu.global.u32 [%0], %1;" ::"l"(p), "r"(v) : "memory");
+}
+
+// one look at a phase, without waiting
+__device__ __forceinline__ bool mbar_test(uint64_t* bar, uint32_t parity)
+{
+    uint32_t ok;
+    asm volatile(
+        "{\n"
+        " .reg .pred p;\n"
+        " mbarrier.test_wait.parity.shared::cta.b64 p, [%1], %2;\n"
+        " selp.u32 %0, 1, 0, p;\n"
+        "}\n"
+        : "=r"(ok)
+        : "r"(smem_u32(bar)), "r"(parity)
+        : "memory");
+    return ok != 0;
 }
 
 __device__ __forceinline__ void mbar_arrive(uint64_t* bar)
@@ -1545,16 +1615,16 @@ __device__ __forceinline__ bool pl_wait(uint64_t* bar, uint32_t parity, volatile
 // The block: the compute warps and one warpgroup whose first two warps control
 // (registers are handed out per warpgroup).  All start with 168 registers a
 // thread; the control group gives up what the compute warps need beyond that
-// (setmaxnreg: 256 x 216 + 128 x 72 = 384 x 168).
-constexpr int kPlStartRegs = 168, kPlComputeRegs = 216, kPlControlRegs = 72;
+// (setmaxnreg: 256 x 216 + 128 x 72 = 256 x 224 + 128 x 56 = 384 x 168).
+constexpr int kPlStartRegs = 168;
 
-template <int kForm, int kN>
-__global__ void __launch_bounds__(32 * (PlGeo<kForm>::kWarps + 4), 1)
+template <int kCfg, int kN>
+__global__ void __launch_bounds__(32 * (PlGeo<kCfg>::kWarps + 4), 1)
     solver_solve_kernel(const __grid_constant__ PlSolve<kN> g, float step, float mom)
 {
-    using G = PlGeo<kForm>;
+    using G = PlGeo<kCfg>;
     static_assert(G::kWarps % 4 == 0 &&
-            G::kWarps * kPlComputeRegs + 4 * kPlControlRegs <= (G::kWarps + 4) * kPlStartRegs &&
+            G::kWarps * G::kComputeRegs + 4 * G::kControlRegs <= (G::kWarps + 4) * kPlStartRegs &&
             32 * (G::kWarps + 4) * kPlStartRegs <= 65536,
         "the warpgroups' registers within the block's");
     extern __shared__ __align__(128) unsigned char smem_raw[];
@@ -1586,7 +1656,7 @@ __global__ void __launch_bounds__(32 * (PlGeo<kForm>::kWarps + 4), 1)
     grid_dependency_wait();
 
     if (warp >= G::kWarps) {
-        asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(kPlControlRegs));
+        asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(G::kControlRegs));
         if (warp == G::kWarps) {
             // ---- loading warp ---------------------------------------------------------
             const int total = g.tile0[g.count] * g.nround;
@@ -1597,14 +1667,19 @@ __global__ void __launch_bounds__(32 * (PlGeo<kForm>::kWarps + 4), 1)
                 ticket = __shfl_sync(0xffffffffu, ticket, 0);
                 const bool valid = ticket < total;
                 PlJob j{};
+                const unsigned* watched = nullptr;
+                bool ready = true;
                 if (valid) {
-                    j = pl_job<kForm>(g, ticket);
-                    int spins = 0;
-                    bool ready;
-                    while (!(ready = pl_deps(g, j, lane)) && ++spins < kWaitSpins && !s_abort)
-                        __nanosleep(20);
-                    if (!ready && lane == 0)
-                        s_abort = 1;
+                    j = pl_job<kCfg>(g, ticket);
+                    // look at the neighbours until they are done or the staging is free
+                    watched = pl_watched<kCfg>(g, j, lane);
+                    ready = pl_look(watched, j.k);
+                    for (int spins = 0; !ready && spins < kWaitSpins && !s_abort; ++spins) {
+                        const bool free = i == 0 || mbar_test(empty_in, (i - 1) & 1);
+                        if (__shfl_sync(0xffffffffu, static_cast<int>(free), 0))
+                            break;
+                        ready = pl_look(watched, j.k);
+                    }
                 }
                 if (lane == 0) {
                     if (i > 0)
@@ -1615,9 +1690,9 @@ __global__ void __launch_bounds__(32 * (PlGeo<kForm>::kWarps + 4), 1)
                         t.oy = j.oy;
                         t.w = j.w;
                         t.h = j.h;
-                        t.k0 = j.k * kTbT;
-                        t.T = min(kTbT, g.num_iter - t.k0);
-                        t.mode = pl_mode<kForm>(j.ox, j.oy, j.w, j.h);
+                        t.k0 = j.k * G::kT;
+                        t.T = min(G::kT, g.num_iter - t.k0);
+                        t.mode = pl_mode<kCfg>(j.ox, j.oy, j.w, j.h);
                         t.k = j.k;
                         t.p = j.p;
                         t.c = j.c;
@@ -1628,13 +1703,30 @@ __global__ void __launch_bounds__(32 * (PlGeo<kForm>::kWarps + 4), 1)
                     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
                     ++phases;
                     if (t.valid) {
-                        pl_job_loads<kForm>(stage, g, j, full_in);
-                        ticket = static_cast<int>(atomicAdd(g.ticket, 1u));
+                        mbar_expect_tx(full_in, G::kPlanes * G::kStageBytes);
+                        if (ready)
+                            pl_load_iterate<kCfg>(stage, g, j, full_in);
+                        pl_load_constants<kCfg>(stage, g, j, full_in);
                     } else {
                         mbar_arrive(full_in);
                     }
                 }
                 __syncwarp();
+                if (!valid || s_abort)
+                    break;
+                if (!ready) {
+                    // late neighbours: the constants are on their way meanwhile
+                    for (int spins = 0; !ready && spins < kWaitSpins && !s_abort; ++spins)
+                        ready = pl_look(watched, j.k);
+                    if (lane == 0) {
+                        if (!ready)
+                            s_abort = 1;
+                        pl_load_iterate<kCfg>(stage, g, j, full_in);  // also when giving up: the phase completes
+                    }
+                    __syncwarp();
+                }
+                if (lane == 0)
+                    ticket = static_cast<int>(atomicAdd(g.ticket, 1u));
                 if (!valid || s_abort)
                     break;
             }
@@ -1652,8 +1744,8 @@ __global__ void __launch_bounds__(32 * (PlGeo<kForm>::kWarps + 4), 1)
                     break;
                 const CUtensorMap* m = g.map[t.p];
                 const int par = (t.k + 1) & 1;
-                tma_store_3d(m + (par ? kPmOo1 : kPmOo0), t.ox + kTbT, t.oy + kTbT, t.c, so);
-                tma_store_3d(m + (par ? kPmUo1 : kPmUo0), t.ox + kTbT, t.oy + kTbT, t.c, su);
+                tma_store_3d(m + (par ? kPmOo1 : kPmOo0), t.ox + G::kT, t.oy + G::kT, t.c, so);
+                tma_store_3d(m + (par ? kPmUo1 : kPmUo0), t.ox + G::kT, t.oy + G::kT, t.c, su);
                 bulk_commit();
                 // publish: the release store orders the completed async-proxy writes,
                 // brought into the generic proxy by the proxy fence, before the counter
@@ -1667,7 +1759,7 @@ __global__ void __launch_bounds__(32 * (PlGeo<kForm>::kWarps + 4), 1)
     }
 
     // ---- compute warps --------------------------------------------------------------------
-    asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(kPlComputeRegs));
+    asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(G::kComputeRegs));
     bool ok = true;
     for (int i = 0;; ++i) {
         ok = pl_wait(full_in, i & 1, &s_abort) && ok;
@@ -1691,18 +1783,18 @@ __global__ void __launch_bounds__(32 * (PlGeo<kForm>::kWarps + 4), 1)
             break;
         }
         const int T = t.T, k0 = t.k0, mode = t.mode;
-        const PlPlace place = pl_place<kForm>(t.ox, t.oy, t.w, t.h, lane, warp);
-        PlState<kForm> s;
+        const PlPlace place = pl_place<kCfg>(t.ox, t.oy, t.w, t.h, lane, warp);
+        PlState<kCfg> s;
         float4 up, dn;
-        pl_take<kForm>(s, up, dn, stage, k0, lane, warp);
+        pl_take<kCfg>(s, up, dn, stage, k0, lane, warp);
         __syncwarp();
         if (lane == 0)
             mbar_arrive(empty_in);
-        pl_round<kForm>(mode, s, up, dn, slots, T, k0, step, mom, lane, warp, place,
+        pl_round<kCfg>(mode, s, up, dn, slots, T, k0, step, mom, lane, warp, place,
             [] { asm volatile("barrier.cta.sync 1, %0;" ::"n"(32 * G::kWarps) : "memory"); });
         if (i > 0)
             ok = pl_wait(empty_out, (i - 1) & 1, &s_abort);
-        pl_put<kForm>(s, so, su, lane, warp);
+        pl_put<kCfg>(s, so, su, lane, warp);
         asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
         __syncwarp();
         if (lane == 0)
@@ -1760,9 +1852,8 @@ template <int kN>
 bool set_group_smem()
 {
     constexpr auto kAttr = cudaFuncAttributeMaxDynamicSharedMemorySize;
-    return cudaFuncSetAttribute(solver_persistent_kernel<kN>, kAttr, kPsSmem) == cudaSuccess &&
-           cudaFuncSetAttribute(solver_tall_kernel<kN>, kAttr, kPSmem) == cudaSuccess &&
-           cudaFuncSetAttribute(solver_solve_kernel<kSolverFma, kN>, kAttr, PlGeo<kSolverFma>::kSmem) == cudaSuccess;
+    return cudaFuncSetAttribute(solver_solve_kernel<kSolverFma, kN>, kAttr, PlGeo<kSolverFma>::kSmem) == cudaSuccess &&
+           cudaFuncSetAttribute(solver_solve_kernel<kSolverExact, kN>, kAttr, PlGeo<kSolverExact>::kSmem) == cudaSuccess;
 }
 
 struct DeviceInfo {
@@ -1791,7 +1882,14 @@ cudaError_t device_info(DeviceInfo** out)
         if ((e = cudaFuncSetAttribute(solver_tb_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kTbSmem)) !=
             cudaSuccess)
             return e;
-        d.ps_smem = set_group_smem<1>() && set_group_smem<4>() && set_group_smem<kGroupMax>() &&
+        constexpr auto kAttr = cudaFuncAttributeMaxDynamicSharedMemorySize;
+        d.ps_smem = cudaFuncSetAttribute(solver_solve_kernel<kSolverFma | kPlLong, 1>, kAttr,
+                        PlGeo<kSolverFma | kPlLong>::kSmem) == cudaSuccess &&
+                    cudaFuncSetAttribute(solver_solve_kernel<kSolverExact | kPlLong, 1>, kAttr,
+                        PlGeo<kSolverExact | kPlLong>::kSmem) == cudaSuccess &&
+                    cudaFuncSetAttribute(solver_persistent_kernel, kAttr, kPsSmem) == cudaSuccess &&
+                    cudaFuncSetAttribute(solver_tall_kernel, kAttr, kPSmem) == cudaSuccess &&
+                    set_group_smem<1>() && set_group_smem<4>() && set_group_smem<kGroupMax>() &&
                     cudaFuncSetAttribute(solver_fma_plain_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                         PlGeo<kSolverFma>::kSmem) == cudaSuccess;
         cudaGetLastError();
@@ -1803,17 +1901,16 @@ cudaError_t device_info(DeviceInfo** out)
 bool aligned16p(const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15) == 0; }
 
 // ---- tile-shape autotuner ------------------------------------------------------------
-// The two persistent kernels of the exact form (64 x 32 and 64 x 48 tiles)
-// give the same results bit for bit; which is faster depends on how their
-// tiles fill the waves of one tile per SM.  solver_group_autotune times both
-// on scratch images of the sizes one launch solves (one image, or one image
-// per stream of a multi-stream step) and keeps the faster per (device, form,
-// sizes); sizes never tuned use a wave model: a 64 x 48 tile costs about 1.91
+// The two persistent kernels of the exact form on interleaved images (64 x 32
+// and 64 x 48 tiles) give the same results bit for bit; which is faster depends
+// on how their tiles fill the waves of one tile per SM.  solver_autotune times
+// both on scratch images of a size and keeps the faster per (device, form,
+// size); sizes never tuned use a wave model: a 64 x 48 tile costs about 1.91
 // times a 64 x 32 one (GB300, 1920x1080 and 960x540).  The FMA form has one
 // shape, 128 x 72 pixels of one channel plane.
 struct ShapeTable {
     std::mutex mu;
-    std::map<std::vector<int>, int> rows;  // {device, form, w0, h0, w1, h1, ...} -> tile rows
+    std::map<std::tuple<int, int, int, int>, int> rows;  // {device, form, w, h} -> tile rows
     bool enabled = true;
 };
 ShapeTable& shape_table()
@@ -1822,39 +1919,25 @@ ShapeTable& shape_table()
     return t;
 }
 
-std::vector<int> shape_key(int dev, const int* w, const int* h, int n, int form)
-{
-    std::vector<int> k{dev, form};
-    for (int i = 0; i < n; ++i) {
-        k.push_back(w[i]);
-        k.push_back(h[i]);
-    }
-    return k;
-}
-
 int tiles_of(int w, int h, int ir) { return ((w + kIW - 1) / kIW) * ((h + ir - 1) / ir); }
 
-int model_rows(const int* w, const int* h, int n, int sms, int form)
+int model_rows(int w, int h, int sms, int form)
 {
     if (form == kSolverFma)
         return PlGeo<kSolverFma>::kRows;
-    int64_t n_short = 0, n_tall = 0;
-    for (int i = 0; i < n; ++i) {
-        n_short += tiles_of(w[i], h[i], kIH);
-        n_tall += tiles_of(w[i], h[i], kPIH);
-    }
+    const int n_short = tiles_of(w, h, kIH), n_tall = tiles_of(w, h, kPIH);
     return 1.91 * ((n_tall + sms - 1) / sms) < 1.0 * ((n_short + sms - 1) / sms) ? kPEY : kTbEY;
 }
 
-// the tile rows a launch over these sizes uses on the current device: tuned, else the model
-int chosen_rows(int dev, const int* w, const int* h, int n, int sms, int form, bool* tuned = nullptr)
+// the tile rows a launch at this size uses on the current device: tuned, else the model
+int chosen_rows(int dev, int w, int h, int sms, int form, bool* tuned = nullptr)
 {
     ShapeTable& t = shape_table();
     std::lock_guard<std::mutex> lock(t.mu);
-    auto it = t.rows.find(shape_key(dev, w, h, n, form));
+    auto it = t.rows.find({dev, form, w, h});
     if (tuned)
         *tuned = it != t.rows.end();
-    return it != t.rows.end() ? it->second : model_rows(w, h, n, sms, form);
+    return it != t.rows.end() ? it->second : model_rows(w, h, sms, form);
 }
 
 int interior_rows(int rows) { return rows - 2 * kTbT; }
@@ -1895,34 +1978,11 @@ bool encode_plane_map(CUtensorMap* m, const float* base, int w, int h, int pitch
                CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
 
-// problem p of a launch: launch li of the solve reads O[c] and U[li & 1] and
-// writes O[c ^ 1] and U[(li + 1) & 1]
-template <int kN>
-void group_set(SolverGroup<kN>& g, int p, const SolveMaps& m, int c, int li, int w, int h, int rows, uint8_t* rgba)
-{
-    g.map[p][kMapO] = m.O[c];
-    g.map[p][kMapU] = m.U[li & 1];
-    g.map[p][kMapA] = m.A;
-    g.map[p][kMapW] = m.W;
-    g.map[p][kMapL] = m.L;
-    g.map[p][kMapOo] = m.Oo[c ^ 1];
-    g.map[p][kMapUo] = m.Uo[(li + 1) & 1];
-    g.w[p] = w;
-    g.h[p] = h;
-    g.tiles_x[p] = (w + kIW - 1) / kIW;
-    g.rgba[p] = rgba;
-    if (p == 0)
-        g.tile0[0] = 0;
-    g.tile0[p + 1] = g.tile0[p] + tiles_of(w, h, interior_rows(rows));
-    g.count = p + 1;
-}
-
-// One launch of a persistent kernel of the exact form (`rows`-row tiles)
-// over a group's tiles, with programmatic dependent launch on the previous
-// launch of the stream.
-template <int kN>
-cudaError_t launch_group(int rows, const SolverGroup<kN>& g, int T, int k0, float step, float mom, int sms,
-    cudaStream_t st)
+// Steps k_first .. num_iter - 1 of a solve in launches of T <= kTbT steps of a
+// persistent kernel (`rows`-row tiles) with programmatic dependent launch.
+// Launch li reads O[c0 ^ (li & 1)] and U[li & 1] and writes the others.
+cudaError_t launch_rounds(const SolveMaps& m, int w, int h, int c0, uint8_t* rgba, int rows, int num_iter, float step,
+    float mom, int sms, cudaStream_t st, int* nl, int k_first = 0)
 {
     cudaLaunchConfig_t cfg = {};
     cudaLaunchAttribute attr[1];
@@ -1931,45 +1991,35 @@ cudaError_t launch_group(int rows, const SolverGroup<kN>& g, int T, int k0, floa
     cfg.stream = st;
     cfg.attrs = attr;
     cfg.numAttrs = 1;
-    cfg.gridDim = dim3(std::min(g.tile0[g.count], sms));
-    if (rows == kPEY) {
-        cfg.blockDim = dim3(kPThreads);
-        cfg.dynamicSmemBytes = kPSmem;
-        return cudaLaunchKernelEx(&cfg, solver_tall_kernel<kN>, g, T, k0, step, mom);
-    }
-    cfg.blockDim = dim3(32, kTbEY / 2);
-    cfg.dynamicSmemBytes = kPsSmem;
-    return cudaLaunchKernelEx(&cfg, solver_persistent_kernel<kN>, g, T, k0, step, mom);
-}
-
-// One image of a grouped solve: its maps and where its iterate starts.
-struct GroupMember {
-    SolveMaps maps;
-    int w, h, c0;  // c0: the ping-pong buffer the first launch reads
-    uint8_t* rgba;
-};
-
-// Steps k_first .. num_iter - 1 of a solve over all members, in launches of
-// T <= kTbT steps, kN problems per launch.
-template <int kN>
-cudaError_t launch_members(const std::vector<GroupMember>& mem, int rows, int num_iter, float step, float mom,
-    int sms, cudaStream_t st, int* nl, int k_first = 0)
-{
+    SolverLaunch g{};
+    g.map[kMapA] = m.A;
+    g.map[kMapW] = m.W;
+    g.map[kMapL] = m.L;
+    g.w = w;
+    g.h = h;
+    g.tiles_x = (w + kIW - 1) / kIW;
+    g.tiles = tiles_of(w, h, interior_rows(rows));
+    cfg.gridDim = dim3(std::min(g.tiles, sms));
     const int nlaunch = (num_iter - k_first + kTbT - 1) / kTbT;
-    SolverGroup<kN> g{};
     cudaError_t e = cudaSuccess;
     int k0 = k_first;
     for (int li = 0; li < nlaunch && e == cudaSuccess; ++li) {
-        const int T = std::min(kTbT, num_iter - k0);
-        for (size_t b = 0; b < mem.size() && e == cudaSuccess; b += kN) {
-            const int cnt = static_cast<int>(std::min(mem.size() - b, static_cast<size_t>(kN)));
-            for (int p = 0; p < cnt; ++p) {
-                const GroupMember& m = mem[b + p];
-                group_set(g, p, m.maps, m.c0 ^ (li & 1), li, m.w, m.h, rows, li == nlaunch - 1 ? m.rgba : nullptr);
-            }
-            e = launch_group(rows, g, T, k0, step, mom, sms, st);
-            ++*nl;
+        const int T = std::min(kTbT, num_iter - k0), c = c0 ^ (li & 1);
+        g.map[kMapO] = m.O[c];
+        g.map[kMapU] = m.U[li & 1];
+        g.map[kMapOo] = m.Oo[c ^ 1];
+        g.map[kMapUo] = m.Uo[(li + 1) & 1];
+        g.rgba = li == nlaunch - 1 ? rgba : nullptr;
+        if (rows == kPEY) {
+            cfg.blockDim = dim3(kPThreads);
+            cfg.dynamicSmemBytes = kPSmem;
+            e = cudaLaunchKernelEx(&cfg, solver_tall_kernel, g, T, k0, step, mom);
+        } else {
+            cfg.blockDim = dim3(32, kTbEY / 2);
+            cfg.dynamicSmemBytes = kPsSmem;
+            e = cudaLaunchKernelEx(&cfg, solver_persistent_kernel, g, T, k0, step, mom);
         }
+        ++*nl;
         k0 += T;
     }
     return e;
@@ -1986,18 +2036,16 @@ void solver_set_autotune(bool on)
         t.rows.clear();
 }
 
-int solver_group_tile_rows(const int* w, const int* h, int n, bool* tuned, int form)
+int solver_tile_rows(int w, int h, bool* tuned, int form)
 {
     int dev = 0;
     DeviceInfo* di = nullptr;
-    if (n < 1 || cudaGetDevice(&dev) != cudaSuccess || device_info(&di) != cudaSuccess)
+    if (cudaGetDevice(&dev) != cudaSuccess || device_info(&di) != cudaSuccess)
         return 0;
-    return chosen_rows(dev, w, h, n, di->sms, form, tuned);
+    return chosen_rows(dev, w, h, di->sms, form, tuned);
 }
 
-int solver_tile_rows(int w, int h, bool* tuned, int form) { return solver_group_tile_rows(&w, &h, 1, tuned, form); }
-
-cudaError_t solver_group_autotune(const int* w, const int* h, int n, cudaStream_t st, int* rows_out, int form)
+cudaError_t solver_autotune(int w, int h, cudaStream_t st, int* rows_out, int form)
 {
     DeviceInfo* di = nullptr;
     int dev = 0;
@@ -2006,27 +2054,22 @@ cudaError_t solver_group_autotune(const int* w, const int* h, int n, cudaStream_
         e = device_info(&di);
     if (e != cudaSuccess)
         return e;
-    if (n < 1)
-        return cudaErrorInvalidValue;
-    bool eligible = di->ps_smem && form != kSolverFma;  // the FMA form has one shape
-    size_t total = 0;  // floats of one image per member, 16-byte multiples
-    for (int i = 0; i < n; ++i) {
-        eligible = eligible && (w[i] % 4) == 0 && w[i] >= 1 && h[i] >= 1;
-        total += static_cast<size_t>(w[i]) * h[i] * 3;
-    }
+    // the FMA form has one shape
+    const bool eligible = di->ps_smem && form != kSolverFma && w % 4 == 0 && w >= 1 && h >= 1;
+    const size_t total = static_cast<size_t>(w) * h * 3;
     ShapeTable& t = shape_table();
-    const std::vector<int> key = shape_key(dev, w, h, n, form);
+    const std::tuple<int, int, int, int> key{dev, form, w, h};
     {
         std::lock_guard<std::mutex> lock(t.mu);
         auto it = t.rows.find(key);
         if (it != t.rows.end() || !t.enabled || !eligible) {
             if (rows_out)
-                *rows_out = it != t.rows.end() ? it->second : model_rows(w, h, n, di->sms, form);
+                *rows_out = it != t.rows.end() ? it->second : model_rows(w, h, di->sms, form);
             return cudaSuccess;
         }
     }
     // scratch images (zeros; the kernels have no data-dependent control flow):
-    // per member O, O2, U0, U1, A, Wt, lap P
+    // O, O2, U0, U1, A, Wt, lap P
     float* buf = nullptr;
     if ((e = cudaMalloc(&buf, 7 * total * sizeof(float))) != cudaSuccess)
         return e;
@@ -2038,42 +2081,28 @@ cudaError_t solver_group_autotune(const int* w, const int* h, int n, cudaStream_
     cudaEvent_t ev[2] = {};
     float best_ms[2] = {1e30f, 1e30f};
     const int shapes[2] = {kTbEY, kPEY};
-    std::vector<GroupMember> mem[2];
+    SolveMaps maps[2];
     e = cudaMemsetAsync(buf, 0, 7 * total * sizeof(float), st);
     for (int i = 0; i < 2 && e == cudaSuccess; ++i)
         e = cudaEventCreate(&ev[i]);
     for (int s = 0; s < 2 && e == cudaSuccess; ++s) {
-        size_t off = 0;
-        for (int i = 0; i < n && e == cudaSuccess; ++i) {
-            float* im[7];
-            for (int k = 0; k < 7; ++k)
-                im[k] = buf + k * total + off;
-            off += static_cast<size_t>(w[i]) * h[i] * 3;
-            GroupMember m{};
-            float* const O[2] = {im[0], im[1]};
-            float* const U[2] = {im[2], im[3]};
-            if (!encode_solve(&m.maps, O, U, im[4], im[5], im[6], w[i], h[i], shapes[s]))
-                e = cudaErrorInvalidValue;
-            m.w = w[i];
-            m.h = h[i];
-            mem[s].push_back(m);
-        }
+        float* const O[2] = {buf, buf + total};
+        float* const U[2] = {buf + 2 * total, buf + 3 * total};
+        if (!encode_solve(&maps[s], O, U, buf + 4 * total, buf + 5 * total, buf + 6 * total, w, h, shapes[s]))
+            e = cudaErrorInvalidValue;
     }
-    // the kernel instantiation the solves will use: one problem, up to 4, up to 16 per launch
-    auto launch = [&](const std::vector<GroupMember>& m, int rows, int num_iter, int* nl) {
-        return n == 1 ? launch_members<1>(m, rows, num_iter, 0.15f, 0.15f, di->sms, st, nl, kTbT)
-             : n <= 4 ? launch_members<4>(m, rows, num_iter, 0.15f, 0.15f, di->sms, st, nl, kTbT)
-                      : launch_members<kGroupMax>(m, rows, num_iter, 0.15f, 0.15f, di->sms, st, nl, kTbT);
+    auto launch = [&](int s, int num_iter, int* nl) {
+        return launch_rounds(maps[s], w, h, 0, nullptr, shapes[s], num_iter, 0.15f, 0.15f, di->sms, st, nl, kTbT);
     };
     for (int round = 0; round < 5 && e == cudaSuccess; ++round) {
         for (int s = 0; s < 2 && e == cudaSuccess; ++s) {
             int nl = 0;
             // a warm-up launch, then four timed ones, all of kTbT steps with momentum
-            e = launch(mem[s], shapes[s], 2 * kTbT, &nl);
+            e = launch(s, 2 * kTbT, &nl);
             if (e == cudaSuccess)
                 e = cudaEventRecord(ev[0], st);
             if (e == cudaSuccess)
-                e = launch(mem[s], shapes[s], 5 * kTbT, &nl);
+                e = launch(s, 5 * kTbT, &nl);
             float ms = 0.0f;
             if (e == cudaSuccess)
                 e = cudaEventRecord(ev[1], st);
@@ -2102,33 +2131,38 @@ cudaError_t solver_group_autotune(const int* w, const int* h, int n, cudaStream_
     return cudaSuccess;
 }
 
-cudaError_t solver_autotune(int w, int h, cudaStream_t st, int* rows_out, int form)
-{
-    return solver_group_autotune(&w, &h, 1, st, rows_out, form);
-}
-
-// The FMA form's workspace ends in the solve kernel's counters: the ticket,
+// A workspace of planes ends in the solve kernel's counters: the ticket,
 // padding to 64 bytes, one finished-round counter per tile; rounded up to
 // 256 bytes so that a workspace placed after it stays aligned.
-int pl_counter_floats(int w, int h) { return (16 + pl_tiles<kSolverFma>(w, h) + 63) / 64 * 64; }
+int pl_tiles_of(int w, int h, int cfg)
+{
+    switch (cfg) {
+        case kSolverFma: return pl_tiles<kSolverFma>(w, h);
+        case kSolverFma | kPlLong: return pl_tiles<kSolverFma | kPlLong>(w, h);
+        case kSolverExact | kPlLong: return pl_tiles<kSolverExact | kPlLong>(w, h);
+        default: return pl_tiles<kSolverExact>(w, h);
+    }
+}
+int pl_counter_floats(int w, int h, int cfg) { return (16 + pl_tiles_of(w, h, cfg) + 63) / 64 * 64; }
 
 // A plane's row in floats where the workspace has room for rows on the 16-byte
 // grid (TMA's), whatever the width.
-// 854x480, 150 steps: 218 us; with plain loads, which a tile's steps wait for,
-// and a launch a round 542 us.
+// 854x480, FMA form, 150 steps: 218 us; with plain loads, which a tile's steps
+// wait for, and a launch a round 542 us.
 int pl_pitch(int w) { return (w + 3) & ~3; }
+
+// planes-images of a form: O, U (two each) and its constants
+constexpr int pl_images(int form) { return form == kSolverFma ? 6 : 7; }
 
 size_t solver_workspace_floats(int w, int h, int form)
 {
     const size_t img = static_cast<size_t>(w) * h * 3;
-    return form == kSolverFma ? 6 * img + pl_counter_floats(w, h) : 4 * img;
+    return form == kSolverFma ? 6 * img + pl_counter_floats(w, h, form) : 4 * img;
 }
 
 size_t solver_workspace_full_floats(int w, int h, int form)
 {
-    if (form != kSolverFma)
-        return solver_workspace_floats(w, h, form);
-    return 6 * static_cast<size_t>(pl_pitch(w)) * h * 3 + pl_counter_floats(w, h);
+    return pl_images(form) * static_cast<size_t>(pl_pitch(w)) * h * 3 + pl_counter_floats(w, h, form | kPlLong);
 }
 
 size_t solver_workspace_any_floats(int w, int h)
@@ -2140,9 +2174,8 @@ int solver_steps_per_launch() { return kTbT; }
 
 namespace {
 
-// launches of a solve, and the buffer its iterate starts in so that the last
-// launch writes O: O itself for an even count, the second buffer otherwise
-int solve_launches(int num_iter) { return num_iter > 0 ? (num_iter + kTbT - 1) / kTbT : 0; }
+// rounds of a solve
+int solve_launches(int num_iter, int steps = kTbT) { return num_iter > 0 ? (num_iter + steps - 1) / steps : 0; }
 
 struct WsView {
     float *L, *U0, *U1, *O2;
@@ -2153,18 +2186,19 @@ WsView ws_view(float* ws, int w, int h)
     return WsView{ws, ws + n, ws + 2 * n, ws + 3 * n};
 }
 
-// The FMA form's workspace: six planar images (three planes of h rows of
-// `pitch` floats each), then the solve kernel's counters.
+// A form's workspace of planes: its planar images (three planes of h rows of
+// `pitch` floats each; A: the exact form's only), then the solve kernel's counters.
 struct PlWs {
-    float *C, *K, *U[2], *O[2];
+    float *C, *K, *U[2], *O[2], *A;
     unsigned* cnt;
     int ncnt, pitch;
 };
-PlWs pl_view(float* ws, int w, int h, int pitch)
+PlWs pl_view(float* ws, int w, int h, int pitch, int cfg)
 {
+    const int form = cfg & 1;
     const size_t n = static_cast<size_t>(pitch) * h * 3;
-    return PlWs{ws, ws + n, {ws + 2 * n, ws + 3 * n}, {ws + 4 * n, ws + 5 * n},
-        reinterpret_cast<unsigned*>(ws + 6 * n), pl_counter_floats(w, h), pitch};
+    return PlWs{ws, ws + n, {ws + 2 * n, ws + 3 * n}, {ws + 4 * n, ws + 5 * n}, ws + 6 * n,
+        reinterpret_cast<unsigned*>(ws + pl_images(form) * n), pl_counter_floats(w, h, cfg), pitch};
 }
 
 bool tma_eligible(const DeviceInfo* di, int w, const float* O, const WsView& v, const float* A, const float* Wt)
@@ -2173,12 +2207,34 @@ bool tma_eligible(const DeviceInfo* di, int w, const float* O, const WsView& v, 
            aligned16p(v.U1) && aligned16p(A) && aligned16p(Wt) && aligned16p(v.L);
 }
 
-// A solve in planes of rows on the 16-byte grid: a 16-byte aligned workspace of
-// solver_workspace_full_floats (for a width that is a multiple of 4 the same
-// as solver_workspace_floats).
-bool pl_tma_eligible(const DeviceInfo* di, int w, int h, const float* ws, size_t ws_floats)
+// A solve in planes of rows on the 16-byte grid: a 16-byte aligned workspace with
+// room for them and for the counters of cfg's tiles.
+bool pl_tma_eligible(const DeviceInfo* di, int w, int h, const float* ws, size_t ws_floats, int cfg)
 {
-    return di->ps_smem && aligned16p(ws) && ws_floats >= solver_workspace_full_floats(w, h, kSolverFma);
+    const size_t planes = pl_images(cfg & 1) * static_cast<size_t>(pl_pitch(w)) * h * 3;
+    return di->ps_smem && aligned16p(ws) && ws_floats >= planes + pl_counter_floats(w, h, cfg);
+}
+
+// Rounds of 16 steps where a solve's rounds are chains of waits (for the
+// neighbours' stores, counters and loads: about 5 us) rather than work.  A ring
+// of 16 pixels leaves 42 % of an FMA tile as interior (exact form 37 %) against
+// 68 % (66 %) with 8, so only while an SM has at most 2.5 (FMA form) or one
+// (exact form) of a long round's tiles.  150 steps, 8-step and 16-step rounds:
+// FMA 320x180 166 and 118 us, 640x360 181 and 136, 854x480 197 and 179, 960x540
+// 220 and 218; exact 320x180 188 and 142, 480x270 194 and 171, 640x360 205 and 209.
+bool pl_long_rounds(const DeviceInfo* di, int w, int h, int num_iter, int form)
+{
+    const int tiles = pl_tiles_of(w, h, form | kPlLong);
+    return num_iter > kTbT && 2 * tiles <= (form == kSolverFma ? 5 : 2) * di->sms;
+}
+
+// The exact form on interleaved images, a launch a round, where one wave of its
+// 64 x 32 tiles is the image (75 steps: 320x180 71 us against 75 in planes,
+// 240x135 70 against 86), or one of the 64 x 48 tiles for two rounds at most
+// (600x338, 16 steps: 28 us against 32).
+bool exact_interleaved(const DeviceInfo* di, int w, int h, int num_iter)
+{
+    return tiles_of(w, h, kIH) <= di->sms || (num_iter <= 2 * kTbT && tiles_of(w, h, kPIH) <= di->sms);
 }
 
 struct PlanarCopy {
@@ -2219,12 +2275,12 @@ cudaError_t launch_planar(const PlanarCopy* c, int n, int to_planar, cudaStream_
 
 // One launch of the FMA form's solve kernel per kN members (each member's
 // counters zeroed beforehand; the first member's ticket serves the launch).
-template <int kForm, int kN>
+template <int kCfg, int kN>
 cudaError_t launch_solve(const std::vector<PlWs>& v, const int* w, const int* h, int n, int num_iter, float step,
     float mom, int sms, cudaStream_t st, int* nl)
 {
-    using G = PlGeo<kForm>;
-    const int nround = solve_launches(num_iter);
+    using G = PlGeo<kCfg>;
+    const int nround = solve_launches(num_iter, G::kT);
     for (int b0 = 0; b0 < n; b0 += kN) {
         PlSolve<kN> g{};
         g.count = std::min(n - b0, kN);
@@ -2237,16 +2293,17 @@ cudaError_t launch_solve(const std::vector<PlWs>& v, const int* w, const int* h,
             for (int c = 0; c < 2 && ok; ++c)
                 ok = encode_plane_map(&mp[c ? kPmO1 : kPmO0], m.O[c], W, H, m.pitch, kPlW, G::kRows) &&
                      encode_plane_map(&mp[c ? kPmU1 : kPmU0], m.U[c], W, H, m.pitch, kPlW, G::kRows) &&
-                     encode_plane_map(&mp[c ? kPmOo1 : kPmOo0], m.O[c], W, H, m.pitch, kPlIW, G::kIRows) &&
-                     encode_plane_map(&mp[c ? kPmUo1 : kPmUo0], m.U[c], W, H, m.pitch, kPlIW, G::kIRows);
+                     encode_plane_map(&mp[c ? kPmOo1 : kPmOo0], m.O[c], W, H, m.pitch, G::kIW, G::kIRows) &&
+                     encode_plane_map(&mp[c ? kPmUo1 : kPmUo0], m.U[c], W, H, m.pitch, G::kIW, G::kIRows);
             if (!ok || !encode_plane_map(&mp[kPmK], m.K, W, H, m.pitch, kPlW, G::kRows) ||
-                !encode_plane_map(&mp[kPmC], m.C, W, H, m.pitch, kPlW, G::kRows))
+                !encode_plane_map(&mp[kPmC], m.C, W, H, m.pitch, kPlW, G::kRows) ||
+                (!G::kFma && !encode_plane_map(&mp[kPmA], m.A, W, H, m.pitch, kPlW, G::kRows)))
                 return cudaErrorInvalidValue;
             g.done[p] = m.cnt + 16;
             g.w[p] = W;
             g.h[p] = H;
-            g.tiles_x[p] = pl_tiles_x(W);
-            g.tile0[p + 1] = g.tile0[p] + pl_tiles<kForm>(W, H);
+            g.tiles_x[p] = pl_tiles_x<kCfg>(W);
+            g.tile0[p + 1] = g.tile0[p] + pl_tiles<kCfg>(W, H);
         }
         g.nround = nround;
         g.num_iter = num_iter;
@@ -2258,10 +2315,13 @@ cudaError_t launch_solve(const std::vector<PlWs>& v, const int* w, const int* h,
         cfg.stream = st;
         cfg.attrs = attr;
         cfg.numAttrs = 1;
-        cfg.gridDim = dim3(static_cast<unsigned>(std::min<int64_t>(static_cast<int64_t>(g.tile0[g.count]) * nround, sms)));
+        // no more CTAs than a round has tiles: a CTA more could only start on the next
+        // round and would wait, holding an SM that another stream's kernel could use
+        // (three 640x360 videos at a time, exact form: 353 -> 303 us a frame; one: the same)
+        cfg.gridDim = dim3(std::min(g.tile0[g.count], sms));
         cfg.blockDim = dim3(32 * (G::kWarps + 4));
         cfg.dynamicSmemBytes = G::kSmem;
-        const cudaError_t e = cudaLaunchKernelEx(&cfg, solver_solve_kernel<kForm, kN>, g, step, mom);
+        const cudaError_t e = cudaLaunchKernelEx(&cfg, solver_solve_kernel<kCfg, kN>, g, step, mom);
         if (e != cudaSuccess)
             return e;
         ++*nl;
@@ -2269,33 +2329,52 @@ cudaError_t launch_solve(const std::vector<PlWs>& v, const int* w, const int* h,
     return cudaGetLastError();
 }
 
-// The FMA form of run_solver: constants, O's planes (or the upsampled coarse
-// solution Oc) and zeroed counters, the solve (one launch; per round on the
-// plain-load path), O (and the RGBA8 copy) back from its planes.
-cudaError_t run_solver_fma(const DeviceInfo* di, const float* P, const float* A, const float* Wt, float* O, int w,
-    int h, int num_iter, float step, float mom, float* workspace, size_t ws_floats, cudaStream_t st, int* nl,
-    uint8_t* rgba_out, const float* Oc, int cw, int ch)
+cudaError_t launch_prep(int form, const float* P, const float* A, const float* Wt, const float* O, const PlWs& v,
+    float* Op, int w, int h, float step, unsigned* cnt, int ncnt, const float* Oc, int cw, int ch, cudaStream_t st)
 {
-    const bool tma = pl_tma_eligible(di, w, h, workspace, ws_floats);
-    const PlWs v = pl_view(workspace, w, h, tma ? pl_pitch(w) : w);
     const dim3 b(32, 8);
-    cudaError_t e = launch_pdl(solver_prep_fma_kernel, grid2d(w, h, b), b, 0, st, P, A, Wt,
-        static_cast<const float*>(O), v.C, v.K, v.O[0], w, h, v.pitch, step, v.cnt, v.ncnt, Oc, cw, ch);
+    auto k = form == kSolverFma ? solver_prep_kernel<kSolverFma> : solver_prep_kernel<kSolverExact>;
+    return launch_pdl(k, grid2d(w, h, b), b, 0, st, P, A, Wt, O, v.C, v.K, v.A, Op, w, h, v.pitch, step, cnt, ncnt, Oc,
+        cw, ch);
+}
+
+// run_solver in planes: constants, the planes of the start Oi (or of the
+// coarse solution Oc upsampled) and zeroed counters, the solve (one launch; for
+// the FMA form in a smaller workspace a launch a round with plain loads), O
+// (and the RGBA8 copy) back from its planes.
+cudaError_t run_solver_planes(const DeviceInfo* di, int form, const float* P, const float* A, const float* Wt,
+    const float* Oi, float* O, int w, int h, int num_iter, float step, float mom, float* workspace, size_t ws_floats,
+    cudaStream_t st, int* nl, uint8_t* rgba_out, const float* Oc, int cw, int ch)
+{
+    const bool tma = pl_tma_eligible(di, w, h, workspace, ws_floats, form);
+    int cfg = form;
+    if (tma && pl_long_rounds(di, w, h, num_iter, form) &&
+        pl_tma_eligible(di, w, h, workspace, ws_floats, form | kPlLong))
+        cfg |= kPlLong;
+    const PlWs v = pl_view(workspace, w, h, tma ? pl_pitch(w) : w, cfg);
+    cudaError_t e = launch_prep(form, P, A, Wt, Oi, v, v.O[0], w, h, step, v.cnt, v.ncnt, Oc, cw, ch, st);
     ++*nl;
-    const int nlaunch = solve_launches(num_iter);
+    const int nlaunch = solve_launches(num_iter, cfg & kPlLong ? 2 * kTbT : kTbT);
     if (e == cudaSuccess && tma) {
         const std::vector<PlWs> one(1, v);
-        e = launch_solve<kSolverFma, 1>(one, &w, &h, 1, num_iter, step, mom, di->sms, st, nl);
+        auto solve = [&](auto c) {
+            return launch_solve<decltype(c)::value, 1>(one, &w, &h, 1, num_iter, step, mom, di->sms, st, nl);
+        };
+        switch (cfg) {
+            case kSolverFma: e = solve(std::integral_constant<int, kSolverFma>{}); break;
+            case kSolverFma | kPlLong: e = solve(std::integral_constant<int, kSolverFma | kPlLong>{}); break;
+            case kSolverExact | kPlLong: e = solve(std::integral_constant<int, kSolverExact | kPlLong>{}); break;
+            default: e = solve(std::integral_constant<int, kSolverExact>{}); break;
+        }
     } else if (e == cudaSuccess) {
         // plain loads and stores
-        const int tx = pl_tiles_x(w), nt = pl_tiles<kSolverFma>(w, h);
+        const int tx = pl_tiles_x<kSolverFma>(w), nt = pl_tiles<kSolverFma>(w, h);
         int k0 = 0;
         for (int li = 0; li < nlaunch && e == cudaSuccess; ++li) {
             const int T = std::min(kTbT, num_iter - k0);
             const PlPlain pl{v.O[li & 1], v.U[li & 1], v.K, v.C, v.O[(li + 1) & 1], v.U[(li + 1) & 1], w, h, tx, nt};
             e = launch_pdl(solver_fma_plain_kernel, dim3(std::min(nt, di->sms)), dim3(32 * PlGeo<kSolverFma>::kWarps),
-                PlGeo<kSolverFma>::kSmem, st, pl, T,
-                k0, step, mom);
+                PlGeo<kSolverFma>::kSmem, st, pl, T, k0, step, mom);
             ++*nl;
             k0 += T;
         }
@@ -2315,52 +2394,12 @@ bool solver_tma_supported()
     return device_info(&di) == cudaSuccess && di->ps_smem;
 }
 
-float* solver_start_buffer(float* O, int w, int h, int num_iter, float* workspace, int form)
-{
-    if (form == kSolverFma)
-        return O;  // the solve copies O into its planes first
-    return solve_launches(num_iter) % 2 == 0 ? O : ws_view(workspace, w, h).O2;
-}
-
-cudaError_t solver_lap(const float* P, int w, int h, float* workspace, cudaStream_t st)
-{
-    const dim3 b(32, 8);
-    const cudaError_t e = launch_pdl(lap_pr_kernel, grid2d(w, h, b), b, 0, st, P, workspace, w, h);
-    if (e != cudaSuccess)
-        return e;
-    return cudaGetLastError();
-}
-
 cudaError_t solver_prep(int form, const float* P, const float* A, const float* Wt, int w, int h, float step,
     float* workspace, cudaStream_t st)
 {
-    if (form != kSolverFma)
-        return solver_lap(P, w, h, workspace, st);
-    const PlWs v = pl_view(workspace, w, h, pl_pitch(w));  // w is a multiple of 4 in a grouped solve
-    const dim3 b(32, 8);
-    const cudaError_t e = launch_pdl(solver_prep_fma_kernel, grid2d(w, h, b), b, 0, st, P, A, Wt,
-        static_cast<const float*>(nullptr), v.C, v.K, static_cast<float*>(nullptr), w, h, v.pitch, step,
-        static_cast<unsigned*>(nullptr), 0, static_cast<const float*>(nullptr), 0, 0);
-    if (e != cudaSuccess)
-        return e;
-    return cudaGetLastError();
-}
-
-bool solver_group_eligible(const SolverImage* im, int n, int form)
-{
-    DeviceInfo* di = nullptr;
-    if (n < 1 || device_info(&di) != cudaSuccess)
-        return false;
-    for (int i = 0; i < n; ++i) {
-        const bool ok = form == kSolverFma
-                            ? im[i].w % 4 == 0 && pl_tma_eligible(di, im[i].w, im[i].h, im[i].workspace,
-                                                        solver_workspace_floats(im[i].w, im[i].h, form))
-                            : tma_eligible(di, im[i].w, im[i].O, ws_view(im[i].workspace, im[i].w, im[i].h), im[i].A,
-                                  im[i].Wt);
-        if (!ok)
-            return false;
-    }
-    return true;
+    const PlWs v = pl_view(workspace, w, h, pl_pitch(w), form);
+    const cudaError_t e = launch_prep(form, P, A, Wt, nullptr, v, nullptr, w, h, step, nullptr, 0, nullptr, 0, 0, st);
+    return e != cudaSuccess ? e : cudaGetLastError();
 }
 
 cudaError_t run_solver_group(const SolverImage* im, int n, int num_iter, float step, float mom, cudaStream_t st,
@@ -2370,7 +2409,7 @@ cudaError_t run_solver_group(const SolverImage* im, int n, int num_iter, float s
     cudaError_t e = device_info(&di);
     if (e != cudaSuccess)
         return e;
-    if (!solver_group_eligible(im, n, form))
+    if (n < 1 || !di->ps_smem)
         return cudaErrorInvalidValue;
     int nl = 0;
     if (num_iter <= 0) {
@@ -2383,70 +2422,52 @@ cudaError_t run_solver_group(const SolverImage* im, int n, int num_iter, float s
             *launches += nl;
         return e;
     }
-    int dev = 0;
-    if ((e = cudaGetDevice(&dev)) != cudaSuccess)
-        return e;
+    // O into planes (counters zeroed), one solve launch per 16 images, O back
     std::vector<int> ws(n), hs(n);
+    std::vector<PlWs> v(n);
+    std::vector<PlanarCopy> to(n), back(n);
     for (int i = 0; i < n; ++i) {
-        ws[i] = im[i].w;
-        hs[i] = im[i].h;
-    }
-    const int rows = chosen_rows(dev, ws.data(), hs.data(), n, di->sms, form);
-    const bool odd = solve_launches(num_iter) % 2 == 1;
-    if (form == kSolverFma) {
-        // O into planes (counters zeroed), one solve launch per 16 images, O back
-        std::vector<PlWs> v(n);
-        std::vector<PlanarCopy> to(n), back(n);
-        for (int i = 0; i < n; ++i) {
-            v[i] = pl_view(im[i].workspace, im[i].w, im[i].h, im[i].w);
-            to[i] = PlanarCopy{im[i].O, v[i].O[0], nullptr, im[i].w, im[i].h, im[i].w, v[i].cnt, v[i].ncnt};
-            back[i] = PlanarCopy{v[i].O[solve_launches(num_iter) & 1], im[i].O, im[i].rgba, im[i].w, im[i].h, im[i].w};
-        }
-        e = launch_planar(to.data(), n, 1, st, &nl);
-        if (e == cudaSuccess)
-            e = n <= 4 ? launch_solve<kSolverFma, 4>(v, ws.data(), hs.data(), n, num_iter, step, mom, di->sms, st, &nl)
-                       : launch_solve<kSolverFma, kGroupMax>(v, ws.data(), hs.data(), n, num_iter, step, mom, di->sms, st, &nl);
-        if (e == cudaSuccess)
-            e = launch_planar(back.data(), n, 0, st, &nl);
-        if (launches)
-            *launches += nl;
-        return e != cudaSuccess ? e : cudaGetLastError();
-    }
-    std::vector<GroupMember> mem(n);
-    for (int i = 0; i < n; ++i) {
-        const WsView v = ws_view(im[i].workspace, im[i].w, im[i].h);
-        float* const O[2] = {im[i].O, v.O2};
-        float* const U[2] = {v.U0, v.U1};
-        if (!encode_solve(&mem[i].maps, O, U, im[i].A, im[i].Wt, v.L, im[i].w, im[i].h, rows))
+        const int w = ws[i] = im[i].w, h = hs[i] = im[i].h;
+        v[i] = pl_view(im[i].workspace, w, h, pl_pitch(w), form);
+        if (!aligned16p(im[i].workspace))
             return cudaErrorInvalidValue;
-        mem[i].c0 = odd ? 1 : 0;
-        mem[i].rgba = im[i].rgba;
-        mem[i].w = im[i].w;
-        mem[i].h = im[i].h;
+        to[i] = PlanarCopy{im[i].O, v[i].O[0], nullptr, w, h, v[i].pitch, v[i].cnt, v[i].ncnt};
+        back[i] = PlanarCopy{v[i].O[solve_launches(num_iter) & 1], im[i].O, im[i].rgba, w, h, v[i].pitch};
     }
-    e = n <= 4 ? launch_members<4>(mem, rows, num_iter, step, mom, di->sms, st, &nl)
-               : launch_members<kGroupMax>(mem, rows, num_iter, step, mom, di->sms, st, &nl);
+    e = launch_planar(to.data(), n, 1, st, &nl);
+    auto solve = [&](auto f, auto group) {
+        return launch_solve<decltype(f)::value, decltype(group)::value>(v, ws.data(), hs.data(), n, num_iter, step, mom,
+            di->sms, st, &nl);
+    };
+    using Fma = std::integral_constant<int, kSolverFma>;
+    using Exact = std::integral_constant<int, kSolverExact>;
+    using Few = std::integral_constant<int, 4>;
+    using Many = std::integral_constant<int, kGroupMax>;
+    if (e == cudaSuccess)
+        e = form == kSolverFma ? (n <= 4 ? solve(Fma{}, Few{}) : solve(Fma{}, Many{}))
+                               : (n <= 4 ? solve(Exact{}, Few{}) : solve(Exact{}, Many{}));
+    if (e == cudaSuccess)
+        e = launch_planar(back.data(), n, 0, st, &nl);
     if (launches)
         *launches += nl;
-    if (e == cudaSuccess)
-        e = cudaGetLastError();
-    return e;
+    return e != cudaSuccess ? e : cudaGetLastError();
 }
 
-cudaError_t run_solver_from_coarse(const float* P, const float* A, const float* Wt, float* O, int w, int h,
-    const float* Oc, int cw, int ch, int num_iter, float step, float mom, float* workspace, size_t ws_floats,
-    cudaStream_t st, int* launches, uint8_t* rgba_out)
+cudaError_t run_solver_planes(int form, const float* P, const float* A, const float* Wt, const float* Oi, float* O,
+    int w, int h, const float* Oc, int cw, int ch, int num_iter, float step, float mom, float* workspace,
+    size_t ws_floats, cudaStream_t st, int* launches, uint8_t* rgba_out)
 {
-    if (num_iter <= 0 || !Oc || cw <= 0 || ch <= 0)
+    if (num_iter <= 0 || !(Oi || (Oc && cw > 0 && ch > 0)))
         return cudaErrorInvalidValue;
     DeviceInfo* di = nullptr;
     cudaError_t e = device_info(&di);
     if (e != cudaSuccess)
         return e;
-    if (!di->ps_smem)
+    if (!di->ps_smem || !pl_tma_eligible(di, w, h, workspace, ws_floats, form))
         return cudaErrorNotSupported;
     int nl = 0;
-    e = run_solver_fma(di, P, A, Wt, O, w, h, num_iter, step, mom, workspace, ws_floats, st, &nl, rgba_out, Oc, cw, ch);
+    e = run_solver_planes(di, form, P, A, Wt, Oi, O, w, h, num_iter, step, mom, workspace, ws_floats, st, &nl, rgba_out,
+        Oc, cw, ch);
     if (launches)
         *launches += nl;
     return e;
@@ -2471,22 +2492,24 @@ cudaError_t run_solver(const float* P, const float* A, const float* Wt, float* O
     cudaError_t e0 = device_info(&di);
     if (e0 != cudaSuccess)
         return e0;
-    if (form == kSolverFma) {
-        if (!di->ps_smem)
-            return cudaErrorNotSupported;
-        const cudaError_t e = run_solver_fma(di, P, A, Wt, O, w, h, num_iter, step, mom, workspace, ws_floats, st, &nl,
-            rgba_out, nullptr, 0, 0);
+    if (form == kSolverFma && !di->ps_smem)
+        return cudaErrorNotSupported;
+    const bool interleaved = tma_eligible(di, w, O, v, A, Wt) && exact_interleaved(di, w, h, num_iter);
+    if (form == kSolverFma || (!interleaved && pl_tma_eligible(di, w, h, workspace, ws_floats, form))) {
+        const cudaError_t e = run_solver_planes(di, form, P, A, Wt, O, O, w, h, num_iter, step, mom, workspace,
+            ws_floats, st, &nl, rgba_out, nullptr, 0, 0);
         if (launches)
             *launches += nl;
         return e;
     }
-    if ((e0 = solver_lap(P, w, h, v.L, st)) != cudaSuccess)
+    const dim3 b(32, 8);
+    if ((e0 = launch_pdl(lap_pr_kernel, grid2d(w, h, b), b, 0, st, P, v.L, w, h)) != cudaSuccess)
         return e0;
     ++nl;
     // Launches of up to kTbT iterations; ping-pong O between O and O2 and U
     // between its two buffers so that the last launch writes O.
     const int nlaunch = solve_launches(num_iter);
-    float* cur = solver_start_buffer(O, w, h, num_iter, workspace, kSolverExact);
+    float* cur = nlaunch % 2 == 0 ? O : v.O2;
     if (cur != O) {
         cudaError_t e = cudaMemcpyAsync(v.O2, O, n * sizeof(float), cudaMemcpyDeviceToDevice, st);
         if (e != cudaSuccess)
@@ -2497,21 +2520,16 @@ cudaError_t run_solver(const float* P, const float* A, const float* Wt, float* O
     int dev = 0;
     if ((e0 = cudaGetDevice(&dev)) != cudaSuccess)
         return e0;
-    const int rows = chosen_rows(dev, &w, &h, 1, di->sms, kSolverExact);
-    GroupMember m{};
+    const int rows = chosen_rows(dev, w, h, di->sms, kSolverExact);
+    SolveMaps m;
     bool tma = tma_eligible(di, w, O, v, A, Wt);
     if (tma) {
         float* const Ob[2] = {O, v.O2};
         float* const Ub[2] = {v.U0, v.U1};
-        tma = encode_solve(&m.maps, Ob, Ub, A, Wt, v.L, w, h, rows);
+        tma = encode_solve(&m, Ob, Ub, A, Wt, v.L, w, h, rows);
     }
     if (tma) {
-        m.w = w;
-        m.h = h;
-        m.c0 = cur == O ? 0 : 1;
-        m.rgba = rgba_out;
-        const std::vector<GroupMember> one(1, m);
-        cudaError_t e = launch_members<1>(one, rows, num_iter, step, mom, di->sms, st, &nl);
+        cudaError_t e = launch_rounds(m, w, h, cur == O ? 0 : 1, rgba_out, rows, num_iter, step, mom, di->sms, st, &nl);
         if (launches)
             *launches += nl;
         return e != cudaSuccess ? e : cudaGetLastError();
