@@ -63,6 +63,29 @@ def test_lowp_correlation_exact_on_representable_values(vsc, oracle, cuda, shape
     vsc.check_device()
 
 
+@pytest.mark.parametrize("shape,md", [
+    ((1, 1, 1, 1), 0),                           # one output element
+    ((1, 96, 6, 33), 4), ((1, 128, 3, 129), 8),  # 32 channels of three chunks, 64 of two
+    ((1, 192, 4, 20), 4), ((1, 208, 3, 40), 1),  # the largest: 64 of three, 16 of thirteen
+    ((12, 20, 37, 130), 4), ((12, 60, 19, 130), 3),  # several output rows an item, the last item short
+    ((14, 33, 19, 130), 1), ((16, 64, 35, 128), 0)])
+def test_lowp_correlation_chunk_widths_and_row_blocks(vsc, oracle, cuda, shape, md):
+    """Values that are exact in 16 bits, sums that are exact in FP32: equal bit
+    for bit for every chunk width and number of rows an item.  The tensors start
+    4 bytes past a 16-byte boundary as well."""
+    import torch
+
+    f1 = (RNG.integers(-3, 4, shape) * 0.25).astype(np.float32)
+    f2 = (RNG.integers(-3, 4, shape) * 0.5).astype(np.float32)
+    want = oracle.correlation(f1, f2, md)
+    a, b = _t(f1, cuda), _t(f2, cuda)
+    assert np.array_equal(vsc.correlation_lowp(a, b, md, "bf16").cpu().numpy(), want)
+    shifted = torch.empty(a.numel() + 1, dtype=torch.float32, device=cuda)[1:].view(shape)
+    shifted.copy_(a)
+    assert np.array_equal(vsc.correlation_lowp(shifted, b, md, "fp16").cpu().numpy(), want)
+    vsc.check_device()
+
+
 @pytest.mark.parametrize("dtype", ["bf16", "fp16"])
 def test_lowp_correlation_pwc_pyramid_640x360(vsc, oracle, cuda, dtype):
     """The five PWC levels of a 640x360 frame pair (C = 32..196); error

@@ -58,22 +58,21 @@ cudaError_t launch_warp_op_f64(const double* in, const double* flow, double* out
 constexpr int kTcMaxMd = 8;                 // max_displacement limit of the tile
 constexpr int kTcMaxChannelsPadded = 208;   // channels, padded to a multiple of 16
 int tc_padded_channels(int C);
+int tc_chunk_channels(int cp);  // channels of a chunk of the layout below: the largest of 64, 32, 16 that divides cp
 size_t corr_tc_workspace_bytes(int N, int C, int H, int W);
 // From float NCHW (scaled per tensor, converted in the workspace).
 cudaError_t launch_corr_tc(const float* f1, const float* f2, float* out, int N, int C, int H, int W, int md,
     bool bf16, void* workspace, cudaStream_t st);
-// From operands already in the chunked 16-bit layout [n][y][c / 16][x][c % 16]
-// (Cp channels) with their scales (2 floats: f1, f2) on the device.
+// From operands already in the chunked 16-bit layout [n][y][c / cw][x][c % cw]
+// (Cp channels, cw = tc_chunk_channels(Cp)) with their scales (2 floats: f1, f2) on the device.
 cudaError_t launch_corr_tc_chunked(const void* f1c, const void* f2c, float* out, const float* scales, int N, int Cp,
     int H, int W, int md, bool bf16, cudaStream_t st);
 // two correlations of the same shape in one launch (f1c / f2c -> out and g1c / g2c -> out2)
 cudaError_t launch_corr_tc_chunked2(const void* f1c, const void* f2c, float* out, const void* g1c, const void* g2c,
     float* out2, const float* scales, int N, int Cp, int H, int W, int md, bool bf16, cudaStream_t st);
 
-// float NCHW -> chunked 16-bit operand layout, multiplied by *scale.
-cudaError_t launch_to_chunked(const float* in, void* out, const float* scale, int N, int C, int H, int W, bool bf16,
-    cudaStream_t st);
-// the same for up to 5 tensors of one image each (a feature pyramid's levels) in one launch
+// float NCHW -> chunked 16-bit operand layout, multiplied by *scale, of up to 5
+// tensors of one image each (a feature pyramid's levels) in one launch
 cudaError_t launch_to_chunked_levels(const float* const* in, void* const* out, const int* C, const int* H,
     const int* W, int n, const float* scale, bool bf16, cudaStream_t st);
 // custom::Warp (single precision) with the chunked 16-bit layout as output;

@@ -67,6 +67,22 @@ __device__ __forceinline__ bool mbar_wait_bounded(uint64_t* bar, uint32_t parity
     return false;
 }
 
+// True in one lane of a converged warp.  A branch on it, unlike one on the lane's
+// number, tells the compiler that one thread runs what follows, which TMA and MMA
+// instructions (their operands live in uniform registers) are generated for.
+__device__ __forceinline__ bool elect_one()
+{
+    uint32_t one;
+    asm volatile(
+        "{\n"
+        " .reg .pred p;\n"
+        " elect.sync _|p, 0xffffffff;\n"
+        " selp.u32 %0, 1, 0, p;\n"
+        "}\n"
+        : "=r"(one)::"memory");
+    return one != 0;
+}
+
 // ---- tiled TMA loads ---------------------------------------------------------------
 __device__ __forceinline__ void tma_load_5d(void* dst, const CUtensorMap* map, int c0, int c1, int c2, int c3, int c4,
     uint64_t* bar)
@@ -114,19 +130,19 @@ __device__ __forceinline__ uint64_t umma_desc_kmajor(uint32_t smem_addr, uint32_
     return d;
 }
 
-// Shared-memory descriptor of a K-major operand in the 32-byte swizzle layout
-// (what a TMA load with CU_TENSOR_MAP_SWIZZLE_32B and a 32-byte inner box
-// writes): rows of 32 bytes (16 K-elements of 16 bits, one MMA's K), 8-row
-// groups 256 bytes apart (the stride offset); the leading offset is unused
-// because an MMA's K spans one swizzle row.  Layout type 6 = 32-byte
-// swizzle in bits [61, 64); the start must sit on a 256-byte boundary.
-__device__ __forceinline__ uint64_t umma_desc_kmajor_sw32(uint32_t smem_addr)
+// Shared-memory descriptor of a K-major operand in the swizzle layout of
+// `row`-byte rows, 32, 64 or 128 (what a TMA load with that swizzle and an inner
+// box of as many bytes writes): 8-row groups 8 x row bytes apart (the stride
+// offset); the leading offset is unused, an MMA's K (32 bytes) lying in one
+// row.  Layout type 6, 4 or 2 in bits [61, 64).  The operand starts on a
+// boundary of 8 x row bytes; K step i of a row is 32 i bytes further on.
+__device__ __forceinline__ uint64_t umma_desc_kmajor_swizzled(uint32_t smem_addr, int row)
 {
     uint64_t d = static_cast<uint64_t>((smem_addr & 0x3FFFFu) >> 4);
-    d |= static_cast<uint64_t>(1) << 16;           // leading offset (unused): 16 bytes
-    d |= static_cast<uint64_t>(256 >> 4) << 32;    // stride offset: 8 rows x 32 bytes
+    d |= static_cast<uint64_t>(1) << 16;              // leading offset (unused): 16 bytes
+    d |= static_cast<uint64_t>((8 * row) >> 4) << 32;  // stride offset
     d |= static_cast<uint64_t>(1) << 46;
-    d |= static_cast<uint64_t>(6) << 61;
+    d |= static_cast<uint64_t>(row == 128 ? 2 : row == 64 ? 4 : 6) << 61;
     return d;
 }
 
