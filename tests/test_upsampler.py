@@ -95,6 +95,29 @@ def test_inference_matches_numpy_and_fallback(vsc, cuda, h, w):
 
 
 @pytest.mark.gpu
+@pytest.mark.parametrize("h,w", [(1, 1), (7, 125), (8, 126), (9, 127), (17, 128), (24, 253), (330, 1000)])
+def test_inference_at_segment_and_group_edges(vsc, cuda, h, w):
+    """Segments of 126 output columns and groups of 8 output rows: one short,
+    exact and one over, and an image of more than two groups a block.  Same FP16
+    operands as the restatement, FP32 vs float64 sums: the bound of the test
+    above."""
+    import torch
+
+    coarse = torch.from_numpy(RNG.normal(0, 1.5, ((h + 1) // 2, (w + 1) // 2, 3)).astype(np.float32)).to(cuda)
+    frame = torch.from_numpy(RNG.random((h, w, 3)).astype(np.float32)).to(cuda)
+    params = RNG.normal(0, 0.08, vsc.Upsampler.param_count()).astype(np.float32)
+    params = params.astype(np.float16).astype(np.float32)
+    up = vsc.Upsampler(params)
+    up.set_max_residual(1e9)
+    inp = vsc.Upsampler.prepare(coarse, frame).cpu().numpy()
+    r = _np_forward(params, inp, half_acts=True)
+    got = up.apply(coarse, frame).cpu().numpy()
+    assert np.allclose(got[..., :2], inp[..., :2] + r, atol=1e-3 * (1 + np.abs(r).max()))
+    assert np.all(got[..., 2] == 0)
+    up.close()
+
+
+@pytest.mark.gpu
 def test_training_overfits_a_batch(vsc, cuda):
     import torch
 

@@ -1155,7 +1155,7 @@ cudaError_t upsampler_apply_pair(vsc_stabilizer* s, cudaStream_t st, int* nl)
     cudaError_t e = upsampler_sync_weights(s->upsampler, st);
     if (e == cudaSuccess)
         e = launch_upsampler_prepare(s->flow_small, s->fw, s->fh, 3, s->orig[(s->head + 1) % 3], input, s->w, s->h, 2,
-            fs, s->orig[(s->head + 2) % 3] - s->orig[(s->head + 1) % 3], npx * 3, st);
+            fs, s->orig[(s->head + 2) % 3] - s->orig[(s->head + 1) % 3], npx * 3, st, up_tc_work(input, 2 * npx * 3));
     *nl += 1;
     if (e == cudaSuccess)
         e = launch_upsampler_tc(s->upsampler->wtc, s->upsampler->prm, input, up_tc_work(input, 2 * npx * 3),
@@ -1691,7 +1691,7 @@ VSC_API vsc_status vsc_upsampler_apply(vsc_upsampler* u, const vsc_image* coarse
     cudaError_t e = upsampler_sync_weights(u, st);
     if (e == cudaSuccess)
         e = launch_upsampler_prepare(coarse_flow->data, coarse_flow->width, coarse_flow->height, coarse_flow->channels,
-            frame->data, input, w, h, 1, 0, 0, 0, st);
+            frame->data, input, w, h, 1, 0, 0, 0, st, up_tc_work(input, npx * 3));
     if (e == cudaSuccess)
         e = launch_upsampler_tc(u->wtc, u->prm, input, up_tc_work(input, npx * 3), flow_out->data, 1, h, w,
             u->max_residual, 0, st, nullptr);

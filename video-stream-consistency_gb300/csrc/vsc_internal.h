@@ -95,15 +95,16 @@ int upsampler_param_count();
 void upsampler_init_params(float* host, uint64_t seed);
 size_t upsampler_train_work_floats(int N, int H, int W);   // activations and gradients of a batch
 // input (N x h x w x 3): the coarse flows bilinearly upsampled with their vectors
-// scaled to the full grid, and the frames' luma; batch n at base + n * stride
+// scaled to the full grid, and the frames' luma; batch n at base + n * stride;
+// plane: launch_upsampler_tc's work, whose first part it writes
 cudaError_t launch_upsampler_prepare(const float* coarse, int cw, int ch, int cfc, const float* img, float* input,
-    int w, int h, int N, int64_t s_coarse, int64_t s_img, int64_t s_in, cudaStream_t st);
+    int w, int h, int N, int64_t s_coarse, int64_t s_img, int64_t s_in, cudaStream_t st, void* plane = nullptr);
 // Tensor-core inference (tcgen05 implicit-GEMM convolutions, FP16 operands,
 // FP32 accumulation).  Packed weights: upsampler_tc_weight_bytes() bytes,
 // written from the FP32 parameters by launch_upsampler_tc_pack.  Work:
 // upsampler_tc_work_bytes(N, H, W) bytes, 16-byte aligned.  Writes the
 // finished flows (u, v, 0) of every batch image (flow + n * s_out floats)
-// from the prepared input (launch_upsampler_prepare's layout).
+// from the prepared input (launch_upsampler_prepare, which was given the work).
 size_t upsampler_tc_weight_bytes();
 size_t upsampler_tc_work_bytes(int N, int H, int W);
 cudaError_t launch_upsampler_tc_pack(const float* prm, void* wtc, cudaStream_t st);

@@ -37,9 +37,12 @@ __device__ __forceinline__ float luma(const float* p) { return 0.299f * p[0] + 0
 
 // ---- input: base flow and luma ------------------------------------------------------
 // base = bilinear(coarse) at the frame's size (kernel_bilinear's sampling,
-// flowconsistency.cu:50-75) times the size ratio per axis.
+// flowconsistency.cu:50-75) times the size ratio per axis.  plane, if given:
+// the same values as the tensor-core inference's first chunk plane (FP16, five
+// zero channels).
 __global__ void prepare_kernel(const float* __restrict__ coarse, int cw, int ch, int cfc, const float* __restrict__ img,
-    float* __restrict__ input, int w, int h, int64_t s_coarse, int64_t s_img, int64_t s_in)
+    float* __restrict__ input, int w, int h, int64_t s_coarse, int64_t s_img, int64_t s_in,
+    uint4* __restrict__ plane)
 {
     const int x = blockIdx.x * blockDim.x + threadIdx.x;
     const int y = blockIdx.y * blockDim.y + threadIdx.y;
@@ -60,9 +63,15 @@ __global__ void prepare_kernel(const float* __restrict__ coarse, int cw, int ch,
         v[k] = v00 * (1 - fx) * (1 - fy) + v10 * fx * (1 - fy) + v01 * (1 - fx) * fy + v11 * fx * fy;
     }
     float* o = input + n * s_in + pix_index(x, y, w) * 3;
-    o[0] = v[0] * sx;
-    o[1] = v[1] * sy;
-    o[2] = luma(img + n * s_img + pix_index(x, y, w) * 3);
+    const float u = v[0] * sx, t = v[1] * sy, l = luma(img + n * s_img + pix_index(x, y, w) * 3);
+    o[0] = u;
+    o[1] = t;
+    o[2] = l;
+    if (plane) {
+        const __half2 a = __floats2half2_rn(u, t), b = __floats2half2_rn(l, 0.0f);
+        plane[(static_cast<int64_t>(n) * h + y) * w + x] =
+            make_uint4(*reinterpret_cast<const uint32_t*>(&a), *reinterpret_cast<const uint32_t*>(&b), 0u, 0u);
+    }
 }
 
 // ---- training: 3x3 convolutions on register tiles ---------------------------------------
@@ -612,11 +621,12 @@ void upsampler_init_params(float* host, uint64_t seed)
 }
 
 cudaError_t launch_upsampler_prepare(const float* coarse, int cw, int ch, int cfc, const float* img, float* input, int w,
-    int h, int N, int64_t s_coarse, int64_t s_img, int64_t s_in, cudaStream_t st)
+    int h, int N, int64_t s_coarse, int64_t s_img, int64_t s_in, cudaStream_t st, void* plane)
 {
     const dim3 b(32, 8);
     const dim3 g((w + 31) / 32, (h + 7) / 8, N);
-    prepare_kernel<<<g, b, 0, st>>>(coarse, cw, ch, cfc, img, input, w, h, s_coarse, s_img, s_in);
+    prepare_kernel<<<g, b, 0, st>>>(coarse, cw, ch, cfc, img, input, w, h, s_coarse, s_img, s_in,
+        static_cast<uint4*>(plane));
     return cudaGetLastError();
 }
 

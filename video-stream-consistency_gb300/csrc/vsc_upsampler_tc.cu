@@ -20,23 +20,25 @@
 // the epilogue of the other: the layer is bound by HBM, not by the
 // accumulator ring.
 //
-// A work item is a segment of kUpRC = 16 output rows (two groups); each
-// group's ten input rows stream through a ring of row buffers (one TMA box
-// {8, 130, 1, chunks} per row: the segment with its one-pixel halo,
-// zero-filled outside the image, which is the convolution's zero padding);
-// the two rows the groups share are loaded for each, so that every buffer has
-// one reader.  The A operand is
-// a row buffer seen from position tx (8 positions x 16 bytes per core
-// matrix, M-adjacent core matrices 128 bytes apart, K-adjacent ones a chunk
-// plane apart).  Weights [tx][chunk][ty * NO + o][8] (FP16, output channels
+// A group's ten input rows stream through row buffers of their own, one TMA box
+// per row: the 128 positions of a segment, of which the outer two are the halo of
+// the 126 it computes (accumulator lanes 126 and 127 hold what nobody reads),
+// zero-filled outside the image, which is the convolution's zero padding.  A row
+// of a chunk plane is contiguous, so the box takes it as 256 elements of 8
+// bytes: the TMA works through a box by its rows, and with boxes of {8 channels,
+// 130 positions} it went through 520 rows of 16 bytes a row of 32 channels and
+// bound the kernel (1920x1080: all layers 260 us, now 193 for 1.0 GB of
+// traffic).  The A operand is a row buffer seen from position tx (8
+// positions x 16 bytes per core matrix, M-adjacent core matrices 128 bytes
+// apart, K-adjacent ones a chunk plane apart; lanes 126 and 127 run 32 bytes
+// past the plane).  Weights [tx][chunk][ty * NO + o][8] (FP16, output channels
 // padded to NO, input channels to the K chunks) stay in shared memory for the
 // launch.  The first layer's three input channels (base flow u, v and luma)
 // occupy one chunk; its second K chunk is a zero plane that is never loaded.
 //
 // Persistent and warp-specialised: warp 0 issues the TMA loads; warp 1 (which
-// owns Tensor Memory) issues the MMAs of every item's first group and warp 18
-// those of its second (one thread issues an MMA about every 90 cycles, twice
-// the tensor pipe's time for these shapes); warps 2-17 are the epilogue, four
+// owns Tensor Memory) issues the MMAs of every second group and warp 18 those of
+// the others; warps 2-17 are the epilogue, four
 // per 32 Tensor Memory lanes, each taking two output rows of a group.  Epilogue:
 // bias, ReLU, FP16 and the chunked store for the inner layers; for the last
 // layer the residual test and the finished flow (base + r where
@@ -54,26 +56,22 @@
 namespace vsc {
 namespace {
 
-constexpr int kUpM = 128;                // output positions per segment (MMA M, Tensor Memory lanes)
+constexpr int kUpM = 128;                // positions of a segment, halo included (MMA M, Tensor Memory lanes)
+constexpr int kUpOut = kUpM - 2;         // output positions per segment
 constexpr int kUpGR = 8;                 // output rows per accumulator group
-constexpr int kUpRC = 16;                // output rows per work item
-constexpr int kUpGPI = kUpRC / kUpGR;    // groups per work item
 constexpr int kUpGRows = kUpGR + 2;      // input rows per group
-constexpr int kUpLoads = kUpGPI * kUpGRows;  // row loads per work item (each group has its own)
-constexpr int kUpTW = kUpM + 2;          // positions loaded per row (one-pixel halo)
-constexpr int kUpRowBufs = 22;           // row buffers in shared memory (more than an item's 18 rows)
-constexpr int kUpSlots = 2;              // group accumulators in Tensor Memory
+constexpr int kUpSlots = 2;              // group accumulators in Tensor Memory, and MMA issuers
+constexpr int kUpRowBufs = kUpSlots * kUpGRows;  // row buffers in shared memory: a group's rows for each issuer
 constexpr uint32_t kUpTmemCols = 512;
 constexpr int kUpEpiWarps = 16;          // 4 lane quarters x 4 pairs of a group's rows
 constexpr int kUpWaitSpins = 1 << 22;    // bounded mbarrier waits (about a second)
 constexpr int kUpIssuerWarp1 = 2 + kUpEpiWarps;  // the second group's MMA issuer (the first: warp 1)
 constexpr int kUpThreads = (3 + kUpEpiWarps) * 32;
-constexpr int kUpPlaneBytes = kUpTW * 16;  // one chunk plane of a row buffer
+constexpr int kUpPlaneBytes = kUpM * 16;  // one chunk plane of a row buffer
 constexpr uint32_t kUpZeroBytes = 8192;  // zero operands of the slot-clearing MMA (A 4 KB, B 8 KB overlapped)
 constexpr int kUpSmemLimit = 232448;
 constexpr uint32_t kUpMinSmem = 120 * 1024;
-static_assert(kUpRC % kUpGR == 0 && kUpEpiWarps == 4 * (kUpGR / 2), "epilogue rows");
-static_assert(kUpRowBufs >= kUpLoads + 2 && kUpGPI == kUpSlots, "row buffers; one slot and issuer per group");
+static_assert(kUpEpiWarps == 4 * (kUpGR / 2), "epilogue rows");
 
 __host__ __device__ constexpr uint32_t up_align1k(uint32_t v) { return (v + 1023u) & ~1023u; }
 // a row buffer: the TMA destination and the MMA operands need 128-byte alignment
@@ -155,10 +153,11 @@ __global__ void __launch_bounds__(kUpThreads, 1)
     uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(drain + kUpSlots);
     volatile int* abort = reinterpret_cast<volatile int*>(drain + kUpSlots + 1);
 
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int nseg = (W + kUpM - 1) / kUpM, nchunk = (H + kUpRC - 1) / kUpRC;
-    const int items = N * nchunk * nseg;
+    const int warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0), lane = threadIdx.x & 31;  // warp: uniform
+    const int nseg = (W + kUpOut - 1) / kUpOut, nchunk = (H + kUpGR - 1) / kUpGR;
+    const int items = N * nchunk * nseg;  // groups
 
+    pdl_enter();
     // weights and bias into shared memory; the zero operands and the K chunks that
     // are never loaded are zero
     for (uint32_t i = threadIdx.x; i < kWBytes / 16; i += blockDim.x)
@@ -196,40 +195,38 @@ __global__ void __launch_bounds__(kUpThreads, 1)
     ptx::tc_fence_after();
     const uint32_t tmem = *tmem_slot;
 
-    // row loads are counted over the whole CTA (u): row buffer u % kUpRowBufs; item
-    // k of the CTA owns loads k * kUpLoads ..., group g's ten input rows from
-    // k * kUpLoads + g * kUpGRows (the two rows the groups share are loaded for
-    // each).  Group g of every item is issued by its own thread (warp 1 for g = 0,
-    // warp kUpIssuerWarp1 for g = 1) into Tensor Memory slot g; the epilogue
-    // counts groups over the CTA (G), slot G % kUpSlots = g.
+    // Groups are counted over the CTA (k).  Those with k % 2 = i have an issuer
+    // (warp 1 for i = 0, warp kUpIssuerWarp1 for i = 1), a Tensor Memory slot and
+    // ten row buffers of their own, so every wait follows its ring in order.
     if (warp == 0) {
         // ---- TMA producer -------------------------------------------------------------
-        if (lane == 0) {
-            int u = 0;
+        if (ptx::elect_one()) {
+            int k = 0, u = 0;
             bool ok = true;
-            for (int it = blockIdx.x; ok && it < items; it += gridDim.x) {
+            for (int it = blockIdx.x; ok && it < items; it += gridDim.x, ++k) {
                 const int seg = it % nseg, rest = it / nseg;
                 const int chunk = rest % nchunk, n = rest / nchunk;
-                for (int j = 0; j < kUpLoads; ++j, ++u) {
-                    const int b = u % kUpRowBufs;
-                    if (!(ok = up_wait(&empty[b], ((u / kUpRowBufs) & 1) ^ 1, abort)))
+                const int b0 = (k & 1) * kUpGRows;
+                for (int r = 0; r < kUpGRows; ++r, ++u) {
+                    const int b = b0 + r;
+                    if (!(ok = up_wait(&empty[b], ((k >> 1) & 1) ^ 1, abort)))
                         break;
-                    const int y = chunk * kUpRC - 1 + (j / kUpGRows) * kUpGR + j % kUpGRows;
                     ptx::mbar_expect_tx(&full[b], LCH * kUpPlaneBytes);
-                    ptx::tma_load_5d(rows + b * kRowBytes, &mIn, 0, seg * kUpM - 1, y, 0, n, &full[b]);
+                    ptx::tma_load_5d(rows + b * kRowBytes, &mIn, 2 * (seg * kUpOut - 1), chunk * kUpGR - 1 + r, 0, n,
+                        0, &full[b]);
                 }
             }
             if (*abort)  // let every copy issued land before the CTA exits
                 for (int i = 0; i < kUpRowBufs && i < u; ++i) {
-                    const int v = u - 1 - i;
+                    const int v = u - 1 - i;  // row v % kUpGRows of group v / kUpGRows
                     ptx::mbar_wait_bounded(&full[v % kUpRowBufs], (v / kUpRowBufs) & 1, kUpWaitSpins);
                 }
         }
     } else if (warp == 1 || warp == kUpIssuerWarp1) {
-        // ---- MMA issuers: group g of every item ------------------------------------------
-        if (lane == 0) {
+        // ---- MMA issuers: every second group each ----------------------------------------
+        if (ptx::elect_one()) {
             const int g = warp == 1 ? 0 : 1;
-            int m = 0;  // items done by this issuer (slot g's uses)
+            int m = 0;  // groups done by this issuer (slot g's uses)
             bool ok = true;
             // Descriptors are built once; an operand at byte offset d from its base is
             // the base descriptor + d / 16 (the start-address field, which cannot carry:
@@ -239,15 +236,15 @@ __global__ void __launch_bounds__(kUpThreads, 1)
             const uint64_t zadesc = ptx::umma_desc_kmajor(ptx::smem_u32(zero), 2048, 128);
             const uint64_t zbdesc = ptx::umma_desc_kmajor(ptx::smem_u32(zero), kSlotCols * 16, 128);
             const uint32_t dslot = tmem + g * kSlotCols;
-            for (int it = blockIdx.x; ok && it < items; it += gridDim.x, ++m) {
+            for (int it = blockIdx.x + g * gridDim.x; ok && it < items; it += 2 * gridDim.x, ++m) {
                 if (!(ok = up_wait(&sempty[g], (m & 1) ^ 1, abort)))
                     break;
                 ptx::tc_fence_after();
                 ptx::umma_f16(dslot, zadesc, zbdesc, idesc0, false);  // clear the group's accumulator
                 // the group's output rows 0 ... 7 read its input rows r = 0 ... 9
                 for (int r = 0; r < kUpGRows; ++r) {
-                    const int u = m * kUpLoads + g * kUpGRows + r, b = u % kUpRowBufs;
-                    if (!(ok = up_wait(&full[b], (u / kUpRowBufs) & 1, abort)))
+                    const int b = g * kUpGRows + r;
+                    if (!(ok = up_wait(&full[b], m & 1, abort)))
                         break;
                     ptx::tc_fence_after();
                     // input row r feeds output row t = r - ty for ty = 0, 1, 2 where
@@ -285,16 +282,17 @@ __global__ void __launch_bounds__(kUpThreads, 1)
         const int rp = e >> 2;                    // its rows of a group: 2 rp, 2 rp + 1
         const uint32_t lane_base = static_cast<uint32_t>(q * 32) << 16;
         const int64_t HW = static_cast<int64_t>(H) * W;
-        int G = 0;
+        int k = 0;
         bool ok = true;
-        for (int it = blockIdx.x; ok && it < items; it += gridDim.x) {
+        for (int it = blockIdx.x; ok && it < items; it += gridDim.x, ++k) {
             const int seg = it % nseg, rest = it / nseg;
             const int chunk = rest % nchunk, n = rest / nchunk;
-            const int x = seg * kUpM + q * 32 + lane;
-            for (int g = 0; g < kUpGPI; ++g, ++G) {
-                const int sl = G % kUpSlots;
+            const int x = seg * kUpOut + q * 32 + lane;
+            const bool inside = q * 32 + lane < kUpOut && x < W;
+            {
+                const int sl = k & 1;
                 // warp-uniform outcome: the Tensor Memory loads below are warp-collective
-                ok = __all_sync(0xffffffffu, up_wait(&sfull[sl], (G / kUpSlots) & 1, abort));
+                ok = __all_sync(0xffffffffu, up_wait(&sfull[sl], (k >> 1) & 1, abort));
                 if (!ok)
                     break;
                 ptx::tc_fence_after();
@@ -320,8 +318,8 @@ __global__ void __launch_bounds__(kUpThreads, 1)
                     ptx::mbar_arrive(&sempty[sl]);
 #pragma unroll
                 for (int r = 0; r < 2; ++r) {
-                    const int y = chunk * kUpRC + g * kUpGR + 2 * rp + r;
-                    if (x >= W || y >= H)
+                    const int y = chunk * kUpGR + 2 * rp + r;
+                    if (!inside || y >= H)
                         continue;
                     const int64_t p = static_cast<int64_t>(y) * W + x;
                     if (!kFinish) {
@@ -377,29 +375,20 @@ __global__ void up_pack_weights_kernel(const float* __restrict__ w, int ci, int 
     wtc[i] = __float2half_rn(o < co && c < ci ? w[(o * 9 + t) * ci + c] : 0.0f);
 }
 
-// prepared input (u, v, luma as floats) -> the first layer's chunk plane (FP16, 5 zero channels)
-__global__ void up_input_half_kernel(const float* __restrict__ input, uint4* __restrict__ in16, int64_t npx)
-{
-    const int64_t p = blockIdx.x * static_cast<int64_t>(blockDim.x) + threadIdx.x;
-    if (p >= npx)
-        return;
-    const __half2 a = __floats2half2_rn(input[p * 3], input[p * 3 + 1]);
-    const __half2 b = __floats2half2_rn(input[p * 3 + 2], 0.0f);
-    in16[p] = make_uint4(*reinterpret_cast<const uint32_t*>(&a), *reinterpret_cast<const uint32_t*>(&b), 0u, 0u);
-}
-
 bool encode_act_map(CUtensorMap* m, const void* base, int N, int H, int W, int chunks)
 {
     EncodeTiledFn fn = tensor_map_encoder();
     if (!fn)
         return false;
-    const cuuint64_t dims[5] = {8, static_cast<cuuint64_t>(W), static_cast<cuuint64_t>(H),
-        static_cast<cuuint64_t>(chunks), static_cast<cuuint64_t>(N)};
-    const cuuint64_t plane = static_cast<cuuint64_t>(H) * W * 16;
-    const cuuint64_t strides[4] = {16, static_cast<cuuint64_t>(W) * 16, plane, plane * chunks};
-    const cuuint32_t box[5] = {8, kUpTW, 1, static_cast<cuuint32_t>(chunks), 1};
+    // a row of a chunk plane is W x 16 contiguous bytes: 2 W elements of 8 bytes,
+    // of which a box takes 256, the segment
+    const cuuint64_t dims[5] = {static_cast<cuuint64_t>(W) * 2, static_cast<cuuint64_t>(H),
+        static_cast<cuuint64_t>(chunks), static_cast<cuuint64_t>(N), 1};
+    const cuuint64_t row = static_cast<cuuint64_t>(W) * 16, plane = row * H;
+    const cuuint64_t strides[4] = {row, plane, plane * chunks, plane * chunks * N};
+    const cuuint32_t box[5] = {2 * kUpM, 1, static_cast<cuuint32_t>(chunks), 1, 1};
     const cuuint32_t estr[5] = {1, 1, 1, 1, 1};
-    return fn(m, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 5, const_cast<void*>(base), dims, strides, box, estr,
+    return fn(m, CU_TENSOR_MAP_DATA_TYPE_UINT64, 5, const_cast<void*>(base), dims, strides, box, estr,
                CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
                CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
@@ -422,11 +411,10 @@ cudaError_t run_layer(int l, const void* wtc, const float* prm, const void* in, 
     CUtensorMap m;
     if (!encode_act_map(&m, in, N, H, W, LCH))
         return cudaErrorInvalidValue;
-    const int items = N * ((H + kUpRC - 1) / kUpRC) * ((W + kUpM - 1) / kUpM);
-    up_conv_tc_kernel<KCH, LCH, NO, kFinish><<<std::min(items, sms), kUpThreads, smem, st>>>(m,
-        reinterpret_cast<const uint4*>(static_cast<const unsigned char*>(wtc) + kTcLayers[l].wt_off),
+    const int items = N * ((H + kUpGR - 1) / kUpGR) * ((W + kUpOut - 1) / kUpOut);
+    return launch_pdl(up_conv_tc_kernel<KCH, LCH, NO, kFinish>, dim3(std::min(items, sms)), dim3(kUpThreads), smem, st,
+        m, reinterpret_cast<const uint4*>(static_cast<const unsigned char*>(wtc) + kTcLayers[l].wt_off),
         prm + kUpLayers[l].b_off, kUpLayers[l].co, out, input, flow, s_out, max_residual, N, H, W, flag);
-    return cudaGetLastError();
 }
 
 }  // namespace
@@ -466,10 +454,6 @@ cudaError_t launch_upsampler_tc(const void* wtc, const float* prm, const float* 
     __half* in16 = reinterpret_cast<__half*>(wb);
     __half* actA = reinterpret_cast<__half*>(wb + npx * 16);
     __half* actB = reinterpret_cast<__half*>(wb + npx * 80);
-    up_input_half_kernel<<<static_cast<unsigned>((npx + 255) / 256), 256, 0, st>>>(input, reinterpret_cast<uint4*>(in16),
-        npx);
-    if ((e = cudaGetLastError()) != cudaSuccess)
-        return e;
     if ((e = run_layer<2, 1, 32, false>(0, wtc, prm, in16, actA, nullptr, nullptr, 0, 0.0f, N, H, W, sms, flag, st)) !=
         cudaSuccess)
         return e;
@@ -481,7 +465,7 @@ cudaError_t launch_upsampler_tc(const void* wtc, const float* prm, const float* 
         return e;
     e = run_layer<4, 4, 16, true>(3, wtc, prm, actA, nullptr, input, flow, s_out, max_residual, N, H, W, sms, flag, st);
     if (launches)
-        *launches += 5;
+        *launches += 4;
     return e;
 }
 
