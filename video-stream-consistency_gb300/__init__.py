@@ -226,10 +226,16 @@ def _check(status: int) -> None:
 
 
 def _stream(stream=None):
+    """The handle of `stream`, or of the current device's current stream (asked
+    for by itself: building the Stream object around it takes 2.9 us a call,
+    a quarter of a small operator's)."""
     import torch
 
-    s = stream if stream is not None else torch.cuda.current_stream()
-    return C.c_void_p(s.cuda_stream)
+    if stream is None:
+        if torch.cuda.is_initialized():
+            return C.c_void_p(torch._C._cuda_getCurrentRawStream(torch._C._cuda_getDevice()))
+        stream = torch.cuda.current_stream()
+    return C.c_void_p(stream.cuda_stream)
 
 
 def _f32(t, name):
