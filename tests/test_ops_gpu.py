@@ -35,6 +35,18 @@ def test_correlation_bit_exact(vsc, oracle, cuda, shape, md):
     assert np.array_equal(out, oracle.correlation(f1, f2, md))
 
 
+@pytest.mark.parametrize("legacy", [0, 1])
+@pytest.mark.parametrize("shape,md", [
+    ((1, 15, 8, 16), 4), ((1, 16, 8, 16), 4), ((2, 17, 3, 43), 4), ((1, 33, 1, 129), 2), ((1, 31, 16, 16), 7)])
+def test_correlation_channel_batches_bit_exact(vsc, oracle, cuda, shape, md, legacy):
+    """Small maps, whose channels are read 16 at a time: one short, exact, one
+    over, and blocks of 128 pixels with one over."""
+    f1 = RNG.standard_normal(shape).astype(np.float32)
+    f2 = RNG.standard_normal(shape).astype(np.float32)
+    out = vsc.correlation(_t(f1, cuda), _t(f2, cuda), md, legacy=legacy).cpu().numpy()
+    assert np.array_equal(out, oracle.correlation(f1, f2, md, legacy=legacy))
+
+
 @pytest.mark.parametrize("shape,md", [((1, 32, 24, 40), 4), ((2, 5, 7, 9), 4), ((1, 3, 6, 6), 2)])
 def test_correlation_legacy(vsc, oracle, cuda, shape, md):
     f1 = RNG.standard_normal(shape).astype(np.float32)
