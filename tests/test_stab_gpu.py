@@ -246,6 +246,24 @@ def test_consist_out_planes(vsc, oracle, cuda, form, w, h, iters):
     vsc.check_device()
 
 
+# Rounds of 12 steps (interiors of 104 x 40, exact, and 104 x 48): one round,
+# several, a short last one; a row left for the last row of tiles (361 = 9 * 40 + 1,
+# 81 = 2 * 40 + 1, 385 = 8 * 48 + 1, 97 = 2 * 48 + 1).
+@pytest.mark.parametrize("form,w,h,iters", [
+    ("exact", 640, 360, 12), ("exact", 641, 361, 35), ("exact", 99, 81, 12), ("exact", 521, 300, 11),
+    ("fma", 720, 404, 36), ("fma", 723, 385, 23), ("fma", 97, 41, 10), ("fma", 100, 97, 24)])
+def test_consist_out_planes_12_step_rounds(vsc, oracle, cuda, form, w, h, iters):
+    P, A, Wt, O0 = _img(h, w), _img(h, w), _img(h, w, hi=2.0), _img(h, w)
+    Wt[Wt < 0.3] = 0.0
+    O = _t(O0, cuda)
+    vsc.get_consist_out(_t(P, cuda), _t(A, cuda), _t(Wt, cuda), iters, 0.15, 0.15, O, form=form)
+    got = O.cpu().numpy()
+    ref = oracle.consist_out(P, A, Wt, iters, 0.15, 0.15, O0, form=form)
+    assert _equal_up_to_zero_sign(got, ref) if form == "exact" else np.array_equal(
+        got.view(np.uint32), ref.view(np.uint32))
+    vsc.check_device()
+
+
 def test_consist_out_fma_single_tile_shape(vsc, cuda):
     """The FMA form has one tile shape (128 x 72 of a plane); the autotuner
     reports it without measuring."""

@@ -861,8 +861,8 @@ constexpr int kGroupMax = 16;             // images of a grouped solve's launch
 constexpr int kPlW = 128;                 // tile width (a warp: 32 lanes x 4 columns)
 
 // How a solve in planes runs: its form (bit 0) and whether its rounds are 16
-// steps with a 16-pixel ring instead of 8 (bit 1).
-constexpr int kPlLong = 2;
+// steps with a 16-pixel ring (bit 1) or 12 with 12 (bit 2) instead of 8.
+constexpr int kPlLong = 2, kPlMid = 4;
 
 // A form's tile: kPlanes input planes, kWarps warps of kRPT rows each, and the
 // registers of the compute and the control warps.
@@ -882,6 +882,8 @@ struct PlG<kSolverExact> {  // O, U, consWt, lap P, A
     static constexpr int kComputeRegs = 224, kControlRegs = 56;
 };
 
+constexpr int pl_steps(int cfg) { return cfg & kPlLong ? 2 * kTbT : cfg & kPlMid ? 3 * kTbT / 2 : kTbT; }
+
 template <int kCfg>
 struct PlGeo : PlG<kCfg & 1> {
     using B = PlG<kCfg & 1>;
@@ -889,10 +891,10 @@ struct PlGeo : PlG<kCfg & 1> {
     using B::kRPT;
     using B::kWarps;
     static constexpr bool kFma = (kCfg & 1) == kSolverFma;
-    static constexpr int kT = kCfg & kPlLong ? 2 * kTbT : kTbT;  // steps a round, the ring's width
-    static constexpr int kIW = kPlW - 2 * kT;            // interior columns: 112, 96 in long rounds
+    static constexpr int kT = pl_steps(kCfg);            // steps a round, the ring's width: 8, 12, 16
+    static constexpr int kIW = kPlW - 2 * kT;            // interior columns: 112, 104, 96
     static constexpr int kRows = kRPT * kWarps;          // 72 (FMA), 64 (exact)
-    static constexpr int kIRows = kRows - 2 * kT;        // interior rows: 56, 48; 40, 32 in long rounds
+    static constexpr int kIRows = kRows - 2 * kT;        // interior rows: 56, 48, 40 (FMA), 48, 40, 32 (exact)
     static constexpr int kStage = kRows * kPlW;          // floats of one input tile
     static constexpr int kStageBytes = kStage * static_cast<int>(sizeof(float));
     static constexpr int kSlots = (kWarps + 2) * 2 * kPlW;  // edge-row slots of one buffer
@@ -1456,7 +1458,7 @@ template <int kCfg>
 __device__ __forceinline__ bool pl_deep(int h, int ty_n)
 {
     using G = PlGeo<kCfg>;
-    return (kCfg & kPlLong) && ty_n >= 3 && h - (ty_n - 1) * G::kIRows < G::kT;
+    return G::kT > kTbT && ty_n >= 3 && h - (ty_n - 1) * G::kIRows < G::kT;
 }
 
 template <int kCfg, int kN>
@@ -1495,8 +1497,8 @@ __device__ __forceinline__ PlJob pl_job(const PlSolve<kN>& g, int ticket)
     // frame's last row (rows h - 2 and h - 1 then sit in fixed rows of fixed
     // warps, where pl_row tests them without per-row tests), when its top ring
     // still lies in the row of tiles above (the 3 x 3 dependency holds) or, in
-    // long rounds, whose 16-pixel ring reaches further than 40 % of the frames'
-    // last rows of tiles, in the two rows above (pl_watched looks two rows up and
+    // longer rounds, whose 16-pixel ring reaches further than 40 % of the frames'
+    // last rows of tiles (12 pixels: 27 %), in the two rows above (pl_watched looks two rows up and
     // down there).  Its interior then overlaps those rows': both compute the
     // shared rows from the same inputs with the same arithmetic and store the
     // same bits.
@@ -1537,7 +1539,7 @@ __device__ __forceinline__ void pl_load_iterate(float* stage, const PlSolve<kN>&
 template <int kCfg, int kN>
 __device__ __forceinline__ const unsigned* pl_watched(const PlSolve<kN>& g, const PlJob& j, int lane)
 {
-    if (j.k == 0 || lane >= (kCfg & kPlLong ? 12 : 9))
+    if (j.k == 0 || lane >= (PlGeo<kCfg>::kT > kTbT ? 12 : 9))
         return nullptr;
     const int tx_n = g.tiles_x[j.p];
     const int per_plane = (g.tile0[j.p + 1] - g.tile0[j.p]) / 3;
@@ -1883,10 +1885,14 @@ cudaError_t device_info(DeviceInfo** out)
             cudaSuccess)
             return e;
         constexpr auto kAttr = cudaFuncAttributeMaxDynamicSharedMemorySize;
-        d.ps_smem = cudaFuncSetAttribute(solver_solve_kernel<kSolverFma | kPlLong, 1>, kAttr,
-                        PlGeo<kSolverFma | kPlLong>::kSmem) == cudaSuccess &&
-                    cudaFuncSetAttribute(solver_solve_kernel<kSolverExact | kPlLong, 1>, kAttr,
-                        PlGeo<kSolverExact | kPlLong>::kSmem) == cudaSuccess &&
+        auto single = [](auto c) {
+            return cudaFuncSetAttribute(solver_solve_kernel<decltype(c)::value, 1>, kAttr,
+                       PlGeo<decltype(c)::value>::kSmem) == cudaSuccess;
+        };
+        d.ps_smem = single(std::integral_constant<int, kSolverFma | kPlLong>{}) &&
+                    single(std::integral_constant<int, kSolverFma | kPlMid>{}) &&
+                    single(std::integral_constant<int, kSolverExact | kPlLong>{}) &&
+                    single(std::integral_constant<int, kSolverExact | kPlMid>{}) &&
                     cudaFuncSetAttribute(solver_persistent_kernel, kAttr, kPsSmem) == cudaSuccess &&
                     cudaFuncSetAttribute(solver_tall_kernel, kAttr, kPSmem) == cudaSuccess &&
                     set_group_smem<1>() && set_group_smem<4>() && set_group_smem<kGroupMax>() &&
@@ -2139,7 +2145,9 @@ int pl_tiles_of(int w, int h, int cfg)
     switch (cfg) {
         case kSolverFma: return pl_tiles<kSolverFma>(w, h);
         case kSolverFma | kPlLong: return pl_tiles<kSolverFma | kPlLong>(w, h);
+        case kSolverFma | kPlMid: return pl_tiles<kSolverFma | kPlMid>(w, h);
         case kSolverExact | kPlLong: return pl_tiles<kSolverExact | kPlLong>(w, h);
+        case kSolverExact | kPlMid: return pl_tiles<kSolverExact | kPlMid>(w, h);
         default: return pl_tiles<kSolverExact>(w, h);
     }
 }
@@ -2147,7 +2155,7 @@ int pl_counter_floats(int w, int h, int cfg) { return (16 + pl_tiles_of(w, h, cf
 
 // A plane's row in floats where the workspace has room for rows on the 16-byte
 // grid (TMA's), whatever the width.
-// 854x480, FMA form, 150 steps: 218 us; with plain loads, which a tile's steps
+// 854x480, FMA form, 150 steps: 164 us; with plain loads, which a tile's steps
 // wait for, and a launch a round 542 us.
 int pl_pitch(int w) { return (w + 3) & ~3; }
 
@@ -2215,17 +2223,38 @@ bool pl_tma_eligible(const DeviceInfo* di, int w, int h, const float* ws, size_t
     return di->ps_smem && aligned16p(ws) && ws_floats >= planes + pl_counter_floats(w, h, cfg);
 }
 
-// Rounds of 16 steps where a solve's rounds are chains of waits (for the
-// neighbours' stores, counters and loads: about 5 us) rather than work.  A ring
-// of 16 pixels leaves 42 % of an FMA tile as interior (exact form 37 %) against
-// 68 % (66 %) with 8, so only while an SM has at most 2.5 (FMA form) or one
-// (exact form) of a long round's tiles.  150 steps, 8-step and 16-step rounds:
-// FMA 320x180 166 and 118 us, 640x360 181 and 136, 854x480 197 and 179, 960x540
-// 220 and 218; exact 320x180 188 and 142, 480x270 194 and 171, 640x360 205 and 209.
-bool pl_long_rounds(const DeviceInfo* di, int w, int h, int num_iter, int form)
+// The rounds of a solve: 8, 12 or 16 steps.  Where an SM has few tiles a round
+// is a chain of waits (for the neighbours' stores, counters and loads: about 5 us)
+// and its steps, and long rounds need fewer of them; where it has many, a round
+// is its tiles' work, and a ring of 16 pixels leaves 42 % of an FMA tile as
+// interior (exact form 37 %), one of 12 54 (51) and one of 8 68 (66).  The time
+// of a round, measured at 17 sizes from 320x180 to 1280x720, is within a tenth
+// of the larger of `least` and base + tile * (tiles per SM); the cheapest
+// number of rounds is taken.  150 steps in us, 8, 12 and 16 a round:
+// FMA 320x180 147, 126, 109; 640x360 177, 145, 131; 854x480 196, 163, 177;
+// 960x540 195, 211, 217; 1280x720 290, 324, 385; exact 480x270 189, 162, 167;
+// 560x316 202, 170, 156; 640x360 204, 174, 199; 800x450 220, 227, 277.
+int pl_rounds_cfg(const DeviceInfo* di, int w, int h, int num_iter, int form)
 {
-    const int tiles = pl_tiles_of(w, h, form | kPlLong);
-    return num_iter > kTbT && 2 * tiles <= (form == kSolverFma ? 5 : 2) * di->sms;
+    struct Cost {
+        int cfg;
+        float least, base, tile;  // us
+    };
+    static constexpr Cost kCost[2][3] = {
+        {{0, 10.5f, 2.8f, 5.3f}, {kPlMid, 12.8f, 5.5f, 6.2f}, {kPlLong, 14.5f, 5.0f, 8.4f}},
+        {{0, 9.5f, 3.5f, 3.8f}, {kPlMid, 11.2f, 3.0f, 5.5f}, {kPlLong, 12.5f, 3.0f, 7.0f}}};
+    int best = form;
+    float best_us = 0.0f;
+    for (const Cost& c : kCost[form == kSolverFma]) {
+        const float tiles = static_cast<float>(pl_tiles_of(w, h, form | c.cfg)) / static_cast<float>(di->sms);
+        const float us = static_cast<float>(solve_launches(num_iter, pl_steps(c.cfg))) *
+                         std::max(c.least, c.base + c.tile * tiles);
+        if (c.cfg == 0 || us < best_us) {
+            best = form | c.cfg;
+            best_us = us;
+        }
+    }
+    return best;
 }
 
 // The exact form on interleaved images, a launch a round, where one wave of its
@@ -2347,14 +2376,13 @@ cudaError_t run_solver_planes(const DeviceInfo* di, int form, const float* P, co
     cudaStream_t st, int* nl, uint8_t* rgba_out, const float* Oc, int cw, int ch)
 {
     const bool tma = pl_tma_eligible(di, w, h, workspace, ws_floats, form);
-    int cfg = form;
-    if (tma && pl_long_rounds(di, w, h, num_iter, form) &&
-        pl_tma_eligible(di, w, h, workspace, ws_floats, form | kPlLong))
-        cfg |= kPlLong;
+    int cfg = tma ? pl_rounds_cfg(di, w, h, num_iter, form) : form;
+    if (!pl_tma_eligible(di, w, h, workspace, ws_floats, cfg))
+        cfg = form;
     const PlWs v = pl_view(workspace, w, h, tma ? pl_pitch(w) : w, cfg);
     cudaError_t e = launch_prep(form, P, A, Wt, Oi, v, v.O[0], w, h, step, v.cnt, v.ncnt, Oc, cw, ch, st);
     ++*nl;
-    const int nlaunch = solve_launches(num_iter, cfg & kPlLong ? 2 * kTbT : kTbT);
+    const int nlaunch = solve_launches(num_iter, pl_steps(cfg));
     if (e == cudaSuccess && tma) {
         const std::vector<PlWs> one(1, v);
         auto solve = [&](auto c) {
@@ -2363,7 +2391,9 @@ cudaError_t run_solver_planes(const DeviceInfo* di, int form, const float* P, co
         switch (cfg) {
             case kSolverFma: e = solve(std::integral_constant<int, kSolverFma>{}); break;
             case kSolverFma | kPlLong: e = solve(std::integral_constant<int, kSolverFma | kPlLong>{}); break;
+            case kSolverFma | kPlMid: e = solve(std::integral_constant<int, kSolverFma | kPlMid>{}); break;
             case kSolverExact | kPlLong: e = solve(std::integral_constant<int, kSolverExact | kPlLong>{}); break;
+            case kSolverExact | kPlMid: e = solve(std::integral_constant<int, kSolverExact | kPlMid>{}); break;
             default: e = solve(std::integral_constant<int, kSolverExact>{}); break;
         }
     } else if (e == cudaSuccess) {
