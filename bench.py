@@ -432,17 +432,16 @@ def solver_roofline(vsc, dev, stream, iters: int = 144, form: str = "exact"):
     A = torch.rand((H, W, 3), device=dev, generator=g)
     Wt = torch.rand((H, W, 3), device=dev, generator=g) * 2
     O = P.clone()
-    wsp = torch.empty(vsc.consist_out_workspace_size(W, H, form=form) // 4, dtype=torch.float32, device=dev)
     T = int(vsc.load().vsc_solver_steps_per_launch())
     torch.cuda.synchronize()
     for _ in range(2):
-        vsc.get_consist_out(P, A, Wt, iters, 0.15, 0.15, O, workspace=wsp, stream=stream, form=form)
+        vsc.get_consist_out(P, A, Wt, iters, 0.15, 0.15, O, stream=stream, form=form)
     ev = [torch.cuda.Event(enable_timing=True) for _ in range(4)]
     ev[0].record(stream)
-    vsc.get_consist_out(P, A, Wt, 8, 0.15, 0.15, O, workspace=wsp, stream=stream, form=form)
+    vsc.get_consist_out(P, A, Wt, 8, 0.15, 0.15, O, stream=stream, form=form)
     ev[1].record(stream)
     ev[2].record(stream)
-    vsc.get_consist_out(P, A, Wt, 8 + iters, 0.15, 0.15, O, workspace=wsp, stream=stream, form=form)
+    vsc.get_consist_out(P, A, Wt, 8 + iters, 0.15, 0.15, O, stream=stream, form=form)
     ev[3].record(stream)
     ev[3].synchronize()
     step_ms = (ev[2].elapsed_time(ev[3]) - ev[0].elapsed_time(ev[1])) / iters
@@ -452,12 +451,9 @@ def solver_roofline(vsc, dev, stream, iters: int = 144, form: str = "exact"):
     achieved = alg_bytes / (round_ms / 1000.0) / 1e9
     eff = SOLVER_BYTES_PER_PX * W * H * T / (round_ms / 1000.0) / 1e9
     traffic = SOLVER_TRAFFIC_BYTES.get(kname)
-    if form == "fma":
-        desc = (f"{kname} (one persistent launch per solve: rounds of {T} Jacobi steps on 128x72 tiles of one "
-                "channel plane, tiles taken in round order, each waiting for its neighbours' previous round; "
-                "1920x1080)")
-    else:
-        desc = f"{kname} (one launch per round of {T} Jacobi steps on 64x48 tiles of three channels; 1920x1080)"
+    desc = (f"{kname} (one persistent launch per solve: rounds of {T} Jacobi steps on 128x{72 if form == 'fma' else 64} "
+            "tiles of one channel plane, tiles taken in round order, each waiting for its neighbours' previous "
+            "round; 1920x1080)")
     line = {"bound": "hbm", "kernel": desc,
             "achieved": achieved, "peak": peak, "unit": "GB/s", "frac": achieved / peak,
             "traffic": traffic, "algorithmic_bytes_per_round": alg_bytes,
@@ -1148,25 +1144,25 @@ def run_gpu(args):
 # The full-resolution solver kernel of each form and its compulsory bytes per
 # 8-step round (per pixel): exact form O, U, A, consWt, lap P in (60) + O, U
 # out (24); FMA form O, U, nK, Cs in (48) + O, U out (24).
-SOLVER_KERNELS = {"exact": ("solver_tall_kernel", 84), "fma": ("solver_fma_solve_kernel", 72)}
+SOLVER_KERNELS = {"exact": ("solver_solve_kernel<exact>", 84), "fma": ("solver_solve_kernel<FMA>", 72)}
 # dram__bytes_read.sum + dram__bytes_write.sum of one 8-step round at
 # 1920x1080 from the ncu captures summarised in profiles/, and where each
 # comes from.
-SOLVER_TRAFFIC_BYTES = {"solver_tall_kernel": 144_198_912, "solver_fma_solve_kernel": 140_631_616}
+SOLVER_TRAFFIC_BYTES = {"solver_solve_kernel<exact>": 172_763_776, "solver_solve_kernel<FMA>": 144_740_288}
 SOLVER_TRAFFIC_SOURCE = {
-    "solver_tall_kernel": "profiles/solver_tall_1080p.md (one launch per round; mean of two launches: "
-                          "124,613,888 + 21,037,568 and 124,601,600 + 18,144,768 bytes)",
-    "solver_fma_solve_kernel": "profiles/solver_fma_solve_1080p.md (one launch per solve; per round, the "
-                               "difference of a 40-step and an 8-step solve over 4 rounds: (466,624,512 - "
-                               "99,649,280) read + (212,874,752 - 17,323,520) written, / 4)",
+    "solver_solve_kernel<exact>": "profiles/solver_solve_1080p.md (one launch per solve; per round, the difference "
+                                  "of a 40-step and an 8-step solve over 4 rounds: (617,573,120 - 124,665,344) read "
+                                  "+ (221,238,784 - 23,091,456) written, / 4)",
+    "solver_solve_kernel<FMA>": "profiles/solver_solve_1080p.md (one launch per solve; per round, the difference of a "
+                                "40-step and an 8-step solve over 4 rounds: (480,915,968 - 99,618,304) read + "
+                                "(215,260,672 - 17,597,184) written, / 4)",
 }
-# What bounds each solver kernel, from the same captures: the FP32 pipe and
-# its latency, not HBM (the time steps stay on chip): the FMA pipe's active
-# cycles per sub-partition cycle (sm__pipe_fma_cycles_active / 4 /
-# sm__cycles_active) and smsp__issue_active.
+# What bounds each solver kernel, from the same captures: FP32 issue and the
+# exchange between warps, not HBM alone (the time steps stay on chip): the FMA
+# pipe's warp instructions per scheduler and cycle, and smsp__issue_active.
 SOLVER_PIPE = {
-    "solver_tall_kernel": {"fma_pipe_active": None, "issue_active": 0.585},
-    "solver_fma_solve_kernel": {"fma_pipe_active": 0.647, "issue_active": 0.448},
+    "solver_solve_kernel<exact>": {"fma_pipe_active": 0.542, "issue_active": 0.622},
+    "solver_solve_kernel<FMA>": {"fma_pipe_active": 0.435, "issue_active": 0.535},
 }
 
 
