@@ -64,8 +64,9 @@ VSC_API vsc_status vsc_check_device(void);
  * returns VSC_ETIMEOUT.  No fault, trap or hang is involved. */
 VSC_API vsc_status vsc_selftest_bounded_wait(int32_t spins, vsc_stream_t stream);
 
-/* Jacobi steps of the blend solver per kernel launch (temporal blocking);
- * a property of the build, for profiling tools. */
+/* Jacobi steps of the blend solver per round of its tiles on large frames
+ * (temporal blocking; small frames take 12 or 16); a property of the build, for
+ * profiling tools. */
 VSC_API int32_t vsc_solver_steps_per_launch(void);
 
 /* Tile-shape autotuner of the blend solver's exact form on interleaved images
