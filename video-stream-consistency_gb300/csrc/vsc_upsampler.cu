@@ -86,7 +86,7 @@ __global__ void prepare_kernel(const float* __restrict__ coarse, int cw, int ch,
 // 64 batch in 274 us forward and 369 us backward; weight gradients with one
 // block per (output, tap), which re-read the whole activation with a stride
 // for each of the 288 blocks, took 919 us.  The layer's 1.2 G FMAs are 30 us
-// at 152 x 128 lanes.
+// at 152 x 128 lanes; now 70 forward, 68 backward, 72 for the weights.
 
 __device__ __forceinline__ void cp_async4(float* dst, const float* src, bool valid)
 {
@@ -110,27 +110,57 @@ constexpr int kPitch = 36;   // its shared-memory pitch: 34 with the halo; 4 mod
 
 enum ConvMode { kConvRelu, kConvLoss, kConvBwd };
 
-// The convolution of one 32 x (8 PG) pixel tile.  A thread keeps 8 adjacent
-// pixels x OCT output channels; a warp covers 32 x 8 pixels of one channel
-// group, so its weight reads are broadcasts and its pixel reads (10 values
-// for the 8 pixels' three horizontal taps) conflict-free 16-byte words: per
-// input channel and tap row, 2.5 + 3 OCT / 4 reads for 24 OCT FMAs.  Channels
-// stream in chunks of CC through two cp.async buffers (zero outside the
-// image, the convolution's padding).
+// The convolution of one 32 x 8 pixel tile.  A thread keeps PX adjacent pixels
+// x OCT output channels; its weight reads are broadcasts.  Every sum runs over
+// the taps in order with the channels of a tap inside, as the per-pixel loops
+// it replaces had it, so activations and ReLU signs keep their bits; all
+// channels of the tile and all weights are therefore in shared memory at once (93
+// KB for 32 channels, two blocks an SM).  The pixels' window at a horizontal
+// tap is 8 of 10 values: two 16-byte words and at most one value more, rows on a
+// pitch that keeps them free of bank conflicts; weights in the parameters' own
+// layout, read four channels (forward) or four outputs (backward) at a time.
+// Per tap and four channels 8 x 8 registers take 8 + 11 reads for 256 FMAs.
+constexpr int kConvPitch = 44;  // columns x0 - 4 ... x0 + 39: x0 on a 16-byte boundary; 12 mod 32
+
 template <int CI, int CO, int OCT>
 struct ConvShape {
-    static constexpr int CC = CI < 8 ? CI : 8;
-    static constexpr int chunks = (CI + CC - 1) / CC;
-    static constexpr int OG = CO / OCT;          // channel groups
-    static constexpr int PG = 4 / OG;            // 32 x 8 pixel groups of the tile
-    static constexpr int rows = 8 * PG;
-    static constexpr int plane = (rows + 2) * kPitch;
-    static constexpr int wp = 9 * CO + 4;        // weights [c][tap][o]; + 4 spreads the transposing writes
-    static constexpr int buf = (CC * plane + CC * wp + 3) / 4 * 4;
-    static constexpr int bufs = chunks > 1 ? 2 : 1;
-    static constexpr int smem = bufs * buf * 4;
-    static_assert(CI % CC == 0 && OG * PG == 4 && (CC * plane) % 4 == 0 && wp % (OCT < 4 ? 2 : 4) == 0, "tile");
+    static constexpr int OG = CO / OCT;             // channel groups
+    static constexpr int rows = 8;
+    static constexpr int PX = 32 * rows * OG / 128;  // pixels a thread
+    static constexpr int kG = kTileW / PX;          // threads of a tile row
+    static constexpr int plane = (rows + 2) * kConvPitch;
+    static constexpr int weights = CI * 9 * CO;
+    static constexpr int smem = (CI * plane + weights) * 4;
+    static_assert((PX == 8 || PX == 2) && weights % 4 == 0 && (CI * plane) % 4 == 0, "tile");
 };
+
+__device__ __forceinline__ void cp_async16(float* dst, const float* src, bool valid)
+{
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(
+                     static_cast<uint32_t>(__cvta_generic_to_shared(dst))),
+        "l"(src), "r"(valid ? 16 : 0)
+        : "memory");
+}
+
+// v[i] = p[kx + i], p four bytes below a 16-byte boundary
+template <int PX>
+__device__ __forceinline__ void conv_window(const float* p, int kx, float (&v)[PX])
+{
+    if constexpr (PX == 8) {
+        const float4 a = *reinterpret_cast<const float4*>(p + 1), b = *reinterpret_cast<const float4*>(p + 5);
+        const float w[8] = {a.x, a.y, a.z, a.w, b.x, b.y, b.z, b.w};
+        const float e = kx == 0 ? p[0] : kx == 2 ? p[9] : 0.0f;
+#pragma unroll
+        for (int i = 0; i < 8; ++i) {
+            const int j = i + kx - 1;
+            v[i] = j < 0 || j > 7 ? e : w[j & 7];
+        }
+    } else {
+#pragma unroll
+        for (int i = 0; i < PX; ++i)
+            v[i] = p[kx + i];
+    }
+}
 
 // x: planes (kInter: interleaved CI-channel pixels).  kConvRelu: y = ReLU(conv
 // + bias).  kConvLoss (the last layer): the L1 loss of base + r against the
@@ -139,114 +169,125 @@ struct ConvShape {
 // nonfinite: set when a value the weight gradients will multiply (the input
 // or an activation) is not finite.
 template <int CI, int CO, int OCT, int kMode, bool kInter>
-__global__ void __launch_bounds__(128, 4) conv3x3_kernel(const float* __restrict__ x, const float* __restrict__ wts,
+__global__ void __launch_bounds__(128, 2) conv3x3_kernel(const float* __restrict__ x, const float* __restrict__ wts,
     const float* __restrict__ bias, const float* __restrict__ a_prev, float* __restrict__ y, int H, int W, int tiles_x,
     const float* __restrict__ input, const float* __restrict__ target, float* __restrict__ loss, float inv,
     int* __restrict__ nonfinite)
 {
     using S = ConvShape<CI, CO, OCT>;
+    constexpr int PX = S::PX;
     extern __shared__ __align__(16) float sm[];
-    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    const int og = warp % S::OG, pg = warp / S::OG;
-    const int g = lane & 3, r = pg * 8 + (lane >> 2);  // this thread's 8-pixel group and tile row
+    float* sw = sm + CI * S::plane;
+    const int tid = threadIdx.x, lane = tid & 31;
+    const int og = tid / (8 * S::kG), g = tid % S::kG, r = tid / S::kG % 8;  // channel group, pixel group, tile row
     const int x0 = (blockIdx.x % tiles_x) * kTileW, y0 = (blockIdx.x / tiles_x) * S::rows;
     const int64_t HW = static_cast<int64_t>(H) * W;
     const int n = blockIdx.y;
     const float* xn = x + static_cast<int64_t>(n) * HW * CI;
 
-    auto stage = [&](int chunk, float* b) {
-        const int c0 = chunk * S::CC;
-        for (int i = tid; i < S::CC * (S::rows + 2) * 34; i += 128) {
-            const int c = i / ((S::rows + 2) * 34), rem = i % ((S::rows + 2) * 34);
-            const int row = rem / 34, col = rem % 34;
+    for (int i = tid; i < S::weights / 4; i += 128)
+        cp_async16(sw + 4 * i, wts + 4 * i, true);
+    if (!kInter && (W & 3) == 0) {  // planes and rows start on the 16-byte grid: a vector is in the image or not
+        for (int i = tid; i < CI * (S::rows + 2) * 8; i += 128) {
+            const int q = i & 7, row = i / 8 % (S::rows + 2), c = i / (8 * (S::rows + 2));
+            const int gy = y0 - 1 + row, gx = x0 + 4 * q;
+            const bool ok = gy >= 0 && gy < H && gx < W;
+            cp_async16(sm + c * S::plane + row * kConvPitch + 4 + 4 * q,
+                xn + c * HW + (ok ? static_cast<int64_t>(gy) * W + gx : 0), ok);
+        }
+        for (int i = tid; i < CI * (S::rows + 2) * 2; i += 128) {
+            const int q = i & 1, row = i / 2 % (S::rows + 2), c = i / (2 * (S::rows + 2));
+            const int gy = y0 - 1 + row, gx = x0 + (q ? 32 : -1);
+            const bool ok = gy >= 0 && gy < H && gx >= 0 && gx < W;
+            cp_async4(sm + c * S::plane + row * kConvPitch + (q ? 36 : 3),
+                xn + c * HW + (ok ? static_cast<int64_t>(gy) * W + gx : 0), ok);
+        }
+    } else {
+        for (int i = tid; i < CI * (S::rows + 2) * 34; i += 128) {
+            const int col = i % 34, row = i / 34 % (S::rows + 2), c = i / (34 * (S::rows + 2));
             const int gy = y0 - 1 + row, gx = x0 - 1 + col;
             const bool ok = gy >= 0 && gy < H && gx >= 0 && gx < W;
             const int64_t p = ok ? static_cast<int64_t>(gy) * W + gx : 0;
-            cp_async4(b + c * S::plane + row * kPitch + col, xn + (kInter ? p * CI + c0 + c : (c0 + c) * HW + p), ok);
+            cp_async4(sm + c * S::plane + row * kConvPitch + 3 + col, xn + (kInter ? p * CI + c : c * HW + p), ok);
         }
-        float* sw = b + S::CC * S::plane;
-        for (int i = tid; i < S::CC * 9 * CO; i += 128) {
-            if (kMode == kConvBwd) {  // the layer's weights [in = its outputs][tap][out], taps flipped
-                const int o = i % CO, t = (i / CO) % 9, c = i / (9 * CO);
-                cp_async4(sw + c * S::wp + t * CO + o, wts + ((c0 + c) * 9 + 8 - t) * CO + o, true);
-            } else {
-                const int c = i % S::CC, t = (i / S::CC) % 9, o = i / (9 * S::CC);
-                cp_async4(sw + c * S::wp + t * CO + o, wts + (o * 9 + t) * CI + c0 + c, true);
-            }
-        }
-        cp_async_commit();
-    };
+    }
+    cp_async_commit();
 
-    float acc[8][OCT];
+    float acc[PX][OCT];
 #pragma unroll
     for (int o = 0; o < OCT; ++o) {
         const float b = kMode == kConvBwd ? 0.0f : bias[og * OCT + o];
 #pragma unroll
-        for (int i = 0; i < 8; ++i)
+        for (int i = 0; i < PX; ++i)
             acc[i][o] = b;
     }
-    stage(0, sm);
     bool bad = false;
-    for (int k = 0; k < S::chunks; ++k) {
-        float* b = sm + (k % S::bufs) * S::buf;
-        if (k + 1 < S::chunks)
-            stage(k + 1, sm + ((k + 1) % S::bufs) * S::buf);
-        if (k + 1 < S::chunks)
-            cp_async_wait<1>();
-        else
-            cp_async_wait<0>();
-        __syncthreads();
-        if (kInter && kMode == kConvRelu)  // the layer's own input feeds its weight gradient
-            for (int i = tid; i < S::CC * (S::rows + 2) * 34; i += 128) {
-                const int c = i / ((S::rows + 2) * 34), rem = i % ((S::rows + 2) * 34);
-                bad = bad || !finite_f(b[c * S::plane + rem / 34 * kPitch + rem % 34]);
-            }
-        const float* xp = b + r * kPitch + 8 * g;
-        const float* wq = b + S::CC * S::plane + og * OCT;
+    cp_async_wait<0>();
+    __syncthreads();
+    if (kInter && kMode == kConvRelu)  // the layer's own input feeds its weight gradient
+        for (int i = tid; i < CI * (S::rows + 2) * 34; i += 128) {
+            const int col = i % 34, row = i / 34 % (S::rows + 2), c = i / (34 * (S::rows + 2));
+            bad = bad || !finite_f(sm[c * S::plane + row * kConvPitch + 3 + col]);
+        }
+    // tap (ky, kx) of the layer; backward reads the output pixel whose tap it was
 #pragma unroll 1
-        for (int c = 0; c < S::CC; ++c, xp += S::plane, wq += S::wp) {
+    for (int ky = 0; ky < 3; ++ky) {
+        const float* xr = sm + (r + (kMode == kConvBwd ? 2 - ky : ky)) * kConvPitch + 3 + PX * g;
 #pragma unroll
-            for (int ky = 0; ky < 3; ++ky) {
-                const float4 v0 = *reinterpret_cast<const float4*>(xp + ky * kPitch);
-                const float4 v1 = *reinterpret_cast<const float4*>(xp + ky * kPitch + 4);
-                const float2 v2 = *reinterpret_cast<const float2*>(xp + ky * kPitch + 8);
-                const float v[10] = {v0.x, v0.y, v0.z, v0.w, v1.x, v1.y, v1.z, v1.w, v2.x, v2.y};
+        for (int kx = 0; kx < 3; ++kx) {
+            constexpr int kC = CI % 4 == 0 ? 4 : 1;
+            const int t = ky * 3 + kx, dx = kMode == kConvBwd ? 2 - kx : kx;
+#pragma unroll 1
+            for (int c0 = 0; c0 < CI; c0 += kC) {
+                float w[kC][OCT];
+                if constexpr (kMode == kConvBwd) {  // [in = its outputs][tap][out]
 #pragma unroll
-                for (int kx = 0; kx < 3; ++kx) {
-                    float w[OCT];
-                    const float* wt = wq + (ky * 3 + kx) * CO;
-                    if constexpr (OCT % 4 == 0) {
+                    for (int c = 0; c < kC; ++c)
 #pragma unroll
                         for (int q = 0; q < OCT / 4; ++q) {
-                            const float4 f = *reinterpret_cast<const float4*>(wt + 4 * q);
-                            w[4 * q] = f.x;
-                            w[4 * q + 1] = f.y;
-                            w[4 * q + 2] = f.z;
-                            w[4 * q + 3] = f.w;
+                            const float4 f =
+                                *reinterpret_cast<const float4*>(sw + ((c0 + c) * 9 + t) * CO + og * OCT + 4 * q);
+                            w[c][4 * q] = f.x;
+                            w[c][4 * q + 1] = f.y;
+                            w[c][4 * q + 2] = f.z;
+                            w[c][4 * q + 3] = f.w;
                         }
-                    } else {
-                        const float2 f = *reinterpret_cast<const float2*>(wt);
-                        w[0] = f.x;
-                        w[1] = f.y;
-                    }
+                } else {  // [out][tap][in]
 #pragma unroll
-                    for (int i = 0; i < 8; ++i)
+                    for (int o = 0; o < OCT; ++o) {
+                        const float* q = sw + ((og * OCT + o) * 9 + t) * CI + c0;
+                        if constexpr (kC == 4) {
+                            const float4 f = *reinterpret_cast<const float4*>(q);
+                            w[0][o] = f.x;
+                            w[1][o] = f.y;
+                            w[2][o] = f.z;
+                            w[3][o] = f.w;
+                        } else {
+                            w[0][o] = q[0];
+                        }
+                    }
+                }
+#pragma unroll
+                for (int c = 0; c < kC; ++c) {
+                    float v[PX];
+                    conv_window<PX>(xr + (c0 + c) * S::plane, dx, v);
+#pragma unroll
+                    for (int i = 0; i < PX; ++i)
 #pragma unroll
                         for (int o = 0; o < OCT; ++o)
-                            acc[i][o] = __fmaf_rn(w[o], v[i + kx], acc[i][o]);
+                            acc[i][o] = __fmaf_rn(w[c][o], v[i], acc[i][o]);
                 }
             }
         }
-        __syncthreads();  // the buffer is refilled two chunks on
     }
 
-    const int py = y0 + r, px = x0 + 8 * g;
+    const int py = y0 + r, px = x0 + PX * g;
     const bool row_in = py < H;
     const int64_t p = static_cast<int64_t>(py) * W + px;
     if constexpr (kMode == kConvLoss) {
         float l = 0.0f;
 #pragma unroll
-        for (int i = 0; i < 8; ++i) {
+        for (int i = 0; i < PX; ++i) {
             if (!row_in || px + i >= W)
                 continue;
             const int64_t q = n * HW + p + i;
@@ -259,8 +300,13 @@ __global__ void __launch_bounds__(128, 4) conv3x3_kernel(const float* __restrict
         }
         for (int o = 16; o > 0; o >>= 1)
             l += __shfl_xor_sync(0xffffffffu, l, o);
+        // one add a block: the running sum is rounded a quarter as often
+        __syncthreads();
         if (lane == 0)
-            atomicAdd(loss, l * inv);
+            sm[tid >> 5] = l;
+        __syncthreads();
+        if (tid == 0)
+            atomicAdd(loss, ((sm[0] + sm[1]) + (sm[2] + sm[3])) * inv);
     } else {
         const bool vec = (W & 3) == 0;  // planes and rows then start on the 16-byte grid
 #pragma unroll
