@@ -86,6 +86,21 @@ def test_lowp_correlation_chunk_widths_and_row_blocks(vsc, oracle, cuda, shape, 
     vsc.check_device()
 
 
+@pytest.mark.parametrize("operand", [0, 1])
+def test_lowp_correlation_result_over_an_operand(vsc, oracle, cuda, operand):
+    """The operands are converted before the result is written, so the result may
+    take an operand's memory."""
+    import torch
+
+    shape = (1, 81, 20, 40)
+    f = [(RNG.integers(-3, 4, shape) * 0.25).astype(np.float32) for _ in range(2)]
+    d = [_t(a, cuda) for a in f]
+    out = vsc.correlation_lowp(d[0], d[1], 4, "bf16", out=d[operand].view(1, 9, 9, 20, 40))
+    assert out.data_ptr() == d[operand].data_ptr()
+    assert np.array_equal(out.cpu().numpy(), oracle.correlation(f[0], f[1], 4))
+    vsc.check_device()
+
+
 @pytest.mark.parametrize("dtype", ["bf16", "fp16"])
 def test_lowp_correlation_pwc_pyramid_640x360(vsc, oracle, cuda, dtype):
     """The five PWC levels of a 640x360 frame pair (C = 32..196); error

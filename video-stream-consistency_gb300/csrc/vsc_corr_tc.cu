@@ -35,6 +35,7 @@
 #include <cuda_bf16.h>
 #include <cuda_fp16.h>
 
+#include <functional>
 #include <mutex>
 
 namespace vsc {
@@ -841,16 +842,20 @@ cudaError_t launch_corr_tc(const float* f1, const float* f2, float* out, int N, 
     if (e != cudaSuccess)
         return e;
     // Three launches: partial maxima (kept at the front of `out`, which the
-    // correlation overwrites; behind the scales when it has no 64 elements), both operands' conversion with the scales
+    // correlation overwrites; behind the scales when it has no 64 elements or shares
+    // memory with an operand), both operands' conversion with the scales
     // worked out by every block, the correlation.  (A memset, a maximum and a
     // conversion per operand and a launch for the scales: a call of 2 x 64 x 136 x
     // 240 then took 60 us back to back, now 35; of 130 x 34 x 60, 29 and 14.)
     const int64_t total = static_cast<int64_t>(N) * C * H * W;
     const int64_t outs = static_cast<int64_t>(N) * (2 * md + 1) * (2 * md + 1) * H * W;
-    float* part = outs >= 64 ? out : scales + 8;
+    auto apart = [&](const float* f) { return std::less_equal<const float*>()(f + total, out) ||
+                                              std::less_equal<const float*>()(out + outs, f); };
+    const bool in_out = outs >= 64 && apart(f1) && apart(f2);
+    float* part = in_out ? out : scales + 8;
     const int64_t want = std::min<int64_t>((total / 4 + 1023) / 1024, 2 * sms);  // 4+ vectors a thread
     const unsigned parts = static_cast<unsigned>(
-        std::max<int64_t>(1, std::min<int64_t>(want, outs >= 64 ? outs / 2 : 28)));
+        std::max<int64_t>(1, std::min<int64_t>(want, in_out ? outs / 2 : 28)));
     auto a16 = [](const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15) == 0; };
     e = launch_pdl(absmax2_kernel, dim3(parts, 2), dim3(256), 0, st, f1, f2, total, a16(f1) && a16(f2) ? 1 : 0, part);
     if (e != cudaSuccess)
