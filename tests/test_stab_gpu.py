@@ -250,8 +250,8 @@ def test_consist_out_planes(vsc, oracle, cuda, form, w, h, iters):
 # several, a short last one; a row left for the last row of tiles (361 = 9 * 40 + 1,
 # 81 = 2 * 40 + 1, 385 = 8 * 48 + 1, 97 = 2 * 48 + 1).
 @pytest.mark.parametrize("form,w,h,iters", [
-    ("exact", 640, 360, 12), ("exact", 641, 361, 35), ("exact", 99, 81, 12), ("exact", 521, 300, 11),
-    ("fma", 720, 404, 36), ("fma", 723, 385, 23), ("fma", 97, 41, 10), ("fma", 100, 97, 24)])
+    ("exact", 640, 360, 36), ("exact", 641, 361, 35), ("exact", 99, 81, 12), ("exact", 521, 300, 35),
+    ("fma", 720, 404, 36), ("fma", 723, 385, 35), ("fma", 97, 41, 10), ("fma", 100, 97, 24)])
 def test_consist_out_planes_12_step_rounds(vsc, oracle, cuda, form, w, h, iters):
     P, A, Wt, O0 = _img(h, w), _img(h, w), _img(h, w, hi=2.0), _img(h, w)
     Wt[Wt < 0.3] = 0.0

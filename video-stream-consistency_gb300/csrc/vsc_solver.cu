@@ -2227,13 +2227,18 @@ bool pl_tma_eligible(const DeviceInfo* di, int w, int h, const float* ws, size_t
 // is a chain of waits (for the neighbours' stores, counters and loads: about 5 us)
 // and its steps, and long rounds need fewer of them; where it has many, a round
 // is its tiles' work, and a ring of 16 pixels leaves 42 % of an FMA tile as
-// interior (exact form 37 %), one of 12 54 (51) and one of 8 68 (66).  The time
-// of a round, measured at 17 sizes from 320x180 to 1280x720, is within a tenth
-// of the larger of `least` and base + tile * (tiles per SM); the cheapest
-// number of rounds is taken.  150 steps in us, 8, 12 and 16 a round:
-// FMA 320x180 147, 126, 109; 640x360 177, 145, 131; 854x480 196, 163, 177;
-// 960x540 195, 211, 217; 1280x720 290, 324, 385; exact 480x270 189, 162, 167;
-// 560x316 202, 170, 156; 640x360 204, 174, 199; 800x450 220, 227, 277.
+// interior (exact form 37 %), one of 12 54 (51) and one of 8 68 (66).  A round's
+// time, measured at 17 sizes from 320x180 to 1280x720, is the larger of `least`
+// and base + tile * (tiles per SM) within a tenth, so longer rounds are taken
+// where their estimate is a tenth below that of 8.  They are not where three
+// 8-step tiles an SM or more make a round work alone (1920x1080, 150 steps in
+// rounds of 8 and 12: FMA 657 and 711 us, exact 913 and 1,009), nor, beyond the
+// smallest frames, for a few rounds, whose first loads nothing hides (exact
+// 854x480, 12 steps: 36 us in two rounds of 8, 42 in one of 12).  150 steps in
+// us, 8, 12 and 16 a round: FMA 320x180 147, 126, 109; 640x360 177, 145, 131;
+// 854x480 196, 163, 177; 960x540 195, 211, 217; 1280x720 290, 324, 385; exact
+// 480x270 189, 162, 167; 560x316 202, 170, 156; 640x360 204, 174, 199; 800x450
+// 220, 227, 277.
 int pl_rounds_cfg(const DeviceInfo* di, int w, int h, int num_iter, int form)
 {
     struct Cost {
@@ -2242,16 +2247,21 @@ int pl_rounds_cfg(const DeviceInfo* di, int w, int h, int num_iter, int form)
     };
     static constexpr Cost kCost[2][3] = {
         {{0, 10.5f, 2.8f, 5.3f}, {kPlMid, 12.8f, 5.5f, 6.2f}, {kPlLong, 14.5f, 5.0f, 8.4f}},
-        {{0, 9.5f, 3.5f, 3.8f}, {kPlMid, 11.2f, 3.0f, 5.5f}, {kPlLong, 12.5f, 3.0f, 7.0f}}};
+        {{0, 9.4f, 5.6f, 2.9f}, {kPlMid, 11.2f, 2.6f, 5.5f}, {kPlLong, 12.5f, 3.0f, 7.0f}}};
+    const int tiles8 = pl_tiles_of(w, h, form);
+    if (tiles8 > 3 * di->sms || (num_iter < 4 * kTbT && 5 * tiles8 > 3 * di->sms))
+        return form;
     int best = form;
-    float best_us = 0.0f;
+    float limit = 0.0f;
     for (const Cost& c : kCost[form == kSolverFma]) {
         const float tiles = static_cast<float>(pl_tiles_of(w, h, form | c.cfg)) / static_cast<float>(di->sms);
         const float us = static_cast<float>(solve_launches(num_iter, pl_steps(c.cfg))) *
                          std::max(c.least, c.base + c.tile * tiles);
-        if (c.cfg == 0 || us < best_us) {
+        if (c.cfg == 0) {
+            limit = 0.9f * us;
+        } else if (us < limit) {
             best = form | c.cfg;
-            best_us = us;
+            limit = us;
         }
     }
     return best;
