@@ -109,6 +109,21 @@ VSC_API vsc_status vsc_solver_autotune_form(int32_t width, int32_t height, int32
     int32_t* tile_rows);
 VSC_API int32_t vsc_solver_tile_rows_form(int32_t width, int32_t height, int32_t form, int32_t* tuned);
 
+/* How a solve of num_iter steps in a 16-byte aligned workspace of
+ * workspace_bytes (0: the library's own, workspace = NULL) runs on a device of
+ * `sms` streaming multiprocessors (0: the current device's; otherwise no device is
+ * asked), for profiling tools and tests: a property of the build, not of its
+ * results.  No counterpart in the reference. */
+typedef struct vsc_solve_plan {
+    int32_t planes;            /* 1: on planes, a channel each; 0: on interleaved images */
+    int32_t steps;             /* Jacobi steps of a round (the last may be shorter) */
+    int32_t rounds;
+    int32_t tiles;             /* of a round */
+    int32_t rounds_per_launch; /* at most; a long solve is several launches */
+} vsc_solve_plan;
+VSC_API vsc_status vsc_solver_plan(int32_t width, int32_t height, int32_t num_iter, int32_t form,
+    size_t workspace_bytes, int32_t sms, vsc_solve_plan* out);
+
 /* ========================================================================
  * ONNX Runtime custom ops (domain "custom")
  * ======================================================================== */

@@ -264,6 +264,31 @@ def test_consist_out_planes_12_step_rounds(vsc, oracle, cuda, form, w, h, iters)
     vsc.check_device()
 
 
+@pytest.mark.parametrize("form,w", [("exact", 1920), ("fma", 1921)])
+def test_solve_of_several_launches(vsc, cuda, form, w):
+    """More steps than a launch of the solve kernel takes: the solve goes on in a
+    second and a third one.  The comparison runs a launch a round in a workspace
+    without room for padded planes (interleaved images; plain loads), with the
+    same bits.  Without weights the solve is a diffusion, which still moves."""
+    import torch
+
+    h = 1080
+    p = vsc.solver_plan(w, h, 1 << 20, form)
+    iters = 2 * p.steps * p.rounds_per_launch + 3
+    assert p.planes and vsc.solver_plan(w, h, iters, form).rounds_per_launch < iters // p.steps // 2 + 1
+    rng = np.random.Generator(np.random.PCG64(w))
+    P, A, O0 = (torch.from_numpy(rng.random((h, w, 3), dtype=np.float32)).to(cuda) for _ in range(3))
+    Wt = torch.zeros_like(P)
+    ws = torch.empty(vsc.consist_out_workspace_size(w, h, form) // 4, dtype=torch.float32, device=cuda)
+    O, ref, before = O0.clone(), O0.clone(), O0.clone()
+    vsc.get_consist_out(P, A, Wt, iters, 0.15, 0.15, O, form=form)
+    vsc.get_consist_out(P, A, Wt, iters, 0.15, 0.15, ref, form=form, workspace=ws)
+    vsc.get_consist_out(P, A, Wt, iters - 1, 0.15, 0.15, before, form=form)
+    assert torch.equal(O.view(torch.int32), ref.view(torch.int32))
+    assert (O != before).float().mean() > 0.01
+    vsc.check_device()
+
+
 def test_consist_out_fma_single_tile_shape(vsc, cuda):
     """The FMA form has one tile shape (128 x 72 of a plane); the autotuner
     reports it without measuring."""

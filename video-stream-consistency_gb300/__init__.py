@@ -48,7 +48,7 @@ EXPORTED = [
     "vsc_multistream_set_fused", "vsc_multistream_fused", "vsc_multistream_set_upsampler",
     "vsc_stabilizer_synchronize", "vsc_stabilizer_wait_output",
     "vsc_get_consist_out_fma", "vsc_consist_out_fma_workspace_size", "vsc_solver_autotune_form",
-    "vsc_solver_tile_rows_form",
+    "vsc_solver_tile_rows_form", "vsc_solver_plan",
     "vsc_stabilizer_set_solver_form", "vsc_multistream_set_solver_form", "vsc_write_jpeg",
 ]
 VSC_DTYPE_F32, VSC_DTYPE_BF16, VSC_DTYPE_F16 = 0, 1, 2
@@ -88,6 +88,10 @@ class FilesConfig(C.Structure):
 
 class StreamDesc(C.Structure):
     _fields_ = [("width", C.c_int32), ("height", C.c_int32), ("flow_downscale", C.c_int32), ("corr_dtype", C.c_int32)]
+
+
+class SolvePlan(C.Structure):
+    _fields_ = [(n, C.c_int32) for n in ("planes", "steps", "rounds", "tiles", "rounds_per_launch")]
 
 
 class StabilizerConfig(C.Structure):
@@ -139,6 +143,7 @@ def load():
         "vsc_get_consist_out": [IP, IP, IP, i32, f32, f32, IP, vp, C.c_size_t, vp],
         "vsc_get_consist_out_fma": [IP, IP, IP, i32, f32, f32, IP, vp, C.c_size_t, vp],
         "vsc_solver_autotune_form": [i32, i32, i32, vp, C.POINTER(i32)],
+        "vsc_solver_plan": [i32, i32, i32, i32, C.c_size_t, i32, C.POINTER(SolvePlan)],
         "vsc_stabilizer_set_solver_form": [vp, i32],
         "vsc_multistream_set_solver_form": [vp, i32],
         "vsc_get_consist_out_noalloc": [IP, IP, IP, i32, f32, f32, IP, vp],
@@ -475,6 +480,15 @@ def solver_tile_rows(w: int, h: int, form: str = "exact"):
 
 def solver_set_autotune(on: bool) -> None:
     load().vsc_solver_set_autotune(1 if on else 0)
+
+
+def solver_plan(w: int, h: int, num_iter: int, form: str = "exact", workspace_bytes: int = 0,
+                sms: int = 0) -> SolvePlan:
+    """How a solve runs (vsc_solver_plan); with `sms` given, no device is asked."""
+    p = SolvePlan()
+    _check(load().vsc_solver_plan(int(w), int(h), int(num_iter), SOLVER_FORMS[form], int(workspace_bytes), int(sms),
+                                  C.byref(p)))
+    return p
 
 
 def consist_out_workspace_size(w: int, h: int, form: str = "exact") -> int:

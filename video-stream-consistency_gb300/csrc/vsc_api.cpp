@@ -500,6 +500,29 @@ VSC_API size_t vsc_consist_out_fma_workspace_size(int32_t width, int32_t height)
     return solver_workspace_floats(width, height, kSolverFma) * sizeof(float);
 }
 
+VSC_API vsc_status vsc_solver_plan(int32_t width, int32_t height, int32_t num_iter, int32_t form,
+    size_t workspace_bytes, int32_t sms, vsc_solve_plan* out)
+{
+    clear_error();
+    if (!out)
+        return set_error(VSC_EINVAL, "solver_plan: null argument");
+    if (!dims_ok(width) || !dims_ok(height) || static_cast<int64_t>(width) * height > (int64_t{1} << 36) || num_iter < 0)
+        return set_error(VSC_EINVAL, "solver_plan: %d steps of a %dx%d image", num_iter, width, height);
+    if (form != VSC_SOLVER_EXACT && form != VSC_SOLVER_FMA)
+        return set_error(VSC_EINVAL, "solver_plan: unknown solver form %d", form);
+    const size_t floats = workspace_bytes ? workspace_bytes / sizeof(float)
+                                          : solver_workspace_full_floats(width, height, form);
+    if (floats < solver_workspace_floats(width, height, form))
+        return set_error(VSC_ENOMEM, "solver_plan: workspace of %zu bytes, need %zu", workspace_bytes,
+            solver_workspace_floats(width, height, form) * sizeof(float));
+    SolverPlan p;
+    const vsc_status s = check_cuda(solver_plan(width, height, num_iter, form, floats, sms, &p), "solver_plan");
+    if (s)
+        return s;
+    *out = vsc_solve_plan{p.planes ? 1 : 0, p.steps, p.rounds, p.tiles, p.rounds_per_launch};
+    return VSC_OK;
+}
+
 namespace {
 
 vsc_status consist_out_form(int form, const vsc_image* crnt_pr, const vsc_image* prev_stab_warp,

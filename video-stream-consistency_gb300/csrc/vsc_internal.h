@@ -151,6 +151,16 @@ enum SolverForm { kSolverExact = 0, kSolverFma = 1 };
 size_t solver_workspace_floats(int w, int h, int form = kSolverExact);
 size_t solver_workspace_full_floats(int w, int h, int form);
 size_t solver_workspace_any_floats(int w, int h);  // the larger form's
+// How run_solver works w x h, num_iter steps in an aligned workspace of ws_floats on a
+// device of `sms` SMs (0: the current device's; else no device is asked): in
+// planes or on interleaved images, the steps of a round, its rounds, the tiles of
+// a round (interleaved: of the shape the wave model gives), and the rounds that
+// one launch runs.
+struct SolverPlan {
+    bool planes;
+    int steps, rounds, tiles, rounds_per_launch;
+};
+cudaError_t solver_plan(int w, int h, int num_iter, int form, size_t ws_floats, int sms, SolverPlan* out);
 int solver_steps_per_launch();  // Jacobi steps one solver launch performs (temporal blocking)
 // Tile-shape autotuner of the exact form's kernels on interleaved images (same
 // results either way): solver_autotune times both shapes at (w, h) on scratch

@@ -1443,7 +1443,8 @@ struct PlSolve {
     unsigned* done[kN];  // per problem and tile: rounds finished (zeroed before the launch)
     int w[kN], h[kN], tiles_x[kN];
     int tile0[kN + 1];   // first tile of problem p in a round's tile list; tile0[count] = N
-    int count, nround, num_iter;
+    int count, num_iter;
+    int round0, nround;  // this launch's rounds: round0 .. round0 + nround - 1
     unsigned* ticket;    // the next ticket (zeroed before the launch)
 };
 
@@ -1467,8 +1468,9 @@ __device__ __forceinline__ PlJob pl_job(const PlSolve<kN>& g, int ticket)
     using G = PlGeo<kCfg>;
     const int N = g.tile0[g.count];
     PlJob j;
-    j.k = ticket / N;
-    const int tile = ticket - j.k * N;
+    const int round = ticket / N;
+    j.k = g.round0 + round;
+    const int tile = ticket - round * N;
     int p = 0;
     if (kN > 1) {
         // the last problem whose first tile is <= tile (binary search)
@@ -1661,7 +1663,7 @@ __global__ void __launch_bounds__(32 * (PlGeo<kCfg>::kWarps + 4), 1)
         asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(G::kControlRegs));
         if (warp == G::kWarps) {
             // ---- loading warp ---------------------------------------------------------
-            const int total = g.tile0[g.count] * g.nround;
+            const int total = g.tile0[g.count] * g.nround;  // (pl_launch_rounds: far below 2^31)
             int ticket = 0, phases = 0;  // full_in phases armed
             if (lane == 0)
                 ticket = static_cast<int>(atomicAdd(g.ticket, 1u));
@@ -2183,7 +2185,14 @@ int solver_steps_per_launch() { return kTbT; }
 namespace {
 
 // rounds of a solve
-int solve_launches(int num_iter, int steps = kTbT) { return num_iter > 0 ? (num_iter + steps - 1) / steps : 0; }
+int solve_launches(int num_iter, int steps = kTbT) { return num_iter > 0 ? (num_iter - 1) / steps + 1 : 0; }
+
+// Rounds of one launch of the solve kernel at `tiles` tiles a round.  A launch
+// counts its tickets, tiles x rounds, in 32 bits, and nothing bounds a caller's
+// num_iter: a solve of more than 2^20 tickets (1920x1080, exact form: 6,752 steps,
+// 39 ms) is several launches, each of whole rounds.
+constexpr int kLaunchTickets = 1 << 20;
+int pl_launch_rounds(int tiles, int nround) { return std::min(nround, std::max(1, kLaunchTickets / tiles)); }
 
 struct WsView {
     float *L, *U0, *U1, *O2;
@@ -2217,10 +2226,14 @@ bool tma_eligible(const DeviceInfo* di, int w, const float* O, const WsView& v, 
 
 // A solve in planes of rows on the 16-byte grid: a 16-byte aligned workspace with
 // room for them and for the counters of cfg's tiles.
-bool pl_tma_eligible(const DeviceInfo* di, int w, int h, const float* ws, size_t ws_floats, int cfg)
+bool pl_fits(int w, int h, size_t ws_floats, int cfg)
 {
     const size_t planes = pl_images(cfg & 1) * static_cast<size_t>(pl_pitch(w)) * h * 3;
-    return di->ps_smem && aligned16p(ws) && ws_floats >= planes + pl_counter_floats(w, h, cfg);
+    return ws_floats >= planes + pl_counter_floats(w, h, cfg);
+}
+bool pl_tma_eligible(const DeviceInfo* di, int w, int h, const float* ws, size_t ws_floats, int cfg)
+{
+    return di->ps_smem && aligned16p(ws) && pl_fits(w, h, ws_floats, cfg);
 }
 
 // The rounds of a solve: 8, 12 or 16 steps.  Where an SM has few tiles a round
@@ -2239,7 +2252,7 @@ bool pl_tma_eligible(const DeviceInfo* di, int w, int h, const float* ws, size_t
 // 854x480 196, 163, 177; 960x540 195, 211, 217; 1280x720 290, 324, 385; exact
 // 480x270 189, 162, 167; 560x316 202, 170, 156; 640x360 204, 174, 199; 800x450
 // 220, 227, 277.
-int pl_rounds_cfg(const DeviceInfo* di, int w, int h, int num_iter, int form)
+int pl_rounds_cfg(int sms, int w, int h, int num_iter, int form)
 {
     struct Cost {
         int cfg;
@@ -2249,12 +2262,12 @@ int pl_rounds_cfg(const DeviceInfo* di, int w, int h, int num_iter, int form)
         {{0, 10.5f, 2.8f, 5.3f}, {kPlMid, 12.8f, 5.5f, 6.2f}, {kPlLong, 14.5f, 5.0f, 8.4f}},
         {{0, 9.4f, 5.6f, 2.9f}, {kPlMid, 11.2f, 2.6f, 5.5f}, {kPlLong, 12.5f, 3.0f, 7.0f}}};
     const int tiles8 = pl_tiles_of(w, h, form);
-    if (tiles8 > 3 * di->sms || (num_iter < 4 * kTbT && 5 * tiles8 > 3 * di->sms))
+    if (tiles8 > 3 * sms || (num_iter < 4 * kTbT && 5 * tiles8 > 3 * sms))
         return form;
     int best = form;
     float limit = 0.0f;
     for (const Cost& c : kCost[form == kSolverFma]) {
-        const float tiles = static_cast<float>(pl_tiles_of(w, h, form | c.cfg)) / static_cast<float>(di->sms);
+        const float tiles = static_cast<float>(pl_tiles_of(w, h, form | c.cfg)) / static_cast<float>(sms);
         const float us = static_cast<float>(solve_launches(num_iter, pl_steps(c.cfg))) *
                          std::max(c.least, c.base + c.tile * tiles);
         if (c.cfg == 0) {
@@ -2271,9 +2284,16 @@ int pl_rounds_cfg(const DeviceInfo* di, int w, int h, int num_iter, int form)
 // 64 x 32 tiles is the image (75 steps: 320x180 71 us against 75 in planes,
 // 240x135 70 against 86), or one of the 64 x 48 tiles for two rounds at most
 // (600x338, 16 steps: 28 us against 32).
-bool exact_interleaved(const DeviceInfo* di, int w, int h, int num_iter)
+bool exact_interleaved(int sms, int w, int h, int num_iter)
 {
-    return tiles_of(w, h, kIH) <= di->sms || (num_iter <= 2 * kTbT && tiles_of(w, h, kPIH) <= di->sms);
+    return tiles_of(w, h, kIH) <= sms || (num_iter <= 2 * kTbT && tiles_of(w, h, kPIH) <= sms);
+}
+
+// The rounds of a solve in a workspace of ws_floats.
+int pl_cfg(int sms, int w, int h, int num_iter, int form, size_t ws_floats)
+{
+    const int cfg = pl_rounds_cfg(sms, w, h, num_iter, form);
+    return pl_fits(w, h, ws_floats, cfg) ? cfg : form;
 }
 
 struct PlanarCopy {
@@ -2312,8 +2332,9 @@ cudaError_t launch_planar(const PlanarCopy* c, int n, int to_planar, cudaStream_
     return cudaGetLastError();
 }
 
-// One launch of the FMA form's solve kernel per kN members (each member's
-// counters zeroed beforehand; the first member's ticket serves the launch).
+// The solve kernel over n members, kN a launch (each member's counters zeroed
+// beforehand; the first member's ticket serves the launch).  The tiles' counters
+// run on from launch to launch of a long solve, the ticket starts again.
 template <int kCfg, int kN>
 cudaError_t launch_solve(const std::vector<PlWs>& v, const int* w, const int* h, int n, int num_iter, float step,
     float mom, int sms, cudaStream_t st, int* nl)
@@ -2344,7 +2365,6 @@ cudaError_t launch_solve(const std::vector<PlWs>& v, const int* w, const int* h,
             g.tiles_x[p] = pl_tiles_x<kCfg>(W);
             g.tile0[p + 1] = g.tile0[p] + pl_tiles<kCfg>(W, H);
         }
-        g.nround = nround;
         g.num_iter = num_iter;
         g.ticket = v[b0].cnt;
         cudaLaunchConfig_t cfg = {};
@@ -2360,10 +2380,17 @@ cudaError_t launch_solve(const std::vector<PlWs>& v, const int* w, const int* h,
         cfg.gridDim = dim3(std::min(g.tile0[g.count], sms));
         cfg.blockDim = dim3(32 * (G::kWarps + 4));
         cfg.dynamicSmemBytes = G::kSmem;
-        const cudaError_t e = cudaLaunchKernelEx(&cfg, solver_solve_kernel<kCfg, kN>, g, step, mom);
-        if (e != cudaSuccess)
-            return e;
-        ++*nl;
+        const int per = pl_launch_rounds(g.tile0[g.count], nround);
+        for (int r0 = 0; r0 < nround; r0 += per) {
+            g.round0 = r0;
+            g.nround = std::min(per, nround - r0);
+            cudaError_t e = r0 > 0 ? cudaMemsetAsync(g.ticket, 0, sizeof(unsigned), st) : cudaSuccess;
+            if (e == cudaSuccess)
+                e = cudaLaunchKernelEx(&cfg, solver_solve_kernel<kCfg, kN>, g, step, mom);
+            if (e != cudaSuccess)
+                return e;
+            ++*nl;
+        }
     }
     return cudaGetLastError();
 }
@@ -2386,9 +2413,7 @@ cudaError_t run_solver_planes(const DeviceInfo* di, int form, const float* P, co
     cudaStream_t st, int* nl, uint8_t* rgba_out, const float* Oc, int cw, int ch)
 {
     const bool tma = pl_tma_eligible(di, w, h, workspace, ws_floats, form);
-    int cfg = tma ? pl_rounds_cfg(di, w, h, num_iter, form) : form;
-    if (!pl_tma_eligible(di, w, h, workspace, ws_floats, cfg))
-        cfg = form;
+    const int cfg = tma ? pl_cfg(di->sms, w, h, num_iter, form, ws_floats) : form;
     const PlWs v = pl_view(workspace, w, h, tma ? pl_pitch(w) : w, cfg);
     cudaError_t e = launch_prep(form, P, A, Wt, Oi, v, v.O[0], w, h, step, v.cnt, v.ncnt, Oc, cw, ch, st);
     ++*nl;
@@ -2440,6 +2465,34 @@ cudaError_t solver_prep(int form, const float* P, const float* A, const float* W
     const PlWs v = pl_view(workspace, w, h, pl_pitch(w), form);
     const cudaError_t e = launch_prep(form, P, A, Wt, nullptr, v, nullptr, w, h, step, nullptr, 0, nullptr, 0, 0, st);
     return e != cudaSuccess ? e : cudaGetLastError();
+}
+
+cudaError_t solver_plan(int w, int h, int num_iter, int form, size_t ws_floats, int sms, SolverPlan* out)
+{
+    if (sms <= 0) {
+        DeviceInfo* di = nullptr;
+        const cudaError_t e = device_info(&di);
+        if (e != cudaSuccess)
+            return e;
+        sms = di->sms;
+    }
+    SolverPlan p{};
+    const bool inter = form == kSolverExact && w % 4 == 0 && exact_interleaved(sms, w, h, num_iter);
+    p.planes = form == kSolverFma || (!inter && pl_fits(w, h, ws_floats, form));
+    const bool one_launch = p.planes && pl_fits(w, h, ws_floats, form);
+    const int cfg = one_launch ? pl_cfg(sms, w, h, num_iter, form, ws_floats) : form;
+    p.steps = pl_steps(cfg);
+    p.rounds = solve_launches(num_iter, p.steps);
+    if (p.planes) {
+        p.tiles = pl_tiles_of(w, h, cfg);
+    } else {
+        const int T = std::min(num_iter, kTbT);  // (solver_tb_kernel's ring is its launch's steps)
+        p.tiles = w % 4 == 0 ? tiles_of(w, h, interior_rows(model_rows(w, h, sms, form)))
+                             : ((w - 1) / (kTbEX - 2 * T) + 1) * ((h - 1) / (kTbEY - 2 * T) + 1);
+    }
+    p.rounds_per_launch = one_launch ? pl_launch_rounds(p.tiles, p.rounds) : std::min(1, p.rounds);
+    *out = p;
+    return cudaSuccess;
 }
 
 cudaError_t run_solver_group(const SolverImage* im, int n, int num_iter, float step, float mom, cudaStream_t st,
@@ -2534,7 +2587,7 @@ cudaError_t run_solver(const float* P, const float* A, const float* Wt, float* O
         return e0;
     if (form == kSolverFma && !di->ps_smem)
         return cudaErrorNotSupported;
-    const bool interleaved = tma_eligible(di, w, O, v, A, Wt) && exact_interleaved(di, w, h, num_iter);
+    const bool interleaved = tma_eligible(di, w, O, v, A, Wt) && exact_interleaved(di->sms, w, h, num_iter);
     if (form == kSolverFma || (!interleaved && pl_tma_eligible(di, w, h, workspace, ws_floats, form))) {
         const cudaError_t e = run_solver_planes(di, form, P, A, Wt, O, O, w, h, num_iter, step, mom, workspace,
             ws_floats, st, &nl, rgba_out, nullptr, 0, 0);
