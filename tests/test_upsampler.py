@@ -244,3 +244,68 @@ def test_training_ignores_values_where_the_gradient_is_zero(vsc, cuda):
         up.close()
     assert np.all(np.isfinite(got[1]))
     assert np.quantile(np.abs(got[0] - got[1]), 0.99) <= 1e-5  # the sums' order varies
+
+
+def _taps_outside(h, w):
+    """Mask over the parameters: weights of taps that lie outside an h x w image at every pixel."""
+    out = []
+    for ci, co in LAYERS:
+        m = np.zeros((co, 3, 3, ci), bool)
+        if h == 1:
+            m[:, [0, 2]] = True
+        if w == 1:
+            m[:, :, [0, 2]] = True
+        out += [m.reshape(-1), np.zeros(co, bool)]
+    return np.concatenate(out)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("h,w", [(1, 40), (40, 1), (1, 1), (1, 7)])
+def test_training_leaves_taps_outside_the_image_out(vsc, cuda, h, w):
+    """A tap outside the image adds nothing whatever its weight: in images of one
+    row (or column) the taps above and below (beside) are never inside, so weights
+    there that are not finite change nothing.  Bounds as in the test above."""
+    import torch
+
+    rng = np.random.Generator(np.random.PCG64(h + 100 * w))
+    lr = 1e-4
+    outside = _taps_outside(h, w)
+    params = rng.normal(0, 0.1, vsc.Upsampler.param_count()).astype(np.float32)
+    params[outside] = 0.0
+    bad = params.copy()
+    bad[outside] = np.resize(np.float32([np.nan, np.inf, -np.inf]), outside.sum())
+    batches = [(rng.normal(0, 1, (2, h, w, 3)).astype(np.float32), rng.normal(0, 1, (2, h, w, 2)).astype(np.float32))
+               for _ in range(2)]
+    up = vsc.Upsampler(bad)
+    for (inp, tgt), (loss, ref) in zip(batches, _reference_steps(params, batches, lr)):
+        got = up.train_step(torch.from_numpy(inp).to(cuda), torch.from_numpy(tgt).to(cuda), lr)
+        assert abs(got - loss) <= 1e-5 * loss
+        p = up.params()
+        assert np.array_equal(p[outside], bad[outside], equal_nan=True)
+        err = np.maximum(np.abs(p - ref)[~outside] - 6e-8, 0) / lr
+        assert np.median(err) <= 1e-4 and np.quantile(err, 0.99) <= 1e-2 and err.max() <= 2.5, err.max()
+    up.close()
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("h,w", [(1, 8), (1, 70), (70, 1)])
+def test_weight_gradients_leave_taps_outside_the_image_out(vsc, cuda, h, w):
+    """The same for the weight gradients where dz is not finite (an overflow on
+    the way back: 3e38 * 1e9): the first layer's taps outside the image keep a
+    gradient of zero, those inside get one that is not finite."""
+    import torch
+
+    params = np.zeros(vsc.Upsampler.param_count(), np.float32)
+    at = 0
+    for (ci, co), value in zip(LAYERS, (1e-30, 3e38, 1e10, 1.0)):
+        params[at + 4 * ci] = value  # output 0, centre tap, channel 0
+        at += co * 9 * ci + co
+    inp = np.zeros((1, h, w, 3), np.float32)
+    inp[..., 0] = 1.0
+    up = vsc.Upsampler(params)
+    up.train_step(torch.from_numpy(inp).to(cuda), torch.zeros((1, h, w, 2), device=cuda), 1e-3)
+    got = up.params()[:27].reshape(3, 3, 3)  # output 0: [ky][kx][channel]
+    outside = _taps_outside(h, w)[:27].reshape(3, 3, 3)
+    assert np.array_equal(got[outside], params[:27].reshape(3, 3, 3)[outside])
+    assert not np.isfinite(got[~outside]).any()
+    up.close()

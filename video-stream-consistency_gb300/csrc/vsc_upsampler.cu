@@ -26,6 +26,7 @@
 #include <algorithm>
 #include <cmath>
 #include <mutex>
+#include <type_traits>
 
 namespace vsc {
 namespace {
@@ -162,12 +163,35 @@ __device__ __forceinline__ void conv_window(const float* p, int kx, float (&v)[P
     }
 }
 
+// Output (thread's pixel i, channel oc) of conv3x3_kernel again, with the taps
+// outside the image left out rather than multiplied with the zeros that the tile
+// holds there: w * 0 is not 0 for a weight that is not finite.  xr: the tile at
+// the thread's first pixel's window; the sum in the kernel's order.
+template <int CI, int CO, int OCT, int kMode>
+__device__ __noinline__ float conv_inside(const float* xr, const float* sw, float b, int oc, int i, int py, int px,
+    int H, int W)
+{
+    using S = ConvShape<CI, CO, OCT>;
+    constexpr bool kBwd = kMode == kConvBwd;
+    float acc = b;
+    for (int t = 0; t < 9; ++t) {
+        const int dy = kBwd ? 2 - t / 3 : t / 3, dx = kBwd ? 2 - t % 3 : t % 3;
+        const int yy = py + dy - 1, xx = px + i + dx - 1;
+        if (yy < 0 || yy >= H || xx < 0 || xx >= W)
+            continue;
+        for (int c = 0; c < CI; ++c)
+            acc = __fmaf_rn(kBwd ? sw[(c * 9 + t) * CO + oc] : sw[(oc * 9 + t) * CI + c],
+                xr[c * S::plane + dy * kConvPitch + i + dx], acc);
+    }
+    return acc;
+}
+
 // x: planes (kInter: interleaved CI-channel pixels).  kConvRelu: y = ReLU(conv
 // + bias).  kConvLoss (the last layer): the L1 loss of base + r against the
 // target and its gradient dr = sign / pixels as planes in y.  kConvBwd: x is
 // dz of the layer's CI outputs, y = dz of its CO inputs where a_prev > 0.
-// nonfinite: set when a value the weight gradients will multiply (the input
-// or an activation) is not finite.
+// nonfinite: set when a value the weight gradients will multiply (the input,
+// an activation or a dz) is not finite.
 template <int CI, int CO, int OCT, int kMode, bool kInter>
 __global__ void __launch_bounds__(128, 2) conv3x3_kernel(const float* __restrict__ x, const float* __restrict__ wts,
     const float* __restrict__ bias, const float* __restrict__ a_prev, float* __restrict__ y, int H, int W, int tiles_x,
@@ -284,7 +308,23 @@ __global__ void __launch_bounds__(128, 2) conv3x3_kernel(const float* __restrict
     const int py = y0 + r, px = x0 + PX * g;
     const bool row_in = py < H;
     const int64_t p = static_cast<int64_t>(py) * W + px;
+    // sums of pixels at the image's edge that are not finite may have come from a tap outside it
+    bool redo = false;
+    const float* const x_thread = sm + r * kConvPitch + 3 + PX * g;
+    if (py == 0 || py == H - 1 || px == 0 || px + PX >= W) {
+#pragma unroll
+        for (int i = 0; i < PX; ++i)
+#pragma unroll
+            for (int o = 0; o < OCT; ++o)
+                redo = redo || !finite_f(acc[i][o]);
+    }
     if constexpr (kMode == kConvLoss) {
+        if (redo)
+#pragma unroll
+            for (int i = 0; i < PX; ++i)
+#pragma unroll
+                for (int o = 0; o < OCT; ++o)
+                    acc[i][o] = conv_inside<CI, CO, OCT, kMode>(x_thread, sw, bias[o], o, i, py, px, H, W);
         float l = 0.0f;
 #pragma unroll
         for (int i = 0; i < PX; ++i) {
@@ -322,6 +362,7 @@ __global__ void __launch_bounds__(128, 2) conv3x3_kernel(const float* __restrict
                     bad = bad || (in && !finite_f(v[i]));
                 } else {
                     v[i] = in && a_prev[q + i] > 0.0f ? v[i] : 0.0f;
+                    bad = bad || !finite_f(v[i]);
                 }
             }
 #pragma unroll
@@ -337,7 +378,21 @@ __global__ void __launch_bounds__(128, 2) conv3x3_kernel(const float* __restrict
                 }
             }
         }
-        if (kMode == kConvRelu && bad)
+        if (redo && row_in) {  // (the thread's own stores, written over)
+#pragma unroll 1
+            for (int k = 0; k < PX * OCT; ++k) {
+                const int i = k % PX, oc = og * OCT + k / PX;
+                if (px + i >= W)
+                    continue;
+                const int64_t q = (static_cast<int64_t>(n) * CO + oc) * HW + p + i;
+                float v = conv_inside<CI, CO, OCT, kMode>(x_thread, sw, kMode == kConvBwd ? 0.0f : bias[oc], oc, i, py,
+                    px, H, W);
+                v = kMode == kConvRelu ? fmaxf(v, 0.0f) : a_prev[q] > 0.0f ? v : 0.0f;
+                bad = bad || !finite_f(v);
+                y[q] = v;
+            }
+        }
+        if (bad)
             atomicOr(nonfinite, 1);
     }
 }
@@ -346,7 +401,8 @@ __global__ void __launch_bounds__(128, 2) conv3x3_kernel(const float* __restrict
 // dw[o][t][c] += sum over pixels of dz[o] * x[tap t][c]; db[o] += sum dz[o].
 // Blocks walk 32 x 2 pixel tiles, two cp.async buffers, and add their sums to
 // the gradient once at the end.  A pixel with dz = 0 adds nothing, whatever x
-// holds there (kSafe, taken when some x is not finite; else 0 * x is 0 anyway).
+// holds there, nor does a tap outside the image, whatever dz is (kSafe, taken
+// when some x or dz is not finite; else the product with 0 is 0 anyway).
 constexpr int kWgRows = 2;
 constexpr int kWgPx = kTileW * kWgRows;
 constexpr int kWgPlane = 148;  // x plane: 4 rows x 36, + 4: 20 mod 32, 16-byte reads across channels conflict-free
@@ -363,9 +419,19 @@ struct WgShape {
     static constexpr int smem = 2 * buf * 4;
 };
 
-__device__ __forceinline__ float wg_add(bool safe, float g, float v, float acc)
+// inside: the tap lies in the image (looked at where safe only)
+__device__ __forceinline__ float wg_add(bool safe, float g, float v, float acc, bool inside)
 {
-    return safe && g == 0.0f ? acc : __fmaf_rn(g, v, acc);
+    return safe && (g == 0.0f || !inside) ? acc : __fmaf_rn(g, v, acc);
+}
+
+// bit i of n: the coordinate first + i lies in [0, size)
+__device__ __forceinline__ unsigned inside_bits(int first, int n, int size)
+{
+    unsigned m = 0;
+    for (int i = 0; i < n; ++i)
+        m |= first + i >= 0 && first + i < size ? 1u << i : 0u;
+    return m;
 }
 
 template <int CO, int OGT, bool kSafe>
@@ -402,8 +468,10 @@ __device__ __forceinline__ void wg_tile(const float* sx, const float* sz, int ks
 #pragma unroll
                 for (int i = 0; i < 4; ++i)
 #pragma unroll
-                    for (int t = 0; t < 9; ++t)
-                        acc[o][t] = wg_add(kSafe, gz[i], v[t / 3][i + t % 3], acc[o][t]);
+                    for (int t = 0; t < 9; ++t) {
+                        const float a = v[t / 3][i + t % 3];
+                        acc[o][t] = wg_add(kSafe, gz[i], a, acc[o][t], a == a);
+                    }
             }
         }
     }
@@ -462,10 +530,19 @@ __global__ void __launch_bounds__(128, 4) wgrad_kernel(const float* __restrict__
         cp_async_wait<1>();
         __syncthreads();
         const float* sz = b + 32 * kWgPlane + og * OGT * S::dzp;
-        if (safe)
+        if (safe) {
+            // x is a ReLU's output, never NaN: NaN marks the tile's places outside the image
+            const int x0 = (tile % tiles % tiles_x) * kTileW, y0 = (tile % tiles / tiles_x) * kWgRows;
+            for (int i = tid; i < 32 * 4 * 34; i += 128) {
+                const int c = i / (4 * 34), q = i % (4 * 34), gy = y0 - 1 + q / 34, gx = x0 - 1 + q % 34;
+                if (gy < 0 || gy >= H || gx < 0 || gx >= W)
+                    sm[(k & 1) * S::buf + c * kWgPlane + q / 34 * kPitch + q % 34] = __int_as_float(0x7fffffff);
+            }
+            __syncthreads();
             wg_tile<CO, OGT, true>(b, sz, ks, lane, acc);
-        else
+        } else {
             wg_tile<CO, OGT, false>(b, sz, ks, lane, acc);
+        }
         if (ks == 0)
 #pragma unroll
             for (int o = 0; o < OGT; ++o)
@@ -542,28 +619,42 @@ __global__ void __launch_bounds__(128) wgrad_first_kernel(const float* __restric
         cp_async_wait<1>();
         __syncthreads();
         const float* sx = b + 32 * kWg1Dz;
+        const int x0 = (tile % tiles % tiles_x) * kTileW, y0 = (tile % tiles / tiles_x) * kWgRows;
+        auto add_tile = [&](auto safe_tile) {
+            constexpr bool kSafe = decltype(safe_tile)::value;
+            const unsigned ym = kSafe ? inside_bits(y0 - 1, kWgRows + 2, H) : 0;
 #pragma unroll 1
-        for (int q = 2 * warp; q < 2 * warp + 2; ++q)  // this warp's 4-pixel groups of each row
+            for (int q = 2 * warp; q < 2 * warp + 2; ++q) {  // this warp's 4-pixel groups of each row
+                const unsigned xm = kSafe ? inside_bits(x0 + 4 * q - 1, 6, W) : 0;
 #pragma unroll
-            for (int row = 0; row < kWgRows; ++row) {
-                const float4 z = *reinterpret_cast<const float4*>(b + lane * kWg1Dz + row * kTileW + 4 * q);
-                const float gz[4] = {z.x, z.y, z.z, z.w};
-                bsum += (z.x + z.y) + (z.z + z.w);
+                for (int row = 0; row < kWgRows; ++row) {
+                    const float4 z = *reinterpret_cast<const float4*>(b + lane * kWg1Dz + row * kTileW + 4 * q);
+                    const float gz[4] = {z.x, z.y, z.z, z.w};
+                    bsum += (z.x + z.y) + (z.z + z.w);
 #pragma unroll
-                for (int c = 0; c < 3; ++c)
+                    for (int c = 0; c < 3; ++c)
 #pragma unroll
-                    for (int ky = 0; ky < 3; ++ky) {
-                        const float* xr = sx + (c * 4 + row + ky) * kPitch + 4 * q;
-                        const float4 v0 = *reinterpret_cast<const float4*>(xr);
-                        const float2 v1 = *reinterpret_cast<const float2*>(xr + 4);
-                        const float v[6] = {v0.x, v0.y, v0.z, v0.w, v1.x, v1.y};
+                        for (int ky = 0; ky < 3; ++ky) {
+                            const float* xr = sx + (c * 4 + row + ky) * kPitch + 4 * q;
+                            const float4 v0 = *reinterpret_cast<const float4*>(xr);
+                            const float2 v1 = *reinterpret_cast<const float2*>(xr + 4);
+                            const float v[6] = {v0.x, v0.y, v0.z, v0.w, v1.x, v1.y};
 #pragma unroll
-                        for (int i = 0; i < 4; ++i)
+                            for (int i = 0; i < 4; ++i)
 #pragma unroll
-                            for (int kx = 0; kx < 3; ++kx)
-                                acc[(ky * 3 + kx) * 3 + c] = wg_add(safe, gz[i], v[i + kx], acc[(ky * 3 + kx) * 3 + c]);
-                    }
+                                for (int kx = 0; kx < 3; ++kx) {
+                                    float& a = acc[(ky * 3 + kx) * 3 + c];
+                                    a = wg_add(kSafe, gz[i], v[i + kx], a,
+                                        (xm >> (i + kx) & ym >> (row + ky) & 1u) != 0);
+                                }
+                        }
+                }
             }
+        };
+        if (safe)
+            add_tile(std::true_type{});
+        else
+            add_tile(std::false_type{});
         __syncthreads();
     }
     __syncthreads();
