@@ -309,3 +309,56 @@ def test_weight_gradients_leave_taps_outside_the_image_out(vsc, cuda, h, w):
     assert np.array_equal(got[outside], params[:27].reshape(3, 3, 3)[outside])
     assert not np.isfinite(got[~outside]).any()
     up.close()
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("n,h,w", [(1, 32, 64), (32, 64, 64), (1, 1024, 2048)])
+def test_weight_gradient_sums_against_float64(vsc, cuda, n, h, w):
+    """The gradients' sums over the pixels, read from one Adam step of a learning
+    rate so large that the update is all that is left of a parameter, and with
+    gradients (1e-10) far below Adam's epsilon, where it is nearly linear in
+    them.  Weights of few bits and a target far below give every pixel the same
+    dz, exactly, so only the inputs' products and their sums round.  A sum of m equal terms
+    in a row is off by about sqrt(m) / 3 units (2^-24) in the root mean square: 32
+    copies in four chains 0.9, 19 or fewer blocks a copy 1.5 and 2,048 pixels a
+    thread 15, averaged over 32 copies and 608 blocks to 0.3 and 0.6, reading
+    the update about 1; all blocks on one sum would be 8.  The largest batch has more
+    than 32 tiles a block."""
+    import torch
+
+    rng = np.random.Generator(np.random.PCG64(n + h))
+    params, at, spans = np.zeros(vsc.Upsampler.param_count(), np.float32), 0, []
+    for li, (ci, co) in enumerate(LAYERS):
+        k = co * 9 * ci
+        params[at:at + k] = rng.integers(1, 4, k) * 2.0 ** (-38 if li == 3 else -8)
+        spans.append((at, k, ci, co))
+        at += k + co
+    x = rng.random((n, h, w, 3), dtype=np.float32)
+    inp = torch.from_numpy(x).to(cuda)
+    lr = 1e6
+    up = vsc.Upsampler(params)
+    up.train_step(inp, torch.full((n, h, w, 2), -10.0, device=cuda), lr)
+    moved = (params.astype(np.float64) - up.params()) / lr  # g / (|g| + 1e-8)
+    up.close()
+    moved[spans[3][0]:] = 0  # (the last layer's gradients are far above the epsilon)
+    grad = moved * 1e-8 / (1 - np.abs(moved))
+
+    acts = [inp.double().permute(0, 3, 1, 2)]
+    wts = []
+    for a, k, ci, co in spans:
+        wts.append(torch.from_numpy(params[a:a + k].astype(np.float64)).to(cuda).reshape(co, 3, 3, ci).permute(0, 3, 1, 2)
+                   .contiguous())
+        if len(wts) < 4:
+            acts.append(torch.nn.functional.conv2d(acts[-1], wts[-1], padding=1))
+    dz = torch.full((n, 2, h, w), 1.0 / (n * h * w), dtype=torch.float64, device=cuda)
+    for li in (2, 1, 0):
+        dz = torch.nn.functional.conv_transpose2d(dz, wts[li + 1], padding=1)
+        a, k, ci, co = spans[li]
+        # correlate x with dz, a tap at a time
+        xp = torch.nn.functional.pad(acts[li], (1, 1, 1, 1))
+        ref = torch.stack([torch.stack([torch.einsum("nohw,nchw->oc", dz, xp[:, :, ky:ky + h, kx:kx + w])
+                                        for kx in range(3)], 1) for ky in range(3)], 1).reshape(-1).cpu().numpy()
+        db = dz.sum((0, 2, 3)).cpu().numpy()
+        for got, want in ((grad[a:a + k], ref), (grad[a + k:a + k + co], db)):
+            rms = np.sqrt(np.mean((got / want - 1) ** 2)) * 2 ** 24
+            assert rms <= 4.0, (li, got.size, rms)

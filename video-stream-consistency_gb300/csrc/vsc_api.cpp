@@ -1591,7 +1591,7 @@ VSC_API vsc_status vsc_upsampler_create(const float* params, vsc_upsampler** out
         upsampler_init_params(host.data(), 0x55505341'4D504C45ULL);  // seeded He-uniform
     cudaError_t e = dalloc(&u->prm, n);
     if (e == cudaSuccess)
-        e = dalloc(&u->grad, n);
+        e = dalloc(&u->grad, upsampler_grad_floats());
     if (e == cudaSuccess)
         e = dalloc(&u->m, n);
     if (e == cudaSuccess)

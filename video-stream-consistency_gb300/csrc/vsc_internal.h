@@ -93,6 +93,7 @@ constexpr UpLayer kUpLayers[4] = {{3, 32, 0, 864}, {32, 32, 896, 896 + 9216}, {3
     {32, 2, 19392, 19392 + 576}};
 int upsampler_param_count();
 void upsampler_init_params(float* host, uint64_t seed);
+size_t upsampler_grad_floats();                            // the gradient's copies, summed by the update
 size_t upsampler_train_work_floats(int N, int H, int W);   // activations and gradients of a batch
 // input (N x h x w x 3): the coarse flows bilinearly upsampled with their vectors
 // scaled to the full grid, and the frames' luma; batch n at base + n * stride;

@@ -400,9 +400,17 @@ __global__ void __launch_bounds__(128, 2) conv3x3_kernel(const float* __restrict
 // ---- weight gradients ---------------------------------------------------------------
 // dw[o][t][c] += sum over pixels of dz[o] * x[tap t][c]; db[o] += sum dz[o].
 // Blocks walk 32 x 2 pixel tiles, two cp.async buffers, and add their sums to
-// the gradient once at the end.  A pixel with dz = 0 adds nothing, whatever x
+// the gradient at the end, and every kWgFlush tiles.  The gradient is kept in
+// copies, one for 16 blocks and 32 at most, which the update sums: all 608 blocks
+// on one sum were 608 additions in a row and five times as far from the float64 sum
+// (32 x 64 x 64 pixels of equal dz: 5.9 units of 2^-24 in the root mean square, now
+// 1.1; the per-pixel kernels 1.7), and slower (a step 550 -> 545 us); a thread's
+// own sum is at most 2,048 products long, whatever the batch.  A pixel with dz = 0 adds nothing, whatever x
 // holds there, nor does a tap outside the image, whatever dz is (kSafe, taken
 // when some x or dz is not finite; else the product with 0 is 0 anyway).
+constexpr int kGradCopies = 32;
+constexpr int kGradPitch = (kParams + 31) / 32 * 32;  // of a copy, in floats
+constexpr int kWgFlush = 32;
 constexpr int kWgRows = 2;
 constexpr int kWgPx = kTileW * kWgRows;
 constexpr int kWgPlane = 148;  // x plane: 4 rows x 36, + 4: 20 mod 32, 16-byte reads across channels conflict-free
@@ -480,7 +488,7 @@ __device__ __forceinline__ void wg_tile(const float* sx, const float* sz, int ks
 template <int CO, int OGT>
 __global__ void __launch_bounds__(128, 4) wgrad_kernel(const float* __restrict__ x, const float* __restrict__ dz,
     float* __restrict__ dw, float* __restrict__ db, int H, int W, int tiles_x, int tiles, int N,
-    const int* __restrict__ nonfinite)
+    int copies, const int* __restrict__ nonfinite)
 {
     using S = WgShape<CO, OGT>;
     extern __shared__ __align__(16) float sm[];
@@ -509,58 +517,62 @@ __global__ void __launch_bounds__(128, 4) wgrad_kernel(const float* __restrict__
         }
     };
 
-    float acc[OGT][9], bsum[OGT];
-#pragma unroll
-    for (int o = 0; o < OGT; ++o) {
-        bsum[o] = 0.0f;
-#pragma unroll
-        for (int t = 0; t < 9; ++t)
-            acc[o][t] = 0.0f;
-    }
+    dw += blockIdx.x % copies * kGradPitch;
+    db += blockIdx.x % copies * kGradPitch;
     const bool safe = *nonfinite != 0;
     int tile = blockIdx.x, k = 0;
     if (tile < total)
         stage(tile, sm);
     cp_async_commit();
-    for (; tile < total; tile += gridDim.x, ++k) {
-        const float* b = sm + (k & 1) * S::buf;
-        if (tile + static_cast<int>(gridDim.x) < total)
-            stage(tile + gridDim.x, sm + ((k + 1) & 1) * S::buf);
-        cp_async_commit();
-        cp_async_wait<1>();
-        __syncthreads();
-        const float* sz = b + 32 * kWgPlane + og * OGT * S::dzp;
-        if (safe) {
-            // x is a ReLU's output, never NaN: NaN marks the tile's places outside the image
-            const int x0 = (tile % tiles % tiles_x) * kTileW, y0 = (tile % tiles / tiles_x) * kWgRows;
-            for (int i = tid; i < 32 * 4 * 34; i += 128) {
-                const int c = i / (4 * 34), q = i % (4 * 34), gy = y0 - 1 + q / 34, gx = x0 - 1 + q % 34;
-                if (gy < 0 || gy >= H || gx < 0 || gx >= W)
-                    sm[(k & 1) * S::buf + c * kWgPlane + q / 34 * kPitch + q % 34] = __int_as_float(0x7fffffff);
-            }
-            __syncthreads();
-            wg_tile<CO, OGT, true>(b, sz, ks, lane, acc);
-        } else {
-            wg_tile<CO, OGT, false>(b, sz, ks, lane, acc);
+    while (tile < total) {
+        float acc[OGT][9], bsum[OGT];
+#pragma unroll
+        for (int o = 0; o < OGT; ++o) {
+            bsum[o] = 0.0f;
+#pragma unroll
+            for (int t = 0; t < 9; ++t)
+                acc[o][t] = 0.0f;
         }
-        if (ks == 0)
+        for (int m = 0; m < kWgFlush && tile < total; ++m, tile += gridDim.x, ++k) {
+            const float* b = sm + (k & 1) * S::buf;
+            if (tile + static_cast<int>(gridDim.x) < total)
+                stage(tile + gridDim.x, sm + ((k + 1) & 1) * S::buf);
+            cp_async_commit();
+            cp_async_wait<1>();
+            __syncthreads();
+            const float* sz = b + 32 * kWgPlane + og * OGT * S::dzp;
+            if (safe) {
+                // x is a ReLU's output, never NaN: NaN marks the tile's places outside the image
+                const int x0 = (tile % tiles % tiles_x) * kTileW, y0 = (tile % tiles / tiles_x) * kWgRows;
+                for (int i = tid; i < 32 * 4 * 34; i += 128) {
+                    const int c = i / (4 * 34), q = i % (4 * 34), gy = y0 - 1 + q / 34, gx = x0 - 1 + q % 34;
+                    if (gy < 0 || gy >= H || gx < 0 || gx >= W)
+                        sm[(k & 1) * S::buf + c * kWgPlane + q / 34 * kPitch + q % 34] = __int_as_float(0x7fffffff);
+                }
+                __syncthreads();
+                wg_tile<CO, OGT, true>(b, sz, ks, lane, acc);
+            } else {
+                wg_tile<CO, OGT, false>(b, sz, ks, lane, acc);
+            }
+            if (ks == 0)
 #pragma unroll
-            for (int o = 0; o < OGT; ++o)
-                bsum[o] += sz[o * S::dzp + lane] + sz[o * S::dzp + 32 + lane];
-        __syncthreads();
-    }
+                for (int o = 0; o < OGT; ++o)
+                    bsum[o] += sz[o * S::dzp + lane] + sz[o * S::dzp + 32 + lane];
+            __syncthreads();
+        }
 #pragma unroll
-    for (int o = 0; o < OGT; ++o) {
-        const int oc = og * OGT + o;
+        for (int o = 0; o < OGT; ++o) {
+            const int oc = og * OGT + o;
 #pragma unroll
-        for (int t = 0; t < 9; ++t)
-            atomicAdd(&dw[(oc * 9 + t) * 32 + lane], acc[o][t]);  // a warp's 32 channels: one 128-byte line
-        if (ks == 0) {
-            float s = bsum[o];
-            for (int d = 16; d > 0; d >>= 1)
-                s += __shfl_xor_sync(0xffffffffu, s, d);
-            if (lane == 0)
-                atomicAdd(&db[oc], s);
+            for (int t = 0; t < 9; ++t)
+                atomicAdd(&dw[(oc * 9 + t) * 32 + lane], acc[o][t]);  // a warp's 32 channels: one 128-byte line
+            if (ks == 0) {
+                float s = bsum[o];
+                for (int d = 16; d > 0; d >>= 1)
+                    s += __shfl_xor_sync(0xffffffffu, s, d);
+                if (lane == 0)
+                    atomicAdd(&db[oc], s);
+            }
         }
     }
 }
@@ -573,7 +585,7 @@ constexpr int kWg1Buf = 32 * kWg1Dz + kWg1X;
 
 __global__ void __launch_bounds__(128) wgrad_first_kernel(const float* __restrict__ x, const float* __restrict__ dz,
     float* __restrict__ dw, float* __restrict__ db, int H, int W, int tiles_x, int tiles, int N,
-    const int* __restrict__ nonfinite)
+    int copies, const int* __restrict__ nonfinite)
 {
     __shared__ __align__(16) float sm[2 * kWg1Buf];
     __shared__ float red[32 * 28];
@@ -602,7 +614,9 @@ __global__ void __launch_bounds__(128) wgrad_first_kernel(const float* __restric
         }
     };
 
-    float acc[27], bsum = 0.0f;
+    dw += blockIdx.x % copies * kGradPitch;
+    db += blockIdx.x % copies * kGradPitch;
+    float acc[27], bsum8 = 0.0f, bsum = 0.0f;  // dz in short chains: of a tile, of 8 tiles, of the eights
 #pragma unroll
     for (int t = 0; t < 27; ++t)
         acc[t] = 0.0f;
@@ -622,6 +636,7 @@ __global__ void __launch_bounds__(128) wgrad_first_kernel(const float* __restric
         const int x0 = (tile % tiles % tiles_x) * kTileW, y0 = (tile % tiles / tiles_x) * kWgRows;
         auto add_tile = [&](auto safe_tile) {
             constexpr bool kSafe = decltype(safe_tile)::value;
+            float tsum = 0.0f;
             const unsigned ym = kSafe ? inside_bits(y0 - 1, kWgRows + 2, H) : 0;
 #pragma unroll 1
             for (int q = 2 * warp; q < 2 * warp + 2; ++q) {  // this warp's 4-pixel groups of each row
@@ -630,7 +645,7 @@ __global__ void __launch_bounds__(128) wgrad_first_kernel(const float* __restric
                 for (int row = 0; row < kWgRows; ++row) {
                     const float4 z = *reinterpret_cast<const float4*>(b + lane * kWg1Dz + row * kTileW + 4 * q);
                     const float gz[4] = {z.x, z.y, z.z, z.w};
-                    bsum += (z.x + z.y) + (z.z + z.w);
+                    tsum += (z.x + z.y) + (z.z + z.w);
 #pragma unroll
                     for (int c = 0; c < 3; ++c)
 #pragma unroll
@@ -650,33 +665,48 @@ __global__ void __launch_bounds__(128) wgrad_first_kernel(const float* __restric
                         }
                 }
             }
+            bsum8 += tsum;
         };
         if (safe)
             add_tile(std::true_type{});
         else
             add_tile(std::false_type{});
+        if ((k & 7) == 7) {
+            bsum += bsum8;
+            bsum8 = 0.0f;
+        }
+        __syncthreads();
+        if ((k + 1) % kWgFlush != 0 && tile + static_cast<int>(gridDim.x) < total)
+            continue;
+        // the four warps' sums, then one coalesced addition per weight and block
+#pragma unroll
+        for (int t = 0; t < 27; ++t) {
+            atomicAdd(&red[lane * 27 + t], acc[t]);
+            acc[t] = 0.0f;
+        }
+        atomicAdd(&red[32 * 27 + lane], bsum + bsum8);
+        bsum = bsum8 = 0.0f;
+        __syncthreads();
+        for (int i = tid; i < 32 * 28; i += 128) {
+            atomicAdd(i < 32 * 27 ? &dw[i] : &db[i - 32 * 27], red[i]);
+            red[i] = 0.0f;
+        }
         __syncthreads();
     }
-    __syncthreads();
-    // the four warps' sums, then one coalesced addition per weight and block
-#pragma unroll
-    for (int t = 0; t < 27; ++t)
-        atomicAdd(&red[lane * 27 + t], acc[t]);
-    atomicAdd(&red[32 * 27 + lane], bsum);
-    __syncthreads();
-    for (int i = tid; i < 32 * 27; i += 128)
-        atomicAdd(&dw[i], red[i]);
-    if (tid < 32)
-        atomicAdd(&db[tid], red[32 * 27 + tid]);
 }
 
 __global__ void adam_kernel(float* __restrict__ prm, const float* __restrict__ g, float* __restrict__ m,
-    float* __restrict__ v, int n, float lr, float b1, float b2, float c1, float c2, float eps)
+    float* __restrict__ v, int n, int copies, float lr, float b1, float b2, float c1, float c2, float eps)
 {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n)
         return;
-    const float gi = g[i];
+    float part[4] = {};  // (copies in four chains: shorter sums, loads ahead)
+    for (int c = 0; c < copies; c += 4)
+#pragma unroll
+        for (int k = 0; k < 4; ++k)
+            part[k] += c + k < copies ? g[(c + k) * kGradPitch + i] : 0.0f;
+    const float gi = (part[0] + part[1]) + (part[2] + part[3]);
     m[i] = b1 * m[i] + (1.0f - b1) * gi;
     v[i] = b2 * v[i] + (1.0f - b2) * gi * gi;
     prm[i] -= lr * (m[i] / c1) / (sqrtf(v[i] / c2) + eps);
@@ -741,6 +771,7 @@ void launch_conv(const float* x, const float* prm, int layer, const float* a_pre
 }  // namespace
 
 int upsampler_param_count() { return kParams; }
+size_t upsampler_grad_floats() { return static_cast<size_t>(kGradCopies) * kGradPitch; }
 
 void upsampler_init_params(float* host, uint64_t seed)
 {
@@ -767,8 +798,8 @@ cudaError_t launch_upsampler_prepare(const float* coarse, int cw, int ch, int cf
     return cudaGetLastError();
 }
 
-// One Adam step on a batch: forward, L1 loss, backward, update.  work:
-// upsampler_train_work_floats floats; state: the loss and, as an int, the
+// One Adam step on a batch: forward, L1 loss, backward, update.  grad:
+// upsampler_grad_floats floats; work: upsampler_train_work_floats; state: the loss and, as an int, the
 // non-finite flag.
 cudaError_t upsampler_train_step(float* prm, float* grad, float* m, float* v, int step, const float* input,
     const float* target, int N, int H, int W, float lr, float* work, float* state, cudaStream_t st)
@@ -786,8 +817,6 @@ cudaError_t upsampler_train_step(float* prm, float* grad, float* m, float* v, in
     float* dz1 = dz2 + px * 32;
     float* dr = dz1 + px * 32;
     int* bad = reinterpret_cast<int*>(state + 1);
-    if ((e = cudaMemsetAsync(grad, 0, kParams * sizeof(float), st)) != cudaSuccess)
-        return e;
     if ((e = cudaMemsetAsync(state, 0, 2 * sizeof(float), st)) != cudaSuccess)
         return e;
     launch_conv<3, 32, 8, kConvRelu, true>(input, prm, 0, nullptr, a1, N, H, W, bad, st);
@@ -798,22 +827,25 @@ cudaError_t upsampler_train_step(float* prm, float* grad, float* m, float* v, in
     // weight gradients: resident blocks walk the tiles, so a block's sums are added once
     const int tx = (W + kTileW - 1) / kTileW, tiles = tx * ((H + kWgRows - 1) / kWgRows);
     const int wb = static_cast<int>(std::min<int64_t>(static_cast<int64_t>(tiles) * N, 4 * sms));
+    const int copies = std::min((wb + 15) / 16, kGradCopies);
+    if ((e = cudaMemsetAsync(grad, 0, static_cast<size_t>(copies) * kGradPitch * sizeof(float), st)) != cudaSuccess)
+        return e;
     float* gw[4];
     float* gb[4];
     for (int l = 0; l < 4; ++l) {
         gw[l] = grad + kUpLayers[l].w_off;
         gb[l] = grad + kUpLayers[l].b_off;
     }
-    wgrad_kernel<2, 2><<<wb, 128, WgShape<2, 2>::smem, st>>>(a3, dr, gw[3], gb[3], H, W, tx, tiles, N, bad);
+    wgrad_kernel<2, 2><<<wb, 128, WgShape<2, 2>::smem, st>>>(a3, dr, gw[3], gb[3], H, W, tx, tiles, N, copies, bad);
     launch_conv<2, 32, 8, kConvBwd, false>(dr, prm, 3, a3, dz3, N, H, W, bad, st);
-    wgrad_kernel<32, 8><<<wb, 128, WgShape<32, 8>::smem, st>>>(a2, dz3, gw[2], gb[2], H, W, tx, tiles, N, bad);
+    wgrad_kernel<32, 8><<<wb, 128, WgShape<32, 8>::smem, st>>>(a2, dz3, gw[2], gb[2], H, W, tx, tiles, N, copies, bad);
     launch_conv<32, 32, 8, kConvBwd, false>(dz3, prm, 2, a2, dz2, N, H, W, bad, st);
-    wgrad_kernel<32, 8><<<wb, 128, WgShape<32, 8>::smem, st>>>(a1, dz2, gw[1], gb[1], H, W, tx, tiles, N, bad);
+    wgrad_kernel<32, 8><<<wb, 128, WgShape<32, 8>::smem, st>>>(a1, dz2, gw[1], gb[1], H, W, tx, tiles, N, copies, bad);
     launch_conv<32, 32, 8, kConvBwd, false>(dz2, prm, 1, a1, dz1, N, H, W, bad, st);
-    wgrad_first_kernel<<<wb, 128, 0, st>>>(input, dz1, gw[0], gb[0], H, W, tx, tiles, N, bad);
+    wgrad_first_kernel<<<wb, 128, 0, st>>>(input, dz1, gw[0], gb[0], H, W, tx, tiles, N, copies, bad);
     const float b1 = 0.9f, b2 = 0.999f;
     const float c1 = 1.0f - std::pow(b1, static_cast<float>(step)), c2 = 1.0f - std::pow(b2, static_cast<float>(step));
-    adam_kernel<<<(kParams + 255) / 256, 256, 0, st>>>(prm, grad, m, v, kParams, lr, b1, b2, c1, c2, 1e-8f);
+    adam_kernel<<<(kParams + 255) / 256, 256, 0, st>>>(prm, grad, m, v, kParams, copies, lr, b1, b2, c1, c2, 1e-8f);
     return cudaGetLastError();
 }
 
