@@ -65,3 +65,28 @@ def test_noalloc_rejects_images_beyond_its_workspace(vsc, cuda):
     assert rc == vsc.VSC_EINVAL
     msg = lib.vsc_last_error().decode()
     assert "limit" in msg and str(vsc.NOALLOC_MAX_PIXELS) in msg
+
+
+def test_noalloc_calls_that_overlap_do_not_wait_for_each_other(vsc, cuda):
+    """Overlapping calls race on the shared array and have no defined results,
+    but neither may wait for the other's bookkeeping: both finish at once and
+    the device reports no timeout.  424 x 300 is a size whose planes would fit
+    the array."""
+    import time
+
+    import torch
+
+    h, w = 300, 424
+    rng = np.random.Generator(np.random.PCG64(5))
+    ins = [_inputs(rng, h, w, cuda) for _ in range(2)]
+    streams = [torch.cuda.Stream() for _ in range(2)]
+    vsc.get_consist_out_noalloc(*ins[0][:3], 8, 0.15, 0.15, ins[0][3])
+    torch.cuda.synchronize()
+    t = time.perf_counter()
+    for _ in range(20):
+        for (P, A, Wt, O), s in zip(ins, streams):
+            with torch.cuda.stream(s):
+                vsc.get_consist_out_noalloc(P, A, Wt, 75, 0.15, 0.15, O)
+    torch.cuda.synchronize()
+    assert time.perf_counter() - t < 0.5  # 40 solves of 0.15 ms
+    vsc.check_device()

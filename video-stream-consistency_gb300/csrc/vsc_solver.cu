@@ -2724,8 +2724,12 @@ cudaError_t run_solver_noalloc(const float* P, const float* A, const float* Wt, 
         return e;
     // Every workspace element (lap P, both momentum images, the second Jacobi
     // buffer) is written before it is read, so nothing is cleared.
-    return run_solver(P, A, Wt, O, w, h, num_iter, step, mom, ws, kNoAllocWorkspaceFloats, st, nullptr, nullptr,
-        kSolverExact);
+    // On interleaved images even where the array has room for planes: the solve on
+    // planes waits for counters in its workspace, and of two calls that overlap (a
+    // race on the shared array that costs their results) the setup of one would
+    // zero the counters that the other's blocks wait for.
+    return run_solver(P, A, Wt, O, w, h, num_iter, step, mom, ws, solver_workspace_floats(w, h, kSolverExact), st,
+        nullptr, nullptr, kSolverExact);
 }
 
 cudaError_t device_timeout_flag(int** flag)
