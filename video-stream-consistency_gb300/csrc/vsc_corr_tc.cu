@@ -28,6 +28,7 @@
 // from its largest magnitude (|f| 2^k in [2^13, 2^14)) before the 16-bit
 // conversion, which keeps FP16 clear of overflow and of its subnormal range;
 // the sums are multiplied by 2^-(k1 + k2) afterwards (exact).
+#include "vsc_device.h"
 #include "vsc_internal.h"
 #include "vsc_math.cuh"
 #include "vsc_ptx.cuh"
@@ -36,7 +37,6 @@
 #include <cuda_fp16.h>
 
 #include <functional>
-#include <mutex>
 
 namespace vsc {
 namespace {
@@ -705,24 +705,17 @@ bool encode_chunked_map(CUtensorMap* m, const void* base, int N, int H, int W, i
 // persistent grid is sized by the device's SM count.
 cudaError_t tc_prepare_device(int* sms)
 {
-    static std::mutex mu;
-    static int count[64] = {};
-    int dev = 0;
-    cudaError_t e = cudaGetDevice(&dev);
-    if (e != cudaSuccess)
-        return e;
-    if (dev < 0 || dev >= 64)
-        return cudaErrorInvalidDevice;
-    std::lock_guard<std::mutex> lock(mu);
-    if (!count[dev]) {
-        if ((e = cudaFuncSetAttribute(corr_tc_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kTcSmemLimit)) !=
-            cudaSuccess)
-            return e;
-        if ((e = cudaDeviceGetAttribute(&count[dev], cudaDevAttrMultiProcessorCount, dev)) != cudaSuccess)
-            return e;
-    }
-    *sms = count[dev];
-    return cudaSuccess;
+    static PerDevice<int> device;
+    return device.get(
+        [](int* count) {
+            cudaError_t e =
+                cudaFuncSetAttribute(corr_tc_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kTcSmemLimit);
+            int dev = 0;
+            if (e == cudaSuccess)
+                e = cudaGetDevice(&dev);
+            return e != cudaSuccess ? e : cudaDeviceGetAttribute(count, cudaDevAttrMultiProcessorCount, dev);
+        },
+        sms);
 }
 
 }  // namespace

@@ -18,6 +18,7 @@
 // cores (vsc_upsampler_tc.cu).  Nothing here has a bit-exact contract
 // (contraction is spelled out with __fmaf_rn, the library being built
 // without automatic contraction).
+#include "vsc_device.h"
 #include "vsc_internal.h"
 #include "vsc_math.cuh"
 
@@ -25,7 +26,6 @@
 
 #include <algorithm>
 #include <cmath>
-#include <mutex>
 #include <type_traits>
 
 namespace vsc {
@@ -723,37 +723,28 @@ uint64_t splitmix(uint64_t* s)
 // Dynamic shared memory of the training kernels, opted into once per device.
 cudaError_t train_prepare_device(int* sms)
 {
-    static std::mutex mu;
-    static int count[64] = {};
-    int dev = 0;
-    cudaError_t e = cudaGetDevice(&dev);
-    if (e != cudaSuccess)
-        return e;
-    if (dev < 0 || dev >= 64)
-        return cudaErrorInvalidDevice;
-    std::lock_guard<std::mutex> lock(mu);
-    if (!count[dev]) {
-        constexpr auto kAttr = cudaFuncAttributeMaxDynamicSharedMemorySize;
-        auto set = [&](auto* k, int smem) {
+    static PerDevice<int> device;
+    return device.get(
+        [](int* count) {
+            constexpr auto kAttr = cudaFuncAttributeMaxDynamicSharedMemorySize;
+            cudaError_t e = cudaSuccess;
+            auto set = [&](auto* k, int smem) {
+                if (e == cudaSuccess)
+                    e = cudaFuncSetAttribute(k, kAttr, smem);
+            };
+            set(conv3x3_kernel<3, 32, 8, kConvRelu, true>, ConvShape<3, 32, 8>::smem);
+            set(conv3x3_kernel<32, 32, 8, kConvRelu, false>, ConvShape<32, 32, 8>::smem);
+            set(conv3x3_kernel<32, 2, 2, kConvLoss, false>, ConvShape<32, 2, 2>::smem);
+            set(conv3x3_kernel<2, 32, 8, kConvBwd, false>, ConvShape<2, 32, 8>::smem);
+            set(conv3x3_kernel<32, 32, 8, kConvBwd, false>, ConvShape<32, 32, 8>::smem);
+            set(wgrad_kernel<2, 2>, WgShape<2, 2>::smem);
+            set(wgrad_kernel<32, 8>, WgShape<32, 8>::smem);
+            int dev = 0;
             if (e == cudaSuccess)
-                e = cudaFuncSetAttribute(k, kAttr, smem);
-        };
-        set(conv3x3_kernel<3, 32, 8, kConvRelu, true>, ConvShape<3, 32, 8>::smem);
-        set(conv3x3_kernel<32, 32, 8, kConvRelu, false>, ConvShape<32, 32, 8>::smem);
-        set(conv3x3_kernel<32, 2, 2, kConvLoss, false>, ConvShape<32, 2, 2>::smem);
-        set(conv3x3_kernel<2, 32, 8, kConvBwd, false>, ConvShape<2, 32, 8>::smem);
-        set(conv3x3_kernel<32, 32, 8, kConvBwd, false>, ConvShape<32, 32, 8>::smem);
-        set(wgrad_kernel<2, 2>, WgShape<2, 2>::smem);
-        set(wgrad_kernel<32, 8>, WgShape<32, 8>::smem);
-        int n = 0;
-        if (e == cudaSuccess)
-            e = cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev);
-        if (e != cudaSuccess)
-            return e;
-        count[dev] = n;
-    }
-    *sms = count[dev];
-    return cudaSuccess;
+                e = cudaGetDevice(&dev);
+            return e != cudaSuccess ? e : cudaDeviceGetAttribute(count, cudaDevAttrMultiProcessorCount, dev);
+        },
+        sms);
 }
 
 template <int CI, int CO, int OCT, int kMode, bool kInter>

@@ -45,13 +45,14 @@
 // max(|r_u|, |r_v|) <= max_residual, else base).  Every mbarrier wait is
 // bounded; a wait that runs out stops all roles and sets the device timeout
 // flag.
+#include "vsc_device.h"
 #include "vsc_internal.h"
 #include "vsc_math.cuh"
 #include "vsc_ptx.cuh"
 
 #include <cuda_fp16.h>
 
-#include <mutex>
+#include <algorithm>
 
 namespace vsc {
 namespace {
@@ -393,26 +394,45 @@ bool encode_act_map(CUtensorMap* m, const void* base, int N, int H, int W, int c
                CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
 
+// at least kUpMinSmem, so that one CTA (and one Tensor Memory allocation) occupies an SM
+template <int KCH, int NO>
+constexpr int up_layer_smem()
+{
+    constexpr uint32_t smem = std::max(up_smem_bytes(KCH, NO), kUpMinSmem);
+    static_assert(smem <= static_cast<uint32_t>(kUpSmemLimit), "shared memory per CTA");
+    return static_cast<int>(smem);
+}
+
+// The layers' dynamic shared memory opt-in on the current device, and its SM count.
+cudaError_t up_prepare_device(int* sms)
+{
+    static PerDevice<int> device;
+    return device.get(
+        [](int* count) {
+            constexpr auto kAttr = cudaFuncAttributeMaxDynamicSharedMemorySize;
+            cudaError_t e = cudaFuncSetAttribute(up_conv_tc_kernel<2, 1, 32, false>, kAttr, up_layer_smem<2, 32>());
+            if (e == cudaSuccess)
+                e = cudaFuncSetAttribute(up_conv_tc_kernel<4, 4, 32, false>, kAttr, up_layer_smem<4, 32>());
+            if (e == cudaSuccess)
+                e = cudaFuncSetAttribute(up_conv_tc_kernel<4, 4, 16, true>, kAttr, up_layer_smem<4, 16>());
+            int dev = 0;
+            if (e == cudaSuccess)
+                e = cudaGetDevice(&dev);
+            return e != cudaSuccess ? e : cudaDeviceGetAttribute(count, cudaDevAttrMultiProcessorCount, dev);
+        },
+        sms);
+}
+
 template <int KCH, int LCH, int NO, bool kFinish>
 cudaError_t run_layer(int l, const void* wtc, const float* prm, const void* in, __half* out, const float* input,
     float* flow, int64_t s_out, float max_residual, int N, int H, int W, int sms, int* flag, cudaStream_t st)
 {
-    // at least kUpMinSmem, so that one CTA (and one Tensor Memory allocation) occupies an SM
-    constexpr uint32_t smem = up_smem_bytes(KCH, NO) > kUpMinSmem ? up_smem_bytes(KCH, NO) : kUpMinSmem;
-    static_assert(smem <= static_cast<uint32_t>(kUpSmemLimit), "shared memory per CTA");
-    static std::once_flag once;
-    static cudaError_t attr = cudaSuccess;
-    std::call_once(once, [] {
-        attr = cudaFuncSetAttribute(up_conv_tc_kernel<KCH, LCH, NO, kFinish>,
-            cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));
-    });
-    if (attr != cudaSuccess)
-        return attr;
     CUtensorMap m;
     if (!encode_act_map(&m, in, N, H, W, LCH))
         return cudaErrorInvalidValue;
     const int items = N * ((H + kUpGR - 1) / kUpGR) * ((W + kUpOut - 1) / kUpOut);
-    return launch_pdl(up_conv_tc_kernel<KCH, LCH, NO, kFinish>, dim3(std::min(items, sms)), dim3(kUpThreads), smem, st,
+    return launch_pdl(up_conv_tc_kernel<KCH, LCH, NO, kFinish>, dim3(std::min(items, sms)), dim3(kUpThreads),
+        up_layer_smem<KCH, NO>(), st,
         m, reinterpret_cast<const uint4*>(static_cast<const unsigned char*>(wtc) + kTcLayers[l].wt_off),
         prm + kUpLayers[l].b_off, kUpLayers[l].co, out, input, flow, s_out, max_residual, N, H, W, flag);
 }
@@ -440,10 +460,8 @@ cudaError_t launch_upsampler_tc(const void* wtc, const float* prm, const float* 
 {
     if (N <= 0 || H <= 0 || W <= 0)
         return cudaSuccess;
-    int dev = 0, sms = 0;
-    cudaError_t e = cudaGetDevice(&dev);
-    if (e == cudaSuccess)
-        e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+    int sms = 0;
+    cudaError_t e = up_prepare_device(&sms);
     int* flag = nullptr;
     if (e == cudaSuccess)
         e = device_timeout_flag(&flag);
