@@ -285,17 +285,22 @@ VSC_API vsc_status vsc_get_bilinear(const vsc_image* input, const vsc_image* out
 /* Bytes of device workspace vsc_get_consist_out needs for a width x height image. */
 VSC_API size_t vsc_consist_out_workspace_size(int32_t width, int32_t height);
 
+/* Bytes of device workspace with which a solve of a form (VSC_SOLVER_EXACT:
+ * vsc_get_consist_out, VSC_SOLVER_FMA: vsc_get_consist_out_fma) runs as it does with
+ * workspace = NULL, at its fastest: about 7/4 of vsc_consist_out_workspace_size,
+ * and a little more than vsc_consist_out_fma_workspace_size. */
+VSC_API size_t vsc_consist_out_full_workspace_size(int32_t width, int32_t height, int32_t form);
+
 /* num_iter gradient-descent steps with momentum on the blend energy
  * (Jacobi form; consis_out holds the initial solution and receives the
  * result).  Replaces get_consist_out / kernel_consist_out
  * (flowconsistency.cu:193-258, :350-374).  workspace: device memory of at
  * least vsc_consist_out_workspace_size bytes, or NULL to let the library
  * take it from the stream-ordered memory pool of the current device.  The
- * faster solve, each channel as its own plane in one launch, needs 7/4 of
- * those bytes (the width rounded up to a multiple of 4) and 4 bytes per tile:
- * NULL takes them, a workspace that has them is used so, a smaller one is
- * solved on interleaved images (same bits, about 1.6 times the time at
- * 1920x1080). */
+ * faster solve of all but the smallest images, each channel as its own plane in
+ * one launch, needs vsc_consist_out_full_workspace_size bytes: NULL takes
+ * them, a workspace that has them is used so, a smaller one is solved on
+ * interleaved images (same bits, about 1.6 times the time at 1920x1080). */
 VSC_API vsc_status vsc_get_consist_out(const vsc_image* crnt_pr, const vsc_image* prev_stab_warp,
     const vsc_image* cons_wt, int32_t num_iter, float step_size, float mom_fac, const vsc_image* consis_out,
     void* workspace, size_t workspace_bytes, vsc_stream_t stream);
@@ -303,10 +308,11 @@ VSC_API vsc_status vsc_get_consist_out(const vsc_image* crnt_pr, const vsc_image
 /* vsc_get_consist_out in the VSC_SOLVER_FMA form: same arguments; its
  * workspace (vsc_consist_out_fma_workspace_size bytes, 16-byte aligned, or
  * NULL for the library's stream-ordered pool) holds the solve as planes, 18
- * floats a pixel.  Where the width is not a multiple of 4, the TMA-fed solve
- * needs the bytes of the width rounded up to one: NULL takes them, and so does
- * a workspace that has them; a smaller one is solved with plain loads (same
- * bits, about 2.5 times the time).  Results within the tolerance stated at VSC_SOLVER_FMA of
+ * floats a pixel.  With vsc_consist_out_full_workspace_size bytes, which NULL
+ * takes, it is at its fastest: in fewer, small images have rounds of fewer steps
+ * (640x360, 150 steps: 145 us against 131), and where the width is not a
+ * multiple of 4 the solve runs with plain loads (about 2.5 times the time); same
+ * bits either way.  Results within the tolerance stated at VSC_SOLVER_FMA of
  * vsc_get_consist_out's.  No counterpart in the reference. */
 VSC_API size_t vsc_consist_out_fma_workspace_size(int32_t width, int32_t height);
 VSC_API vsc_status vsc_get_consist_out_fma(const vsc_image* crnt_pr, const vsc_image* prev_stab_warp,

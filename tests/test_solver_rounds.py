@@ -30,3 +30,36 @@ def test_plan_rejects_what_no_solve_takes(vsc):
     with pytest.raises(vsc.VscError):
         vsc.solver_plan(64, 64, 8, workspace_bytes=64 * 64 * 12 * 4 - 4, sms=SMS)
     assert vsc.solver_plan(64, 64, 0, sms=SMS).rounds == 0
+
+
+SIZES = [(1, 1), (5, 200), (64, 36), (240, 135), (426, 240), (427, 240), (640, 360), (720, 404), (800, 450), (854, 480),
+         (856, 480), (960, 540), (1279, 719), (1920, 1080), (3840, 2160)]
+
+
+def _fields(p):
+    return [getattr(p, f) for f, _ in p._fields_]
+
+
+@pytest.mark.parametrize("form", ["exact", "fma"])
+@pytest.mark.parametrize("w,h", SIZES)
+@pytest.mark.parametrize("iters", [8, 20, 150])
+def test_full_workspace_is_as_good_as_none(vsc, form, w, h, iters):
+    """A workspace of the full size takes the path of the library's own."""
+    full = vsc.consist_out_workspace_size(w, h, form, full=True)
+    assert full >= vsc.consist_out_workspace_size(w, h, form)
+    assert _fields(vsc.solver_plan(w, h, iters, form, full, SMS)) == _fields(vsc.solver_plan(w, h, iters, form, 0, SMS))
+
+
+def test_full_workspace_size_of_no_image(vsc):
+    assert vsc.consist_out_workspace_size(0, 10, full=True) == 0
+    assert vsc.load().vsc_consist_out_full_workspace_size(8, 8, 2) == 0
+
+
+@pytest.mark.parametrize("w,h,null_steps,small_steps", [(640, 360, 16, 12), (320, 180, 16, 12), (64, 36, 16, 16), (960, 540, 8, 8),
+                                                        (856, 480, 12, 8)])
+def test_a_smaller_workspace_gets_the_longest_rounds_it_has_counters_for(vsc, w, h, null_steps, small_steps):
+    """FMA form, 150 steps: the documented workspace has counters for the 8-step
+    tiles, rounded up to 64, which may be enough for 12-step or 16-step ones."""
+    assert vsc.solver_plan(w, h, 150, "fma", 0, SMS).steps == null_steps
+    p = vsc.solver_plan(w, h, 150, "fma", vsc.consist_out_workspace_size(w, h, "fma"), SMS)
+    assert p.planes and p.steps == small_steps

@@ -289,6 +289,25 @@ def test_solve_of_several_launches(vsc, cuda, form, w):
     vsc.check_device()
 
 
+@pytest.mark.parametrize("form,w,h", [("exact", 641, 361), ("exact", 640, 360), ("fma", 427, 240), ("fma", 640, 360)])
+def test_consist_out_in_workspaces_of_both_sizes(vsc, oracle, cuda, form, w, h):
+    """A caller's workspace of the full size, of the documented one and the
+    library's own: the same bits, whatever path each takes."""
+    import torch
+
+    P, A, Wt, O0 = _img(h, w), _img(h, w), _img(h, w, hi=2.0), _img(h, w)
+    ref = oracle.consist_out(P, A, Wt, 37, 0.15, 0.15, O0, form=form)
+    got = []
+    for size in (vsc.consist_out_workspace_size(w, h, form), vsc.consist_out_workspace_size(w, h, form, full=True), 0):
+        ws = torch.full((size // 4,), float("nan"), device=cuda) if size else None
+        O = _t(O0, cuda)
+        vsc.get_consist_out(_t(P, cuda), _t(A, cuda), _t(Wt, cuda), 37, 0.15, 0.15, O, form=form, workspace=ws)
+        got.append(O.cpu().numpy())
+        assert _equal_up_to_zero_sign(got[-1], ref)
+        assert np.array_equal(got[-1].view(np.uint32), got[0].view(np.uint32))
+    vsc.check_device()
+
+
 def test_consist_out_fma_single_tile_shape(vsc, cuda):
     """The FMA form has one tile shape (128 x 72 of a plane); the autotuner
     reports it without measuring."""

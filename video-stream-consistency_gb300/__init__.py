@@ -48,7 +48,7 @@ EXPORTED = [
     "vsc_multistream_set_fused", "vsc_multistream_fused", "vsc_multistream_set_upsampler",
     "vsc_stabilizer_synchronize", "vsc_stabilizer_wait_output",
     "vsc_get_consist_out_fma", "vsc_consist_out_fma_workspace_size", "vsc_solver_autotune_form",
-    "vsc_solver_tile_rows_form", "vsc_solver_plan",
+    "vsc_solver_tile_rows_form", "vsc_solver_plan", "vsc_consist_out_full_workspace_size",
     "vsc_stabilizer_set_solver_form", "vsc_multistream_set_solver_form", "vsc_write_jpeg",
 ]
 VSC_DTYPE_F32, VSC_DTYPE_BF16, VSC_DTYPE_F16 = 0, 1, 2
@@ -215,6 +215,8 @@ def load():
     L.vsc_consist_out_workspace_size.argtypes = [i32, i32]
     L.vsc_consist_out_fma_workspace_size.restype = C.c_size_t
     L.vsc_consist_out_fma_workspace_size.argtypes = [i32, i32]
+    L.vsc_consist_out_full_workspace_size.restype = C.c_size_t
+    L.vsc_consist_out_full_workspace_size.argtypes = [i32, i32, i32]
     L.vsc_default_hyper_params.restype = None
     L.vsc_default_hyper_params.argtypes = [C.POINTER(HyperParams)]
     L.vsc_stabilizer_hyper_params.restype = C.POINTER(HyperParams)
@@ -491,7 +493,10 @@ def solver_plan(w: int, h: int, num_iter: int, form: str = "exact", workspace_by
     return p
 
 
-def consist_out_workspace_size(w: int, h: int, form: str = "exact") -> int:
+def consist_out_workspace_size(w: int, h: int, form: str = "exact", full: bool = False) -> int:
+    """Bytes get_consist_out needs; with `full`, those with which it is as fast as with no workspace given."""
+    if full:
+        return int(load().vsc_consist_out_full_workspace_size(w, h, SOLVER_FORMS[form]))
     fn = load().vsc_consist_out_fma_workspace_size if form == "fma" else load().vsc_consist_out_workspace_size
     return int(fn(w, h))
 

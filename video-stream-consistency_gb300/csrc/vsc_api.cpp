@@ -500,6 +500,13 @@ VSC_API size_t vsc_consist_out_fma_workspace_size(int32_t width, int32_t height)
     return solver_workspace_floats(width, height, kSolverFma) * sizeof(float);
 }
 
+VSC_API size_t vsc_consist_out_full_workspace_size(int32_t width, int32_t height, int32_t form)
+{
+    if (!dims_ok(width) || !dims_ok(height) || (form != VSC_SOLVER_EXACT && form != VSC_SOLVER_FMA))
+        return 0;
+    return solver_workspace_full_floats(width, height, form) * sizeof(float);
+}
+
 VSC_API vsc_status vsc_solver_plan(int32_t width, int32_t height, int32_t num_iter, int32_t form,
     size_t workspace_bytes, int32_t sms, vsc_solve_plan* out)
 {

@@ -147,7 +147,8 @@ cudaError_t launch_bilinear_group(const Img* in, const Img* out, int n, cudaStre
 // 16-byte grid.  In a workspace of solver_workspace_floats only, the exact form
 // (4 images: lap P, two momentum images, the second iterate) runs a launch a
 // round on interleaved images, and the FMA form, where its width is not a
-// multiple of 4 (else the two sizes are the same), one with plain loads.
+// multiple of 4, one with plain loads; at other widths the FMA form's smaller
+// workspace holds the planes and counters for rounds of 8 steps, perhaps of 12.
 enum SolverForm { kSolverExact = 0, kSolverFma = 1 };
 size_t solver_workspace_floats(int w, int h, int form = kSolverExact);
 size_t solver_workspace_full_floats(int w, int h, int form);

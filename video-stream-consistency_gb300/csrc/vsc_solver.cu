@@ -2251,8 +2251,9 @@ bool pl_tma_eligible(const DeviceInfo* di, int w, int h, const float* ws, size_t
 // us, 8, 12 and 16 a round: FMA 320x180 147, 126, 109; 640x360 177, 145, 131;
 // 854x480 196, 163, 177; 960x540 195, 211, 217; 1280x720 290, 324, 385; exact
 // 480x270 189, 162, 167; 560x316 202, 170, 156; 640x360 204, 174, 199; 800x450
-// 220, 227, 277.
-int pl_rounds_cfg(int sms, int w, int h, int num_iter, int form)
+// 220, 227, 277.  Of the rounds that a workspace of ws_floats has counters for: a
+// smaller one may have them for 12 steps and not for 16.
+int pl_rounds_cfg(int sms, int w, int h, int num_iter, int form, size_t ws_floats)
 {
     struct Cost {
         int cfg;
@@ -2267,6 +2268,8 @@ int pl_rounds_cfg(int sms, int w, int h, int num_iter, int form)
     int best = form;
     float limit = 0.0f;
     for (const Cost& c : kCost[form == kSolverFma]) {
+        if (c.cfg != 0 && !pl_fits(w, h, ws_floats, form | c.cfg))
+            continue;
         const float tiles = static_cast<float>(pl_tiles_of(w, h, form | c.cfg)) / static_cast<float>(sms);
         const float us = static_cast<float>(solve_launches(num_iter, pl_steps(c.cfg))) *
                          std::max(c.least, c.base + c.tile * tiles);
@@ -2287,13 +2290,6 @@ int pl_rounds_cfg(int sms, int w, int h, int num_iter, int form)
 bool exact_interleaved(int sms, int w, int h, int num_iter)
 {
     return tiles_of(w, h, kIH) <= sms || (num_iter <= 2 * kTbT && tiles_of(w, h, kPIH) <= sms);
-}
-
-// The rounds of a solve in a workspace of ws_floats.
-int pl_cfg(int sms, int w, int h, int num_iter, int form, size_t ws_floats)
-{
-    const int cfg = pl_rounds_cfg(sms, w, h, num_iter, form);
-    return pl_fits(w, h, ws_floats, cfg) ? cfg : form;
 }
 
 struct PlanarCopy {
@@ -2413,7 +2409,7 @@ cudaError_t run_solver_planes(const DeviceInfo* di, int form, const float* P, co
     cudaStream_t st, int* nl, uint8_t* rgba_out, const float* Oc, int cw, int ch)
 {
     const bool tma = pl_tma_eligible(di, w, h, workspace, ws_floats, form);
-    const int cfg = tma ? pl_cfg(di->sms, w, h, num_iter, form, ws_floats) : form;
+    const int cfg = tma ? pl_rounds_cfg(di->sms, w, h, num_iter, form, ws_floats) : form;
     const PlWs v = pl_view(workspace, w, h, tma ? pl_pitch(w) : w, cfg);
     cudaError_t e = launch_prep(form, P, A, Wt, Oi, v, v.O[0], w, h, step, v.cnt, v.ncnt, Oc, cw, ch, st);
     ++*nl;
@@ -2480,7 +2476,7 @@ cudaError_t solver_plan(int w, int h, int num_iter, int form, size_t ws_floats, 
     const bool inter = form == kSolverExact && w % 4 == 0 && exact_interleaved(sms, w, h, num_iter);
     p.planes = form == kSolverFma || (!inter && pl_fits(w, h, ws_floats, form));
     const bool one_launch = p.planes && pl_fits(w, h, ws_floats, form);
-    const int cfg = one_launch ? pl_cfg(sms, w, h, num_iter, form, ws_floats) : form;
+    const int cfg = one_launch ? pl_rounds_cfg(sms, w, h, num_iter, form, ws_floats) : form;
     p.steps = pl_steps(cfg);
     p.rounds = solve_launches(num_iter, p.steps);
     if (p.planes) {
