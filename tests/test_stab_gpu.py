@@ -308,6 +308,33 @@ def test_consist_out_in_workspaces_of_both_sizes(vsc, oracle, cuda, form, w, h):
     vsc.check_device()
 
 
+def test_consist_out_where_the_full_workspace_does_not_fit(vsc, cuda):
+    """On a device with room for the documented workspace but not for the
+    planes, a solve without a workspace still runs, on interleaved images."""
+    import torch
+
+    w, h = 8192, 4096
+    need, full = (vsc.consist_out_workspace_size(w, h, full=f) for f in (False, True))
+    g = torch.Generator(device=cuda).manual_seed(3)
+    P, A, O0 = (torch.rand((h, w, 3), generator=g, device=cuda) for _ in range(3))
+    Wt = torch.zeros_like(P)
+    ref, O = O0.clone(), O0.clone()
+    ws = torch.empty(need // 4, dtype=torch.float32, device=cuda)
+    vsc.get_consist_out(P, A, Wt, 9, 0.15, 0.15, ref, workspace=ws)
+    del ws
+    torch.cuda.synchronize()
+    torch.cuda.empty_cache()
+    filler = torch.empty(torch.cuda.mem_get_info()[0] - (need + full) // 2, dtype=torch.uint8, device=cuda)
+    try:
+        vsc.get_consist_out(P, A, Wt, 9, 0.15, 0.15, O)
+        torch.cuda.synchronize()
+    finally:
+        del filler
+        torch.cuda.empty_cache()
+    assert torch.equal(O.view(torch.int32), ref.view(torch.int32))
+    vsc.check_device()
+
+
 def test_consist_out_fma_single_tile_shape(vsc, cuda):
     """The FMA form has one tile shape (128 x 72 of a plane); the autotuner
     reports it without measuring."""

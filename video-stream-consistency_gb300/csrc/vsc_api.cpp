@@ -555,8 +555,15 @@ vsc_status consist_out_form(int form, const vsc_image* crnt_pr, const vsc_image*
         if (reinterpret_cast<uintptr_t>(ws) & 15)
             return set_error(VSC_EINVAL, "consist_out: workspace not 16-byte aligned");
     } else if (num_iter > 0) {
+        // the full size, or where the device has no room for it the least a solve needs
         ws_bytes = solver_workspace_full_floats(w, h, form) * sizeof(float);
-        if ((s = check_cuda(pool_alloc(&ws, ws_bytes, cs(stream)), "consist_out workspace")))
+        cudaError_t e = pool_alloc(&ws, ws_bytes, cs(stream));
+        if (e == cudaErrorMemoryAllocation) {
+            cudaGetLastError();
+            ws_bytes = need;
+            e = pool_alloc(&ws, ws_bytes, cs(stream));
+        }
+        if ((s = check_cuda(e, "consist_out workspace")))
             return s;
         pooled = true;
     }
