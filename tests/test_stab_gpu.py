@@ -335,6 +335,16 @@ def test_consist_out_where_the_full_workspace_does_not_fit(vsc, cuda):
     vsc.check_device()
 
 
+@pytest.mark.parametrize("w,h,iters", [(1280, 720, 3), (1280, 720, 4), (1920, 1080, 1), (1920, 1080, 7), (1920, 1080, 8)])
+def test_consist_out_few_steps_of_a_large_image(vsc, oracle, cuda, w, h, iters):
+    """The last step counts on interleaved images and the first on planes."""
+    P, A, Wt, O0 = _img(h, w), _img(h, w), _img(h, w, hi=2.0), _img(h, w)
+    O = _t(O0, cuda)
+    vsc.get_consist_out(_t(P, cuda), _t(A, cuda), _t(Wt, cuda), iters, 0.15, 0.15, O)
+    assert _equal_up_to_zero_sign(O.cpu().numpy(), oracle.consist_out(P, A, Wt, iters, 0.15, 0.15, O0))
+    vsc.check_device()
+
+
 def test_consist_out_fma_single_tile_shape(vsc, cuda):
     """The FMA form has one tile shape (128 x 72 of a plane); the autotuner
     reports it without measuring."""

@@ -2285,11 +2285,18 @@ int pl_rounds_cfg(int sms, int w, int h, int num_iter, int form, size_t ws_float
 
 // The exact form on interleaved images, a launch a round, where one wave of its
 // 64 x 32 tiles is the image (75 steps: 320x180 71 us against 75 in planes,
-// 240x135 70 against 86), or one of the 64 x 48 tiles for two rounds at most
-// (600x338, 16 steps: 28 us against 32).
+// 240x135 70 against 86), one of the 64 x 48 tiles for two rounds at most
+// (600x338, 16 steps: 28 us against 32), or where a few steps of a large image do not
+// pay for the planes' conversions (us, interleaved and in planes: 1280x720 1 step 31
+// and 37, 3 steps 37 and 40, 4 steps 41 and 41; 1600x900 3 steps 58 and 59, 4
+// steps 64 and 61; 1920x1080 1 step 61 and 81, 5 steps 77 and 89, 7 steps 93 and
+// 95, 8 steps 106 and 99; 3840x2160 2 steps 209 and 300, 7 steps 326 and 324; 960x540
+// 1 step 24 and 22).
 bool exact_interleaved(int sms, int w, int h, int num_iter)
 {
-    return tiles_of(w, h, kIH) <= sms || (num_iter <= 2 * kTbT && tiles_of(w, h, kPIH) <= sms);
+    const int tall = tiles_of(w, h, kPIH);
+    return tiles_of(w, h, kIH) <= sms || (num_iter <= 2 * kTbT && tall <= sms) || (num_iter <= 3 && tall > 4 * sms) ||
+           (num_iter < kTbT && tall > 8 * sms);
 }
 
 struct PlanarCopy {
