@@ -335,7 +335,7 @@ def test_consist_out_where_the_full_workspace_does_not_fit(vsc, cuda):
     vsc.check_device()
 
 
-@pytest.mark.parametrize("w,h,iters", [(1280, 720, 3), (1280, 720, 4), (1920, 1080, 1), (1920, 1080, 7), (1920, 1080, 8)])
+@pytest.mark.parametrize("w,h,iters", [(1280, 720, 3), (1280, 720, 4), (1920, 1080, 1), (1920, 1080, 6), (1920, 1080, 7)])
 def test_consist_out_few_steps_of_a_large_image(vsc, oracle, cuda, w, h, iters):
     """The last step counts on interleaved images and the first on planes."""
     P, A, Wt, O0 = _img(h, w), _img(h, w), _img(h, w, hi=2.0), _img(h, w)

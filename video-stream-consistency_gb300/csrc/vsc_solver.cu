@@ -1523,6 +1523,8 @@ __device__ __forceinline__ void pl_load_constants(float* stage, const PlSolve<kN
         tma_load_3d(stage + 4 * G::kStage, m + kPmA, j.ox, j.oy, j.c, bar);
 }
 
+// The first round has no U to load, and the last one's U is not stored: 3840x2160,
+// FMA form, 1 step 250 -> 236 us, 8 steps 292 -> 271.
 template <int kCfg, int kN>
 __device__ __forceinline__ void pl_load_iterate(float* stage, const PlSolve<kN>& g, const PlJob& j, uint64_t* bar)
 {
@@ -1531,7 +1533,8 @@ __device__ __forceinline__ void pl_load_iterate(float* stage, const PlSolve<kN>&
     const CUtensorMap* m = g.map[j.p];
     const int par = j.k & 1;
     tma_load_3d(stage, m + (par ? kPmO1 : kPmO0), j.ox, j.oy, j.c, bar);
-    tma_load_3d(stage + G::kStage, m + (par ? kPmU1 : kPmU0), j.ox, j.oy, j.c, bar);
+    if (j.k > 0)  // (there is no U before the first round)
+        tma_load_3d(stage + G::kStage, m + (par ? kPmU1 : kPmU0), j.ox, j.oy, j.c, bar);
 }
 
 // A job waits for round k - 1 of the tile's 3x3 neighbourhood and, where the
@@ -1707,7 +1710,7 @@ __global__ void __launch_bounds__(32 * (PlGeo<kCfg>::kWarps + 4), 1)
                     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
                     ++phases;
                     if (t.valid) {
-                        mbar_expect_tx(full_in, G::kPlanes * G::kStageBytes);
+                        mbar_expect_tx(full_in, (G::kPlanes - (j.k == 0 ? 1 : 0)) * G::kStageBytes);
                         if (ready)
                             pl_load_iterate<kCfg>(stage, g, j, full_in);
                         pl_load_constants<kCfg>(stage, g, j, full_in);
@@ -1749,7 +1752,8 @@ __global__ void __launch_bounds__(32 * (PlGeo<kCfg>::kWarps + 4), 1)
                 const CUtensorMap* m = g.map[t.p];
                 const int par = (t.k + 1) & 1;
                 tma_store_3d(m + (par ? kPmOo1 : kPmOo0), t.ox + G::kT, t.oy + G::kT, t.c, so);
-                tma_store_3d(m + (par ? kPmUo1 : kPmUo0), t.ox + G::kT, t.oy + G::kT, t.c, su);
+                if (t.k0 + t.T < g.num_iter)  // (nor is U read after the last)
+                    tma_store_3d(m + (par ? kPmUo1 : kPmUo0), t.ox + G::kT, t.oy + G::kT, t.c, su);
                 bulk_commit();
                 // publish: the release store orders the completed async-proxy writes,
                 // brought into the generic proxy by the proxy fence, before the counter
@@ -2286,17 +2290,21 @@ int pl_rounds_cfg(int sms, int w, int h, int num_iter, int form, size_t ws_float
 // The exact form on interleaved images, a launch a round, where one wave of its
 // 64 x 32 tiles is the image (75 steps: 320x180 71 us against 75 in planes,
 // 240x135 70 against 86), one of the 64 x 48 tiles for two rounds at most
-// (600x338, 16 steps: 28 us against 32), or where a few steps of a large image do not
-// pay for the planes' conversions (us, interleaved and in planes: 1280x720 1 step 31
-// and 37, 3 steps 37 and 40, 4 steps 41 and 41; 1600x900 3 steps 58 and 59, 4
-// steps 64 and 61; 1920x1080 1 step 61 and 81, 5 steps 77 and 89, 7 steps 93 and
-// 95, 8 steps 106 and 99; 3840x2160 2 steps 209 and 300, 7 steps 326 and 324; 960x540
-// 1 step 24 and 22).
+// (600x338, 16 steps: 28 us against 32), or where a few steps do not pay for the
+// planes' conversions: of a large image, and where the eight images of a solve
+// stay in L2 (100 of its 129 MB) and eleven do not (us, interleaved and in planes:
+// 1120x630 1 step 27 and 24; 1280x720 1 step 29 and 32, 3 steps 35 and 37, 4 steps 39
+// and 38; 1440x810 1 step 47 and 42; 1600x900 1 step 57 and 53; 1760x990 3 steps 59
+// and 67, 5 steps 70 and 72, 6 steps 77 and 75; 1920x1080 1 step 62 and 75, 6 steps 85
+// and 89, 7 steps 93 and 94, 8 steps 107 and 98; 3840x2160 2 steps 210 and 288, 6
+// steps 298 and 309, 7 steps 326 and 320).
 bool exact_interleaved(int sms, int w, int h, int num_iter)
 {
     const int tall = tiles_of(w, h, kPIH);
-    return tiles_of(w, h, kIH) <= sms || (num_iter <= 2 * kTbT && tall <= sms) || (num_iter <= 3 && tall > 4 * sms) ||
-           (num_iter < kTbT && tall > 8 * sms);
+    const int64_t image = int64_t{12} * w * h, l2 = 100 << 20;  // bytes
+    return tiles_of(w, h, kIH) <= sms || (num_iter <= 2 * kTbT && tall <= sms) ||
+           (num_iter <= 3 && 8 * image <= l2 && 11 * image > l2) ||
+           (num_iter <= 6 && tall > 7 * sms);
 }
 
 struct PlanarCopy {
