@@ -345,6 +345,32 @@ def test_consist_out_few_steps_of_a_large_image(vsc, oracle, cuda, w, h, iters):
     vsc.check_device()
 
 
+@pytest.mark.parametrize("w,h", [(128, 72), (640, 360), (960, 540)])
+def test_step_solves_levels_as_the_solver_does(vsc, oracle, cuda, w, h):
+    """A step's exact solves of small levels run a launch a round on interleaved
+    images, as vsc_get_consist_out's do: both levels of 128x72, the coarse one of
+    640x360, none of 960x540; the bytes equal the restatement's."""
+    fr = _frames(w, h, 3, seed=w)
+    launches = {}
+    for form in ("fma", "exact"):  # (the FMA form runs every level on planes)
+        st = vsc.Stabilizer(w, h, solver_form=form)
+        for f in fr:
+            st.load_frame(*f)
+        out = st.step().cpu().numpy()
+        launches[form] = st.last_launches
+        st.close()
+    plans = [vsc.solver_plan(w >> j, h >> j, 150 // (j + 1)) for j in range(2)]
+    assert [p.planes for p in plans] == {128: [0, 0], 640: [1, 0], 960: [1, 1]}[w]
+    # a launch a round (and at most two more, for the start) in place of the planes' three
+    more = [(p.rounds - 2, p.rounds) for p in plans if not p.planes]
+    assert sum(m[0] for m in more) <= launches["exact"] - launches["fma"] <= sum(m[1] for m in more)
+    of = [oracle.rgba_to_float(o) for o, _ in fr]
+    pf = [oracle.rgba_to_float(p) for _, p in fr]
+    ff, fb = oracle.flow_estimate(of[1], of[2]), oracle.flow_estimate(of[2], of[1])
+    _, ref = oracle.stab_pass(of, pf, ff, fb, pf[2])
+    assert np.array_equal(out, ref)
+
+
 def test_consist_out_fma_single_tile_shape(vsc, cuda):
     """The FMA form has one tile shape (128 x 72 of a plane); the autotuner
     reports it without measuring."""

@@ -1329,10 +1329,11 @@ cudaError_t enqueue_step(vsc_stabilizer* s, const vsc_hyper_params& hp, uint8_t*
         uint8_t* rgba = j == 0 ? rgba_dev : nullptr;
         // The solution is initialised with the processed frame and carried down
         // with the same bilinear chain, so at the coarsest level it equals P;
-        // the solve's setup reads it from there, or upsamples the coarser
-        // solution.
+        // a solve in planes reads it from there in its setup, or upsamples the
+        // coarser solution.
         const bool coarsest = j == L - 1;
-        if (iters > 0 && solver_tma_supported()) {
+        if (iters > 0 && solver_tma_supported() &&
+            !solver_step_interleaved(s->solver_form, A[j], W[j], O[j], s->lw[j], s->lh[j], iters, s->solver_ws)) {
             run(run_solver_planes(s->solver_form, P[j], A[j], W[j], coarsest ? P[j] : nullptr, O[j], s->lw[j], s->lh[j],
                 coarsest ? nullptr : O[j + 1], coarsest ? 0 : s->lw[j + 1], coarsest ? 0 : s->lh[j + 1], iters,
                 hp.step_size, hp.mom_fac, s->solver_ws, ws_floats, st, &nl, rgba));

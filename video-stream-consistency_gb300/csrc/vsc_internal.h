@@ -179,6 +179,12 @@ void solver_set_autotune(bool on);
 cudaError_t run_solver(const float* P, const float* A, const float* Wt, float* O, int w, int h, int num_iter,
     float step, float mom, float* workspace, size_t ws_floats, cudaStream_t st, int* launches,
     uint8_t* rgba_out = nullptr, int form = kSolverExact);
+// Whether run_solver solves a level of a step on interleaved images.  The step
+// follows it there, although planes save it the launch that writes the start:
+// exact frames of 150 steps in us, interleaved and in planes: 128x72 303 and 331,
+// 256x144 315 and 357, 320x180 323 and 326, 416x240 338 and 362, 96x64 293 and 283.
+bool solver_step_interleaved(int form, const float* A, const float* Wt, const float* O, int w, int h, int num_iter,
+    float* workspace);
 // run_solver in a workspace of solver_workspace_full_floats, started from the
 // image Oi or, with Oi null, from the cw x ch solution Oc upsampled to w x h with
 // kernel_bilinear's expression (the pyramid's next level), the upsampling fused

@@ -2478,6 +2478,14 @@ cudaError_t solver_prep(int form, const float* P, const float* A, const float* W
     return e != cudaSuccess ? e : cudaGetLastError();
 }
 
+bool solver_step_interleaved(int form, const float* A, const float* Wt, const float* O, int w, int h, int num_iter,
+    float* workspace)
+{
+    DeviceInfo* di = nullptr;
+    return form == kSolverExact && device_info(&di) == cudaSuccess &&
+           tma_eligible(di, w, O, ws_view(workspace, w, h), A, Wt) && exact_interleaved(di->sms, w, h, num_iter);
+}
+
 cudaError_t solver_plan(int w, int h, int num_iter, int form, size_t ws_floats, int sms, SolverPlan* out)
 {
     if (sms <= 0) {
