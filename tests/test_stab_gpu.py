@@ -878,6 +878,22 @@ def test_multistream_grouped_few_iterations(vsc, cuda, num_iter):
     assert grouped
 
 
+@pytest.mark.parametrize("sizes,num_iter,more", [
+    ([(96, 64), (128, 72), (80, 48)], 60, (8 - 3) + (4 - 3)),   # 14 and 6 tiles at most: both levels interleaved
+    ([(320, 184)] * 3, 45, 3 - 3),                              # 252 tiles: on planes; 72 at the half size
+    ([(64 + 8 * (i % 5), 40) for i in range(18)], 24, 2 * ((3 - 3) + (2 - 3)))])  # groups of 16 and 2
+def test_multistream_small_exact_groups_run_interleaved(vsc, cuda, sizes, num_iter, more):
+    """Groups of one wave of the interleaved kernels' tiles run a launch a round
+    there, others on planes (three launches a level and group, as the FMA form
+    always has); the outputs equal the stabilizers' either way."""
+    n = {}
+    for form in ("exact", "fma"):
+        n[form], grouped = _multistream_vs_singles(vsc, sizes, [(1, "f32")] * len(sizes), True, num_iter, steps=3,
+                                                   solver_form=form)
+        assert grouped
+    assert n["exact"] - n["fma"] == more
+
+
 def test_multistream_ungroupable_size_runs_ungrouped(vsc, cuda):
     """A level width that is not a multiple of 4 (70 -> 35) keeps the step
     ungrouped, with the same results."""

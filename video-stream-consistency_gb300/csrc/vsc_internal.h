@@ -195,20 +195,28 @@ cudaError_t run_solver_planes(int form, const float* P, const float* A, const fl
 
 // Grouped solve: n images of any sizes, the same iterations, each launch of
 // the solve kernel walking the tiles of all of them (up to 16 images per
-// launch).  Per image, before run_solver_group on the same stream:
-// solver_prep(form, ...) into its workspace, and the initial solution in O.
+// launch); on interleaved images, a launch a round, where solver_group_interleaved
+// says so.  Per image, before run_solver_group on the same stream:
+// solver_prep(form, ...) into its workspace, and the initial solution in
+// solver_group_start.
 struct SolverImage {
+    const float *A, *Wt;
     float* O;
     int w, h;
     float* workspace;  // solver_workspace_full_floats(w, h, form)
     uint8_t* rgba;     // RGBA8 copy of the result, or null
 };
 bool solver_tma_supported();  // the solve kernel runs on the current device
+// Exact images of one wave of 64 x 32 tiles in all (of each launch), as run_solver
+// keeps them: three videos of 96x64 318 us a step, 385 on planes; eight 355 and
+// 414; three of 320x180, 252 tiles, 494 and 447.
+bool solver_group_interleaved(const int* w, const int* h, int n, int form);
+float* solver_group_start(float* O, float* workspace, int w, int h, int num_iter, bool interleaved);
 // a form's per-solve constants, into the workspace
 cudaError_t solver_prep(int form, const float* P, const float* A, const float* Wt, int w, int h, float step,
-    float* workspace, cudaStream_t st);
+    float* workspace, bool interleaved, cudaStream_t st);
 cudaError_t run_solver_group(const SolverImage* im, int n, int num_iter, float step, float mom, cudaStream_t st,
-    int* launches, int form = kSolverExact);
+    int* launches, int form, bool interleaved);
 
 // Device-side bounded waits record a timeout in a device flag instead of
 // hanging; this reads and clears it for the current device.

@@ -386,23 +386,37 @@ __device__ __forceinline__ void store_interior(const CUtensorMap* mOo, const CUt
 // (O, U; interior box).
 enum { kMapO, kMapU, kMapA, kMapW, kMapL, kMapOo, kMapUo, kMaps };
 
-// One launch of a persistent kernel on interleaved images: the tensor maps, the
-// size and the tiles.  Passed by value as a __grid_constant__ parameter, so the
+constexpr int kGroupMax = 16;  // images of a grouped solve's launch
+
+// One launch of a persistent kernel on interleaved images, kN of any sizes (one
+// per video of a grouped solve): each one's tensor maps, size and first tile in
+// the launch's list.  Passed by value as a __grid_constant__ parameter, so the
 // maps stay in parameter memory, where TMA reads them.
+template <int kN>
 struct SolverLaunch {
-    CUtensorMap map[kMaps];
-    int w, h, tiles_x, tiles;
-    uint8_t* rgba;  // RGBA8 output of the last launch, or null
+    CUtensorMap map[kN][kMaps];
+    int w[kN], h[kN], tiles_x[kN];
+    int tile0[kN + 1];  // first tile of image p; tile0[count] = tiles in all
+    uint8_t* rgba[kN];  // RGBA8 output of the last launch, or null
+    int count;
 };
 
 struct TileLoc {
+    int p;       // image
     int ox, oy;  // tile origin (ring included)
 };
 
-template <int kRows>
-__device__ __forceinline__ TileLoc locate(const SolverLaunch& g, int tile)
+template <int kRows, int kN>
+__device__ __forceinline__ TileLoc locate(const SolverLaunch<kN>& g, int tile)
 {
-    return TileLoc{(tile % g.tiles_x) * kIW - kTbT, (tile / g.tiles_x) * kRows - kTbT};
+    int p = 0;
+    if (kN > 1) {
+#pragma unroll 1
+        while (p + 1 < g.count && tile >= g.tile0[p + 1])
+            ++p;
+    }
+    const int t = tile - g.tile0[p];
+    return TileLoc{p, (t % g.tiles_x[p]) * kIW - kTbT, (t / g.tiles_x[p]) * kRows - kTbT};
 }
 
 // input tiles first .. last - 1 (map order) of a tile at (ox, oy), into consecutive stages
@@ -440,8 +454,9 @@ __device__ __forceinline__ void issue_first_loads(float* stage, const CUtensorMa
         issue_loads(stage, m, ox, oy, stage_floats, bytes, bar);
 }
 
+template <int kN>
 __global__ void __launch_bounds__(kTbEX / 2 * kTbEY / 2, 1)
-    solver_persistent_kernel(const __grid_constant__ SolverLaunch g, int T, int k0, float step, float mom)
+    solver_persistent_kernel(const __grid_constant__ SolverLaunch<kN> g, int T, int k0, float step, float mom)
 {
     extern __shared__ __align__(128) unsigned char smem_raw[];
     float* stage = reinterpret_cast<float*>(smem_raw);
@@ -456,11 +471,11 @@ __global__ void __launch_bounds__(kTbEX / 2 * kTbEY / 2, 1)
     if (tid == 0)
         mbar_init(bar, 1);
     __syncthreads();
-    const int ntiles = g.tiles;
+    const int ntiles = g.tile0[g.count];
     int tile = blockIdx.x;
     if (tid == 0 && tile < ntiles) {
         const TileLoc n = locate<kIH>(g, tile);
-        issue_first_loads(stage, g.map, n.ox, n.oy, kStageFloats, kStageBytes, bar, k0 > 0);
+        issue_first_loads(stage, g.map[n.p], n.ox, n.oy, kStageFloats, kStageBytes, bar, k0 > 0);
     }
     grid_dependency_wait();
     uint32_t parity = 0;
@@ -468,7 +483,7 @@ __global__ void __launch_bounds__(kTbEX / 2 * kTbEY / 2, 1)
         if (tile + static_cast<int>(gridDim.x) >= ntiles)
             allow_dependent_launch();
         const TileLoc c = locate<kIH>(g, tile);
-        const int ox = c.ox, oy = c.oy, w = g.w, h = g.h;
+        const int ox = c.ox, oy = c.oy, w = g.w[c.p], h = g.h[c.p];
         if (!mbar_wait_bounded(bar, parity, kWaitSpins)) {
             // the outputs are invalid and vsc_check_device reports VSC_ETIMEOUT; the
             // second bounded wait gives copies still in flight a chance to land
@@ -531,7 +546,7 @@ __global__ void __launch_bounds__(kTbEX / 2 * kTbEY / 2, 1)
         if (tid == 0 && tile + static_cast<int>(gridDim.x) < ntiles) {
             asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
             const TileLoc n = locate<kIH>(g, tile + gridDim.x);
-            issue_loads(stage, g.map, n.ox, n.oy, kStageFloats, kStageBytes, bar);
+            issue_loads(stage, g.map[n.p], n.ox, n.oy, kStageFloats, kStageBytes, bar);
         }
 
         const bool interior = ox >= 1 && oy >= 1 && ox + kTbEX - 1 <= w - 3 && oy + kTbEY - 1 <= h - 3;
@@ -568,8 +583,8 @@ __global__ void __launch_bounds__(kTbEX / 2 * kTbEY / 2, 1)
         asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
         __syncthreads();
         if (tid == 0)
-            store_interior(g.map + kMapOo, g.map + kMapUo, ox, oy, so, su);
-        if (uint8_t* rgba = g.rgba) {
+            store_interior(g.map[c.p] + kMapOo, g.map[c.p] + kMapUo, ox, oy, so, su);
+        if (uint8_t* rgba = g.rgba[c.p]) {
 #pragma unroll
             for (int q = 0; q < 4; ++q) {
                 const int px = px0 + (q & 1), py = py0 + (q >> 1);
@@ -701,7 +716,7 @@ __device__ __forceinline__ void p8_iterate(P8State& s, float* obuf, int T, int k
 }
 
 __global__ void __launch_bounds__(kPThreads, 1)
-    solver_tall_kernel(const __grid_constant__ SolverLaunch g, int T, int k0, float step, float mom)
+    solver_tall_kernel(const __grid_constant__ SolverLaunch<1> g, int T, int k0, float step, float mom)
 {
     extern __shared__ __align__(128) unsigned char smem_raw[];
     float* stage = reinterpret_cast<float*>(smem_raw);
@@ -715,11 +730,11 @@ __global__ void __launch_bounds__(kPThreads, 1)
     if (threadIdx.x == 0)
         mbar_init(bar, 1);
     __syncthreads();
-    const int ntiles = g.tiles;
+    const int ntiles = g.tile0[g.count];
     int tile = blockIdx.x;
     if (threadIdx.x == 0 && tile < ntiles) {
         const TileLoc n = locate<kPIH>(g, tile);
-        issue_first_loads(stage, g.map, n.ox, n.oy, kPStageFloats, kPStageBytes, bar, k0 > 0);
+        issue_first_loads(stage, g.map[n.p], n.ox, n.oy, kPStageFloats, kPStageBytes, bar, k0 > 0);
     }
     grid_dependency_wait();
     uint32_t parity = 0;
@@ -727,7 +742,7 @@ __global__ void __launch_bounds__(kPThreads, 1)
         if (tile + static_cast<int>(gridDim.x) >= ntiles)
             allow_dependent_launch();
         const TileLoc c = locate<kPIH>(g, tile);
-        const int ox = c.ox, oy = c.oy, w = g.w, h = g.h;
+        const int ox = c.ox, oy = c.oy, w = g.w[c.p], h = g.h[c.p];
         if (!mbar_wait_bounded(bar, parity, kWaitSpins)) {
             // the outputs are invalid and vsc_check_device reports VSC_ETIMEOUT; the
             // second bounded wait gives copies still in flight a chance to land
@@ -775,7 +790,7 @@ __global__ void __launch_bounds__(kPThreads, 1)
         if (threadIdx.x == 0 && tile + static_cast<int>(gridDim.x) < ntiles) {
             asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
             const TileLoc n = locate<kPIH>(g, tile + gridDim.x);
-            issue_loads(stage, g.map, n.ox, n.oy, kPStageFloats, kPStageBytes, bar);
+            issue_loads(stage, g.map[n.p], n.ox, n.oy, kPStageFloats, kPStageBytes, bar);
         }
 
         const int gx0 = ox + px0, gy0 = oy + py0;
@@ -814,8 +829,8 @@ __global__ void __launch_bounds__(kPThreads, 1)
         asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
         __syncthreads();
         if (threadIdx.x == 0)
-            store_interior(g.map + kMapOo, g.map + kMapUo, ox, oy, so, su);
-        if (uint8_t* rgba = g.rgba) {
+            store_interior(g.map[c.p] + kMapOo, g.map[c.p] + kMapUo, ox, oy, so, su);
+        if (uint8_t* rgba = g.rgba[c.p]) {
 #pragma unroll
             for (int q = 0; q < 8; ++q) {
                 const int px = px0 + (q & 1), py = py0 + (q >> 1);
@@ -857,7 +872,6 @@ __global__ void __launch_bounds__(kPThreads, 1)
 // shuffles per row for four pixels, and each warp publishes its top and
 // bottom row as two 16-byte stores per thread.
 
-constexpr int kGroupMax = 16;             // images of a grouped solve's launch
 constexpr int kPlW = 128;                 // tile width (a warp: 32 lanes x 4 columns)
 
 // How a solve in planes runs: its form (bit 0) and whether its rounds are 16
@@ -1861,7 +1875,8 @@ bool set_group_smem()
 {
     constexpr auto kAttr = cudaFuncAttributeMaxDynamicSharedMemorySize;
     return cudaFuncSetAttribute(solver_solve_kernel<kSolverFma, kN>, kAttr, PlGeo<kSolverFma>::kSmem) == cudaSuccess &&
-           cudaFuncSetAttribute(solver_solve_kernel<kSolverExact, kN>, kAttr, PlGeo<kSolverExact>::kSmem) == cudaSuccess;
+           cudaFuncSetAttribute(solver_solve_kernel<kSolverExact, kN>, kAttr, PlGeo<kSolverExact>::kSmem) == cudaSuccess &&
+           cudaFuncSetAttribute(solver_persistent_kernel<kN>, kAttr, kPsSmem) == cudaSuccess;
 }
 
 struct DeviceInfo {
@@ -1899,7 +1914,6 @@ cudaError_t device_info(DeviceInfo** out)
                     single(std::integral_constant<int, kSolverFma | kPlMid>{}) &&
                     single(std::integral_constant<int, kSolverExact | kPlLong>{}) &&
                     single(std::integral_constant<int, kSolverExact | kPlMid>{}) &&
-                    cudaFuncSetAttribute(solver_persistent_kernel, kAttr, kPsSmem) == cudaSuccess &&
                     cudaFuncSetAttribute(solver_tall_kernel, kAttr, kPSmem) == cudaSuccess &&
                     set_group_smem<1>() && set_group_smem<4>() && set_group_smem<kGroupMax>() &&
                     cudaFuncSetAttribute(solver_fma_plain_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
@@ -1990,11 +2004,24 @@ bool encode_plane_map(CUtensorMap* m, const float* base, int w, int h, int pitch
                CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
 
-// Steps k_first .. num_iter - 1 of a solve in launches of T <= kTbT steps of a
-// persistent kernel (`rows`-row tiles) with programmatic dependent launch.
-// Launch li reads O[c0 ^ (li & 1)] and U[li & 1] and writes the others.
-cudaError_t launch_rounds(const SolveMaps& m, int w, int h, int c0, uint8_t* rgba, int rows, int num_iter, float step,
-    float mom, int sms, cudaStream_t st, int* nl, int k_first = 0)
+// rounds of a solve
+int solve_launches(int num_iter, int steps = kTbT) { return num_iter > 0 ? (num_iter - 1) / steps + 1 : 0; }
+
+// One image of a solve in rounds on interleaved images; c0: the buffer of O that the
+// first round reads.
+struct RoundsImage {
+    SolveMaps maps;
+    int w, h, c0;
+    uint8_t* rgba;
+};
+
+// Steps k_first .. num_iter - 1 of a solve of n images in launches of T <= kTbT
+// steps of a persistent kernel (`rows`-row tiles; the tall one takes one image)
+// with programmatic dependent launch, kN images a launch.  Round li reads O[c0 ^
+// (li & 1)] and U[li & 1] and writes the others.
+template <int kN>
+cudaError_t launch_rounds(const RoundsImage* im, int n, int rows, int num_iter, float step, float mom, int sms,
+    cudaStream_t st, int* nl, int k_first = 0)
 {
     cudaLaunchConfig_t cfg = {};
     cudaLaunchAttribute attr[1];
@@ -2003,35 +2030,45 @@ cudaError_t launch_rounds(const SolveMaps& m, int w, int h, int c0, uint8_t* rgb
     cfg.stream = st;
     cfg.attrs = attr;
     cfg.numAttrs = 1;
-    SolverLaunch g{};
-    g.map[kMapA] = m.A;
-    g.map[kMapW] = m.W;
-    g.map[kMapL] = m.L;
-    g.w = w;
-    g.h = h;
-    g.tiles_x = (w + kIW - 1) / kIW;
-    g.tiles = tiles_of(w, h, interior_rows(rows));
-    cfg.gridDim = dim3(std::min(g.tiles, sms));
-    const int nlaunch = (num_iter - k_first + kTbT - 1) / kTbT;
+    const int nlaunch = solve_launches(num_iter - k_first);
     cudaError_t e = cudaSuccess;
+    SolverLaunch<kN> g{};
     int k0 = k_first;
     for (int li = 0; li < nlaunch && e == cudaSuccess; ++li) {
-        const int T = std::min(kTbT, num_iter - k0), c = c0 ^ (li & 1);
-        g.map[kMapO] = m.O[c];
-        g.map[kMapU] = m.U[li & 1];
-        g.map[kMapOo] = m.Oo[c ^ 1];
-        g.map[kMapUo] = m.Uo[(li + 1) & 1];
-        g.rgba = li == nlaunch - 1 ? rgba : nullptr;
-        if (rows == kPEY) {
-            cfg.blockDim = dim3(kPThreads);
-            cfg.dynamicSmemBytes = kPSmem;
-            e = cudaLaunchKernelEx(&cfg, solver_tall_kernel, g, T, k0, step, mom);
-        } else {
-            cfg.blockDim = dim3(32, kTbEY / 2);
-            cfg.dynamicSmemBytes = kPsSmem;
-            e = cudaLaunchKernelEx(&cfg, solver_persistent_kernel, g, T, k0, step, mom);
+        const int T = std::min(kTbT, num_iter - k0);
+        for (int b0 = 0; b0 < n && e == cudaSuccess; b0 += kN) {  // (a round of one group in the tail of another's)
+            g.count = std::min(n - b0, kN);
+            for (int p = 0; p < g.count; ++p) {
+                const RoundsImage& m = im[b0 + p];
+                const int c = m.c0 ^ (li & 1);
+                g.map[p][kMapO] = m.maps.O[c];
+                g.map[p][kMapU] = m.maps.U[li & 1];
+                g.map[p][kMapA] = m.maps.A;
+                g.map[p][kMapW] = m.maps.W;
+                g.map[p][kMapL] = m.maps.L;
+                g.map[p][kMapOo] = m.maps.Oo[c ^ 1];
+                g.map[p][kMapUo] = m.maps.Uo[(li + 1) & 1];
+                g.w[p] = m.w;
+                g.h[p] = m.h;
+                g.tiles_x[p] = (m.w + kIW - 1) / kIW;
+                g.tile0[p + 1] = g.tile0[p] + tiles_of(m.w, m.h, interior_rows(rows));
+                g.rgba[p] = li == nlaunch - 1 ? m.rgba : nullptr;
+            }
+            cfg.gridDim = dim3(std::min(g.tile0[g.count], sms));
+            if constexpr (kN == 1) {
+                if (rows == kPEY) {
+                    cfg.blockDim = dim3(kPThreads);
+                    cfg.dynamicSmemBytes = kPSmem;
+                    e = cudaLaunchKernelEx(&cfg, solver_tall_kernel, g, T, k0, step, mom);
+                }
+            }
+            if (rows != kPEY) {
+                cfg.blockDim = dim3(32, kTbEY / 2);
+                cfg.dynamicSmemBytes = kPsSmem;
+                e = cudaLaunchKernelEx(&cfg, solver_persistent_kernel<kN>, g, T, k0, step, mom);
+            }
+            ++*nl;
         }
-        ++*nl;
         k0 += T;
     }
     return e;
@@ -2104,7 +2141,8 @@ cudaError_t solver_autotune(int w, int h, cudaStream_t st, int* rows_out, int fo
             e = cudaErrorInvalidValue;
     }
     auto launch = [&](int s, int num_iter, int* nl) {
-        return launch_rounds(maps[s], w, h, 0, nullptr, shapes[s], num_iter, 0.15f, 0.15f, di->sms, st, nl, kTbT);
+        const RoundsImage im{maps[s], w, h, 0, nullptr};
+        return launch_rounds<1>(&im, 1, shapes[s], num_iter, 0.15f, 0.15f, di->sms, st, nl, kTbT);
     };
     for (int round = 0; round < 5 && e == cudaSuccess; ++round) {
         for (int s = 0; s < 2 && e == cudaSuccess; ++s) {
@@ -2187,9 +2225,6 @@ size_t solver_workspace_any_floats(int w, int h)
 int solver_steps_per_launch() { return kTbT; }
 
 namespace {
-
-// rounds of a solve
-int solve_launches(int num_iter, int steps = kTbT) { return num_iter > 0 ? (num_iter - 1) / steps + 1 : 0; }
 
 // Rounds of one launch of the solve kernel at `tiles` tiles a round.  A launch
 // counts its tickets, tiles x rounds, in 32 bits, and nothing bounds a caller's
@@ -2470,9 +2505,37 @@ bool solver_tma_supported()
     return device_info(&di) == cudaSuccess && di->ps_smem;
 }
 
-cudaError_t solver_prep(int form, const float* P, const float* A, const float* Wt, int w, int h, float step,
-    float* workspace, cudaStream_t st)
+bool solver_group_interleaved(const int* w, const int* h, int n, int form)
 {
+    DeviceInfo* di = nullptr;
+    if (form != kSolverExact || device_info(&di) != cudaSuccess || !di->ps_smem)
+        return false;
+    for (int b0 = 0; b0 < n; b0 += kGroupMax) {
+        int64_t tiles = 0;
+        for (int i = b0; i < std::min(n, b0 + kGroupMax); ++i) {
+            if (w[i] % 4 != 0)
+                return false;
+            tiles += tiles_of(w[i], h[i], kIH);
+        }
+        if (tiles > di->sms)
+            return false;
+    }
+    return true;
+}
+
+float* solver_group_start(float* O, float* workspace, int w, int h, int num_iter, bool interleaved)
+{
+    return interleaved && solve_launches(num_iter) % 2 == 1 ? ws_view(workspace, w, h).O2 : O;
+}
+
+cudaError_t solver_prep(int form, const float* P, const float* A, const float* Wt, int w, int h, float step,
+    float* workspace, bool interleaved, cudaStream_t st)
+{
+    if (interleaved) {
+        const dim3 b(32, 8);
+        const cudaError_t e = launch_pdl(lap_pr_kernel, grid2d(w, h, b), b, 0, st, P, ws_view(workspace, w, h).L, w, h);
+        return e != cudaSuccess ? e : cudaGetLastError();
+    }
     const PlWs v = pl_view(workspace, w, h, pl_pitch(w), form);
     const cudaError_t e = launch_prep(form, P, A, Wt, nullptr, v, nullptr, w, h, step, nullptr, 0, nullptr, 0, 0, st);
     return e != cudaSuccess ? e : cudaGetLastError();
@@ -2515,7 +2578,7 @@ cudaError_t solver_plan(int w, int h, int num_iter, int form, size_t ws_floats, 
 }
 
 cudaError_t run_solver_group(const SolverImage* im, int n, int num_iter, float step, float mom, cudaStream_t st,
-    int* launches, int form)
+    int* launches, int form, bool interleaved)
 {
     DeviceInfo* di = nullptr;
     cudaError_t e = device_info(&di);
@@ -2533,6 +2596,26 @@ cudaError_t run_solver_group(const SolverImage* im, int n, int num_iter, float s
         if (launches)
             *launches += nl;
         return e;
+    }
+    if (interleaved) {
+        std::vector<RoundsImage> ri(n);
+        for (int i = 0; i < n; ++i) {
+            const WsView v = ws_view(im[i].workspace, im[i].w, im[i].h);
+            float* const O[2] = {im[i].O, v.O2};
+            float* const U[2] = {v.U0, v.U1};
+            if (!tma_eligible(di, im[i].w, im[i].O, v, im[i].A, im[i].Wt) ||
+                !encode_solve(&ri[i].maps, O, U, im[i].A, im[i].Wt, v.L, im[i].w, im[i].h, kTbEY))
+                return cudaErrorInvalidValue;
+            ri[i].w = im[i].w;
+            ri[i].h = im[i].h;
+            ri[i].c0 = solve_launches(num_iter) % 2;
+            ri[i].rgba = im[i].rgba;
+        }
+        e = n <= 4 ? launch_rounds<4>(ri.data(), n, kTbEY, num_iter, step, mom, di->sms, st, &nl)
+                   : launch_rounds<kGroupMax>(ri.data(), n, kTbEY, num_iter, step, mom, di->sms, st, &nl);
+        if (launches)
+            *launches += nl;
+        return e != cudaSuccess ? e : cudaGetLastError();
     }
     // O into planes (counters zeroed), one solve launch per 16 images, O back
     std::vector<int> ws(n), hs(n);
@@ -2641,7 +2724,8 @@ cudaError_t run_solver(const float* P, const float* A, const float* Wt, float* O
         tma = encode_solve(&m, Ob, Ub, A, Wt, v.L, w, h, rows);
     }
     if (tma) {
-        cudaError_t e = launch_rounds(m, w, h, cur == O ? 0 : 1, rgba_out, rows, num_iter, step, mom, di->sms, st, &nl);
+        const RoundsImage im{m, w, h, cur == O ? 0 : 1, rgba_out};
+        cudaError_t e = launch_rounds<1>(&im, 1, rows, num_iter, step, mom, di->sms, st, &nl);
         if (launches)
             *launches += nl;
         return e != cudaSuccess ? e : cudaGetLastError();
