@@ -371,6 +371,23 @@ def test_step_solves_levels_as_the_solver_does(vsc, oracle, cuda, w, h):
     assert np.array_equal(out, ref)
 
 
+@pytest.mark.parametrize("w,h", [(1, 1), (1, 70), (113, 57), (115, 73), (225, 120), (853, 60), (338, 128)])
+@pytest.mark.parametrize("iters", [1, 8, 9, 17])
+def test_consist_out_fma_plain_loads(vsc, oracle, cuda, w, h, iters):
+    """In the documented workspace a width that is not a multiple of 4 runs with
+    plain loads, a launch a round: one round, which reads and writes no U, two with
+    a short last one, three; the workspace starts as NaN."""
+    import torch
+
+    P, A, Wt, O0 = _img(h, w), _img(h, w), _img(h, w, hi=2.0), _img(h, w)
+    ws = torch.full((vsc.consist_out_workspace_size(w, h, "fma") // 4,), float("nan"), device=cuda)
+    assert vsc.solver_plan(w, h, iters, "fma", ws.numel() * 4).rounds_per_launch == 1
+    O = _t(O0, cuda)
+    vsc.get_consist_out(_t(P, cuda), _t(A, cuda), _t(Wt, cuda), iters, 0.15, 0.15, O, form="fma", workspace=ws)
+    ref = oracle.consist_out(P, A, Wt, iters, 0.15, 0.15, O0, form="fma")
+    assert np.array_equal(O.cpu().numpy().view(np.uint32), ref.view(np.uint32))
+
+
 def test_consist_out_fma_single_tile_shape(vsc, cuda):
     """The FMA form has one tile shape (128 x 72 of a plane); the autotuner
     reports it without measuring."""

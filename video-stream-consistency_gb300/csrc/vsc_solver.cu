@@ -1339,12 +1339,16 @@ __device__ __forceinline__ void tma_store_3d(const CUtensorMap* map, int x, int 
 // are not a multiple of 4, or planes off the 16-byte grid).
 struct PlPlain {
     const float *O, *U, *K, *C;
-    float *Oo, *Uo;
+    float *Oo, *Uo;  // (Uo: null in the last round)
     int w, h, tiles_x, ntiles;
 };
 
-// Stage <- tile (c, ox, oy) of the four planes, zero outside the image.
-__device__ __forceinline__ void pl_plain_load(float* stage, const PlPlain& p, int c, int ox, int oy)
+// Stage <- tile (c, ox, oy) of the four planes, zero outside the image; U (not read
+// in a solve's first round) from round 1 on.  Copied asynchronously, 4 bytes at a
+// time: through registers, four elements ahead, the eight warps had too few loads
+// in flight (854x480, 75 steps 296 us, twelve ahead 271, and 239 so; twelve warps
+// of the kernel before, four ahead, 280).
+__device__ __forceinline__ void pl_plain_load(float* stage, const PlPlain& p, int c, int ox, int oy, bool with_u)
 {
     using G = PlGeo<kSolverFma>;
     const float* src[4] = {p.O, p.U, p.K, p.C};
@@ -1357,8 +1361,12 @@ __device__ __forceinline__ void pl_plain_load(float* stage, const PlPlain& p, in
         const int64_t idx = in ? base + pix_index(gx, gy, p.w) : 0;
 #pragma unroll
         for (int a = 0; a < 4; ++a)
-            stage[a * G::kStage + i] = in ? src[a][idx] : 0.0f;
+            if (a != 1 || with_u)
+                asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;" ::"r"(smem_u32(stage + a * G::kStage + i)),
+                    "l"(src[a] + idx), "r"(in ? 4 : 0)
+                    : "memory");
     }
+    asm volatile("cp.async.wait_all;" ::: "memory");
 }
 
 // The plain-load form (widths that are not a multiple of 4 in a caller's
@@ -1387,7 +1395,7 @@ __global__ void __launch_bounds__(32 * PlGeo<kSolverFma>::kWarps, 1)
         const int ox = (r % pl.tiles_x) * G::kIW - G::kT, oy = (r / pl.tiles_x) * G::kIRows - G::kT;
         const int w = pl.w, h = pl.h;
         __syncthreads();  // the previous tile has left the staging
-        pl_plain_load(stage, pl, c, ox, oy);
+        pl_plain_load(stage, pl, c, ox, oy, k0 > 0);
         __syncthreads();
         PlState<kSolverFma> s;
         float4 up, dn;
@@ -1398,13 +1406,15 @@ __global__ void __launch_bounds__(32 * PlGeo<kSolverFma>::kWarps, 1)
         pl_put<kSolverFma>(s, so, su, lane, warp);
         __syncthreads();
         const int64_t base = static_cast<int64_t>(c) * w * h;
-        for (int i = threadIdx.x; i < G::kOut; i += blockDim.x) {
+#pragma unroll 4
+        for (int i = threadIdx.x; i < G::kOut; i += 32 * G::kWarps) {
             const int iy = i / G::kIW, ix = i - iy * G::kIW;
             const int gy = oy + G::kT + iy, gx = ox + G::kT + ix;
             if (gx < w && gy < h) {
                 const int64_t idx = base + pix_index(gx, gy, w);
                 pl.Oo[idx] = so[i];
-                pl.Uo[idx] = su[i];
+                if (pl.Uo)
+                    pl.Uo[idx] = su[i];
             }
         }
     }
@@ -2483,7 +2493,8 @@ cudaError_t run_solver_planes(const DeviceInfo* di, int form, const float* P, co
         int k0 = 0;
         for (int li = 0; li < nlaunch && e == cudaSuccess; ++li) {
             const int T = std::min(kTbT, num_iter - k0);
-            const PlPlain pl{v.O[li & 1], v.U[li & 1], v.K, v.C, v.O[(li + 1) & 1], v.U[(li + 1) & 1], w, h, tx, nt};
+            const PlPlain pl{v.O[li & 1], v.U[li & 1], v.K, v.C, v.O[(li + 1) & 1],
+                li + 1 < nlaunch ? v.U[(li + 1) & 1] : nullptr, w, h, tx, nt};
             e = launch_pdl(solver_fma_plain_kernel, dim3(std::min(nt, di->sms)), dim3(32 * PlGeo<kSolverFma>::kWarps),
                 PlGeo<kSolverFma>::kSmem, st, pl, T, k0, step, mom);
             ++*nl;
