@@ -388,6 +388,33 @@ def test_consist_out_fma_plain_loads(vsc, oracle, cuda, w, h, iters):
     assert np.array_equal(O.cpu().numpy().view(np.uint32), ref.view(np.uint32))
 
 
+# (form, steps of a round at 152 SMs, w, h, iterations): both kinds of width, rows
+# left for the last row of tiles from one (which then reads two rows of tiles up, in
+# rounds of 12 and 16) to nearly a whole one, short and odd last rounds
+@pytest.mark.parametrize("form,steps,w,h,iters", [
+    ("exact", 16, 97, 65, 37), ("exact", 16, 241, 135, 75), ("exact", 16, 481, 257, 37), ("exact", 16, 480, 270, 75),
+    ("exact", 16, 640, 328, 75), ("exact", 16, 640, 340, 75), ("exact", 12, 113, 97, 20), ("exact", 12, 400, 289, 20),
+    ("exact", 12, 99, 81, 20), ("exact", 12, 241, 135, 20), ("exact", 12, 640, 360, 75), ("exact", 8, 640, 337, 20),
+    ("exact", 8, 723, 385, 20), ("exact", 8, 960, 540, 9), ("exact", 8, 961, 541, 37),
+    ("fma", 16, 240, 121, 37), ("fma", 16, 193, 161, 75), ("fma", 16, 641, 361, 37), ("fma", 16, 241, 135, 37),
+    ("fma", 16, 400, 289, 75), ("fma", 16, 640, 340, 37), ("fma", 12, 113, 97, 20), ("fma", 12, 400, 289, 9),
+    ("fma", 12, 801, 449, 75), ("fma", 12, 193, 161, 20), ("fma", 8, 640, 337, 20), ("fma", 8, 720, 404, 37),
+    ("fma", 8, 961, 541, 75)])
+def test_consist_out_every_round_length(vsc, oracle, cuda, form, steps, w, h, iters):
+    assert vsc.solver_plan(w, h, iters, form, sms=152).steps == steps
+    p = vsc.solver_plan(w, h, iters, form)
+    assert p.planes and p.steps in (8, 12, 16)
+    P, A, Wt, O0 = _img(h, w), _img(h, w), _img(h, w, hi=2.0), _img(h, w)
+    Wt[Wt < 0.3] = 0.0
+    O = _t(O0, cuda)
+    vsc.get_consist_out(_t(P, cuda), _t(A, cuda), _t(Wt, cuda), iters, 0.15, 0.15, O, form=form)
+    got = O.cpu().numpy()
+    ref = oracle.consist_out(P, A, Wt, iters, 0.15, 0.15, O0, form=form)
+    assert _equal_up_to_zero_sign(got, ref) if form == "exact" else np.array_equal(
+        got.view(np.uint32), ref.view(np.uint32))
+    vsc.check_device()
+
+
 def test_consist_out_fma_single_tile_shape(vsc, cuda):
     """The FMA form has one tile shape (128 x 72 of a plane); the autotuner
     reports it without measuring."""

@@ -24,7 +24,7 @@ INCLUDE = PKG.parent / "include"
 
 SOURCES = ["vsc_ops.cu", "vsc_stab.cu", "vsc_solver.cu", "vsc_flow.cu", "vsc_corr_tc.cu", "vsc_upsampler.cu",
            "vsc_upsampler_tc.cu", "vsc_api.cpp", "vsc_files.cpp", "vsc_jpeg.cpp"]
-HEADERS = ["vsc_internal.h", "vsc_device.h", "vsc_math.cuh", "vsc_ptx.cuh"]
+HEADERS = ["vsc_internal.h", "vsc_device.h", "vsc_solver_geo.h", "vsc_math.cuh", "vsc_ptx.cuh"]
 
 ARCH = ["-gencode", "arch=compute_103a,code=sm_103a"]
 COMMON = ["-O3", "-std=c++17", "-lineinfo", "-fmad=false", "-Xcompiler", "-fPIC", "-Xcompiler",

@@ -11,6 +11,7 @@
 #include <stdint.h>
 
 #include "../../include/vsc.h"
+#include "vsc_solver_geo.h"
 
 namespace vsc {
 
@@ -149,7 +150,6 @@ cudaError_t launch_bilinear_group(const Img* in, const Img* out, int n, cudaStre
 // round on interleaved images, and the FMA form, where its width is not a
 // multiple of 4, one with plain loads; at other widths the FMA form's smaller
 // workspace holds the planes and counters for rounds of 8 steps, perhaps of 12.
-enum SolverForm { kSolverExact = 0, kSolverFma = 1 };
 size_t solver_workspace_floats(int w, int h, int form = kSolverExact);
 size_t solver_workspace_full_floats(int w, int h, int form);
 size_t solver_workspace_any_floats(int w, int h);  // the larger form's

@@ -74,12 +74,8 @@ __global__ void lap_pr_kernel(const float* __restrict__ P, float* __restrict__ L
 // shuffle (one warp spans the full tile width).  Tiles away from the image
 // border skip the reference's neighbour-validity selects.  The result equals
 // the one-iteration-per-launch Jacobi bit for bit.
-#ifndef VSC_SOLVER_T
-#define VSC_SOLVER_T 8
-#endif
 constexpr int kTbEX = 64;
 constexpr int kTbEY = 32;
-constexpr int kTbT = VSC_SOLVER_T;             // iterations per launch
 constexpr int kTbPX = kTbEX + 4;               // shared row pitch (2-column apron each side)
 constexpr int kTbPlane = kTbPX * (kTbEY + 2);  // one colour plane with a 1-row apron
 constexpr int kTbSmem = 2 * 3 * kTbPlane * static_cast<int>(sizeof(float));
@@ -872,61 +868,6 @@ __global__ void __launch_bounds__(kPThreads, 1)
 // shuffles per row for four pixels, and each warp publishes its top and
 // bottom row as two 16-byte stores per thread.
 
-constexpr int kPlW = 128;                 // tile width (a warp: 32 lanes x 4 columns)
-
-// How a solve in planes runs: its form (bit 0) and whether its rounds are 16
-// steps with a 16-pixel ring (bit 1) or 12 with 12 (bit 2) instead of 8.
-constexpr int kPlLong = 2, kPlMid = 4;
-
-// A form's tile: kPlanes input planes, kWarps warps of kRPT rows each, and the
-// registers of the compute and the control warps.
-template <int kForm>
-struct PlG;
-template <>
-struct PlG<kSolverFma> {  // O, U, nK, Cs
-    static constexpr int kPlanes = 4, kWarps = 8, kRPT = 9;
-    static constexpr int kComputeRegs = 216, kControlRegs = 72;
-};
-// The exact form's step needs three constants of a pixel, consWt, lap P and A:
-// 160 registers of state for 4 x 8 blocks, a tile of 128 x 64 (interior 112 x
-// 48, 66 %).
-template <>
-struct PlG<kSolverExact> {  // O, U, consWt, lap P, A
-    static constexpr int kPlanes = 5, kWarps = 8, kRPT = 8;
-    static constexpr int kComputeRegs = 224, kControlRegs = 56;
-};
-
-constexpr int pl_steps(int cfg) { return cfg & kPlLong ? 2 * kTbT : cfg & kPlMid ? 3 * kTbT / 2 : kTbT; }
-
-template <int kCfg>
-struct PlGeo : PlG<kCfg & 1> {
-    using B = PlG<kCfg & 1>;
-    using B::kPlanes;
-    using B::kRPT;
-    using B::kWarps;
-    static constexpr bool kFma = (kCfg & 1) == kSolverFma;
-    static constexpr int kT = pl_steps(kCfg);            // steps a round, the ring's width: 8, 12, 16
-    static constexpr int kIW = kPlW - 2 * kT;            // interior columns: 112, 104, 96
-    static constexpr int kRows = kRPT * kWarps;          // 72 (FMA), 64 (exact)
-    static constexpr int kIRows = kRows - 2 * kT;        // interior rows: 56, 48, 40 (FMA), 48, 40, 32 (exact)
-    static constexpr int kStage = kRows * kPlW;          // floats of one input tile
-    static constexpr int kStageBytes = kStage * static_cast<int>(sizeof(float));
-    static constexpr int kSlots = (kWarps + 2) * 2 * kPlW;  // edge-row slots of one buffer
-    static constexpr int kOut = kIRows * kIW;            // floats of one interior tile
-    static constexpr int kSmem =
-        kPlanes * kStageBytes + (2 * kSlots + 2 * kOut) * static_cast<int>(sizeof(float)) + 128;
-    static_assert(kSmem <= 232448, "dynamic shared memory per CTA");
-    static_assert((kPlanes * kStageBytes) % 128 == 0 && (2 * kSlots * 4) % 128 == 0 && (kOut * 4) % 128 == 0,
-        "TMA sources and destinations on the 128-byte grid");
-    static_assert(kT <= kIW && kT <= kIRows, "a tile reads only its 3 x 3 neighbours' interiors");
-    static_assert((kIW * 4) % 16 == 0 && (kT * 4) % 16 == 0, "TMA x coordinates must be 16-byte aligned");
-    // rows of the tile that the frame's rows 0 (tiles at oy = -kT) and h - 2, h - 1
-    // (tiles that end on the frame's last row) sit in, as warp and row
-    static constexpr int kTopWarp = kT / kRPT, kTopRow = kT % kRPT;
-    static constexpr int kBot2Warp = (kRows - kT - 2) / kRPT, kBot2Row = (kRows - kT - 2) % kRPT;
-    static constexpr int kBot1Warp = (kRows - kT - 1) / kRPT, kBot1Row = (kRows - kT - 1) % kRPT;
-};
-
 // Cs = step * fma(wt, A, -lap P) and nK = -(step * (cnt + wt)) as planes
 // (lap P, cnt as lap_pr_kernel computes them); with O non-null, also O as
 // planes into Op, or with Oc non-null the cw x ch image Oc upsampled to w x h
@@ -1053,39 +994,6 @@ struct PlState {
 __device__ __forceinline__ float& f4(float4& v, int j) { return j == 0 ? v.x : j == 1 ? v.y : j == 2 ? v.z : v.w; }
 __device__ __forceinline__ float f4c(const float4& v, int j) { return j == 0 ? v.x : j == 1 ? v.y : j == 2 ? v.z : v.w; }
 
-// Neighbour tests of the planar step.  kernel_consist_out reads a neighbour as
-// +0 unless it lies in [0, w - 2] x [0, h - 2] (left: gx - 1 >= 0, right:
-// gx + 1 < w - 1, up: gy - 1 >= 0, down: gy + 1 < h - 1), so the only pixels of
-// the frame with a neighbour read as +0 are column 0 (left), columns w - 2 and
-// w - 1 (right), row 0 (up) and rows h - 2 and h - 1 (down); every other read
-// of a pixel inside the frame is of a pixel inside the frame.  Pixels outside
-// the frame (the ring of a border tile) are computed too, but no pixel inside
-// the frame reads them unmasked, so their values never reach the output.
-//   kPlAll:   an interior tile, no test.
-//   kPlLanes: a border tile of a frame whose width, like the tile origins, is
-//             a multiple of 4: column 0 is then column j = 0 of the thread
-//             with gx0 = 0 and columns w - 2, w - 1 are j = 2, 3 of the thread
-//             with gx0 = w - 4 (three selects a row); row 0 of a tile at
-//             oy = -8 and rows h - 2, h - 1 of a tile at oy = h - 64 are fixed
-//             rows of fixed warps (kTopRow ..: a select of a row's up or down
-//             neighbours in every warp, true only in that one).  A tile
-//             holding row 0, h - 2 or h - 1 elsewhere (frames of few rows)
-//             takes kPlEvery.
-//   kPlCols:  the same for any other width: columns w - 2 and w - 1 may be any
-//             column of a thread (five selects a row).
-//   kPlEvery: rows 0, h - 2 and h - 1 anywhere, too (a select of every row's up
-//             and down neighbours).
-enum { kPlAll, kPlLanes, kPlCols, kPlEvery };
-
-// What a step needs to know of its thread's place.  zl / zr: it holds column 0 /
-// columns w - 4 .. w - 1; zt / zb2 / zb1 (kPlLanes, kPlCols): its row kTopRow /
-// kBot2Row / kBot1Row is the frame's row 0 / h - 2 / h - 1.
-struct PlPlace {
-    int xlim;      // its first column that is column w - 2 or beyond
-    int top, bot;  // kPlEvery: its row that is row 0, its first one that is row h - 2 or beyond
-    bool zl, zr, zt, zb2, zb1;
-};
-
 // The columns left and right of a thread's block, from the neighbouring lanes
 // (the outer lanes keep their own value: the tile's outer columns never reach
 // the interior).
@@ -1171,21 +1079,6 @@ __device__ __forceinline__ void pl_step(PlState<kCfg>& s, PlSides<kCfg>& x, floa
         s.o[r] = on[r];
 }
 
-// The planar step's test mode for a tile at (ox, oy) of a w x h frame.
-template <int kCfg>
-__device__ __forceinline__ int pl_mode(int ox, int oy, int w, int h)
-{
-    using G = PlGeo<kCfg>;
-    constexpr int kRows = G::kRows;
-    if (ox >= 1 && oy >= 1 && ox + kPlW - 1 <= w - 3 && oy + kRows - 1 <= h - 3)
-        return kPlAll;
-    const bool row0 = oy <= 0 && oy + kRows - 1 >= 0;
-    const bool last2 = oy <= h - 1 && oy + kRows - 1 >= h - 2;
-    if ((!row0 || oy == -G::kT) && (!last2 || oy == h - kRows + G::kT))  // ox is a multiple of 4
-        return (w & 3) == 0 ? kPlLanes : kPlCols;
-    return kPlEvery;
-}
-
 // The steps of one tile's round.  After each step a warp publishes its top and
 // bottom row to a slot buffer (slot w + 1 is warp w's; even steps write buffer
 // 0 and odd ones buffer 1) and bar() joins the warps; `up` and `dn` are the
@@ -1242,24 +1135,6 @@ __device__ __forceinline__ void pl_round(int mode, PlState<kCfg>& s, float4 up, 
         pl_steps<kCfg, kPlEvery>(s, up, dn, slots, T, k0, step, mom, lane, warp, t, bar);
 }
 
-// A thread's place in a tile at (ox, oy).
-template <int kCfg>
-__device__ __forceinline__ PlPlace pl_place(int ox, int oy, int w, int h, int lane, int warp)
-{
-    using G = PlGeo<kCfg>;
-    const int gx0 = ox + 4 * lane, gy0 = oy + G::kRPT * warp;
-    PlPlace t;
-    t.xlim = w - 2 - gx0;
-    t.top = -gy0;
-    t.bot = h - 2 - gy0;
-    t.zl = gx0 == 0;
-    t.zr = gx0 == w - 4;
-    t.zt = oy == -G::kT && warp == G::kTopWarp;
-    t.zb2 = oy == h - G::kRows + G::kT && warp == G::kBot2Warp;
-    t.zb1 = oy == h - G::kRows + G::kT && warp == G::kBot1Warp;
-    return t;
-}
-
 // A thread's block out of the staged tile, with the O rows above and below it
 // (zero outside the tile: values the ring never passes on to the interior).
 template <int kCfg>
@@ -1305,17 +1180,6 @@ __device__ __forceinline__ void pl_put(const PlState<kCfg>& s, float* so, float*
         *reinterpret_cast<float4*>(so + iy * G::kIW + ix) = s.o[r];
         *reinterpret_cast<float4*>(su + iy * G::kIW + ix) = s.u[r];
     }
-}
-
-template <int kCfg>
-int pl_tiles_x(int w)
-{
-    return (w + PlGeo<kCfg>::kIW - 1) / PlGeo<kCfg>::kIW;
-}
-template <int kCfg>
-int pl_tiles(int w, int h)
-{
-    return 3 * pl_tiles_x<kCfg>(w) * ((h + PlGeo<kCfg>::kIRows - 1) / PlGeo<kCfg>::kIRows);
 }
 
 __device__ __forceinline__ void tma_load_3d(void* dst, const CUtensorMap* map, int x, int y, int z, uint64_t* bar)
@@ -1473,18 +1337,11 @@ struct PlSolve {
 };
 
 struct PlJob {
-    int k;                   // round
-    int p, c, tx, ty, local;  // problem, plane, tile position, tile index within the problem
-    int ox, oy, w, h;
+    int k;                    // round
+    int p, local, per_plane;  // problem, tile index within it, its tiles of a plane
+    int w, h;
+    PlTileAt t;
 };
-
-// The moved bottom row of tiles reads two rows of tiles up.
-template <int kCfg>
-__device__ __forceinline__ bool pl_deep(int h, int ty_n)
-{
-    using G = PlGeo<kCfg>;
-    return G::kT > kTbT && ty_n >= 3 && h - (ty_n - 1) * G::kIRows < G::kT;
-}
 
 template <int kCfg, int kN>
 __device__ __forceinline__ PlJob pl_job(const PlSolve<kN>& g, int ticket)
@@ -1510,27 +1367,10 @@ __device__ __forceinline__ PlJob pl_job(const PlSolve<kN>& g, int ticket)
     }
     j.p = p;
     j.local = tile - g.tile0[p];
-    const int per_plane = (g.tile0[p + 1] - g.tile0[p]) / 3;
-    j.c = j.local / per_plane;
-    const int r = j.local - j.c * per_plane;
-    j.tx = r % g.tiles_x[p];
-    j.ty = r / g.tiles_x[p];
-    j.ox = j.tx * G::kIW - G::kT;
-    j.oy = j.ty * G::kIRows - G::kT;
     j.w = g.w[p];
     j.h = g.h[p];
-    // The bottom row of tiles is moved up until its interior ends on the
-    // frame's last row (rows h - 2 and h - 1 then sit in fixed rows of fixed
-    // warps, where pl_row tests them without per-row tests), when its top ring
-    // still lies in the row of tiles above (the 3 x 3 dependency holds) or, in
-    // longer rounds, whose 16-pixel ring reaches further than 40 % of the frames'
-    // last rows of tiles (12 pixels: 27 %), in the two rows above (pl_watched looks two rows up and
-    // down there).  Its interior then overlaps those rows': both compute the
-    // shared rows from the same inputs with the same arithmetic and store the
-    // same bits.
-    const int ty_n = per_plane / g.tiles_x[p];
-    if (j.ty == ty_n - 1 && j.ty > 0 && (j.h - j.ty * G::kIRows >= G::kT || pl_deep<kCfg>(j.h, ty_n)))
-        j.oy = j.h - G::kRows + G::kT;
+    j.per_plane = (g.tile0[p + 1] - g.tile0[p]) / 3;
+    j.t = pl_tile<kCfg>(j.h, g.tiles_x[p], j.per_plane, j.local);
     return j;
 }
 
@@ -1541,10 +1381,10 @@ __device__ __forceinline__ void pl_load_constants(float* stage, const PlSolve<kN
 {
     using G = PlGeo<kCfg>;
     const CUtensorMap* m = g.map[j.p];
-    tma_load_3d(stage + 2 * G::kStage, m + kPmK, j.ox, j.oy, j.c, bar);
-    tma_load_3d(stage + 3 * G::kStage, m + kPmC, j.ox, j.oy, j.c, bar);
+    tma_load_3d(stage + 2 * G::kStage, m + kPmK, j.t.ox, j.t.oy, j.t.c, bar);
+    tma_load_3d(stage + 3 * G::kStage, m + kPmC, j.t.ox, j.t.oy, j.t.c, bar);
     if (!G::kFma)
-        tma_load_3d(stage + 4 * G::kStage, m + kPmA, j.ox, j.oy, j.c, bar);
+        tma_load_3d(stage + 4 * G::kStage, m + kPmA, j.t.ox, j.t.oy, j.t.c, bar);
 }
 
 // The first round has no U to load, and the last one's U is not stored: 3840x2160,
@@ -1556,28 +1396,20 @@ __device__ __forceinline__ void pl_load_iterate(float* stage, const PlSolve<kN>&
     asm volatile("fence.proxy.async.global;" ::: "memory");  // the acquired stores, before the async-proxy reads
     const CUtensorMap* m = g.map[j.p];
     const int par = j.k & 1;
-    tma_load_3d(stage, m + (par ? kPmO1 : kPmO0), j.ox, j.oy, j.c, bar);
+    tma_load_3d(stage, m + (par ? kPmO1 : kPmO0), j.t.ox, j.t.oy, j.t.c, bar);
     if (j.k > 0)  // (there is no U before the first round)
-        tma_load_3d(stage + G::kStage, m + (par ? kPmU1 : kPmU0), j.ox, j.oy, j.c, bar);
+        tma_load_3d(stage + G::kStage, m + (par ? kPmU1 : kPmU0), j.t.ox, j.t.oy, j.t.c, bar);
 }
 
-// A job waits for round k - 1 of the tile's 3x3 neighbourhood and, where the
-// bottom row of tiles reads two rows up, of the tiles it reads there, whose
-// writers wait for it in turn.  Lanes 0..8, 9..11 of the loading warp each
-// watch one counter (null: none to watch).
+// Lane i of the loading warp watches the counter of the job's watched tile i (null:
+// none to watch).
 template <int kCfg, int kN>
 __device__ __forceinline__ const unsigned* pl_watched(const PlSolve<kN>& g, const PlJob& j, int lane)
 {
-    if (j.k == 0 || lane >= (PlGeo<kCfg>::kT > kTbT ? 12 : 9))
+    if (j.k == 0)
         return nullptr;
-    const int tx_n = g.tiles_x[j.p];
-    const int per_plane = (g.tile0[j.p + 1] - g.tile0[j.p]) / 3;
-    const int ty_n = per_plane / tx_n;
-    const int x = j.tx + lane % 3 - 1;
-    int y = j.ty + lane / 3 - 1;
-    if (lane >= 9)
-        y = !pl_deep<kCfg>(j.h, ty_n) ? -1 : j.ty == ty_n - 1 ? ty_n - 3 : j.ty == ty_n - 3 ? ty_n - 1 : -1;
-    return x >= 0 && x < tx_n && y >= 0 && y < ty_n ? g.done[j.p] + j.c * per_plane + y * tx_n + x : nullptr;
+    const int tile = pl_watched_tile<kCfg>(j.h, g.tiles_x[j.p], j.t, lane);
+    return tile >= 0 ? g.done[j.p] + j.t.c * j.per_plane + tile : nullptr;
 }
 
 // One look by the whole warp, an L2 round trip: the acquiring loads and the
@@ -1717,16 +1549,16 @@ __global__ void __launch_bounds__(32 * (PlGeo<kCfg>::kWarps + 4), 1)
                         pl_wait(empty_in, (i - 1) & 1, &s_abort);
                     PlTile t{};
                     if (valid) {
-                        t.ox = j.ox;
-                        t.oy = j.oy;
+                        t.ox = j.t.ox;
+                        t.oy = j.t.oy;
                         t.w = j.w;
                         t.h = j.h;
                         t.k0 = j.k * G::kT;
                         t.T = min(G::kT, g.num_iter - t.k0);
-                        t.mode = pl_mode<kCfg>(j.ox, j.oy, j.w, j.h);
+                        t.mode = pl_mode<kCfg>(j.t.ox, j.t.oy, j.w, j.h);
                         t.k = j.k;
                         t.p = j.p;
-                        t.c = j.c;
+                        t.c = j.t.c;
                         t.local = j.local;
                         t.valid = !s_abort;
                     }
@@ -2320,7 +2152,7 @@ int pl_rounds_cfg(int sms, int w, int h, int num_iter, int form, size_t ws_float
         if (c.cfg != 0 && !pl_fits(w, h, ws_floats, form | c.cfg))
             continue;
         const float tiles = static_cast<float>(pl_tiles_of(w, h, form | c.cfg)) / static_cast<float>(sms);
-        const float us = static_cast<float>(solve_launches(num_iter, pl_steps(c.cfg))) *
+        const float us = static_cast<float>(solve_launches(num_iter, pl_round_steps(c.cfg))) *
                          std::max(c.least, c.base + c.tile * tiles);
         if (c.cfg == 0) {
             limit = 0.9f * us;
@@ -2473,7 +2305,7 @@ cudaError_t run_solver_planes(const DeviceInfo* di, int form, const float* P, co
     const PlWs v = pl_view(workspace, w, h, tma ? pl_pitch(w) : w, cfg);
     cudaError_t e = launch_prep(form, P, A, Wt, Oi, v, v.O[0], w, h, step, v.cnt, v.ncnt, Oc, cw, ch, st);
     ++*nl;
-    const int nlaunch = solve_launches(num_iter, pl_steps(cfg));
+    const int nlaunch = solve_launches(num_iter, pl_round_steps(cfg));
     if (e == cudaSuccess && tma) {
         const std::vector<PlWs> one(1, v);
         auto solve = [&](auto c) {
@@ -2574,7 +2406,7 @@ cudaError_t solver_plan(int w, int h, int num_iter, int form, size_t ws_floats, 
     p.planes = form == kSolverFma || (!inter && pl_fits(w, h, ws_floats, form));
     const bool one_launch = p.planes && pl_fits(w, h, ws_floats, form);
     const int cfg = one_launch ? pl_rounds_cfg(sms, w, h, num_iter, form, ws_floats) : form;
-    p.steps = pl_steps(cfg);
+    p.steps = pl_round_steps(cfg);
     p.rounds = solve_launches(num_iter, p.steps);
     if (p.planes) {
         p.tiles = pl_tiles_of(w, h, cfg);
