@@ -86,6 +86,18 @@ def test_lowp_correlation_chunk_widths_and_row_blocks(vsc, oracle, cuda, shape, 
     vsc.check_device()
 
 
+@pytest.mark.parametrize("shape", [(2, 48, 150, 641), (1, 33, 300, 511), (3, 16, 257, 400)])
+def test_lowp_correlation_many_narrow_chunks(vsc, oracle, cuda, shape):
+    """Chunks of 16 channels of large maps: a block of the conversion walks several
+    items and more than one block of partial maxima a SM is reduced.  Small
+    integers with one largest value: exact, as in the test above."""
+    rng = np.random.Generator(np.random.PCG64(shape[1]))
+    f1, f2 = (rng.integers(-3, 4, shape).astype(np.float32) for _ in range(2))
+    f1[-1, -1, -1, -1] = 4.0  # (the last element decides the scale)
+    out = vsc.correlation_lowp(_t(f1, cuda), _t(f2, cuda), 1, "bf16").cpu().numpy()
+    assert np.array_equal(out, oracle.correlation(f1, f2, 1))
+
+
 @pytest.mark.parametrize("operand", [0, 1])
 def test_lowp_correlation_result_over_an_operand(vsc, oracle, cuda, operand):
     """The operands are converted before the result is written, so the result may

@@ -507,7 +507,9 @@ __device__ __forceinline__ uint32_t pack2(float a, float b)
 // further apart than they are long, which spreads them over the banks) and
 // written out whole, 16 bytes a thread side by side.  2 x 64 x 136 x 240 take 11.4 us,
 // and 13.4 when the reading threads stored their 32 bytes of every pixel
-// themselves; the loads of the first item do not wait for the scales.
+// themselves; the loads of the first item do not wait for the scales.  A thread of
+// the narrowest chunk has one 16-byte piece and stores it itself, the next item's
+// loads on their way, without barriers.
 template <bool kBf16, int kCw>
 __global__ void __launch_bounds__(256) to_chunked2_kernel(const float* __restrict__ f1, const float* __restrict__ f2,
     uint4* __restrict__ c1, uint4* __restrict__ c2, const float* __restrict__ part, int nparts,
@@ -517,7 +519,7 @@ __global__ void __launch_bounds__(256) to_chunked2_kernel(const float* __restric
     constexpr int kPx = kCw == 16 ? 128 : 64;      // pixels of an item
     constexpr int kCh = kCw * kPx / 256;           // channels a thread reads
     constexpr int kPitch = kPer + 1;
-    __shared__ uint4 tile[kPx * kPitch];
+    __shared__ uint4 tile[kCw == 16 ? 1 : kPx * kPitch];
     __shared__ float wm[8];
     pdl_enter();
     const unsigned HW = static_cast<unsigned>(H) * W;  // < 2^30
@@ -553,6 +555,22 @@ __global__ void __launch_bounds__(256) to_chunked2_kernel(const float* __restric
     }
     for (unsigned it = blockIdx.x;;) {
         const float sc = t ? s2 : s1;
+        if constexpr (kCw == 16) {
+            static_assert(kCw != 16 || kCh == 8, "a piece a thread");
+            const uint4 packed = make_uint4(pack2<kBf16>(v[0] * sc, v[1] * sc), pack2<kBf16>(v[2] * sc, v[3] * sc),
+                pack2<kBf16>(v[4] * sc, v[5] * sc), pack2<kBf16>(v[6] * sc, v[7] * sc));
+            const unsigned p = pb + px, y = p / W, x = p - y * W;
+            uint4* const dst = (t ? c2 : c1) + ((static_cast<int64_t>(n) * H + y) * nq + q) * W * kPer + x * kPer + part_of;
+            const bool in = p < HW;
+            it += gridDim.x;
+            if (it < items)
+                fetch(it);
+            if (in)
+                *dst = packed;
+            if (it >= items)
+                break;
+            continue;
+        }
 #pragma unroll
         for (int h = 0; h < kCh / 8; ++h)
             tile[px * kPitch + part_of * (kCh / 8) + h] =
@@ -846,7 +864,7 @@ cudaError_t launch_corr_tc(const float* f1, const float* f2, float* out, int N, 
                                               std::less_equal<const float*>()(out + outs, f); };
     const bool in_out = outs >= 64 && apart(f1) && apart(f2);
     float* part = in_out ? out : scales + 8;
-    const int64_t want = std::min<int64_t>((total / 4 + 1023) / 1024, 2 * sms);  // 4+ vectors a thread
+    const int64_t want = std::min<int64_t>((total / 4 + 1023) / 1024, 4 * sms);  // 4+ vectors a thread, every SM full
     const unsigned parts = static_cast<unsigned>(
         std::max<int64_t>(1, std::min<int64_t>(want, in_out ? outs / 2 : 28)));
     auto a16 = [](const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15) == 0; };
