@@ -47,6 +47,17 @@ def test_correlation_channel_batches_bit_exact(vsc, oracle, cuda, shape, md, leg
     assert np.array_equal(out, oracle.correlation(f1, f2, md, legacy=legacy))
 
 
+@pytest.mark.parametrize("legacy", [0, 1])
+@pytest.mark.parametrize("shape,md", [((1, 3, 34, 60), 32), ((2, 1, 45, 61), 10), ((1, 15, 34, 60), 9),
+                                      ((3, 16, 20, 31), 7), ((1, 2, 130, 129), 5)])
+def test_correlation_few_channels_many_displacements_bit_exact(vsc, oracle, cuda, shape, md, legacy):
+    """Few channels: a block takes up to 32 / C displacements, the last one fewer."""
+    f1 = RNG.standard_normal(shape).astype(np.float32)
+    f2 = RNG.standard_normal(shape).astype(np.float32)
+    out = vsc.correlation(_t(f1, cuda), _t(f2, cuda), md, legacy=legacy).cpu().numpy()
+    assert np.array_equal(out, oracle.correlation(f1, f2, md, legacy=legacy))
+
+
 @pytest.mark.parametrize("shape,md", [((1, 32, 24, 40), 4), ((2, 5, 7, 9), 4), ((1, 3, 6, 6), 2)])
 def test_correlation_legacy(vsc, oracle, cuda, shape, md):
     f1 = RNG.standard_normal(shape).astype(np.float32)

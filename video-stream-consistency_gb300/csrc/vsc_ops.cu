@@ -221,9 +221,11 @@ __global__ void __launch_bounds__(8 * kCorrTH * (2 * MD + 1))
 // Any max_displacement, and the small pyramid levels (where the tile kernel
 // would run on a handful of CTAs): one thread per output element, pixels in x,
 // displacements in y, batches in z; the channel sum in channel order; batch n
-// at base + n * stride.  A small level is bound by the latency of the channel
-// loop, so kCorrBatch channels' loads are issued before their sums: 196 x 17 x 30
-// (8 warps a SM) take 9.0 us, and 11.3 with the compiler's four.
+// at base + n * stride.  A block of few channels takes several displacements (3 x 34 x
+// 60, max_displacement 32: 69 us with 67,600 blocks of one, 46 with 6,800).  A
+// small level is bound by the latency of the channel loop, so kCorrBatch channels'
+// loads are issued before their sums: 196 x 17 x 30 (8 warps a SM) take 9.0 us, and
+// 11.3 with the compiler's four.
 constexpr int kCorrBatch = 16;
 
 // a read-only load that stays where it is written (the compiler sinks plain
@@ -235,6 +237,7 @@ __device__ __forceinline__ float load_ahead(const float* p)
     return v;
 }
 
+template <bool kMany>  // displacements a block: several, else one
 __global__ void __launch_bounds__(128) corr_generic_kernel(const float* __restrict__ in1,
     const float* __restrict__ in2, float* __restrict__ out, int N, int C, int H, int W, int md, int legacy, int64_t s1,
     int64_t s2, int64_t so)
@@ -242,37 +245,45 @@ __global__ void __launch_bounds__(128) corr_generic_kernel(const float* __restri
     pdl_enter();
     const int P = 2 * md + 1;
     const int64_t HW = static_cast<int64_t>(H) * W;
-    const int d = blockIdx.y, dy = d / P - md, dx = d - d / P * P - md;
-    for (int n = blockIdx.z; n < N; n += gridDim.z) {
-        for (int64_t pix = blockIdx.x * 128 + static_cast<int>(threadIdx.x); pix < HW;
-             pix += static_cast<int64_t>(gridDim.x) * 128) {
-            const int y = HW <= 0x7fffffff ? static_cast<int>(static_cast<unsigned>(pix) / static_cast<unsigned>(W))
-                                           : static_cast<int>(pix / W);
-            const int x = static_cast<int>(pix - static_cast<int64_t>(y) * W);
-            const int y2 = y + dy, x2 = x + dx;
-            float acc = 0.0f;
-            if (y2 >= 0 && y2 < H && x2 >= 0 && x2 < W) {
-                const float* a = in1 + n * s1 + pix;
-                const float* b = in2 + n * s2 + static_cast<int64_t>(y2) * W + x2;
-                int c = 0;
-                for (; c + kCorrBatch <= C; c += kCorrBatch) {
-                    float va[kCorrBatch], vb[kCorrBatch];
+    auto displacement = [&](int d) {
+        const int dy = d / P - md, dx = d - d / P * P - md;
+        for (int n = blockIdx.z; n < N; n += gridDim.z) {
+            for (int64_t pix = blockIdx.x * 128 + static_cast<int>(threadIdx.x); pix < HW;
+                 pix += static_cast<int64_t>(gridDim.x) * 128) {
+                const int y = HW <= 0x7fffffff ? static_cast<int>(static_cast<unsigned>(pix) / static_cast<unsigned>(W))
+                                               : static_cast<int>(pix / W);
+                const int x = static_cast<int>(pix - static_cast<int64_t>(y) * W);
+                const int y2 = y + dy, x2 = x + dx;
+                float acc = 0.0f;
+                if (y2 >= 0 && y2 < H && x2 >= 0 && x2 < W) {
+                    const float* a = in1 + n * s1 + pix;
+                    const float* b = in2 + n * s2 + static_cast<int64_t>(y2) * W + x2;
+                    int c = 0;
+                    for (; c + kCorrBatch <= C; c += kCorrBatch) {
+                        float va[kCorrBatch], vb[kCorrBatch];
 #pragma unroll
-                    for (int i = 0; i < kCorrBatch; ++i) {
-                        va[i] = load_ahead(a + (c + i) * HW);
-                        vb[i] = load_ahead(b + (c + i) * HW);
+                        for (int i = 0; i < kCorrBatch; ++i) {
+                            va[i] = load_ahead(a + (c + i) * HW);
+                            vb[i] = load_ahead(b + (c + i) * HW);
+                        }
+#pragma unroll
+                        for (int i = 0; i < kCorrBatch; ++i)
+                            acc = acc + va[i] * vb[i];
                     }
-#pragma unroll
-                    for (int i = 0; i < kCorrBatch; ++i)
-                        acc = acc + va[i] * vb[i];
+                    for (; c < C; ++c)
+                        acc = acc + __ldg(a + c * HW) * __ldg(b + c * HW);
                 }
-                for (; c < C; ++c)
-                    acc = acc + __ldg(a + c * HW) * __ldg(b + c * HW);
+                if (legacy)
+                    acc = __fdiv_rn(acc, static_cast<float>(C));
+                out[n * so + static_cast<int64_t>(d) * HW + pix] = acc;
             }
-            if (legacy)
-                acc = __fdiv_rn(acc, static_cast<float>(C));
-            out[n * so + static_cast<int64_t>(d) * HW + pix] = acc;
         }
+    };
+    if constexpr (kMany) {
+        for (int d = blockIdx.y; d < P * P; d += gridDim.y)
+            displacement(d);
+    } else {
+        displacement(blockIdx.y);
     }
 }
 
@@ -281,10 +292,13 @@ cudaError_t launch_corr_generic(const float* f1, const float* f2, float* out, in
 {
     const int P = 2 * md + 1;
     const int64_t blocks = (static_cast<int64_t>(H) * W + 127) / 128;
-    const dim3 grid(static_cast<unsigned>(std::min<int64_t>(blocks, 152 * 64)), P * P,
-        static_cast<unsigned>(std::min(N, 65535)));
-    const cudaError_t e =
-        launch_pdl(corr_generic_kernel, grid, dim3(128), 0, st, f1, f2, out, N, C, H, W, md, legacy, s1, s2, so);
+    // few channels: several displacements a block, as long as the blocks fill the SMs
+    // (16 of 128 threads each)
+    const int64_t per = std::max<int64_t>(1, std::min<int64_t>({32 / C, P * P, blocks * N * P * P / (152 * 16)}));
+    const dim3 grid(static_cast<unsigned>(std::min<int64_t>(blocks, 152 * 64)),
+        static_cast<unsigned>((P * P + per - 1) / per), static_cast<unsigned>(std::min(N, 65535)));
+    const cudaError_t e = launch_pdl(per > 1 ? corr_generic_kernel<true> : corr_generic_kernel<false>, grid, dim3(128), 0,
+        st, f1, f2, out, N, C, H, W, md, legacy, s1, s2, so);
     return e != cudaSuccess ? e : cudaGetLastError();
 }
 
