@@ -179,10 +179,8 @@ void solver_set_autotune(bool on);
 cudaError_t run_solver(const float* P, const float* A, const float* Wt, float* O, int w, int h, int num_iter,
     float step, float mom, float* workspace, size_t ws_floats, cudaStream_t st, int* launches,
     uint8_t* rgba_out = nullptr, int form = kSolverExact);
-// Whether run_solver solves a level of a step on interleaved images.  The step
-// follows it there, although planes save it the launch that writes the start:
-// exact frames of 150 steps in us, interleaved and in planes: 128x72 303 and 331,
-// 256x144 315 and 357, 320x180 323 and 326, 416x240 338 and 362, 96x64 293 and 283.
+// Whether a level of a step is better solved by run_solver on interleaved images, its
+// start written to O beforehand, than by run_solver_planes.
 bool solver_step_interleaved(int form, const float* A, const float* Wt, const float* O, int w, int h, int num_iter,
     float* workspace);
 // run_solver in a workspace of solver_workspace_full_floats, started from the

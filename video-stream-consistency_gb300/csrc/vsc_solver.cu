@@ -2184,6 +2184,20 @@ bool exact_interleaved(int sms, int w, int h, int num_iter)
            (num_iter <= 6 && tall > 7 * sms);
 }
 
+// The same for a level of a step, where planes save a launch (the start is
+// upsampled in the setup) and, with fewer blocks, leave room for other streams'
+// steps: more than two rounds of one wave's frames stay on planes unless a row of
+// their tiles in rounds of 16 steps takes the per-row tests, which cost a round a
+// quarter.  Exact frames of 150 steps, us a frame of one video and of three at a
+// time, interleaved and in planes: 320x180 321, 327; 144, 128; 400x224 337, 359;
+// 188, 170; with row tests 128x72 301, 335; 104, 115; 256x144 313, 357; 122, 127;
+// 416x240 336, 363; 198, 199.
+bool step_interleaved(int sms, int w, int h, int num_iter)
+{
+    return exact_interleaved(sms, w, h, num_iter) &&
+           (num_iter <= 2 * kTbT || tiles_of(w, h, kIH) > sms || pl_row_tests<kSolverExact | kPlLong>(w, h));
+}
+
 struct PlanarCopy {
     const float* src;
     float* dst;
@@ -2388,8 +2402,10 @@ bool solver_step_interleaved(int form, const float* A, const float* Wt, const fl
     float* workspace)
 {
     DeviceInfo* di = nullptr;
-    return form == kSolverExact && device_info(&di) == cudaSuccess &&
-           tma_eligible(di, w, O, ws_view(workspace, w, h), A, Wt) && exact_interleaved(di->sms, w, h, num_iter);
+    if (form != kSolverExact || device_info(&di) != cudaSuccess ||
+        !tma_eligible(di, w, O, ws_view(workspace, w, h), A, Wt))
+        return false;
+    return step_interleaved(di->sms, w, h, num_iter);
 }
 
 cudaError_t solver_plan(int w, int h, int num_iter, int form, size_t ws_floats, int sms, SolverPlan* out)

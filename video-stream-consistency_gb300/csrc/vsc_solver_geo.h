@@ -190,6 +190,19 @@ VSC_HD int pl_mode(int ox, int oy, int w, int h)
     return kPlEvery;
 }
 
+// Whether some row of tiles of a solve takes kPlEvery.
+template <int kCfg>
+VSC_HD bool pl_row_tests(int w, int h)
+{
+    const int tx_n = pl_tiles_x<kCfg>(w), per_plane = pl_tiles<kCfg>(w, h) / 3;
+    for (int first = 0; first < per_plane; first += tx_n) {
+        const PlTileAt t = pl_tile<kCfg>(h, tx_n, per_plane, first);
+        if (pl_mode<kCfg>(t.ox, t.oy, w, h) == kPlEvery)
+            return true;
+    }
+    return false;
+}
+
 // A thread's place in a tile at (ox, oy).
 template <int kCfg>
 VSC_HD PlPlace pl_place(int ox, int oy, int w, int h, int lane, int warp)
