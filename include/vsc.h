@@ -77,7 +77,8 @@ VSC_API int32_t vsc_solver_steps_per_launch(void);
  * depends on how the tiles fill the GPU's waves.  vsc_solver_autotune times
  * both at width x height on scratch images and keeps the faster for the
  * current device (it synchronises the stream and is refused while the stream
- * is being captured); vsc_stabilizer_create tunes its pyramid's sizes.
+ * is being captured); vsc_stabilizer_create tunes those sizes of its pyramid
+ * that are one wave of tiles, whose steps may run on these kernels.
  * vsc_solver_tile_rows returns the tile rows (32 or 48) a solve at that size
  * uses, with *tuned = 1 when they were measured (else the wave model's
  * choice).  vsc_solver_set_autotune(0) forgets the measurements and stops
@@ -452,9 +453,9 @@ VSC_API int32_t vsc_stabilizer_last_launches(vsc_stabilizer* s);
 VSC_API vsc_status vsc_stabilizer_set_occlusion_mask(vsc_stabilizer* s, int32_t on);
 
 /* The solver form of every following step: VSC_SOLVER_EXACT (the default,
- * the reference's arithmetic) or VSC_SOLVER_FMA (see there).  Tunes the
- * form's tile shape for the pyramid's sizes on the stabilizer's stream
- * (synchronising it) unless the stream is being captured.  No counterpart
+ * the reference's arithmetic) or VSC_SOLVER_FMA (see there).  A change to
+ * VSC_SOLVER_EXACT tunes as vsc_stabilizer_create does (what is measured already is
+ * kept).  No counterpart
  * in the reference. */
 VSC_API vsc_status vsc_stabilizer_set_solver_form(vsc_stabilizer* s, int32_t form);
 

@@ -1073,6 +1073,14 @@ def test_solver_autotune(vsc, oracle, cuda):
     st.close()
 
 
+def test_stabilizer_tunes_only_what_its_steps_run(vsc, cuda):
+    """Levels of more than one wave of the interleaved kernels' tiles are solved on
+    planes: their shape is not measured at creation."""
+    st = vsc.Stabilizer(1296, 728)
+    assert [vsc.solver_tile_rows(1296 >> j, 728 >> j)[1] for j in range(3)] == [False, False, True]
+    st.close()
+
+
 def test_flow_estimate_equals_restatement(vsc, oracle, cuda):
     w, h = 112, 80
     fr = _frames(w, h, 2, seed=61)

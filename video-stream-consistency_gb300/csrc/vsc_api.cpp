@@ -981,14 +981,16 @@ vsc_status alloc_all(vsc_stabilizer* s)
     return check_cuda(e, "stabilizer allocation");
 }
 
-// The solver's tile shape of a form for the pyramid's sizes (a stream being
-// captured keeps the wave model; a failed measurement too).
+// The tile shape of the interleaved kernels for the pyramid's sizes of one wave, whose
+// steps may run on them (a stream being captured keeps the wave model; a failed
+// measurement too).  Larger levels are solved on planes but for a few steps.
 void tune_pyramid(vsc_stabilizer* s, int form)
 {
     cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
     if (cudaStreamIsCapturing(s->st, &cap) == cudaSuccess && cap == cudaStreamCaptureStatusNone)
         for (int j = 0; j < std::min(s->levels_alloc, 4); ++j)
-            if (solver_autotune(s->lw[j], s->lh[j], s->st, nullptr, form) != cudaSuccess) {
+            if (solver_one_wave(s->lw[j], s->lh[j]) &&
+                solver_autotune(s->lw[j], s->lh[j], s->st, nullptr, form) != cudaSuccess) {
                 cudaGetLastError();
                 break;
             }

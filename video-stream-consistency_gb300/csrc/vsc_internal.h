@@ -172,6 +172,7 @@ int solver_steps_per_launch();  // Jacobi steps one solver launch performs (temp
 // model's choice); per solver form.
 cudaError_t solver_autotune(int w, int h, cudaStream_t st, int* rows_out, int form = kSolverExact);
 int solver_tile_rows(int w, int h, bool* tuned, int form = kSolverExact);
+bool solver_one_wave(int w, int h);  // of 64 x 48 tiles, on the current device
 void solver_set_autotune(bool on);
 // Runs num_iter iterations; O holds the initial solution and receives the
 // result; workspace: ws_floats floats, at least solver_workspace_floats.

@@ -1936,6 +1936,12 @@ int solver_tile_rows(int w, int h, bool* tuned, int form)
     return chosen_rows(dev, w, h, di->sms, form, tuned);
 }
 
+bool solver_one_wave(int w, int h)
+{
+    DeviceInfo* di = nullptr;
+    return device_info(&di) == cudaSuccess && tiles_of(w, h, kPIH) <= di->sms;
+}
+
 cudaError_t solver_autotune(int w, int h, cudaStream_t st, int* rows_out, int form)
 {
     DeviceInfo* di = nullptr;
