@@ -58,6 +58,20 @@ def test_correlation_few_channels_many_displacements_bit_exact(vsc, oracle, cuda
     assert np.array_equal(out, oracle.correlation(f1, f2, md, legacy=legacy))
 
 
+@pytest.mark.parametrize("shape", [(1, 25, 30, 51), (1, 40, 30, 51), (1, 33, 30, 53), (1, 47, 33, 54), (2, 24, 22, 40),
+                                   (2, 50, 15, 51), (1, 48, 5, 300)])
+@pytest.mark.parametrize("legacy", [0, 1])
+def test_correlation_small_maps_bit_exact(vsc, oracle, cuda, shape, legacy):
+    """Small maps of one displacement a block: 24 channels' loads ahead where an SM
+    has up to 6.5 blocks (12 of 128 pixels, 81 displacements: 972 in all), 16 up to 7
+    (13: 1,053) and beyond (14: 1,134); channel counts around the batches."""
+    rng = np.random.default_rng(53)
+    f1 = rng.standard_normal(shape).astype(np.float32)
+    f2 = rng.standard_normal(shape).astype(np.float32)
+    out = vsc.correlation(_t(f1, cuda), _t(f2, cuda), 4, legacy=legacy).cpu().numpy()
+    assert np.array_equal(out, oracle.correlation(f1, f2, 4, legacy=legacy))
+
+
 @pytest.mark.parametrize("shape,md", [((1, 32, 24, 40), 4), ((2, 5, 7, 9), 4), ((1, 3, 6, 6), 2)])
 def test_correlation_legacy(vsc, oracle, cuda, shape, md):
     f1 = RNG.standard_normal(shape).astype(np.float32)

@@ -223,10 +223,10 @@ __global__ void __launch_bounds__(8 * kCorrTH * (2 * MD + 1))
 // displacements in y, batches in z; the channel sum in channel order; batch n
 // at base + n * stride.  A block of few channels takes several displacements (3 x 34 x
 // 60, max_displacement 32: 69 us with 67,600 blocks of one, 46 with 6,800).  A
-// small level is bound by the latency of the channel loop, so kCorrBatch channels'
-// loads are issued before their sums: 196 x 17 x 30 (8 warps a SM) take 9.0 us, and
-// 11.3 with the compiler's four.
-constexpr int kCorrBatch = 16;
+// small level is bound by the latency of the channel loop, so kBatch channels'
+// loads are issued before their sums, in registers that kBlocks blocks an SM leave:
+// 196 x 17 x 30 takes 6.1 us; 8.7 where the compiler is free to take 32 registers,
+// into which no such batch fits, and 10.7 with its own four loads ahead.
 
 // a read-only load that stays where it is written (the compiler sinks plain
 // ones to their uses, four at a time)
@@ -237,8 +237,8 @@ __device__ __forceinline__ float load_ahead(const float* p)
     return v;
 }
 
-template <bool kMany>  // displacements a block: several, else one
-__global__ void __launch_bounds__(128) corr_generic_kernel(const float* __restrict__ in1,
+template <bool kMany, int kBatch, int kBlocks>  // kMany: several displacements a block, else one
+__global__ void __launch_bounds__(128, kBlocks) corr_generic_kernel(const float* __restrict__ in1,
     const float* __restrict__ in2, float* __restrict__ out, int N, int C, int H, int W, int md, int legacy, int64_t s1,
     int64_t s2, int64_t so)
 {
@@ -259,15 +259,15 @@ __global__ void __launch_bounds__(128) corr_generic_kernel(const float* __restri
                     const float* a = in1 + n * s1 + pix;
                     const float* b = in2 + n * s2 + static_cast<int64_t>(y2) * W + x2;
                     int c = 0;
-                    for (; c + kCorrBatch <= C; c += kCorrBatch) {
-                        float va[kCorrBatch], vb[kCorrBatch];
+                    for (; c + kBatch <= C; c += kBatch) {
+                        float va[kBatch], vb[kBatch];
 #pragma unroll
-                        for (int i = 0; i < kCorrBatch; ++i) {
+                        for (int i = 0; i < kBatch; ++i) {
                             va[i] = load_ahead(a + (c + i) * HW);
                             vb[i] = load_ahead(b + (c + i) * HW);
                         }
 #pragma unroll
-                        for (int i = 0; i < kCorrBatch; ++i)
+                        for (int i = 0; i < kBatch; ++i)
                             acc = acc + va[i] * vb[i];
                     }
                     for (; c < C; ++c)
@@ -297,8 +297,18 @@ cudaError_t launch_corr_generic(const float* f1, const float* f2, float* out, in
     const int64_t per = std::max<int64_t>(1, std::min<int64_t>({32 / C, P * P, blocks * N * P * P / (152 * 16)}));
     const dim3 grid(static_cast<unsigned>(std::min<int64_t>(blocks, 152 * 64)),
         static_cast<unsigned>((P * P + per - 1) / per), static_cast<unsigned>(std::min(N, 65535)));
-    const cudaError_t e = launch_pdl(per > 1 ? corr_generic_kernel<true> : corr_generic_kernel<false>, grid, dim3(128), 0,
-        st, f1, f2, out, N, C, H, W, md, legacy, s1, s2, so);
+    // One displacement a block: 24 channels ahead where the SMs hold the blocks at
+    // once (6 each, or a few more), 16 beyond, in 64 registers where that takes
+    // another block an SM.  us with 24, with 16 and with 16 in 64 registers: 196 x 28 x
+    // 50 (5.9 blocks an SM) 10.6, 11.9, 13.2; 128 x 30 x 53 (6.9) 10.2, 8.6, 9.4; 128 x
+    // 34 x 56 (8) 10.7, 10.4, 9.2; 128 x 34 x 60 (8.5) 11.2, 11.1, 10.7.  In 32
+    // registers the first two 12.7 and 11.0, the last 16.2.
+    const int64_t all = blocks * N * P * P;
+    auto kernel = per > 1               ? corr_generic_kernel<true, 16, 16>
+                  : 2 * all <= 13 * 152 ? corr_generic_kernel<false, 24, 6>
+                  : all <= 7 * 152      ? corr_generic_kernel<false, 16, 1>
+                                        : corr_generic_kernel<false, 16, 8>;
+    const cudaError_t e = launch_pdl(kernel, grid, dim3(128), 0, st, f1, f2, out, N, C, H, W, md, legacy, s1, s2, so);
     return e != cudaSuccess ? e : cudaGetLastError();
 }
 
