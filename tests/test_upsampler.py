@@ -362,3 +362,17 @@ def test_weight_gradient_sums_against_float64(vsc, cuda, n, h, w):
         for got, want in ((grad[a:a + k], ref), (grad[a + k:a + k + co], db)):
             rms = np.sqrt(np.mean((got / want - 1) ** 2)) * 2 ** 24
             assert rms <= 4.0, (li, got.size, rms)
+
+
+@pytest.mark.gpu
+def test_training_loss_sum_is_exact(vsc, cuda):
+    """512 blocks' equal sums: with parameters of zero and a distance c of 22 bits every
+    block's sum is exact in FP32 and so is the loss, 2 c, whatever the order of the
+    blocks; added up in FP32 they are 43 units of 2^-24 off."""
+    import torch
+
+    c = 1 + 838861 * 2.0**-21
+    up = vsc.Upsampler(np.zeros(vsc.Upsampler.param_count(), np.float32))
+    inp = torch.zeros((32, 64, 64, 3), device=cuda)
+    assert up.train_step(inp, torch.full((32, 64, 64, 2), c, device=cuda), 1e-3) == 2 * c
+    up.close()

@@ -1164,7 +1164,7 @@ struct vsc_upsampler {
     int step = 0;
     float* work = nullptr;
     size_t work_floats = 0;
-    float* loss = nullptr;  // the step's loss and its non-finite flag
+    float* loss = nullptr;  // the step's loss, its non-finite flag and the loss's sum
     float max_residual = 0.5f;
 };
 namespace {
@@ -1616,7 +1616,7 @@ VSC_API vsc_status vsc_upsampler_create(const float* params, vsc_upsampler** out
     if (e == cudaSuccess)
         e = cudaMalloc(&u->wtc, upsampler_tc_weight_bytes());
     if (e == cudaSuccess)
-        e = dalloc(&u->loss, 2);
+        e = dalloc(&u->loss, 4);
     if (e == cudaSuccess)
         e = cudaMemcpy(u->prm, host.data(), n * sizeof(float), cudaMemcpyHostToDevice);
     if (e == cudaSuccess)

@@ -187,15 +187,15 @@ __device__ __noinline__ float conv_inside(const float* xr, const float* sw, floa
 }
 
 // x: planes (kInter: interleaved CI-channel pixels).  kConvRelu: y = ReLU(conv
-// + bias).  kConvLoss (the last layer): the L1 loss of base + r against the
-// target and its gradient dr = sign / pixels as planes in y.  kConvBwd: x is
+// + bias).  kConvLoss (the last layer): the L1 sum of base + r against the
+// target and the loss's gradient dr = sign / pixels as planes in y.  kConvBwd: x is
 // dz of the layer's CI outputs, y = dz of its CO inputs where a_prev > 0.
 // nonfinite: set when a value the weight gradients will multiply (the input,
 // an activation or a dz) is not finite.
 template <int CI, int CO, int OCT, int kMode, bool kInter>
 __global__ void __launch_bounds__(128, 2) conv3x3_kernel(const float* __restrict__ x, const float* __restrict__ wts,
     const float* __restrict__ bias, const float* __restrict__ a_prev, float* __restrict__ y, int H, int W, int tiles_x,
-    const float* __restrict__ input, const float* __restrict__ target, float* __restrict__ loss, float inv,
+    const float* __restrict__ input, const float* __restrict__ target, double* __restrict__ loss, float inv,
     int* __restrict__ nonfinite)
 {
     using S = ConvShape<CI, CO, OCT>;
@@ -340,13 +340,14 @@ __global__ void __launch_bounds__(128, 2) conv3x3_kernel(const float* __restrict
         }
         for (int o = 16; o > 0; o >>= 1)
             l += __shfl_xor_sync(0xffffffffu, l, o);
-        // one add a block: the running sum is rounded a quarter as often
+        // One add a block, in 64 bits: 512 additions in a row in 32 were up to 8 units
+        // of 2^-24 off (32 x 64 x 64 pixels), in the order in which the blocks end.
         __syncthreads();
         if (lane == 0)
             sm[tid >> 5] = l;
         __syncthreads();
         if (tid == 0)
-            atomicAdd(loss, ((sm[0] + sm[1]) + (sm[2] + sm[3])) * inv);
+            atomicAdd(loss, static_cast<double>((sm[0] + sm[1]) + (sm[2] + sm[3])));
     } else {
         const bool vec = (W & 3) == 0;  // planes and rows then start on the 16-byte grid
 #pragma unroll
@@ -695,10 +696,14 @@ __global__ void __launch_bounds__(128) wgrad_first_kernel(const float* __restric
     }
 }
 
+// The update; also the loss, from its sum over the batch's pixels.
 __global__ void adam_kernel(float* __restrict__ prm, const float* __restrict__ g, float* __restrict__ m,
-    float* __restrict__ v, int n, int copies, float lr, float b1, float b2, float c1, float c2, float eps)
+    float* __restrict__ v, int n, int copies, float lr, float b1, float b2, float c1, float c2, float eps,
+    const double* __restrict__ sum, double px, float* __restrict__ loss)
 {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i == 0)
+        *loss = static_cast<float>(*sum / px);
     if (i >= n)
         return;
     float part[4] = {};  // (copies in four chains: shorter sums, loads ahead)
@@ -750,7 +755,7 @@ cudaError_t train_prepare_device(int* sms)
 template <int CI, int CO, int OCT, int kMode, bool kInter>
 void launch_conv(const float* x, const float* prm, int layer, const float* a_prev, float* y, int N, int H, int W,
     int* nonfinite, cudaStream_t st, const float* input = nullptr, const float* target = nullptr,
-    float* loss = nullptr, float inv = 0.0f)
+    double* loss = nullptr, float inv = 0.0f)
 {
     using S = ConvShape<CI, CO, OCT>;
     const int tx = (W + kTileW - 1) / kTileW, ty = (H + S::rows - 1) / S::rows;
@@ -790,8 +795,8 @@ cudaError_t launch_upsampler_prepare(const float* coarse, int cw, int ch, int cf
 }
 
 // One Adam step on a batch: forward, L1 loss, backward, update.  grad:
-// upsampler_grad_floats floats; work: upsampler_train_work_floats; state: the loss and, as an int, the
-// non-finite flag.
+// upsampler_grad_floats floats; work: upsampler_train_work_floats; state (4 floats, 8-byte
+// aligned): the loss, as an int the non-finite flag, as a double the loss's sum.
 cudaError_t upsampler_train_step(float* prm, float* grad, float* m, float* v, int step, const float* input,
     const float* target, int N, int H, int W, float lr, float* work, float* state, cudaStream_t st)
 {
@@ -808,12 +813,13 @@ cudaError_t upsampler_train_step(float* prm, float* grad, float* m, float* v, in
     float* dz1 = dz2 + px * 32;
     float* dr = dz1 + px * 32;
     int* bad = reinterpret_cast<int*>(state + 1);
-    if ((e = cudaMemsetAsync(state, 0, 2 * sizeof(float), st)) != cudaSuccess)
+    double* sum = reinterpret_cast<double*>(state + 2);
+    if ((e = cudaMemsetAsync(state, 0, 4 * sizeof(float), st)) != cudaSuccess)
         return e;
     launch_conv<3, 32, 8, kConvRelu, true>(input, prm, 0, nullptr, a1, N, H, W, bad, st);
     launch_conv<32, 32, 8, kConvRelu, false>(a1, prm, 1, nullptr, a2, N, H, W, bad, st);
     launch_conv<32, 32, 8, kConvRelu, false>(a2, prm, 2, nullptr, a3, N, H, W, bad, st);
-    launch_conv<32, 2, 2, kConvLoss, false>(a3, prm, 3, nullptr, dr, N, H, W, bad, st, input, target, state,
+    launch_conv<32, 2, 2, kConvLoss, false>(a3, prm, 3, nullptr, dr, N, H, W, bad, st, input, target, sum,
         1.0f / static_cast<float>(px));
     // weight gradients: resident blocks walk the tiles, so a block's sums are added once
     const int tx = (W + kTileW - 1) / kTileW, tiles = tx * ((H + kWgRows - 1) / kWgRows);
@@ -836,7 +842,8 @@ cudaError_t upsampler_train_step(float* prm, float* grad, float* m, float* v, in
     wgrad_first_kernel<<<wb, 128, 0, st>>>(input, dz1, gw[0], gb[0], H, W, tx, tiles, N, copies, bad);
     const float b1 = 0.9f, b2 = 0.999f;
     const float c1 = 1.0f - std::pow(b1, static_cast<float>(step)), c2 = 1.0f - std::pow(b2, static_cast<float>(step));
-    adam_kernel<<<(kParams + 255) / 256, 256, 0, st>>>(prm, grad, m, v, kParams, copies, lr, b1, b2, c1, c2, 1e-8f);
+    adam_kernel<<<(kParams + 255) / 256, 256, 0, st>>>(prm, grad, m, v, kParams, copies, lr, b1, b2, c1, c2, 1e-8f, sum,
+        static_cast<double>(px), state);
     return cudaGetLastError();
 }
 
