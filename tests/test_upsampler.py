@@ -376,3 +376,19 @@ def test_training_loss_sum_is_exact(vsc, cuda):
     inp = torch.zeros((32, 64, 64, 3), device=cuda)
     assert up.train_step(inp, torch.full((32, 64, 64, 2), c, device=cuda), 1e-3) == 2 * c
     up.close()
+
+
+@pytest.mark.gpu
+def test_creation_allocates_nothing_for_training(vsc, cuda):
+    """An upsampler that only infers holds its parameters, their moments and the packed
+    weights, less than half a MiB; the gradient's copies (2.5 MiB) come with the first
+    training step."""
+    import torch
+
+    torch.cuda.synchronize()
+    free = torch.cuda.mem_get_info()[0]
+    ups = [vsc.Upsampler() for _ in range(64)]
+    held = free - torch.cuda.mem_get_info()[0]
+    for up in ups:
+        up.close()
+    assert held <= 64 * 2**19

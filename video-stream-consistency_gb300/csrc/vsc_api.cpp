@@ -1156,13 +1156,12 @@ namespace {
 struct vsc_upsampler {
     int device = 0;
     float* prm = nullptr;  // FP32 master parameters
-    float* grad = nullptr;
     float* m = nullptr;
     float* v = nullptr;
     void* wtc = nullptr;  // FP16 weights packed for the tensor-core inference
     bool wtc_valid = false;
     int step = 0;
-    float* work = nullptr;
+    float* work = nullptr;  // of training: the gradient's copies, the activations and their gradients
     size_t work_floats = 0;
     float* loss = nullptr;  // the step's loss, its non-finite flag and the loss's sum
     float max_residual = 0.5f;
@@ -1608,8 +1607,6 @@ VSC_API vsc_status vsc_upsampler_create(const float* params, vsc_upsampler** out
         upsampler_init_params(host.data(), 0x55505341'4D504C45ULL);  // seeded He-uniform
     cudaError_t e = dalloc(&u->prm, n);
     if (e == cudaSuccess)
-        e = dalloc(&u->grad, upsampler_grad_floats());
-    if (e == cudaSuccess)
         e = dalloc(&u->m, n);
     if (e == cudaSuccess)
         e = dalloc(&u->v, n);
@@ -1637,7 +1634,7 @@ VSC_API vsc_status vsc_upsampler_destroy(vsc_upsampler* u)
         return VSC_OK;
     DeviceGuard g(u->device);
     cudaDeviceSynchronize();
-    for (void* p : {static_cast<void*>(u->prm), static_cast<void*>(u->grad), static_cast<void*>(u->m),
+    for (void* p : {static_cast<void*>(u->prm), static_cast<void*>(u->m),
              static_cast<void*>(u->v), u->wtc, static_cast<void*>(u->work),
              static_cast<void*>(u->loss)})
         if (p)
@@ -1687,7 +1684,7 @@ VSC_API vsc_status vsc_upsampler_train_step(vsc_upsampler* u, const float* input
         return set_error(VSC_EINVAL, "upsampler_train_step: bad arguments");
     DeviceGuard g(u->device);
     cudaStream_t st = cs(stream);
-    const size_t need = upsampler_train_work_floats(n, h, w);
+    const size_t grads = upsampler_grad_floats(), need = grads + upsampler_train_work_floats(n, h, w);
     if (need > u->work_floats) {
         cudaStreamSynchronize(st);
         if (u->work)
@@ -1700,8 +1697,8 @@ VSC_API vsc_status vsc_upsampler_train_step(vsc_upsampler* u, const float* input
         u->work_floats = need;
     }
     u->wtc_valid = false;
-    vsc_status s = check_cuda(upsampler_train_step(u->prm, u->grad, u->m, u->v, ++u->step, input, target, n, h, w, lr,
-                                  u->work, u->loss, st),
+    vsc_status s = check_cuda(upsampler_train_step(u->prm, u->work, u->m, u->v, ++u->step, input, target, n, h, w, lr,
+                                  u->work + grads, u->loss, st),
         "upsampler_train_step");
     if (s || !loss_out)
         return s;
