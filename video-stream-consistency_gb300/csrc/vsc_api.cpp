@@ -1826,10 +1826,11 @@ VSC_API vsc_status vsc_stabilizer_stage_ms(vsc_stabilizer* s, float* ms, int32_t
 // window position as one CUDA graph (all streams advance in lockstep).
 struct vsc_multistream {
     std::vector<vsc_stabilizer*> st;
-    // grouped solves: one persistent-kernel launch per 8 Jacobi steps walks
-    // the tiles of every stream's image at a pyramid level
+    // grouped solves: a pyramid level's whole solve is one launch that walks the
+    // tiles of every stream's image (of up to 16; a launch a round for small
+    // exact groups)
     bool fused = true;      // requested (vsc_multistream_set_fused)
-    bool fused_ok = false;  // every stream's level sizes take the TMA path
+    bool fused_ok = false;  // the level workspaces exist
     std::vector<float*> lvl_ws;  // per stream: solver workspaces of levels 1 ..
     int solver_form = kSolverExact;
     std::vector<cudaStream_t> side;
@@ -1901,7 +1902,7 @@ cudaError_t ms_enqueue(vsc_multistream* m, const std::vector<uint8_t*>& outs, in
 }
 
 // Level j's solver workspace of stream i: the stabilizer's own at level 0,
-// the multistream's per-level ones above (every level's Laplacian is
+// the multistream's per-level ones above (every level's constants are
 // computed before the first grouped solve).
 float* ms_level_ws(vsc_multistream* m, size_t i, int j)
 {
@@ -1914,10 +1915,10 @@ float* ms_level_ws(vsc_multistream* m, size_t i, int j)
     return p;
 }
 
-// The step with grouped solves: each stream's flows, front pass, pyramid and
-// Laplacians on its own CUDA stream; then, on the multistream's stream, per
-// pyramid level one bilinear launch over all streams and the level's solve
-// as launches of the persistent kernel over every stream's tiles.
+// The step with grouped solves: each stream's flows, front pass, pyramid and its
+// levels' solve constants on its own CUDA stream; then, on the multistream's stream,
+// per pyramid level one bilinear launch over all streams and the level's solves
+// grouped (run_solver_group).
 cudaError_t ms_enqueue_fused(vsc_multistream* m, const std::vector<uint8_t*>& outs, int* launches)
 {
     const vsc_hyper_params& hp = m->hp;
@@ -1980,9 +1981,10 @@ cudaError_t ms_enqueue_fused(vsc_multistream* m, const std::vector<uint8_t*>& ou
 }
 
 // the grouped form when requested and possible for the current
-// hyper-parameters: the device runs the TMA kernels and every level width
-// is a multiple of 4 (buffers come from cudaMalloc, offsets are 16-byte
-// multiples then)
+// hyper-parameters: the device runs the solve kernel, every stream has the levels,
+// and every level's width is a multiple of 4.  The solve kernel's planes take any
+// width; the last condition is what vsc.h promises of vsc_multistream_fused, and
+// the small exact groups on interleaved images need it.
 bool ms_use_fused(vsc_multistream* m)
 {
     if (!m->fused || !m->fused_ok || !solver_tma_supported())
@@ -2119,8 +2121,7 @@ VSC_API vsc_status vsc_multistream_create(const vsc_stream_desc* desc, int32_t n
     }
     if (!s && e != cudaSuccess)
         s = check_cuda(e, "multistream_create");
-    // grouped solves: per-level workspaces above level 0, and the tile shape
-    // of each level's group (a stream being captured keeps the wave model)
+    // grouped solves: per-level workspaces above level 0
     m->fused_ok = !s;
     for (size_t i = 0; i < m->st.size() && !s; ++i) {
         vsc_stabilizer* st = m->st[i];
