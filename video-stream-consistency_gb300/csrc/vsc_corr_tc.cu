@@ -373,6 +373,7 @@ __global__ void __launch_bounds__((2 + 4 * kMaxEpiGroups) * 32, 1)
                     ok = __shfl_sync(0xffffffffu, lane == 0 ? tc_wait(&sh.full_d[sd], phase, sh.abort) : 0, 0);
                     if (!ok)
                         break;
+                    __syncwarp();  // orders the other lanes' loads after lane 0's wait (a shuffle does not)
                     ptx::tc_fence_after();
                     uint32_t v0[32], v1[16];
                     const uint32_t ta = tmem + lane_base + sd * kDStride + q * 32;
