@@ -563,7 +563,7 @@ def multistream_measure(vsc, dev, form: str, steps: int, warmup: int, grouped: b
                    "px_per_step": px, "form": form,
                    "per_stream": [{"size": [w, h], "flow_downscale": d, "corr_dtype": c}
                                   for (w, h), (d, c) in zip(MULTI_STREAMS, forms)],
-                   "solves": "grouped: one persistent-kernel launch per 8 Jacobi steps covers all 16 images"
+                   "solves": "grouped: one launch per pyramid level runs the whole solves of all 16 images"
                              if is_grouped else "per stream, each on its own CUDA stream"},
         "grouped_solves": is_grouped, "gpu_launches_per_step": ms.last_launches, "clocks": clk,
     }
@@ -1148,21 +1148,21 @@ SOLVER_KERNELS = {"exact": ("solver_solve_kernel<exact>", 84), "fma": ("solver_s
 # dram__bytes_read.sum + dram__bytes_write.sum of one 8-step round at
 # 1920x1080 from the ncu captures summarised in profiles/, and where each
 # comes from.
-SOLVER_TRAFFIC_BYTES = {"solver_solve_kernel<exact>": 172_763_776, "solver_solve_kernel<FMA>": 144_740_288}
+SOLVER_TRAFFIC_BYTES = {"solver_solve_kernel<exact>": 173_306_304, "solver_solve_kernel<FMA>": 142_168_128}
 SOLVER_TRAFFIC_SOURCE = {
     "solver_solve_kernel<exact>": "profiles/solver_solve_1080p.md (one launch per solve; per round, the difference "
-                                  "of a 40-step and an 8-step solve over 4 rounds: (617,573,120 - 124,665,344) read "
-                                  "+ (221,238,784 - 23,091,456) written, / 4)",
+                                  "of a 40-step and an 8-step solve over 4 rounds: (591,841,024 - 99,814,400) read "
+                                  "+ (209,186,560 - 7,987,968) written, / 4)",
     "solver_solve_kernel<FMA>": "profiles/solver_solve_1080p.md (one launch per solve; per round, the difference of a "
-                                "40-step and an 8-step solve over 4 rounds: (480,915,968 - 99,618,304) read + "
-                                "(215,260,672 - 17,597,184) written, / 4)",
+                                "40-step and an 8-step solve over 4 rounds: (443,653,120 - 74,732,032) read + "
+                                "(203,782,656 - 4,031,232) written, / 4)",
 }
 # What bounds each solver kernel, from the same captures: FP32 issue and the
 # exchange between warps, not HBM alone (the time steps stay on chip): the FMA
 # pipe's warp instructions per scheduler and cycle, and smsp__issue_active.
 SOLVER_PIPE = {
-    "solver_solve_kernel<exact>": {"fma_pipe_active": 0.542, "issue_active": 0.622},
-    "solver_solve_kernel<FMA>": {"fma_pipe_active": 0.435, "issue_active": 0.535},
+    "solver_solve_kernel<exact>": {"fma_pipe_active": 0.543, "issue_active": 0.627},
+    "solver_solve_kernel<FMA>": {"fma_pipe_active": 0.434, "issue_active": 0.538},
 }
 
 

@@ -312,7 +312,7 @@ VSC_API vsc_status vsc_get_consist_out(const vsc_image* crnt_pr, const vsc_image
  * floats a pixel.  With vsc_consist_out_full_workspace_size bytes, which NULL
  * takes, it is at its fastest: in fewer, small images have rounds of fewer steps
  * (640x360, 150 steps: 145 us against 131), and where the width is not a
- * multiple of 4 the solve runs with plain loads (about 2.5 times the time); same
+ * multiple of 4 the solve runs with plain loads (about 2.7 times the time); same
  * bits either way.  Results within the tolerance stated at VSC_SOLVER_FMA of
  * vsc_get_consist_out's.  No counterpart in the reference. */
 VSC_API size_t vsc_consist_out_fma_workspace_size(int32_t width, int32_t height);
@@ -536,8 +536,8 @@ VSC_API int32_t vsc_multistream_last_launches(vsc_multistream* m);
 VSC_API vsc_status vsc_multistream_set_fused(vsc_multistream* m, int32_t on);
 VSC_API int32_t vsc_multistream_fused(vsc_multistream* m);
 /* The solver form (VSC_SOLVER_EXACT or VSC_SOLVER_FMA) of every stream's
- * solves, grouped or not; tunes the form's tile shapes (synchronises the
- * multistream's stream).  No counterpart in the reference. */
+ * solves, grouped or not; tunes as vsc_stabilizer_set_solver_form (synchronises
+ * the multistream's stream).  No counterpart in the reference. */
 VSC_API vsc_status vsc_multistream_set_solver_form(vsc_multistream* m, int32_t form);
 /* The learned flow upsampler for stream `index` (-1: every stream created
  * with flow_downscale > 1), as vsc_stabilizer_set_upsampler; NULL: bilinear.

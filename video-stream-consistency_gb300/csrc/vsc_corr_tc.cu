@@ -857,8 +857,9 @@ cudaError_t launch_corr_tc(const float* f1, const float* f2, float* out, int N, 
     // correlation overwrites; behind the scales when it has no 64 elements or shares
     // memory with an operand), both operands' conversion with the scales
     // worked out by every block, the correlation.  (A memset, a maximum and a
-    // conversion per operand and a launch for the scales: a call of 2 x 64 x 136 x
-    // 240 then took 60 us back to back, now 35; of 130 x 34 x 60, 29 and 14.)
+    // conversion per operand and a launch for the scales, with the correlation of
+    // that time: 2 x 64 x 136 x 240 67.7 us a call, now 38.7; 130 x 34 x 60 on one
+    // pair of operands 29 and 14.)
     const int64_t total = static_cast<int64_t>(N) * C * H * W;
     const int64_t outs = static_cast<int64_t>(N) * (2 * md + 1) * (2 * md + 1) * H * W;
     auto apart = [&](const float* f) { return std::less_equal<const float*>()(f + total, out) ||

@@ -2047,8 +2047,8 @@ int pl_counter_floats(int w, int h, int cfg) { return (16 + pl_tiles_of(w, h, cf
 
 // A plane's row in floats where the workspace has room for rows on the 16-byte
 // grid (TMA's), whatever the width.
-// 854x480, FMA form, 150 steps: 164 us; with plain loads, which a tile's steps
-// wait for, and a launch a round 542 us.
+// 854x480, FMA form, 150 steps: 162 us; with plain loads, which a tile's steps
+// wait for, and a launch a round 454 us.
 int pl_pitch(int w) { return (w + 3) & ~3; }
 
 // planes-images of a form: O, U (two each) and its constants
@@ -2138,8 +2138,10 @@ bool pl_tma_eligible(const DeviceInfo* di, int w, int h, const float* ws, size_t
 // us, 8, 12 and 16 a round: FMA 320x180 147, 126, 109; 640x360 177, 145, 131;
 // 854x480 196, 163, 177; 960x540 195, 211, 217; 1280x720 290, 324, 385; exact
 // 480x270 189, 162, 167; 560x316 202, 170, 156; 640x360 204, 174, 199; 800x450
-// 220, 227, 277.  Of the rounds that a workspace of ws_floats has counters for: a
-// smaller one may have them for 12 steps and not for 16.
+// 220, 227, 277 (calls in place, back to back on one image; on another image each
+// time, its start copied, the 854x480 FMA call takes 172).  Of the rounds that a
+// workspace of ws_floats has counters for: a smaller one may have them for 12 steps
+// and not for 16.
 int pl_rounds_cfg(int sms, int w, int h, int num_iter, int form, size_t ws_floats)
 {
     struct Cost {

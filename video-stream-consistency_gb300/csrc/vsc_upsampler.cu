@@ -405,7 +405,7 @@ __global__ void __launch_bounds__(128, 2) conv3x3_kernel(const float* __restrict
 // copies, one for 16 blocks and 32 at most, which the update sums: all 608 blocks
 // on one sum were 608 additions in a row and five times as far from the float64 sum
 // (32 x 64 x 64 pixels of equal dz: 5.9 units of 2^-24 in the root mean square, now
-// 1.1; the per-pixel kernels 1.7), and slower (a step 550 -> 545 us); a thread's
+// 1.1; the per-pixel kernels 1.7), and slower (a step 590 us, now 560); a thread's
 // own sum is at most 2,048 products long, whatever the batch.  A pixel with dz = 0 adds nothing, whatever x
 // holds there, nor does a tap outside the image, whatever dz is (kSafe, taken
 // when some x or dz is not finite; else the product with 0 is 0 anyway).
