@@ -335,6 +335,48 @@ def test_consist_out_where_the_full_workspace_does_not_fit(vsc, cuda):
     vsc.check_device()
 
 
+@pytest.mark.parametrize("w", [2560, 2562])
+@pytest.mark.parametrize("form", ["exact", "fma"])
+def test_stabilizer_on_a_nearly_full_device(vsc, cuda, form, w):
+    """Where the device has no room for the solver's planes, a stabilizer is created
+    with what a solve needs at least (an image less), and its frames are the same."""
+    import torch
+
+    h = 1440
+    rng = np.random.default_rng(11)
+    frames = [tuple(torch.from_numpy(rng.integers(0, 256, (h, w, 4), dtype=np.uint8)).to(cuda) for _ in range(2))
+              for _ in range(3)]
+    out = torch.empty((h, w, 4), dtype=torch.uint8, device=cuda)
+
+    def run():
+        stream = torch.cuda.Stream()
+        torch.cuda.synchronize()
+        free = torch.cuda.mem_get_info()[0]
+        st = vsc.Stabilizer(w, h, flow_downscale=2, stream=stream, solver_form=form)
+        st.hyper_params.num_iter = 20
+        need = free - torch.cuda.mem_get_info()[0]
+        for f in frames:
+            st.load_frame(*f)
+        st.step(out)
+        stream.synchronize()
+        st.close()
+        return need, out.cpu()
+
+    run()
+    need, ref = run()
+    torch.cuda.empty_cache()
+    image = 12 * w * h
+    filler = torch.empty(torch.cuda.mem_get_info()[0] - need + image // 2, dtype=torch.uint8, device=cuda)
+    try:
+        less, got = run()
+    finally:
+        del filler
+        torch.cuda.empty_cache()
+    assert less <= need - image // 2
+    assert torch.equal(got, ref)
+    vsc.check_device()
+
+
 @pytest.mark.parametrize("w,h,iters", [(1280, 720, 3), (1280, 720, 4), (1920, 1080, 1), (1920, 1080, 6), (1920, 1080, 7)])
 def test_consist_out_few_steps_of_a_large_image(vsc, oracle, cuda, w, h, iters):
     """The last step counts on interleaved images and the first on planes."""

@@ -745,6 +745,7 @@ struct vsc_stabilizer {
     float* pyrO[8] = {};
     int lw[8] = {}, lh[8] = {};
     float* solver_ws = nullptr;
+    size_t ws_floats = 0;  // its size
     float* feat_scratch = nullptr;
     float* flow_scratch = nullptr;
     // tensor-core correlations (corr_dtype BF16 / F16): chunked 16-bit
@@ -946,7 +947,6 @@ vsc_status alloc_all(vsc_stabilizer* s)
         A(dalloc(&s->pyrW[j], m));
         A(dalloc(&s->pyrO[j], m));
     }
-    A(dalloc(&s->solver_ws, solver_workspace_any_floats(s->w, s->h)));
     if (s->compute_flow) {
         s->fd = flow_dims(s->fw, s->fh);
         // the three frames' features in one allocation, so a flow pair can
@@ -977,6 +977,15 @@ vsc_status alloc_all(vsc_stabilizer* s)
             A(dalloc(&s->flow_small, 2 * static_cast<size_t>(s->fw) * s->fh * 3));
         }
         A(flow_upload_weights());
+    }
+    // last, with room for the planes of either form; on a device too full for that,
+    // what a solve of either form needs at least
+    s->ws_floats = solver_workspace_any_floats(s->w, s->h);
+    if (e == cudaSuccess && (e = dalloc(&s->solver_ws, s->ws_floats)) == cudaErrorMemoryAllocation) {
+        cudaGetLastError();
+        s->ws_floats = std::max(solver_workspace_floats(s->w, s->h, kSolverExact),
+            solver_workspace_floats(s->w, s->h, kSolverFma));
+        e = dalloc(&s->solver_ws, s->ws_floats);
     }
     return check_cuda(e, "stabilizer allocation");
 }
@@ -1321,7 +1330,6 @@ cudaError_t enqueue_step(vsc_stabilizer* s, const vsc_hyper_params& hp, uint8_t*
     float** A = lv.A;
     float** W = lv.W;
     float** O = lv.O;
-    const size_t ws_floats = solver_workspace_any_floats(s->w, s->h);
     mark(s, kEvFront);
     for (int j = L - 1; j >= 0; --j) {
         if (j == 0)
@@ -1334,10 +1342,11 @@ cudaError_t enqueue_step(vsc_stabilizer* s, const vsc_hyper_params& hp, uint8_t*
         // coarser solution.
         const bool coarsest = j == L - 1;
         if (iters > 0 && solver_tma_supported() &&
+            solver_planes_fit(s->solver_form, s->lw[j], s->lh[j], s->ws_floats) &&
             !solver_step_interleaved(s->solver_form, A[j], W[j], O[j], s->lw[j], s->lh[j], iters, s->solver_ws)) {
             run(run_solver_planes(s->solver_form, P[j], A[j], W[j], coarsest ? P[j] : nullptr, O[j], s->lw[j], s->lh[j],
                 coarsest ? nullptr : O[j + 1], coarsest ? 0 : s->lw[j + 1], coarsest ? 0 : s->lh[j + 1], iters,
-                hp.step_size, hp.mom_fac, s->solver_ws, ws_floats, st, &nl, rgba));
+                hp.step_size, hp.mom_fac, s->solver_ws, s->ws_floats, st, &nl, rgba));
             continue;
         }
         if (coarsest) {
@@ -1348,7 +1357,7 @@ cudaError_t enqueue_step(vsc_stabilizer* s, const vsc_hyper_params& hp, uint8_t*
             ++nl;
         }
         run(run_solver(P[j], A[j], W[j], O[j], s->lw[j], s->lh[j], iters, hp.step_size, hp.mom_fac, s->solver_ws,
-            ws_floats, st, &nl, rgba, s->solver_form));
+            s->ws_floats, st, &nl, rgba, s->solver_form));
     }
     mark(s, kEvStep1);
     *launches = nl;
@@ -1830,7 +1839,7 @@ struct vsc_multistream {
     // tiles of every stream's image (of up to 16; a launch a round for small
     // exact groups)
     bool fused = true;      // requested (vsc_multistream_set_fused)
-    bool fused_ok = false;  // the level workspaces exist
+    bool fused_ok = false;  // every level's workspace has room for its planes
     std::vector<float*> lvl_ws;  // per stream: solver workspaces of levels 1 ..
     int solver_form = kSolverExact;
     std::vector<cudaStream_t> side;
@@ -2121,16 +2130,22 @@ VSC_API vsc_status vsc_multistream_create(const vsc_stream_desc* desc, int32_t n
     }
     if (!s && e != cudaSuccess)
         s = check_cuda(e, "multistream_create");
-    // grouped solves: per-level workspaces above level 0
+    // grouped solves: per-level workspaces above level 0; on a device too full for
+    // them every stream solves on its own
     m->fused_ok = !s;
-    for (size_t i = 0; i < m->st.size() && !s; ++i) {
+    for (size_t i = 0; i < m->st.size() && m->fused_ok; ++i) {
         vsc_stabilizer* st = m->st[i];
         size_t floats = 0;
         for (int j = 1; j < st->levels_alloc; ++j)
             floats += solver_workspace_any_floats(st->lw[j], st->lh[j]);
         float* p = nullptr;
-        if (floats && (s = check_cuda(dalloc(&p, floats), "multistream_create level workspaces")))
+        e = floats ? dalloc(&p, floats) : cudaSuccess;
+        if (e != cudaSuccess && e != cudaErrorMemoryAllocation) {
+            s = check_cuda(e, "multistream_create level workspaces");
             break;
+        }
+        cudaGetLastError();
+        m->fused_ok = e == cudaSuccess && st->ws_floats >= solver_workspace_any_floats(st->w, st->h);
         m->lvl_ws.push_back(p);
     }
     if (s) {

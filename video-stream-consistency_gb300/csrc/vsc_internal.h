@@ -180,6 +180,8 @@ void solver_set_autotune(bool on);
 cudaError_t run_solver(const float* P, const float* A, const float* Wt, float* O, int w, int h, int num_iter,
     float step, float mom, float* workspace, size_t ws_floats, cudaStream_t st, int* launches,
     uint8_t* rgba_out = nullptr, int form = kSolverExact);
+// Whether a workspace has room for a form's planes.
+bool solver_planes_fit(int form, int w, int h, size_t ws_floats);
 // Whether a level of a step is better solved by run_solver on interleaved images, its
 // start written to O beforehand, than by run_solver_planes.
 bool solver_step_interleaved(int form, const float* A, const float* Wt, const float* O, int w, int h, int num_iter,

@@ -2406,6 +2406,8 @@ cudaError_t solver_prep(int form, const float* P, const float* A, const float* W
     return e != cudaSuccess ? e : cudaGetLastError();
 }
 
+bool solver_planes_fit(int form, int w, int h, size_t ws_floats) { return pl_fits(w, h, ws_floats, form); }
+
 bool solver_step_interleaved(int form, const float* A, const float* Wt, const float* O, int w, int h, int num_iter,
     float* workspace)
 {
