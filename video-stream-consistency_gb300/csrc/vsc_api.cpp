@@ -1935,14 +1935,11 @@ cudaError_t ms_enqueue_fused(vsc_multistream* m, const std::vector<uint8_t*>& ou
     const size_t n = m->st.size();
     std::vector<LevelImages> lv(n);
     std::vector<int> ws(n), hs(n);
-    std::vector<bool> interleaved(L);
-    for (int j = 0; j < L; ++j) {
-        for (size_t i = 0; i < n; ++i) {
-            ws[i] = m->st[i]->lw[j];
-            hs[i] = m->st[i]->lh[j];
-        }
-        interleaved[j] = solver_group_interleaved(ws.data(), hs.data(), static_cast<int>(n), m->solver_form);
+    for (size_t i = 0; i < n; ++i) {
+        ws[i] = m->st[i]->w;
+        hs[i] = m->st[i]->h;
     }
+    const bool interleaved = solver_group_interleaved(ws.data(), hs.data(), static_cast<int>(n), m->solver_form);
     cudaError_t e = cudaEventRecord(m->fork, m->main);
     int nl = 0;
     for (size_t i = 0; i < n && e == cudaSuccess; ++i) {
@@ -1952,13 +1949,13 @@ cudaError_t ms_enqueue_fused(vsc_multistream* m, const std::vector<uint8_t*>& ou
         e = enqueue_pre_solve(s, hp, &lv[i], &nl);
         for (int j = 0; j < L && e == cudaSuccess; ++j) {
             e = solver_prep(m->solver_form, lv[i].P[j], lv[i].A[j], lv[i].W[j], s->lw[j], s->lh[j], hp.step_size,
-                ms_level_ws(m, i, j), interleaved[j], s->st);
+                ms_level_ws(m, i, j), interleaved, s->st);
             ++nl;
         }
         // videostabilizer.cpp:212-217: the coarsest level starts from P
         if (e == cudaSuccess)
             e = cudaMemcpyAsync(solver_group_start(lv[i].O[L - 1], ms_level_ws(m, i, L - 1), s->lw[L - 1], s->lh[L - 1],
-                                    hp.num_iter / L, interleaved[L - 1]),
+                                    hp.num_iter / L, interleaved),
                 lv[i].P[L - 1], static_cast<size_t>(s->lw[L - 1]) * s->lh[L - 1] * 3 * sizeof(float), cudaMemcpyDeviceToDevice, s->st);
         if (e == cudaSuccess && (e = cudaEventRecord(m->joined[i], m->side[i])) == cudaSuccess)
             e = cudaStreamWaitEvent(m->main, m->joined[i], 0);
@@ -1973,7 +1970,7 @@ cudaError_t ms_enqueue_fused(vsc_multistream* m, const std::vector<uint8_t*>& ou
             im[i] = SolverImage{lv[i].A[j], lv[i].W[j], lv[i].O[j], s->lw[j], s->lh[j], ws_j, j == 0 ? outs[i] : nullptr};
             if (j != L - 1) {
                 up_in[i] = Img{lv[i].O[j + 1], s->lw[j + 1], s->lh[j + 1], 3};
-                up_out[i] = Img{solver_group_start(lv[i].O[j], ws_j, s->lw[j], s->lh[j], it, interleaved[j]), s->lw[j],
+                up_out[i] = Img{solver_group_start(lv[i].O[j], ws_j, s->lw[j], s->lh[j], it, interleaved), s->lw[j],
                     s->lh[j], 3};
             }
         }
@@ -1983,7 +1980,7 @@ cudaError_t ms_enqueue_fused(vsc_multistream* m, const std::vector<uint8_t*>& ou
         }
         if (e == cudaSuccess)
             e = run_solver_group(im.data(), static_cast<int>(n), it, hp.step_size, hp.mom_fac, m->main, &nl,
-                m->solver_form, interleaved[j]);
+                m->solver_form, interleaved);
     }
     *launches = nl;
     return e;

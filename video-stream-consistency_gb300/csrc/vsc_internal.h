@@ -209,8 +209,11 @@ struct SolverImage {
 };
 bool solver_tma_supported();  // the solve kernel runs on the current device
 // Exact images of one wave of 64 x 32 tiles in all (of each launch), as run_solver
-// keeps them: three videos of 96x64 318 us a step, 385 on planes; eight 355 and
-// 414; three of 320x180, 252 tiles, 494 and 447.
+// keeps them: three videos of 96x64 329 us a step, 395 on planes; eight 396 and
+// 460; three of 320x184, 252 tiles, 473 and 427.  Asked for a step's finest level and
+// followed by all of it: where that one is on planes, the coarser ones are faster
+// interleaved in a step alone (320x184 and 608x328: 434 us, 454 with both on planes)
+// but not beside another one's (365 and 349).
 bool solver_group_interleaved(const int* w, const int* h, int n, int form);
 float* solver_group_start(float* O, float* workspace, int w, int h, int num_iter, bool interleaved);
 // a form's per-solve constants, into the workspace
